@@ -1,0 +1,76 @@
+"""Shortcuts in the tick's headers against the general path they stand for, on the CPU: the headers are host code too,
+so they are compiled as they are and, for the general path, with the shortcut's line taken out."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from rocketgpu_b200 import build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "rocketgpu_b200", "csrc")
+
+
+def _build(tmp, name, edits=()):
+    """The headers with `edits` [(file, line to take out)] as a shared library."""
+    src = os.path.join(tmp, name)
+    shutil.copytree(CSRC, src)
+    for f, line in edits:
+        path = os.path.join(src, f)
+        with open(path) as h:
+            text = h.read()
+        assert text.count(line) == 1, (f, line)
+        with open(path, "w") as h:
+            h.write(text.replace(line, ""))
+    out = os.path.join(tmp, name + ".so")
+    cuda = os.path.dirname(os.path.dirname(build.nvcc()))  # rg_mesh.cpp holds the mesh upload too
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-ffp-contract=off", "-w", "-I", src, "-I",
+                    os.path.join(ROOT, "include"), "-I", os.path.join(cuda, "include"),
+                    os.path.join(ROOT, "tests", "host_paths.cpp"), os.path.join(src, "rg_mesh.cpp"), "-o", out,
+                    "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath," + os.path.join(cuda, "lib64")],
+                   check=True)
+    return ctypes.CDLL(out)
+
+
+def _same(a, b):
+    """Bitwise, a NaN equal to any NaN."""
+    return bool(((a.view(np.uint32) == b.view(np.uint32)) | (np.isnan(a) & np.isnan(b))).all())
+
+
+@pytest.fixture(scope="module")
+def libs(tmp_path_factory):
+    tmp = str(tmp_path_factory.mktemp("host_paths"))
+    return (_build(tmp, "as_is"),
+            _build(tmp, "general", [("rg_gjk.cuh", "    if (any_nan(xa.o) || any_nan(xb.o)) return false;\n")]))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf, 3.0e38])
+def test_pair_detector_of_a_body_without_a_position(libs, bad):
+    """Boxes, triangles and spheres with a bad value at each place of the box's position, basis, offset and of the
+    other shape, and with none: the same contacts with the shortcut as through the whole loop."""
+    rng = np.random.default_rng(11)
+    n = 9 + 3 + 3 + 9 + 24
+    q = np.linalg.qr(rng.normal(size=(n, 3, 3)))[0]
+    basis = np.ascontiguousarray(q, np.float32)
+    pos = rng.uniform(-1, 1, (n, 3)).astype(np.float32)
+    offset = np.tile(np.float32([0.27, 0.0, 0.41]), (n, 1))
+    half = np.tile(np.float32([1.18, 0.84, 0.36]), (n, 1))
+    tri = rng.uniform(-3, 3, (n, 3, 3)).astype(np.float32)
+    ball = rng.uniform(-2, 2, (n, 3)).astype(np.float32)
+    places = [(basis, k) for k in range(9)] + [(pos, k) for k in range(3)] + [(offset, k) for k in range(3)] + \
+        [(tri, k) for k in range(9)]
+    for case, (a, k) in enumerate(places):
+        a.reshape(n, -1)[case, k] = bad
+        ball[case, k % 3] = bad if a is tri else ball[case, k % 3]
+    ptr = [x.ctypes.data_as(ctypes.c_void_p) for x in (basis, pos, offset, half)]
+    got = {}
+    for name, fn, other, width in (("triangle", "hp_box_triangle", tri, 5), ("ball", "hp_ball_box", ball, 17)):
+        for k, lib in enumerate(libs):
+            out = np.zeros((n, width), np.float32)
+            getattr(lib, fn)(*ptr, other.ctypes.data_as(ctypes.c_void_p), out.ctypes.data_as(ctypes.c_void_p), n)
+            got[name, k] = out
+        assert _same(got[name, 0], got[name, 1]), name
+        assert got[name, 0][len(places):, 0].any(), name  # some of the sound cases touch
