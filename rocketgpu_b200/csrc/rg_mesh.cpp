@@ -330,31 +330,53 @@ MeshHost build_mesh_host(const float* v, int64_t nv, const int32_t* idx, int64_t
     // query grid over the quantized leaf bounds, each cell grown by the largest single-cell query
     h.grid_lo = h.quant.aabb_min;
     const V3 span = h.quant.aabb_max - h.quant.aabb_min;
-    h.grid_dims[0] = static_cast<int32_t>(std::ceil(span.x / kQueryCellBt)) + 1;
-    h.grid_dims[1] = static_cast<int32_t>(std::ceil(span.y / kQueryCellBt)) + 1;
-    h.grid_dims[2] = static_cast<int32_t>(std::ceil(span.z / kQueryCellBt)) + 1;
-    const int64_t cells = static_cast<int64_t>(h.grid_dims[0]) * h.grid_dims[1] * h.grid_dims[2];
-    std::vector<std::vector<int32_t>> lists(static_cast<size_t>(cells));
-    for (int32_t r = 0; r < nt; ++r) {
-        const DevTri& d = h.dev_tris[r];
-        const V3 lo = unquantize(h.quant, d.qmin);
-        const V3 hi = unquantize(h.quant, d.qmax);
-        int c0[3], c1[3];
-        const float lo3[3] = {lo.x - h.grid_lo.x, lo.y - h.grid_lo.y, lo.z - h.grid_lo.z};
-        const float hi3[3] = {hi.x - h.grid_lo.x, hi.y - h.grid_lo.y, hi.z - h.grid_lo.z};
-        for (int a = 0; a < 3; ++a) {
-            // a cell c serves queries whose min corner lies in it; such a query reaches at most
-            // (c + 1) * cell + extent, so the triangle belongs to every cell from (lo - extent) / cell to hi / cell.
-            c0[a] = std::max(0, static_cast<int>(std::floor((lo3[a] - kQueryExtentBt) / kQueryCellBt)) - 1);
-            c1[a] = std::min(h.grid_dims[a] - 1, static_cast<int>(std::floor(hi3[a] / kQueryCellBt)) + 1);
+    struct CellRange {
+        int32_t lo[3], hi[3];
+    };
+    std::vector<CellRange> ranges(static_cast<size_t>(nt));
+    // the cells of every triangle at one cell size; returns how many list entries they make
+    auto cell_ranges = [&](float cell) {
+        const float span3[3] = {span.x, span.y, span.z};
+        const float scale3[3] = {h.quant.scale.x, h.quant.scale.y, h.quant.scale.z};
+        for (int a = 0; a < 3; ++a) h.grid_dims[a] = static_cast<int32_t>(std::ceil(span3[a] / cell)) + 1;
+        int64_t entries = 0;
+        for (int32_t r = 0; r < nt; ++r) {
+            const DevTri& d = h.dev_tris[r];
+            const V3 lo = unquantize(h.quant, d.qmin) - h.grid_lo, hi = unquantize(h.quant, d.qmax) - h.grid_lo;
+            const float lo3[3] = {lo.x, lo.y, lo.z}, hi3[3] = {hi.x, hi.y, hi.z};
+            int64_t n = 1;
+            for (int a = 0; a < 3; ++a) {
+                // a cell c serves queries whose min corner lies in it; such a query reaches at most
+                // (c + 1) * cell + extent, so the triangle belongs to every cell from (lo - extent) / cell to
+                // hi / cell. Quantized overlap reaches two quantization steps past the real one on each side (min
+                // corners round down to even, max corners up to odd); four steps and 0.001 bt cover the rounding.
+                const float eps = 4.0f / scale3[a] + 1.0e-3f;
+                CellRange& c = ranges[r];
+                c.lo[a] = std::clamp(static_cast<int>(std::floor((lo3[a] - kQueryExtentBt - eps) / cell)), 0,
+                                     h.grid_dims[a] - 1);
+                c.hi[a] = std::clamp(static_cast<int>(std::floor((hi3[a] + eps) / cell)), 0, h.grid_dims[a] - 1);
+                n *= c.hi[a] - c.lo[a] + 1;
+            }
+            entries += n;
         }
-        for (int z = c0[2]; z <= c1[2]; ++z)
-            for (int y = c0[1]; y <= c1[1]; ++y)
-                for (int x = c0[0]; x <= c1[0]; ++x)
-                    lists[(static_cast<size_t>(z) * h.grid_dims[1] + y) * h.grid_dims[0] + x].push_back(r);
+        return entries;
+    };
+    h.query_cell = kQueryCellBt;
+    if (cell_ranges(h.query_cell) > kQueryEntriesMax) {
+        h.query_cell = kQueryCellLargeBt;
+        cell_ranges(h.query_cell);
     }
+    const int64_t cells = static_cast<int64_t>(h.grid_dims[0]) * h.grid_dims[1] * h.grid_dims[2];
+    auto each_cell = [&](int32_t r, auto&& f) {
+        const CellRange& c = ranges[r];
+        for (int z = c.lo[2]; z <= c.hi[2]; ++z)
+            for (int y = c.lo[1]; y <= c.hi[1]; ++y)
+                for (int x = c.lo[0]; x <= c.hi[0]; ++x)
+                    f((static_cast<size_t>(z) * h.grid_dims[1] + y) * h.grid_dims[0] + x);
+    };
     h.cell_start.assign(static_cast<size_t>(cells) + 1, 0);
-    for (int64_t c = 0; c < cells; ++c) h.cell_start[c + 1] = h.cell_start[c] + static_cast<int32_t>(lists[c].size());
+    for (int32_t r = 0; r < nt; ++r) each_cell(r, [&](size_t c) { ++h.cell_start[c + 1]; });
+    for (int64_t c = 0; c < cells; ++c) h.cell_start[c + 1] += h.cell_start[c];
     auto entry_of = [&](int32_t r) {
         CellEntry e;
         for (int a = 0; a < 3; ++a) {
@@ -364,9 +386,12 @@ MeshHost build_mesh_host(const float* v, int64_t nv, const int32_t* idx, int64_t
         e.rank = r;
         return e;
     };
-    h.cell_entries.reserve(static_cast<size_t>(h.cell_start[cells]));
-    for (auto& l : lists)
-        for (int32_t r : l) h.cell_entries.push_back(entry_of(r));
+    h.cell_entries.resize(static_cast<size_t>(h.cell_start[cells]));
+    std::vector<int32_t> next(h.cell_start.begin(), h.cell_start.end() - 1);
+    for (int32_t r = 0; r < nt; ++r) {
+        const CellEntry e = entry_of(r);
+        each_cell(r, [&](size_t c) { h.cell_entries[next[c]++] = e; });  // in rank order within each cell
+    }
     h.rank_entries.reserve(static_cast<size_t>(nt));
     for (int32_t r = 0; r < nt; ++r) h.rank_entries.push_back(entry_of(r));
     return h;
@@ -398,6 +423,7 @@ MeshDevice upload_mesh(const MeshHost& h) {
     d.aabb_min = h.aabb_min;
     d.aabb_max = h.aabb_max;
     d.grid_lo = h.grid_lo;
+    d.inv_query_cell = 1.0f / h.query_cell;
     for (int a = 0; a < 3; ++a) d.grid_dims[a] = h.grid_dims[a];
     d.cell_start = upload_array(h.cell_start, "mesh grid");
     d.cell_entries = upload_array(h.cell_entries, "mesh grid lists");

@@ -44,8 +44,15 @@ struct HostTri {
     uint16_t qmin[3], qmax[3];
 };
 
-constexpr float kQueryCellBt = 4.0f;
+// The query grid's cell, and the largest query box that one cell serves. Entries read per query on the ~11k-triangle
+// arena in play: 8 with 2 bt cells, 29 with 4 bt cells and a whole cell of slack on each side (geometry and vehicle
+// updates of a tick 292 -> 260 us at 1,024 mixed arenas, 84 -> 69 us for one 1v1 arena). A mesh of so many large
+// triangles that the finer grid's lists would pass kQueryEntriesMax (64 MB) gets the coarser one. Both sizes are powers
+// of two, so the query's division by the cell is an exact multiplication.
+constexpr float kQueryCellBt = 2.0f;
+constexpr float kQueryCellLargeBt = 4.0f;
 constexpr float kQueryExtentBt = 4.0f;
+constexpr int64_t kQueryEntriesMax = 4 << 20;
 
 // One query-grid entry: a triangle's quantized leaf bounds and its rank, so the overlap test needs no triangle load.
 struct alignas(16) CellEntry {
@@ -63,6 +70,7 @@ struct MeshHost {
     // query grid
     V3 grid_lo{0, 0, 0};
     int32_t grid_dims[3] = {0, 0, 0};
+    float query_cell = kQueryCellBt;
     std::vector<int32_t> cell_start;       // grid cell -> first entry, size cells + 1
     std::vector<CellEntry> cell_entries;   // per cell, in rank order
     std::vector<CellEntry> rank_entries;   // every triangle in rank order (queries larger than one cell)
@@ -76,6 +84,7 @@ struct MeshDevice {
     V3 aabb_min{0, 0, 0}, aabb_max{0, 0, 0};
     V3 grid_lo{0, 0, 0};
     int32_t grid_dims[3] = {0, 0, 0};
+    float inv_query_cell = 1.0f / kQueryCellBt;
     const int32_t* cell_start = nullptr;
     const CellEntry* cell_entries = nullptr;
     const CellEntry* rank_entries = nullptr;

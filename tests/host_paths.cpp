@@ -1,4 +1,6 @@
 // Host build of the tick's headers for test_host_paths.py: entry points over plain arrays.
+#include <vector>
+
 #include "rg_tick.cuh"
 
 extern "C" {
@@ -36,6 +38,43 @@ void hp_ball_box(const float* basis, const float* pos, const float* offset, cons
         out[17 * i + 1] = c.distance_bt;
         memcpy(out + 17 * i + 2, vs, sizeof(vs));
     }
+}
+
+// n box queries (lo, hi per box) on a mesh: how many visit other triangles, or in another order, than a scan of all
+// triangles in leaf order with the quantized overlap test; `cell` receives the query grid's cell size
+int hp_query_boxes(const float* vertices_uu, long long nv, const int* indices, long long ni, const float* boxes, int n,
+                   float* cell) {
+    using rg::V3;
+    const rg::MeshHost h = rg::build_mesh_host(vertices_uu, nv, indices, ni);
+    rg::MeshDevice m;
+    m.tris = h.dev_tris.data();
+    m.tri_count = static_cast<int32_t>(h.dev_tris.size());
+    m.quant = h.quant;
+    m.grid_lo = h.grid_lo;
+    for (int a = 0; a < 3; ++a) m.grid_dims[a] = h.grid_dims[a];
+    m.inv_query_cell = 1.0f / h.query_cell;
+    m.cell_start = h.cell_start.data();
+    m.cell_entries = h.cell_entries.data();
+    m.rank_entries = h.rank_entries.data();
+    *cell = h.query_cell;
+    int wrong = 0;
+    for (int i = 0; i < n; ++i) {
+        const float* b = boxes + 6 * i;
+        const V3 lo{b[0], b[1], b[2]}, hi{b[3], b[4], b[5]};
+        std::vector<int> got, want;
+        rg::mesh_query_box(m, lo, hi, [&](const rg::DevTri& t) { got.push_back(static_cast<int>(&t - m.tris)); });
+        uint16_t qmin[3], qmax[3];
+        rg::quantize_point(m.quant, lo, 0, qmin);
+        rg::quantize_point(m.quant, hi, 1, qmax);
+        for (int r = 0; r < m.tri_count; ++r) {
+            const rg::DevTri& t = m.tris[r];
+            bool over = true;
+            for (int a = 0; a < 3; ++a) over = over && !(qmin[a] > t.qmax[a] || qmax[a] < t.qmin[a]);
+            if (over) want.push_back(r);
+        }
+        wrong += got != want;
+    }
+    return wrong;
 }
 
 }  // extern "C"

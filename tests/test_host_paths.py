@@ -74,3 +74,40 @@ def test_pair_detector_of_a_body_without_a_position(libs, bad):
             got[name, k] = out
         assert _same(got[name, 0], got[name, 1]), name
         assert got[name, 0][len(places):, 0].any(), name  # some of the sound cases touch
+
+
+def _boxes(rng, v, n):
+    """Boxes around mesh vertices and anywhere, from a point to the largest that one cell serves and past it, on cell
+    and quantization edges, and a few that are not finite."""
+    bt = v * np.float32(1 / 50)
+    at = bt[rng.integers(0, len(bt), n)] + rng.normal(0, 1, (n, 3)) * rng.choice([0.0, 0.01, 1.0, 5.0], (n, 1))
+    at[: n // 8] = np.round(at[: n // 8] / 2) * 2
+    lo, hi = bt.min(0) - 3, bt.max(0) + 3
+    at[n // 8: n // 4] = rng.uniform(lo, hi, (n // 4 - n // 8, 3))
+    size = rng.choice([0.0, 0.002, 0.5, 3.9999, 4.0, 4.001, 9.0], (n, 3))
+    out = np.concatenate([at, at + size], 1).astype(np.float32)
+    out[-3:] = [[np.nan] * 6, [np.inf] * 3 + [np.nan] * 3, [-np.inf] * 3 + [np.inf] * 3]
+    return out
+
+
+@pytest.mark.parametrize("mesh", ["arena", "fine", "coarse box", "largest coordinates", "many large triangles"])
+def test_query_grid_visits_what_a_scan_of_all_triangles_does(libs, mesh, arena_mesh):
+    from rocketgpu_b200 import arena
+    rng = np.random.default_rng(5)
+    if mesh == "arena":
+        v, i = arena_mesh
+    elif mesh == "fine":
+        v, i = arena.generate_fine()
+    else:  # triangles across the whole range: 2 bt cells until their lists would grow too long
+        n, scale = {"coarse box": (12, 4000.0), "largest coordinates": (4, 11500.0),
+                    "many large triangles": (60, 6000.0)}[mesh]
+        v = (rng.uniform(-1, 1, (3 * n, 3)) * scale).astype(np.float32)
+        i = np.arange(3 * n, dtype=np.int32)
+    v, i = np.ascontiguousarray(v, np.float32), np.ascontiguousarray(i, np.int32)
+    boxes = _boxes(rng, v, 1500)
+    cell = ctypes.c_float()
+    ptr = [x.ctypes.data_as(ctypes.c_void_p) for x in (v, i, boxes)]
+    wrong = libs[0].hp_query_boxes(ptr[0], ctypes.c_longlong(len(v)), ptr[1], ctypes.c_longlong(len(i)), ptr[2],
+                                   len(boxes), ctypes.byref(cell))
+    assert wrong == 0
+    assert cell.value == (4.0 if mesh in ("largest coordinates", "many large triangles") else 2.0)
