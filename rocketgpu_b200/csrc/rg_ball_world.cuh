@@ -555,23 +555,32 @@ RG_HDI void append_velocity_rows(BallContactRows& rows, V3 normal, float restitu
 }
 
 // --- queries -------------------------------------------------------------------------------------------------------
-// Visits, in BVH leaf order, every triangle whose quantized bounds overlap the box [lo, hi] (Bullet units).
-template <class F>
-RG_HDI void mesh_query_box(const MeshDevice& m, V3 lo, V3 hi, F&& visit) {
+// The list entries that answer a box query [lo, hi] (Bullet units), in BVH leaf order, and the query's quantized box.
+struct MeshQuery {
+    const CellEntry* list;
+    int begin, end;
+    uint16_t qmin[3], qmax[3];
+    RG_HD bool overlaps(const CellEntry& t) const {
+        return !(qmin[0] > t.qmax[0] || qmax[0] < t.qmin[0] || qmin[1] > t.qmax[1] || qmax[1] < t.qmin[1] ||
+                 qmin[2] > t.qmax[2] || qmax[2] < t.qmin[2]);
+    }
+};
+RG_HDI MeshQuery mesh_query(const MeshDevice& m, V3 lo, V3 hi) {
     // Clamp to the quantization bounds first, exactly as quantize_point does: the box quantizes to the same cells, a
     // box reaching past the mesh shrinks to the part it can overlap, and a box with a non-finite coordinate (a car
     // whose state went NaN, which the reference's EPA can produce on a flat landing) collapses onto the bounds' corner
     // like the reference's quantized BVH walk does, instead of scanning every triangle in one lane.
     lo = vmin(vmax(lo, m.quant.aabb_min), m.quant.aabb_max);
     hi = vmin(vmax(hi, m.quant.aabb_min), m.quant.aabb_max);
-    uint16_t qmin[3], qmax[3];
-    quantize_point(m.quant, lo, 0, qmin);
-    quantize_point(m.quant, hi, 1, qmax);
+    MeshQuery q;
+    quantize_point(m.quant, lo, 0, q.qmin);
+    quantize_point(m.quant, hi, 1, q.qmax);
     const float l3[3] = {lo.x - m.grid_lo.x, lo.y - m.grid_lo.y, lo.z - m.grid_lo.z};
     const bool small = (hi.x - lo.x) <= kQueryExtentBt && (hi.y - lo.y) <= kQueryExtentBt &&
                        (hi.z - lo.z) <= kQueryExtentBt;
-    int begin = 0, end = m.tri_count;
-    const CellEntry* list = m.rank_entries;
+    q.begin = 0;
+    q.end = m.tri_count;
+    q.list = m.rank_entries;
     if (small) {
         int cell[3];
         for (int a = 0; a < 3; ++a) {
@@ -580,29 +589,65 @@ RG_HDI void mesh_query_box(const MeshDevice& m, V3 lo, V3 hi, F&& visit) {
             cell[a] = ci;
         }
         const int ci = (cell[2] * m.grid_dims[1] + cell[1]) * m.grid_dims[0] + cell[0];
-        begin = m.cell_start[ci];
-        end = m.cell_start[ci + 1];
-        list = m.cell_entries;
+        q.begin = m.cell_start[ci];
+        q.end = m.cell_start[ci + 1];
+        q.list = m.cell_entries;
     }
+    return q;
+}
+
+// Visits, in BVH leaf order, every triangle whose quantized bounds overlap the box [lo, hi] (Bullet units).
+template <class F>
+RG_HDI void mesh_query_box(const MeshDevice& m, V3 lo, V3 hi, F&& visit) {
+    const MeshQuery q = mesh_query(m, lo, hi);
     // entries are tested four at a time: the four 16-byte loads are independent, so their latencies overlap
-    auto overlaps = [&](const CellEntry& t) {
-        return !(qmin[0] > t.qmax[0] || qmax[0] < t.qmin[0] || qmin[1] > t.qmax[1] || qmax[1] < t.qmin[1] ||
-                 qmin[2] > t.qmax[2] || qmax[2] < t.qmin[2]);
-    };
-    for (int e = begin; e < end; e += 4) {
+    for (int e = q.begin; e < q.end; e += 4) {
         int rank[4];
         unsigned hits = 0u;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const CellEntry en = list[e + k < end ? e + k : e];
+            const CellEntry en = q.list[e + k < q.end ? e + k : e];
             rank[k] = en.rank;
-            hits |= (e + k < end && overlaps(en)) ? (1u << k) : 0u;
+            hits |= (e + k < q.end && q.overlaps(en)) ? (1u << k) : 0u;
         }
         while (hits != 0u) {
             const int k = ctz32(hits);
             hits &= hits - 1u;
             const int r = k == 0 ? rank[0] : (k == 1 ? rank[1] : (k == 2 ? rank[2] : rank[3]));
             visit(m.tris[r]);
+        }
+    }
+}
+
+// One thread doing a query alone (see mesh_query_box_lanes).
+struct OneLane {
+    static constexpr int kLanes = 1;
+    RG_HD int lane() const { return 0; }
+    RG_HD void sync() const {}
+    RG_HD unsigned ballot(bool p) const { return p ? 1u : 0u; }
+    template <class T>
+    RG_HD T from(const T& v, int) const {
+        return v;
+    }
+};
+// mesh_query_box with the list shared by the lanes of `lanes` (threads of one warp that hold the same query): each lane
+// tests its entries of a round, `test(triangle, result)`, and lane 0 visits the results that hold in the list's order.
+template <class R, class L, class Test, class Visit>
+RG_HDI void mesh_query_box_lanes(const L& lanes, const MeshDevice& m, V3 lo, V3 hi, Test&& test, Visit&& visit) {
+    const MeshQuery q = mesh_query(m, lo, hi);
+    for (int e = q.begin; e < q.end; e += L::kLanes) {
+        const int k = e + lanes.lane();
+        R r;
+        bool holds = false;
+        if (k < q.end) {
+            const CellEntry en = q.list[k];
+            holds = q.overlaps(en) && test(m.tris[en.rank], r);
+        }
+        unsigned hits = lanes.ballot(holds);
+        while (hits != 0u) {
+            const R v = lanes.from(r, ctz32(hits));
+            hits &= hits - 1u;
+            if (lanes.lane() == 0) visit(v);
         }
     }
 }

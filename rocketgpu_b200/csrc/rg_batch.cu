@@ -423,13 +423,58 @@ __global__ void __launch_bounds__(256) car_pre_kernel(CarTickArgs a, int t) {
     a.wheels[idx] = wr;
 }
 
-// Tick part 3, one thread per active car: the vehicle update (four suspension rays against the arena mesh and the
-// ball, tyres, drive, air control) and the car's staged world-step parts, for cars whose wheels can land on no other
-// car and under whose car no other wheel can land (rg::arena_free_cars); the others are left to part 4.
-// Tick part 3a, one thread per wheel of an active car: the wheel's suspension ray against the arena mesh, cast ahead of
-// the car's vehicle update (it reads only the car's pose and config, final once the car's tick start has run).
-__global__ void __launch_bounds__(256) car_rays_kernel(CarTickArgs a, int t) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+// Four lanes of a warp that share one car: lane threadIdx.x & 3 of the group.
+struct FourLanes {
+    static constexpr int kLanes = 4;
+    unsigned mask;
+    int base;  // the group's first lane in the warp
+    __device__ FourLanes() : base(static_cast<int>(threadIdx.x & 28u)) { mask = 15u << base; }
+    __device__ int lane() const { return static_cast<int>(threadIdx.x & 3u); }
+    __device__ void sync() const { __syncwarp(mask); }
+    __device__ unsigned ballot(bool p) const { return (__ballot_sync(mask, p) >> base) & 15u; }
+    // lane `src`'s value (a struct of 32-bit words)
+    template <class T>
+    __device__ T from(const T& v, int src) const {
+        static_assert(sizeof(T) % 4 == 0, "whole words");
+        constexpr int kWords = sizeof(T) / 4;
+        uint32_t w[kWords];
+        memcpy(w, &v, sizeof(T));
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) w[i] = __shfl_sync(mask, w[i], src, 4);
+        T out;
+        memcpy(&out, w, sizeof(T));
+        return out;
+    }
+};
+
+// Tick part 3a, what reads only poses and so runs ahead of the vehicle updates, in blocks of three kinds that the chip
+// runs side by side: [0, mesh_blocks) four lanes per active car, the geometry of its arena contacts (triangles shared by
+// the lanes); [mesh_blocks, mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact
+// geometry; the rest one thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets
+// another car's box.
+__global__ void __launch_bounds__(256) car_geometry_kernel(CarTickArgs a, int t, int mesh_blocks, int ball_blocks) {
+    const int block = static_cast<int>(blockIdx.x);
+    if (block < mesh_blocks) {
+        const int k = static_cast<int>(block * blockDim.x + threadIdx.x) >> 2;
+        if (k >= a.active_car_count) return;
+        const int idx = a.active_cars[k];
+        const int e = idx / a.max_cars;
+        if (arena_idle(a, e)) return;
+        rg::car_mesh_stage(FourLanes(), a.cars[idx], a.car_cfgs[idx], a.car_world[idx], arena_mesh(a.base, e),
+                           a.stages[idx]);
+        return;
+    }
+    if (block < mesh_blocks + ball_blocks) {
+        const int k = static_cast<int>((block - mesh_blocks) * blockDim.x + threadIdx.x);
+        if (k >= a.active_car_count) return;
+        const int idx = a.active_cars[k];
+        const int e = idx / a.max_cars;
+        if (arena_idle(a, e)) return;
+        rg::car_proxy_ball_stage(a.base.balls[e], a.snaps[e].ball_vel_bt, a.cars[idx], a.car_cfgs[idx], a.base.tc,
+                                 a.records[idx].vel_bt, a.records[idx].ang_vel, a.ball_car[idx], a.stages[idx]);
+        return;
+    }
+    const int g = static_cast<int>((block - mesh_blocks - ball_blocks) * blockDim.x + threadIdx.x);
     const int k = g >> 2, wheel = g & 3;
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
@@ -443,42 +488,81 @@ __global__ void __launch_bounds__(256) car_rays_kernel(CarTickArgs a, int t) {
     }
     const int base = e * a.max_cars, count = a.base.env_car_count[e], slot = idx - base;
     const uint32_t excluded = rg::wheel_ray_excluded_bodies(car, a.car_cfgs[idx], a.broadphase + e, slot, count);
+    uint8_t meets = 0;
     rg::wheel_mesh_ray_ahead(car, a.car_cfgs[idx], arena_mesh(a.base, e), wheel,
                              rg::WheelOthers{a.cars + base, a.car_cfgs + base, count, slot, excluded},
-                             st.wheel_mesh[wheel], st.wheel_meets_car[wheel]);
+                             st.wheel_mesh[wheel], meets);
+    st.wheel_meets_car[wheel] = static_cast<uint8_t>((meets ? rg::kWheelMeetsCar : 0) |
+                                                     ((excluded & 1u) ? rg::kWheelBallExcluded : 0));
 }
 
-__global__ void __launch_bounds__(256) car_vehicle_kernel(CarTickArgs a, int t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// Tick part 3b, four lanes per active car: the vehicle update (tyres, drive, air control) and the car's staged
+// world-step parts, for cars whose wheels can land on no other car and under whose car no other wheel can land
+// (rg::arena_free_cars); the others are left to part 4. The car, its wheel record and its config are worked on in shared
+// memory: one thread per car on the structs in HBM took 893 us at 16,384 mixed arenas (11 warps per SM, 37 cycles per
+// instruction waiting for lines of 880-byte-strided structs that the L1 could not hold).
+struct alignas(16) VehicleSlot {
+    rg::CarState car;
+    rg::WheelRuntime wheels;
+    alignas(8) rg::CarConfig cfg;
+    rg::VehicleTick tick;
+};
+// lanes_copy's words: 16 bytes for the car, 4 for the wheel record (292 bytes), 8 for the config
+static_assert(offsetof(VehicleSlot, car) % 16 == 0 && offsetof(VehicleSlot, cfg) % 8 == 0, "aligned copies");
+// An odd number of 16-byte units, so that the same field of a warp's eight cars falls into eight different banks.
+constexpr size_t kVehicleSlotBytes = sizeof(VehicleSlot) / 16 % 2 == 1 ? sizeof(VehicleSlot) : sizeof(VehicleSlot) + 16;
+constexpr int kVehicleThreads = 64;
+
+// A struct copied by the four lanes of a group, word l, l + 4, ... by lane l.
+template <class Word, class T>
+__device__ __forceinline__ void lanes_copy(T* dst, const T* src, int lane) {
+    static_assert(sizeof(T) % sizeof(Word) == 0, "whole words: every struct of an array is aligned to one");
+    constexpr int kWords = sizeof(T) / sizeof(Word), kRounds = (kWords + 3) / 4;
+    const Word* s = reinterpret_cast<const Word*>(src);
+    Word* d = reinterpret_cast<Word*>(dst);
+    Word w[kRounds];
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i)
+        if (4 * i + lane < kWords) w[i] = s[4 * i + lane];
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i)
+        if (4 * i + lane < kWords) d[4 * i + lane] = w[i];
+}
+
+__global__ void __launch_bounds__(kVehicleThreads) car_vehicle_kernel(CarTickArgs a, int t) {
+    __shared__ __align__(16) unsigned char shared[kVehicleThreads / 4 * kVehicleSlotBytes];
+    const FourLanes lanes;
+    const int k = static_cast<int>(blockIdx.x * (kVehicleThreads / 4) + (threadIdx.x >> 2));
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
     const int e = idx / a.max_cars;
     if (arena_idle(a, e)) return;
     const int base = e * a.max_cars;
     const int count = a.base.env_car_count[e];
+    VehicleSlot& s = *reinterpret_cast<VehicleSlot*>(shared + (threadIdx.x >> 2) * kVehicleSlotBytes);
+    lanes_copy<uint4>(&s.car, a.cars + idx, lanes.lane());
+    lanes_copy<uint32_t>(&s.wheels, a.wheels + idx, lanes.lane());
+    lanes_copy<uint2>(&s.cfg, a.car_cfgs + idx, lanes.lane());
     // the car's update runs here when no wheel of the arena meets another car, or when the sweep-box rule shows that
     // no other car can be under its wheels nor it under theirs
     const bool free =
         !rg::arena_wheels_meet_cars(a.stages + base, count) ||
         ((rg::arena_free_cars(a.cars + base, a.car_cfgs + base, a.broadphase[e], count) >> (idx - base)) & 1u);
-    a.stages[idx].in_car_thread = free ? 1u : 0u;
-    // every car's ball contact geometry, before its vehicle update (it reads poses only)
-    rg::car_ball_stage(a.base.balls[e], a.snaps[e].ball_vel_bt, a.cars[idx], a.car_cfgs[idx], a.base.tc,
-                       a.records[idx].vel_bt, a.records[idx].ang_vel, a.ball_car[idx], a.stages[idx]);
+    rg::CarStage& st = a.stages[idx];
+    if (lanes.lane() == 0) st.in_car_thread = free ? 1u : 0u;
     if (!free) return;  // the arena thread updates this car in the game's car order
+    lanes.sync();
     const rg::CarControls& ctrl =
         a.controls[control_row(a, e, t) * static_cast<size_t>(a.control_stride) + static_cast<size_t>(idx)];
-    const uint32_t excluded =
-        a.cars[idx].is_demoed ? 0u
-                              : rg::wheel_ray_excluded_bodies(a.cars[idx], a.car_cfgs[idx], a.broadphase + e, idx - base,
-                                                              count);
+    const uint32_t excluded = (st.wheel_meets_car[0] & rg::kWheelBallExcluded) ? 1u : 0u;
     const rg::MeshDevice& mesh = arena_mesh(a.base, e);
-    rg::vehicle_update(a.cars[idx], ctrl, a.car_cfgs[idx], a.base.tc, a.wheels[idx], a.base.balls[e], mesh,
-                       rg::WheelOthers{nullptr, nullptr, 0, -1, excluded}, a.records[idx].pushes,
-                       a.stages[idx].wheel_mesh);
+    rg::vehicle_update(lanes, s.car, ctrl, s.cfg, a.base.tc, s.wheels, a.base.balls[e], mesh,
+                       rg::WheelOthers{nullptr, nullptr, 0, -1, excluded}, a.records[idx].pushes, st.wheel_mesh, s.tick);
     // the car's own part of the world step, while this thread has the car (rg::CarStage)
-    rg::car_stage_compute(a.cars[idx], a.car_cfgs[idx], a.wheels[idx], a.car_world[idx], a.base.tc, mesh, idx - base,
-                          a.records[idx].vel_bt, a.records[idx].ang_vel, a.stages[idx]);
+    if (lanes.lane() == 0) rg::car_stage_compute(s.car, s.cfg, s.wheels, a.base.tc, mesh, idx - base, st);
+    lanes.sync();
+    lanes_copy<uint4>(a.cars + idx, &s.car, lanes.lane());
+    lanes_copy<uint32_t>(a.wheels + idx, &s.wheels, lanes.lane());
 }
 
 // Tick part 4, one thread per arena in step order: the vehicle updates (and staged parts) of cars whose wheels may
@@ -590,6 +674,7 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
     const int ct = b->car_threads;
     const int car_blocks = (b->active_car_count + ct - 1) / ct;
     const int wheel_blocks = (4 * b->active_car_count + ct - 1) / ct;
+    const int vehicle_blocks = (4 * b->active_car_count + kVehicleThreads - 1) / kVehicleThreads;
     auto mark = [&] {
         if (!b->timing) return;
         if (b->events_used == b->events.size()) {
@@ -605,9 +690,10 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         mark();
         if (car_blocks) car_pre_kernel<<<car_blocks, ct, 0, s>>>(a, t);
         mark();
-        // phase 2 (timing) is the wheel rays and the vehicle updates
-        if (car_blocks) car_rays_kernel<<<wheel_blocks, ct, 0, s>>>(a, t);
-        if (car_blocks) car_vehicle_kernel<<<car_blocks, ct, 0, s>>>(a, t);
+        // phase 2 (timing) is the geometry and the vehicle updates
+        if (car_blocks)
+            car_geometry_kernel<<<2 * wheel_blocks + car_blocks, ct, 0, s>>>(a, t, wheel_blocks, car_blocks);
+        if (car_blocks) car_vehicle_kernel<<<vehicle_blocks, kVehicleThreads, 0, s>>>(a, t);
         mark();
         arena_finish_kernel<<<blocks, threads, 0, s>>>(a, t);
         mark();

@@ -376,24 +376,13 @@ struct MeshContactEvents {
     V3 normal[4];
 };
 
-// The car's contacts with the arena mesh for this tick: refresh the retained manifold, collect candidates from the
-// triangles the box overlaps, merge them into the manifold and emit rows (body index `body`, source tag 100).
-// `listed`: the car/mesh manifold exists in the broadphase list.
-// The car does not change here: a hit (res.hit) is recorded by the caller (car_record_world_surface(c, true), once
-// for the points the reference records one by one: the record is idempotent), at the place in the tick where the
-// reference's query runs.
-template <class Rows>
-RG_NOINL CarWorldContactResult car_mesh_contacts(const CarState& c, const CarConfig& cfg, CarWorldScratch& ws,
-                                               bool listed, const MeshDevice& mesh, const TickConfig& tc, int body,
-                                               Rows& rows, MeshContactEvents* events = nullptr) {
-    CarWorldContactResult res;
-    res.hit = false;
-    res.latest_normal = V3{0.0f, 0.0f, 1.0f};
-    if (events) events->count = 0;
-    if (!listed) {
-        ws.count = 0;
-        return res;
-    }
+// The geometry of the car's contacts with the arena mesh for this tick: refresh the retained manifold, collect
+// candidates from the triangles the box overlaps and merge them into the manifold. It reads the car's pose and config
+// only, so it runs ahead of the car's vehicle update. The lanes of `lanes` share the triangles; lane 0 holds the
+// manifold and returns the last contact's triangle normal.
+template <class L>
+RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& cfg, CarWorldScratch& ws,
+                            const MeshDevice& mesh) {
     const float thr = car_contact_threshold_bt(cfg);
     V3 f, r, u;
     car_basis(c, f, r, u);
@@ -424,7 +413,7 @@ RG_NOINL CarWorldContactResult car_mesh_contacts(const CarState& c, const CarCon
         }
     };
     bool seeded = false;
-    if (ws.count > 0) {
+    if (lanes.lane() == 0 && ws.count > 0) {
         refresh();
         for (int k = 0; k < ws.count; ++k) {
             const CarMeshPoint& p = ws.pts[k];
@@ -445,10 +434,12 @@ RG_NOINL CarWorldContactResult car_mesh_contacts(const CarState& c, const CarCon
     }
     V3 last_normal{0.0f, 0.0f, 1.0f};
     const CarQueryFrame qf = car_query_frame(c, cfg);
-    mesh_query_box(mesh, qf.lo, qf.hi, [&](const DevTri& t) {
-        if (car_triangle_query(t, qf, thr) != 2) return;
-        const CarTriHit h = car_triangle_hit(f, r, u, pos, cfg, t, thr);
-        if (!h.hit || h.distance > thr) return;
+    auto test = [&](const DevTri& t, CarTriHit& h) {
+        if (car_triangle_query(t, qf, thr) != 2) return false;
+        h = car_triangle_hit(f, r, u, pos, cfg, t, thr);
+        return h.hit && !(h.distance > thr);
+    };
+    mesh_query_box_lanes<CarTriHit>(lanes, mesh, qf.lo, qf.hi, test, [&](const CarTriHit& h) {
         MeshCandidate m;
         m.normal = h.normal;
         m.raw_normal = h.raw_normal;
@@ -488,12 +479,11 @@ RG_NOINL CarWorldContactResult car_mesh_contacts(const CarState& c, const CarCon
         }
         cand[mesh_replace_index(cand, m)] = m;
     });
+    if (lanes.lane() != 0) return last_normal;
     // the manifold keeps this tick's candidates (seeded points carry over unchanged)
     if (seeded) {
         refresh();
         ws.count = 0;
-    } else if (n == 0) {
-        return res;
     }
     for (int k = 0; k < n; ++k) {
         if (seeded && cand[k].seed >= 0) {
@@ -507,8 +497,25 @@ RG_NOINL CarWorldContactResult car_mesh_contacts(const CarState& c, const CarCon
         p.distance = dot(car_world_point(f, r, u, pos, p.local_a) - p.local_b, p.normal);
         ws.pts[ws.count++] = p;
     }
-    n = ws.count;
+    return last_normal;
+}
+
+// The contact rows of the manifold that car_mesh_geometry left, from the car's velocities as they stand now (body index
+// `body`, source tag 100). The car does not change here: a hit (res.hit) is recorded by the caller
+// (car_record_world_surface(c, true), once for the points the reference records one by one: the record is idempotent),
+// at the place in the tick where the reference's query runs.
+template <class Rows>
+RG_HDI CarWorldContactResult car_mesh_rows(const CarState& c, const CarConfig& cfg, const CarWorldScratch& ws,
+                                           V3 last_normal, const TickConfig& tc, int body, Rows& rows,
+                                           MeshContactEvents* events = nullptr) {
+    CarWorldContactResult res;
+    res.hit = false;
+    res.latest_normal = V3{0.0f, 0.0f, 1.0f};
+    const int n = ws.count;
     if (n <= 0) return res;
+    V3 f, r, u;
+    car_basis(c, f, r, u);
+    const V3 pos = c.pos_bt;
     // rows (reference emit_candidates)
     V3 i0, i1, i2, u0, u1, u2;
     car_inv_inertia_world_bt(c, cfg, tc.car_mass, i0, i1, i2);

@@ -1234,14 +1234,17 @@ RG_HDI bool ball_car_box_overlaps(const BallState& b, const CarState& car, const
 
 // ---- a car's part of the world step, staged ------------------------------------------------------------------
 // What one car of an arena contributes to the world step before the arena's shared stages, computed by the per-car
-// kernel right after the car's vehicle update (one thread per car instead of one per arena): the prestep, the car's
-// predictive contact and its query against the arena mesh, with the retained manifold and the rows that query leaves
-// (as if its manifold is listed, which the arena checks later). Exact: these read and write only the car, its wheel
-// record and its car/mesh manifold (not the ball, the other cars or the broadphase), nothing the arena does between
-// the vehicle update and their place in the world step changes what they read (car/car and car/ball contacts touch
-// only the cars' contact bookkeeping), and their effects on the car (the world-surface record, the contact normal)
-// are applied by the arena where the reference makes them. A car whose vehicle update must run in the arena's car
-// order (arena_free_cars) has its stage computed by the arena thread after all those updates.
+// kernels: the geometry of its arena and ball contacts and its broadphase proxy, which read only the car's pose and
+// config (car_geometry_kernel, every car), then the prestep, the car's predictive contact and the rows of its arena
+// contacts (as if its manifold is listed, which the arena checks later), which read the velocities its vehicle update
+// leaves (car_vehicle_kernel). Exact: these read and write only the car, its wheel record and its car/mesh manifold (not
+// the ball's velocity, the other cars or the broadphase), nothing the arena does between the vehicle update and their
+// place in the world step changes what they read (car/car and car/ball contacts touch only the cars' contact
+// bookkeeping), and their effects on the car (the world-surface record, the contact normal) are applied by the arena
+// where the reference makes them. A car whose vehicle update must run in the arena's car order (arena_free_cars) has
+// its second part computed by the arena thread after all those updates.
+// Per wheel: its ray meets another car's box; the car's rays skip the ball (wheel_ray_excluded_bodies).
+constexpr uint8_t kWheelMeetsCar = 1, kWheelBallExcluded = 2;
 struct CarStage {
     PreContactCar pre;
     V3 pred_n;
@@ -1255,7 +1258,7 @@ struct CarStage {
     PadContacts pads;    // the car's pad contacts after its post-tick (pad_contacts_stage)
     uint32_t in_car_thread;  // this tick's vehicle update and stage ran in the car's own thread (arena_free_cars)
     RayHit wheel_mesh[4];    // the wheels' arena-mesh rays, cast ahead of the vehicle update (wheel_mesh_ray_ahead)
-    uint8_t wheel_meets_car[4];  // the wheel's ray meets another car's box (0 for a demolished car)
+    uint8_t wheel_meets_car[4];  // kWheelMeetsCar, kWheelBallExcluded (0 for a demolished car)
     BallCarScratch ball_manifold;  // the car/ball manifold after this tick's geometry (car_ball_stage)
     uint32_t ball_staged;          // ball_manifold holds this tick's update
     MeshContactEvents mesh_events;  // the query's car-world events (when events are on)
@@ -1272,48 +1275,69 @@ RG_HDI void car_body_proxy(BpProxy& p, const CarState& car, const CarConfig& cfg
               dt);
 }
 
-// The car's ball contact geometry ahead of the world step (one thread per car). The manifold update reads only the
-// two bodies' poses, and neither body moves between the tick start and the world step's car-ball stage (vehicle
-// updates, wheel pushes, bumps and demolitions change velocities and flags only). Staged when the car's box or swept
-// proxy meets the ball's, a superset of the world step's test; the world step takes it when its own test passes.
-RG_HDI void car_ball_stage(const BallState& b, V3 ball_start_vel_bt, const CarState& car, const CarConfig& cfg,
-                           const TickConfig& c, V3 start_vel_bt, V3 start_ang_vel, const BallCarScratch& m_in,
-                           CarStage& st) {
+// The car's broadphase proxy and its ball contact geometry ahead of the world step (one thread per car). The manifold
+// update reads only the two bodies' poses, and neither body moves between the tick start and the world step's car-ball
+// stage (vehicle updates, wheel pushes, bumps and demolitions change velocities and flags only). Staged when the car's
+// box or swept proxy meets the ball's, a superset of the world step's test; the world step takes it when its own test
+// passes.
+RG_HDI void car_proxy_ball_stage(const BallState& b, V3 ball_start_vel_bt, const CarState& car, const CarConfig& cfg,
+                                 const TickConfig& c, V3 start_vel_bt, V3 start_ang_vel, const BallCarScratch& m_in,
+                                 CarStage& st) {
     st.ball_staged = 0u;
-    if (car.is_demoed || car.just_respawned) return;  // the world step's tests fail for both
+    st.proxy.valid = 0;
+    if (car.is_demoed) return;
+    BpProxy pc;
+    car_body_proxy(pc, car, cfg, start_vel_bt, start_ang_vel, c.tick_dt);
+    st.proxy = pc;
+    if (car.just_respawned) return;  // the world step's tests fail for a car demolished or just back
     bool meet = ball_car_box_overlaps(b, car, cfg, c, true);
     if (!meet) {
-        BpProxy pb, pc;
+        BpProxy pb;
         ball_proxy(pb, b.pos_bt, ball_start_vel_bt, c.ball_radius, c.tick_dt);
-        car_body_proxy(pc, car, cfg, start_vel_bt, start_ang_vel, c.tick_dt);
-        meet = pc.valid != 0 && !(pc.child_min.x > pb.child_max.x || pc.child_max.x < pb.child_min.x ||
-                                  pc.child_min.y > pb.child_max.y || pc.child_max.y < pb.child_min.y ||
-                                  pc.child_min.z > pb.child_max.z || pc.child_max.z < pb.child_min.z);
+        meet = !(pc.child_min.x > pb.child_max.x || pc.child_max.x < pb.child_min.x ||
+                 pc.child_min.y > pb.child_max.y || pc.child_max.y < pb.child_min.y ||
+                 pc.child_min.z > pb.child_max.z || pc.child_max.z < pb.child_min.z);
     }
     if (!meet) return;
-    st.ball_manifold = m_in;
-    ball_car_manifold_update(st.ball_manifold, b, car, cfg, c);
+    BallCarScratch m = m_in;
+    ball_car_manifold_update(m, b, car, cfg, c);
+    st.ball_manifold = m;
     st.ball_staged = 1u;
 }
 
-RG_HDI void car_stage_compute(CarState& car, const CarConfig& cfg, WheelRuntime& w, const CarWorldScratch& ws_in,
-                              const TickConfig& c, const MeshDevice& mesh, int slot, V3 start_vel_bt, V3 start_ang_vel,
-                              CarStage& st) {
-    const float sub_dt = c.tick_dt;
-    car_world_prestep(car, cfg, w, c, sub_dt, st.pre);
-    st.proxy.valid = 0;
-    if (!st.pre.is_demoed) car_body_proxy(st.proxy, car, cfg, start_vel_bt, start_ang_vel, sub_dt);
-    st.pred_hit = !st.pre.is_demoed && car_predictive_hit(car, cfg, mesh, sub_dt, st.pred_n, st.pred_d) ? 1u : 0u;
-    st.mesh_ran = !(st.pre.is_demoed || car.just_respawned) ? 1u : 0u;
-    st.rows.nv = st.rows.nf = st.rows.ns = 0;
-    st.res.hit = false;
-    st.res.latest_normal = V3{0.0f, 0.0f, 1.0f};
-    st.mesh_events.count = 0;
-    if (st.mesh_ran) {
-        st.ws = ws_in;
-        st.res = car_mesh_contacts(car, cfg, st.ws, true, mesh, c, slot, st.rows,
-                                   c.events.windows ? &st.mesh_events : nullptr);
+// The geometry of the car's arena contacts ahead of its vehicle update (car_mesh_geometry), by the lanes that share it.
+template <class L>
+RG_HDI void car_mesh_stage(const L& lanes, const CarState& car, const CarConfig& cfg, const CarWorldScratch& ws_in,
+                           const MeshDevice& mesh, CarStage& st) {
+    const bool runs = !(car.is_demoed || car.just_respawned);
+    if (lanes.lane() == 0) st.mesh_ran = runs ? 1u : 0u;
+    if (!runs) return;
+    CarWorldScratch ws;
+    if (lanes.lane() == 0) ws = ws_in;
+    const V3 last_normal = car_mesh_geometry(lanes, car, cfg, ws, mesh);
+    if (lanes.lane() == 0) {
+        st.ws = ws;
+        st.res.latest_normal = last_normal;
     }
+}
+
+// The rest of the car's staged part, after its vehicle update.
+RG_HDI void car_stage_compute(CarState& car, const CarConfig& cfg, const WheelRuntime& w, const TickConfig& c,
+                              const MeshDevice& mesh, int slot, CarStage& st) {
+    const float sub_dt = c.tick_dt;
+    PreContactCar pre;
+    car_world_prestep(car, cfg, w, c, sub_dt, pre);
+    st.pre = pre;
+    st.pred_hit = !pre.is_demoed && car_predictive_hit(car, cfg, mesh, sub_dt, st.pred_n, st.pred_d) ? 1u : 0u;
+    st.rows.nv = st.rows.nf = st.rows.ns = 0;
+    st.mesh_events.count = 0;
+    CarWorldContactResult res;
+    res.hit = false;
+    res.latest_normal = V3{0.0f, 0.0f, 1.0f};
+    if (st.mesh_ran)
+        res = car_mesh_rows(car, cfg, st.ws, st.res.latest_normal, c, slot, st.rows,
+                            c.events.windows ? &st.mesh_events : nullptr);
+    st.res = res;
 }
 
 // One arena's world step with cars (reference WorldStepSoccar, env_step.hpp:4727-5623, on the path a custom-mesh
@@ -1324,7 +1348,7 @@ RG_HDI void car_stage_compute(CarState& car, const CarConfig& cfg, WheelRuntime&
 RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp, CarWorldScratch* cws,
                             BallCarScratch* bcs, const TickConfig& c, const MeshDevice& mesh, const ArenaCars& A,
                             PreContactCar* pre, const TickSnap& snap, uint64_t env_tick,
-                            const CarStage* stages = nullptr) {
+                            const CarStage* stages) {
     const int count = A.count;
     const float sub_dt = c.tick_dt;
     const bool vehicle_woke = (b.sleeping & 4u) != 0;
@@ -1332,11 +1356,7 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
     const bool ball_sleeping = ball_resolve_activation(b);
     if (vehicle_woke) b.deactivation_time = 0.0f;
     const V3 ext_delta = ball_sleeping ? V3{0.0f, 0.0f, 0.0f} : V3{0.0f, 0.0f, c.gravity_z * sub_dt};
-    if (stages) {
-        for (int i = 0; i < count; ++i) pre[i] = stages[i].pre;
-    } else {
-        for (int i = 0; i < count; ++i) car_world_prestep(A.cars[i], A.cfgs[i], A.wheels[i], c, sub_dt, pre[i]);
-    }
+    for (int i = 0; i < count; ++i) pre[i] = stages[i].pre;
     const V3 solver_vel_bt = b.vel_bt;
     // where the bodies stand at the step's start, for the ball-hit records (reference record_ball_car_info)
     const V3 hit_ball_pos = b.pos;
@@ -1354,29 +1374,20 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
     float pred_d[kBpBodies];
     if (!(ball_sleeping && !vehicle_woke) && ball_predictive_hit(b, mesh, sub_dt, pred_n[0], pred_d[0])) pred_mask |= 1u;
     for (int i = 0; i + 1 < body_count; ++i) {
-        if (pre[i].is_demoed) continue;
-        if (stages) {
-            if (stages[i].pred_hit) {
-                pred_n[i + 1] = stages[i].pred_n;
-                pred_d[i + 1] = stages[i].pred_d;
-                pred_mask |= 1u << (i + 1);
-            }
-        } else if (car_predictive_hit(A.cars[i], A.cfgs[i], mesh, sub_dt, pred_n[i + 1], pred_d[i + 1])) {
-            pred_mask |= 1u << (i + 1);
-        }
+        if (pre[i].is_demoed || !stages[i].pred_hit) continue;
+        pred_n[i + 1] = stages[i].pred_n;
+        pred_d[i + 1] = stages[i].pred_d;
+        pred_mask |= 1u << (i + 1);
     }
     // broadphase proxies and the manifold list (reference BuildBulletManifoldList + SortBulletManifoldListByIsland)
     BpProxy proxies[kBpBodies];
     ball_proxy(proxies[0], b.pos_bt, snap.ball_vel_bt, c.ball_radius, sub_dt);
     for (int i = 0; i + 1 < body_count; ++i) {
         BpProxy& p = proxies[i + 1];
-        if (pre[i].is_demoed) {
+        if (pre[i].is_demoed)
             p.valid = 0;
-        } else if (stages) {
+        else
             p = stages[i].proxy;
-        } else {
-            car_body_proxy(p, A.cars[i], A.cfgs[i], snap.car_vel_bt[i], snap.car_ang_vel[i], sub_dt);
-        }
     }
     BpEntry list[kBpMaxEntries];
     const int n_list = bp_build_manifold_list(bp, proxies, body_count, mesh.aabb_min, mesh.aabb_max, pred_mask,
@@ -1454,7 +1465,7 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
             bcs[i].count = 0;
             continue;
         }
-        if (stages && stages[i].ball_staged) {
+        if (stages[i].ball_staged) {
             bcs[i] = stages[i].ball_manifold;
             ball_car_manifold_rows(bcs[i], b, car, A.cfgs[i], c, i, ext_delta, solver_vel_bt, sub_dt, bc);
         } else {
@@ -1487,21 +1498,14 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
             listed = listed || (bp_kind(key) == 2 && bp_body_a(key) == i && bp_static(key) == 0);
         }
         if (!listed && cws[i].count == 0) continue;
-        CarWorldContactResult res;
-        MeshContactEvents ev;
-        const MeshContactEvents* events = nullptr;
-        if (!stages) {
-            res = car_mesh_contacts(car, A.cfgs[i], cws[i], listed, mesh, c, i, cr, c.events.windows ? &ev : nullptr);
-            events = &ev;
-        } else if (!listed) {
+        if (!listed) {
             cws[i].count = 0;  // what the query does for an unlisted manifold
             continue;
-        } else {
-            cws[i] = stages[i].ws;
-            append_car_rows(cr, stages[i].rows);
-            res = stages[i].res;
-            events = &stages[i].mesh_events;
         }
+        cws[i] = stages[i].ws;
+        append_car_rows(cr, stages[i].rows);
+        const CarWorldContactResult res = stages[i].res;
+        const MeshContactEvents* events = &stages[i].mesh_events;
         if (c.events.windows) {
             for (uint32_t k = 0; k < events->count; ++k) {
                 PhysicsEvent e = new_event(kEventCarWorldContact);
@@ -1705,7 +1709,7 @@ RG_HDI bool arena_wheels_meet_cars(const CarStage* stages, int count) {
     for (int i = 0; i < count; ++i)
         any |= stages[i].wheel_meets_car[0] | stages[i].wheel_meets_car[1] | stages[i].wheel_meets_car[2] |
                stages[i].wheel_meets_car[3];
-    return any != 0u;
+    return (any & kWheelMeetsCar) != 0u;
 }
 
 RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, Broadphase& bp, CarWorldScratch* cws,
@@ -1731,13 +1735,12 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
         if (stages[i].in_car_thread) continue;
         left |= 1u << i;
         const uint32_t excluded = A.cars[i].is_demoed ? 0u : wheel_ray_excluded_bodies(A.cars[i], A.cfgs[i], &bp, i, count);
-        vehicle_update(A.cars[i], A.controls[i], A.cfgs[i], c, A.wheels[i], b, mesh,
-                       WheelOthers{A.cars, A.cfgs, count, i, excluded}, recs[i].pushes, stages[i].wheel_mesh);
+        VehicleTick v;
+        vehicle_update(OneLane{}, A.cars[i], A.controls[i], A.cfgs[i], c, A.wheels[i], b, mesh,
+                       WheelOthers{A.cars, A.cfgs, count, i, excluded}, recs[i].pushes, stages[i].wheel_mesh, v);
     }
     for (int i = 0; i < count; ++i)
-        if ((left >> i) & 1u)
-            car_stage_compute(A.cars[i], A.cfgs[i], A.wheels[i], cws[i], c, mesh, i, recs[i].vel_bt, recs[i].ang_vel,
-                              stages[i]);
+        if ((left >> i) & 1u) car_stage_compute(A.cars[i], A.cfgs[i], A.wheels[i], c, mesh, i, stages[i]);
     if (c.events.windows) {
         // the vehicle updates' car-world events, in the game's car order (each update emits its own in the reference)
         for (int k = 0; k < count; ++k) {

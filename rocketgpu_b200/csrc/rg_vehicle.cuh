@@ -655,9 +655,9 @@ RG_HDI void world_wheel_pushback(const CarState& c, const TickConfig& tc, WheelS
 }
 
 // ---- drive (reference :1501-1535, 1697-1796) ----------------------------------------------------------------------
-RG_HDI V3 wheel_steered_right_col(const WheelStep& w, float steer_angle) {
-    const V3 up = -w.wheel_dir_ws;
-    const V3 right = w.wheel_axle_ws;
+RG_HDI V3 wheel_steered_right_col(const CarFrame& f, float steer_angle) {
+    const V3 up = -(-f.up);  // through the wheel's direction and axle, as the reference reads them
+    const V3 right = -f.right;
     const float half_angle = steer_angle * 0.5f;
     const float sin_scale = (half_angle == 0.0f && len2(up) > 0.0f) ? half_angle : (game_sinf(half_angle) / len(up));
     const float cos_half = (half_angle == 0.0f) ? 1.0f : game_cosf(half_angle);
@@ -772,58 +772,55 @@ RG_HDI void combine_wheel_impulses(CarState& c, const WheelImpulse* o) {
         c.ang_vel = ang_vel;
     }
 }
-RG_HDI void wheel_suspension_and_friction(CarState& c, const TickConfig& tc, WheelStep* wh, const CarFrame& f) {
-    if (!(wh[0].is_in_contact || wh[1].is_in_contact || wh[2].is_in_contact || wh[3].is_in_contact)) return;
-    const float dt = tc.tick_dt;
-    WheelImpulse o[4];
-    for (int i = 0; i < 4; ++i) {
-        WheelStep& w = wh[i];
-        o[i].applied = false;
-        if (!w.is_in_contact) continue;
-        const float force_bt = (w.suspension_rest_length * kUuToBt - w.suspension_len_bt) *
-                               kWheelSuspensionStiffness * w.clipped_inv_contact_dot_suspension;
-        const float damping =
-            w.suspension_relative_velocity < 0.0f ? kWheelDampingCompression : kWheelDampingRelaxation;
-        float susp = (force_bt - damping * w.suspension_relative_velocity_bt) * w.suspension_force_scale;
-        if (susp < 0.0f) susp = 0.0f;
-        if (susp * 50.0f > 0.0f) {
-            const V3 rel_bt = w.contact_point_bt - c.pos_bt;
-            const float scale = (susp * dt) + w.extra_pushback;
-            o[i] = wheel_impulse_at(tc.car_mass, f, w.contact_normal_ws * scale, rel_bt);
-        }
+// One wheel's suspension impulse.
+RG_HDI WheelImpulse wheel_suspension_impulse(const CarState& c, const TickConfig& tc, const WheelStep& w,
+                                             const CarFrame& f) {
+    WheelImpulse o;
+    o.applied = false;
+    if (!w.is_in_contact) return o;
+    const float force_bt = (w.suspension_rest_length * kUuToBt - w.suspension_len_bt) * kWheelSuspensionStiffness *
+                           w.clipped_inv_contact_dot_suspension;
+    const float damping = w.suspension_relative_velocity < 0.0f ? kWheelDampingCompression : kWheelDampingRelaxation;
+    float susp = (force_bt - damping * w.suspension_relative_velocity_bt) * w.suspension_force_scale;
+    if (susp < 0.0f) susp = 0.0f;
+    if (susp * 50.0f > 0.0f) {
+        const V3 rel_bt = w.contact_point_bt - c.pos_bt;
+        const float scale = (susp * tc.tick_dt) + w.extra_pushback;
+        o = wheel_impulse_at(tc.car_mass, f, w.contact_normal_ws * scale, rel_bt);
     }
-    combine_wheel_impulses(c, o);
-    // the bilateral body after the suspension impulses (reference MakeBilateralCarBodyBt)
+    return o;
+}
+// One wheel's tyre impulse on the body as the suspension impulses left it (reference MakeBilateralCarBodyBt).
+RG_HDI WheelImpulse wheel_friction_impulse(const CarState& c, const TickConfig& tc, const WheelStep& w,
+                                           const CarFrame& f) {
+    WheelImpulse o;
+    o.applied = false;
+    if (!w.is_in_contact) return o;
+    const float dt = tc.tick_dt;
     const V3 com = c.pos_bt, lin = c.vel_bt, ang = c.ang_vel;
     const float inv_mass = tc.car_mass != 0.0f ? 1.0f / tc.car_mass : 0.0f;
-    for (int i = 0; i < 4; ++i) {
-        WheelStep& w = wh[i];
-        o[i].applied = false;
-        if (!w.is_in_contact) continue;
-        float side_impulse = 0.0f;
-        {
-            const V3 rel_pos1 = w.contact_point_bt - com;
-            const V3 vel = lin + cross(ang, rel_pos1);
-            const V3 cj = cross(rel_pos1, w.cal_axle_dir);
-            const V3 a_j{dot(f.fwd, cj), dot(f.right, cj), dot(f.up, cj)};
-            const V3 minv{f.inv_inertia_local_bt.x * a_j.x, f.inv_inertia_local_bt.y * a_j.y,
-                          f.inv_inertia_local_bt.z * a_j.z};
-            const float a_diag = inv_mass + dot(minv, a_j);
-            const float rel_vel = dot(w.cal_axle_dir, vel);
-            if (!(a_diag <= 0.0f)) side_impulse = -0.2f * rel_vel * (1.0f / a_diag);
-        }
-        const float roll = w.cal_rolling_friction * w.cal_long_friction;
-        const float side = (side_impulse * (dt * w.cal_friction_scale)) * w.cal_lat_friction;
-        const V3 imp{roll * w.cal_forward_dir.x + side * w.cal_axle_dir.x,
-                     roll * w.cal_forward_dir.y + side * w.cal_axle_dir.y,
-                     roll * w.cal_forward_dir.z + side * w.cal_axle_dir.z};
-        if (len2(imp) == 0.0f) continue;
-        const V3 car_up = f.up;
-        const V3 rel = w.contact_point_bt - c.pos_bt;
-        const V3 wheel_rel = rel - car_up * dot(car_up, rel);
-        o[i] = wheel_impulse_at(tc.car_mass, f, imp, wheel_rel);
+    float side_impulse = 0.0f;
+    {
+        const V3 rel_pos1 = w.contact_point_bt - com;
+        const V3 vel = lin + cross(ang, rel_pos1);
+        const V3 cj = cross(rel_pos1, w.cal_axle_dir);
+        const V3 a_j{dot(f.fwd, cj), dot(f.right, cj), dot(f.up, cj)};
+        const V3 minv{f.inv_inertia_local_bt.x * a_j.x, f.inv_inertia_local_bt.y * a_j.y,
+                      f.inv_inertia_local_bt.z * a_j.z};
+        const float a_diag = inv_mass + dot(minv, a_j);
+        const float rel_vel = dot(w.cal_axle_dir, vel);
+        if (!(a_diag <= 0.0f)) side_impulse = -0.2f * rel_vel * (1.0f / a_diag);
     }
-    combine_wheel_impulses(c, o);
+    const float roll = w.cal_rolling_friction * w.cal_long_friction;
+    const float side = (side_impulse * (dt * w.cal_friction_scale)) * w.cal_lat_friction;
+    const V3 imp{roll * w.cal_forward_dir.x + side * w.cal_axle_dir.x,
+                 roll * w.cal_forward_dir.y + side * w.cal_axle_dir.y,
+                 roll * w.cal_forward_dir.z + side * w.cal_axle_dir.z};
+    if (len2(imp) == 0.0f) return o;
+    const V3 car_up = f.up;
+    const V3 rel = w.contact_point_bt - c.pos_bt;
+    const V3 wheel_rel = rel - car_up * dot(car_up, rel);
+    return wheel_impulse_at(tc.car_mass, f, imp, wheel_rel);
 }
 
 // ---- auto-roll (reference ApplyAutoRollReference, :1021-1087) ------------------------------------------------------
@@ -1064,16 +1061,21 @@ RG_HDI void apply_wheel_ball_pushes(BallState& ball, const WheelBallPushes& p, c
 // The update's car-world event: the wheel on the arena with the most upward normal, unless a wheel stood on the same
 // triangle with the same normal last tick (reference PreTickCar, env_step.hpp:3426-3469). Kept out of line: only a
 // batch with an event stream calls it.
-RG_NOINL void wheel_world_event(const CarState& c, const WheelRuntime& wr, const WheelStep* wh,
+struct WheelContact {
+    V3 normal;
+    int32_t static_id;
+    uint8_t in_contact, world, ball;
+};
+RG_NOINL void wheel_world_event(const CarState& c, const WheelRuntime& wr, const WheelContact* wh,
                                 WheelBallPushes& pushes) {
     bool has = false;
     V3 normal{0.0f, 0.0f, 0.0f};
     int32_t id = -1;
     for (int i = 0; i < 4; ++i) {
-        if (wh[i].is_in_contact && wh[i].is_in_contact_with_world && (!has || wh[i].contact_normal_ws.z > normal.z)) {
+        if (wh[i].in_contact && wh[i].world && (!has || wh[i].normal.z > normal.z)) {
             has = true;
-            normal = wh[i].contact_normal_ws;
-            id = wh[i].ground_static_id;
+            normal = wh[i].normal;
+            id = wh[i].static_id;
         }
     }
     bool previous = false;
@@ -1091,193 +1093,227 @@ RG_NOINL void wheel_world_event(const CarState& c, const WheelRuntime& wr, const
     pushes.world_event_on_ground = c.is_on_ground;
 }
 
-// `mesh_hits`: the four wheels' arena-mesh rays cast ahead (wheel_mesh_ray_ahead), or null to cast them here.
-RG_NOINL void vehicle_update(CarState& c, CarControls k_raw, const CarConfig& cfg, const TickConfig& tc,
-                           WheelRuntime& wr, const BallState& ball, const MeshDevice& mesh, const WheelOthers& oth,
-                           WheelBallPushes& pushes, const RayHit* mesh_hits = nullptr) {
-    pushes.count = 0;
-    pushes.world_event = 0u;
-    const float dt = tc.tick_dt;
-    c.demo_no_contact_response = c.is_demoed ? 1 : 0;
-    if (c.is_demoed) return;
-    float raw_pitch = 2.0f;
-    const CarControls k = pre_tick_controls(c, k_raw, raw_pitch);
-    const uint8_t cal_pre = c.cal_pre_flags;
+// What the parts of one car's vehicle update hand one another: the controls and the frame, the wheels' contacts and
+// impulses, and what was read before it changed.
+struct VehicleTick {
     CarFrame f;
-    make_car_frame(f, c, cfg, tc.car_mass);
-    f.queue_forces = true;
+    CarControls k;
+    float raw_pitch, pitchlock_restart_time, forward_speed_uu, abs_snapshot_forward_speed;
+    float min_hit_dist_sq, front_scale, back_scale, front_bone, back_bone;
+    V3 autoroll_normal_sum, sticky_prev_world_normal_sum, world_normal_sum;
+    int32_t autoroll_world_contacts, sticky_prev_world_contacts, world_contacts, num_contact, prev_wheel_contacts;
+    uint8_t flipping_at_start, flip_started, air_jump_started, was_jumping, air_jump_used_before, set_v3_tick,
+        autoroll_prev_contact;
+    DriveShared ds;
+    WheelContact wheel[4];
+    V3 contact_point[4];
+    WheelImpulse impulse[4];
+};
+
+// Before the wheel rays.
+RG_HDI void vehicle_begin(CarState& c, CarControls k_raw, const CarConfig& cfg, const TickConfig& tc, WheelRuntime& wr,
+                          VehicleTick& v) {
+    v.raw_pitch = 2.0f;
+    v.k = pre_tick_controls(c, k_raw, v.raw_pitch);
+    const uint8_t cal_pre = c.cal_pre_flags;
+    make_car_frame(v.f, c, cfg, tc.car_mass);
+    v.f.queue_forces = true;
     wr.pre_solve_rot = c.rot;
     wr.pre_solve_basis_forward = c.tick_start_basis_forward;
     wr.pre_solve_basis_right = c.tick_start_basis_right;
     wr.pre_solve_basis_up = c.tick_start_basis_up;
     wr.pre_solve_basis_authoritative = 1;
-    const uint8_t flipping_at_start = (cal_pre & kCalPreFlippingAtStart) ? 1 : 0;
-    const bool flip_started = (cal_pre & kCalPreFlipStarted) != 0;
-    const float pitchlock_restart_time = c.cal_pre_pitchlock_restart_time;
-    const bool air_jump_started = (cal_pre & kCalPreAirJumpStarted) != 0;
-    const uint8_t was_jumping = (cal_pre & kCalPreWasJumping) ? 1 : 0;
-    float forward_speed_uu = c.cal_pre_forward_speed_uu;
-    const uint8_t air_jump_used_before = (cal_pre & kCalPreAirJumpUsedBefore) ? 1 : 0;
-    const bool set_v3_tick = (cal_pre & kCalPreSetV3Tick) != 0;
-    const int prev_wheel_contacts = (c.wheels_with_contact[0] != 0) + (c.wheels_with_contact[1] != 0) +
-                                    (c.wheels_with_contact[2] != 0) + (c.wheels_with_contact[3] != 0);
-    const bool autoroll_prev_contact = c.tick_count_since_update != 0;
-    V3 autoroll_normal_sum = autoroll_prev_contact ? wr.cal_prev_wheel_normal_sum : V3{0.0f, 0.0f, 0.0f};
-    int autoroll_world_contacts = autoroll_prev_contact ? wr.cal_prev_world_wheel_contacts : 0;
+    v.flipping_at_start = (cal_pre & kCalPreFlippingAtStart) ? 1 : 0;
+    v.flip_started = (cal_pre & kCalPreFlipStarted) ? 1 : 0;
+    v.pitchlock_restart_time = c.cal_pre_pitchlock_restart_time;
+    v.air_jump_started = (cal_pre & kCalPreAirJumpStarted) ? 1 : 0;
+    v.was_jumping = (cal_pre & kCalPreWasJumping) ? 1 : 0;
+    v.forward_speed_uu = c.cal_pre_forward_speed_uu;
+    v.air_jump_used_before = (cal_pre & kCalPreAirJumpUsedBefore) ? 1 : 0;
+    v.set_v3_tick = (cal_pre & kCalPreSetV3Tick) ? 1 : 0;
+    v.prev_wheel_contacts = (c.wheels_with_contact[0] != 0) + (c.wheels_with_contact[1] != 0) +
+                            (c.wheels_with_contact[2] != 0) + (c.wheels_with_contact[3] != 0);
+    v.autoroll_prev_contact = c.tick_count_since_update != 0 ? 1 : 0;
+    v.autoroll_normal_sum = v.autoroll_prev_contact ? wr.cal_prev_wheel_normal_sum : V3{0.0f, 0.0f, 0.0f};
+    v.autoroll_world_contacts = v.autoroll_prev_contact ? wr.cal_prev_world_wheel_contacts : 0;
+    c.world_contact.wheel_ball_mask = 0;
+    v.sticky_prev_world_contacts = wr.cal_prev_world_wheel_contacts;
+    v.sticky_prev_world_normal_sum = wr.cal_prev_wheel_normal_sum;
+    suspension_force_scales(cfg, tc.car_mass, v.front_scale, v.back_scale);
+    v.min_hit_dist_sq = min_wheel_hit_dist_sq_bt(cfg);
+    wheel_bone_z(cfg, v.front_bone, v.back_bone);
+}
 
-    // -- PreTickVehicleDynamics
-    WheelStep wh[4];
-    int num_contact = 0;
-    bool wheel_world_contact = false;
-    float abs_snapshot_forward_speed;
+// Wheel i's ray and what the wheel gets from it.
+RG_HDI void vehicle_wheel_cast(const CarState& c, const CarConfig& cfg, const TickConfig& tc, const WheelRuntime& wr,
+                               const BallState& ball, const MeshDevice& mesh, const WheelOthers& oth,
+                               const RayHit* mesh_hits, const VehicleTick& v, int i, WheelStep& w) {
+    init_wheel(w, c, cfg, i, v.f, i < 2 ? v.front_bone : v.back_bone);
+    w.suspension_force_scale = w.is_front_wheel ? v.front_scale : v.back_scale;
+    w.extra_pushback = wr.extra_pushback[i];
+    wheel_ray_cast(c, w, ball, tc, mesh, v.min_hit_dist_sq, oth, mesh_hits ? mesh_hits + i : nullptr);
+    if (w.is_in_contact) w.extra_pushback = 0.0f;
+    if (w.is_in_contact_with_world) world_wheel_pushback(c, tc, w, v.f);
+}
+// A wheel on another car pushes that car down (and back out when pressed in) at once (reference WheelRayPhase,
+// :2196-2219; ResolveCarCarWheelPushbackMagnitudeBtInputs, ApplyImpulseAtPointBtRoundtripBtInputs,
+// host_validation_and_contact_debug.hpp:413-482).
+RG_HDI void vehicle_wheel_on_car(const CarState& c, const CarConfig& cfg, const TickConfig& tc, const WheelOthers& oth,
+                                 WheelStep& w) {
+    if (!(w.is_in_contact && !w.is_in_contact_with_world && w.ground_kind == kRayHitCar && oth.cars &&
+          w.ground_car_idx >= 0 && w.ground_car_idx < oth.count && w.ground_car_idx != oth.self))
+        return;
+    CarState& o = oth.cars[w.ground_car_idx];
+    const CarConfig& ocfg = oth.cfgs[w.ground_car_idx];
+    const V3 n_bt = w.contact_normal_ws, cp_bt = w.contact_point_bt;
+    const float solver_dt = 1.0f / 60.0f;
+    const float thresh = (w.suspension_rest_length * kUuToBt + w.wheel_radius * kUuToBt) - 0.05f;
+    w.extra_pushback = 0.0f;
+    if (w.wheel_trace_len_bt < thresh)
+        w.extra_pushback = car_car_wheel_pushback(c, cfg, o, ocfg, tc.car_mass, cp_bt, n_bt,
+                                                  w.wheel_trace_len_bt - thresh, solver_dt) /
+                           4.0f;
+    if (w.extra_pushback > 0.0f) {
+        const float full = w.extra_pushback * 4.0f;
+        car_impulse_at_point_bt(o, ocfg, tc.car_mass, -n_bt * full, cp_bt - o.pos_bt);
+    }
+    car_impulse_at_point_bt(o, ocfg, tc.car_mass, -n_bt, cp_bt - o.pos_bt);
+}
+// Hands wheel i's contact to the car's parts.
+RG_HDI void vehicle_wheel_share(WheelRuntime& wr, VehicleTick& v, int i, const WheelStep& w) {
+    wr.extra_pushback[i] = w.extra_pushback;
+    WheelContact& x = v.wheel[i];
+    x.in_contact = w.is_in_contact;
+    x.world = w.is_in_contact_with_world;
+    x.ball = w.ground_kind == kRayHitBall ? 1 : 0;
+    x.normal = w.contact_normal_ws;
+    x.static_id = w.ground_static_id;
+    v.contact_point[i] = w.contact_point_bt;
+}
+
+// The wheels' contacts together (CombineWheelContacts), then the drive train's shared inputs.
+RG_HDI void vehicle_contacts(CarState& c, const CarConfig& cfg, const TickConfig& tc, WheelRuntime& wr, VehicleTick& v,
+                             WheelBallPushes& pushes) {
+    const float dt = tc.tick_dt;
+    const CarControls& k = v.k;
+    int push_count = 0;
+    for (int kk = 0; kk < 4; ++kk) {
+        const int i = kk ^ 1;
+        // a ray on the ball pushes it down (reference WheelRayPhase, :2200-2207); the caller applies the push in the
+        // arena's car order (apply_wheel_ball_pushes)
+        if (v.wheel[i].in_contact && !v.wheel[i].world && v.wheel[i].ball) {
+            pushes.point_bt[push_count] = v.contact_point[i];
+            pushes.normal[push_count] = v.wheel[i].normal;
+            ++push_count;
+        }
+    }
+    pushes.count = push_count;
+    V3 world_normal_sum{0.0f, 0.0f, 0.0f};
+    int world_contacts = 0, num_contact = 0;
+    for (int kk = 0; kk < 4; ++kk) {
+        const int i = kk ^ 1;
+        const bool in_contact = v.wheel[i].in_contact != 0;
+        c.wheels_with_contact[i] = in_contact;
+        c.world_contact.wheel_ball_mask |= static_cast<uint8_t>((in_contact && v.wheel[i].ball) << i);
+        num_contact += in_contact ? 1 : 0;
+    }
+    c.is_on_ground = num_contact >= 3 ? 1 : 0;
+    for (int kk = 0; kk < 4; ++kk) {
+        const int i = kk ^ 1;
+        if (v.wheel[i].in_contact && v.wheel[i].world) {
+            world_normal_sum += v.wheel[i].normal;
+            ++world_contacts;
+        }
+    }
+    wr.cal_prev_wheel_normal_sum = world_normal_sum;
+    wr.cal_prev_world_wheel_contacts = static_cast<uint8_t>(world_contacts);
+    v.world_normal_sum = world_normal_sum;
+    v.world_contacts = world_contacts;
+    v.num_contact = num_contact;
+    v.abs_snapshot_forward_speed = fabs_(v.forward_speed_uu);
+    float forward_speed_uu;
     {
-        c.world_contact.wheel_ball_mask = 0;
-        const uint8_t sticky_prev_world_contacts = wr.cal_prev_world_wheel_contacts;
-        const V3 sticky_prev_world_normal_sum = wr.cal_prev_wheel_normal_sum;
-        float front_scale, back_scale, front_bone, back_bone;
-        suspension_force_scales(cfg, tc.car_mass, front_scale, back_scale);
-        const float min_hit_dist_sq = min_wheel_hit_dist_sq_bt(cfg);
-        wheel_bone_z(cfg, front_bone, back_bone);
-        uint32_t flags[4];
-        for (int kk = 0; kk < 4; ++kk) {
-            const int i = kk ^ 1;
-            WheelStep& w = wh[i];
-            init_wheel(w, c, cfg, i, f, i < 2 ? front_bone : back_bone);
-            w.suspension_force_scale = w.is_front_wheel ? front_scale : back_scale;
-            w.extra_pushback = wr.extra_pushback[i];
-            wheel_ray_cast(c, w, ball, tc, mesh, min_hit_dist_sq, oth, mesh_hits ? mesh_hits + i : nullptr);
-            if (w.is_in_contact) w.extra_pushback = 0.0f;
-            if (w.is_in_contact_with_world) world_wheel_pushback(c, tc, w, f);
-            if (w.is_in_contact && !w.is_in_contact_with_world && w.ground_kind == kRayHitCar && oth.cars &&
-                w.ground_car_idx >= 0 && w.ground_car_idx < oth.count && w.ground_car_idx != oth.self) {
-                // a wheel on another car pushes that car down (and back out when pressed in) at once (reference
-                // WheelRayPhase, :2196-2219; ResolveCarCarWheelPushbackMagnitudeBtInputs, ApplyImpulseAtPointBt-
-                // RoundtripBtInputs, host_validation_and_contact_debug.hpp:413-482)
-                CarState& o = oth.cars[w.ground_car_idx];
-                const CarConfig& ocfg = oth.cfgs[w.ground_car_idx];
-                const V3 n_bt = w.contact_normal_ws, cp_bt = w.contact_point_bt;
-                const float solver_dt = 1.0f / 60.0f;
-                const float thresh = (w.suspension_rest_length * kUuToBt + w.wheel_radius * kUuToBt) - 0.05f;
-                w.extra_pushback = 0.0f;
-                if (w.wheel_trace_len_bt < thresh)
-                    w.extra_pushback = car_car_wheel_pushback(c, cfg, o, ocfg, tc.car_mass, cp_bt, n_bt,
-                                                              w.wheel_trace_len_bt - thresh, solver_dt) /
-                                       4.0f;
-                if (w.extra_pushback > 0.0f) {
-                    const float full = w.extra_pushback * 4.0f;
-                    car_impulse_at_point_bt(o, ocfg, tc.car_mass, -n_bt * full, cp_bt - o.pos_bt);
-                }
-                car_impulse_at_point_bt(o, ocfg, tc.car_mass, -n_bt, cp_bt - o.pos_bt);
-            } else if (w.is_in_contact && !w.is_in_contact_with_world && w.ground_kind == kRayHitBall) {
-                // the ray pushes the ball down (reference WheelRayPhase, :2200-2207); the caller applies the push in
-                // the arena's car order (apply_wheel_ball_pushes)
-                pushes.point_bt[pushes.count] = w.contact_point_bt;
-                pushes.normal[pushes.count] = w.contact_normal_ws;
-                ++pushes.count;
+        // FreshCarRbSnapshot (:940-988)
+        V3 vel = c.vel_bt * 50.0f;
+        const float l2 = (vel.y * vel.y + vel.x * vel.x) + vel.z * vel.z;
+        if (tc.car_max_speed > 0.0f && tc.car_max_speed * tc.car_max_speed < l2) {
+            const float inv = 1.0f / sqrtf(l2);
+            vel = V3{tc.car_max_speed * (inv * vel.x), tc.car_max_speed * (inv * vel.y),
+                     tc.car_max_speed * (inv * vel.z)};
+        }
+        const V3 snap_vel{quant_trunc_offset(vel.x, 100.0f), quant_trunc_offset(vel.y, 100.0f),
+                          quant_trunc_offset(vel.z, 100.0f)};
+        const Q4 snap_rot = game_quantize_quat(game_rot_from_basis(v.f.fwd, v.f.right, v.f.up));
+        forward_speed_uu = snapshot_forward_speed(snap_rot, snap_vel);
+    }
+    const float abs_forward_speed = fabs_(forward_speed_uu);
+    if (k.handbrake) {
+        c.handbrake_val = clampf(c.handbrake_val + 5.0f * dt, 0.0f, 1.0f);
+    } else {
+        c.handbrake_val = clampf(c.handbrake_val - 2.0f * dt, 0.0f, 1.0f);
+    }
+    const float real_throttle = k.throttle;
+    float real_brake = 0.0f;
+    float engine_throttle = c.driving_disabled ? 0.0f : real_throttle;
+    if (!k.handbrake && !c.driving_disabled) {
+        const float abs_throttle = fabs_(real_throttle);
+        if (abs_throttle > 0.01f) {
+            if (abs_forward_speed > 25.0f && sgnf(real_throttle) != sgnf(forward_speed_uu)) {
+                real_brake = 1.0f;
+                if (abs_forward_speed > 0.01f) engine_throttle = 0.0f;
             }
-            wr.extra_pushback[i] = w.extra_pushback;
-            flags[i] = (w.is_in_contact ? 1u : 0u) | (w.is_in_contact_with_world ? 2u : 0u) |
-                       (w.ground_kind == kRayHitBall ? 4u : 0u);
-        }
-        // CombineWheelContacts
-        V3 world_normal_sum{0.0f, 0.0f, 0.0f};
-        int world_contacts = 0;
-        for (int kk = 0; kk < 4; ++kk) {
-            const int i = kk ^ 1;
-            const bool in_contact = (flags[i] & 1u) != 0;
-            c.wheels_with_contact[i] = in_contact;
-            c.world_contact.wheel_ball_mask |= static_cast<uint8_t>((in_contact && (flags[i] & 4u)) << i);
-            num_contact += in_contact ? 1 : 0;
-        }
-        c.is_on_ground = num_contact >= 3 ? 1 : 0;
-        for (int kk = 0; kk < 4; ++kk) {
-            const int i = kk ^ 1;
-            if ((flags[i] & 1u) && (flags[i] & 2u)) {
-                world_normal_sum += wh[i].contact_normal_ws;
-                ++world_contacts;
-            }
-        }
-        wr.cal_prev_wheel_normal_sum = world_normal_sum;
-        wr.cal_prev_world_wheel_contacts = static_cast<uint8_t>(world_contacts);
-        wheel_world_contact = world_contacts > 0;
-
-        abs_snapshot_forward_speed = fabs_(forward_speed_uu);
-        {
-            // FreshCarRbSnapshot (:940-988)
-            V3 v = c.vel_bt * 50.0f;
-            const float l2 = (v.y * v.y + v.x * v.x) + v.z * v.z;
-            if (tc.car_max_speed > 0.0f && tc.car_max_speed * tc.car_max_speed < l2) {
-                const float inv = 1.0f / sqrtf(l2);
-                v = V3{tc.car_max_speed * (inv * v.x), tc.car_max_speed * (inv * v.y), tc.car_max_speed * (inv * v.z)};
-            }
-            const V3 snap_vel{quant_trunc_offset(v.x, 100.0f), quant_trunc_offset(v.y, 100.0f),
-                              quant_trunc_offset(v.z, 100.0f)};
-            const Q4 snap_rot = game_quantize_quat(game_rot_from_basis(f.fwd, f.right, f.up));
-            forward_speed_uu = snapshot_forward_speed(snap_rot, snap_vel);
-        }
-        const float abs_forward_speed = fabs_(forward_speed_uu);
-        const float friction_scale = tc.car_mass / 3.0f;
-        if (k.handbrake) {
-            c.handbrake_val = clampf(c.handbrake_val + 5.0f * dt, 0.0f, 1.0f);
         } else {
-            c.handbrake_val = clampf(c.handbrake_val - 2.0f * dt, 0.0f, 1.0f);
+            engine_throttle = 0.0f;
+            real_brake = abs_forward_speed < 25.0f ? 1.0f : 0.15f;
         }
-        const float real_throttle = k.throttle;
-        float real_brake = 0.0f;
-        float engine_throttle = c.driving_disabled ? 0.0f : real_throttle;
-        if (!k.handbrake && !c.driving_disabled) {
-            const float abs_throttle = fabs_(real_throttle);
-            if (abs_throttle > 0.01f) {
-                if (abs_forward_speed > 25.0f && sgnf(real_throttle) != sgnf(forward_speed_uu)) {
-                    real_brake = 1.0f;
-                    if (abs_forward_speed > 0.01f) engine_throttle = 0.0f;
-                }
-            } else {
-                engine_throttle = 0.0f;
-                real_brake = abs_forward_speed < 25.0f ? 1.0f : 0.15f;
-            }
+    }
+    const float drive_speed_scale = engine_throttle != 0.0f ? drive_torque_factor(forward_speed_uu) : 1.0f;
+    float engine_uu = (drive_speed_scale * (engine_throttle * 288000.0f)) * 0.25f;
+    if (num_contact < 3) engine_uu *= 0.25f;
+    DriveShared& ds = v.ds;
+    ds.drive_engine_force = engine_uu * kUuToBt;
+    ds.drive_brake_force = ((real_brake * 10500.0f) * 0.25f) * kUuToBt;
+    {
+        float steer_deg = steer_angle_from_speed(cfg.steer_angle_curve_deg, abs_forward_speed);
+        if (c.handbrake_val > 0.0f)
+            steer_deg += (powerslide_steer_angle_from_speed(cfg.powerslide_steer_angle_curve_deg, abs_forward_speed) -
+                          steer_deg) *
+                         c.handbrake_val;
+        ds.next_steer_angle = (steer_deg * k.steer) * kSteerDegToRad;
+    }
+    ds.real_throttle = real_throttle;
+    ds.friction_scale = tc.car_mass / 3.0f;
+    ds.front_right_col = ds.back_right_col = V3{0.0f, 0.0f, 0.0f};
+    const bool front_in = v.wheel[0].in_contact || v.wheel[1].in_contact;
+    const bool back_in = v.wheel[2].in_contact || v.wheel[3].in_contact;
+    if (front_in) ds.front_right_col = wheel_steered_right_col(v.f, ds.next_steer_angle);
+    if (back_in) {
+        const bool positive_zero = ds.next_steer_angle == 0.0f && !signbit(ds.next_steer_angle);
+        if (front_in && positive_zero) {
+            ds.back_right_col = ds.front_right_col;
+        } else {
+            ds.back_right_col = wheel_steered_right_col(v.f, 0.0f);
         }
-        const float drive_speed_scale = engine_throttle != 0.0f ? drive_torque_factor(forward_speed_uu) : 1.0f;
-        float engine_uu = (drive_speed_scale * (engine_throttle * 288000.0f)) * 0.25f;
-        if (num_contact < 3) engine_uu *= 0.25f;
-        DriveShared ds;
-        ds.drive_engine_force = engine_uu * kUuToBt;
-        ds.drive_brake_force = ((real_brake * 10500.0f) * 0.25f) * kUuToBt;
-        {
-            float steer_deg = steer_angle_from_speed(cfg.steer_angle_curve_deg, abs_forward_speed);
-            if (c.handbrake_val > 0.0f)
-                steer_deg +=
-                    (powerslide_steer_angle_from_speed(cfg.powerslide_steer_angle_curve_deg, abs_forward_speed) -
-                     steer_deg) *
-                    c.handbrake_val;
-            ds.next_steer_angle = (steer_deg * k.steer) * kSteerDegToRad;
-        }
-        ds.real_throttle = real_throttle;
-        ds.friction_scale = friction_scale;
-        ds.front_right_col = ds.back_right_col = V3{0.0f, 0.0f, 0.0f};
-        const bool front_in = wh[0].is_in_contact || wh[1].is_in_contact;
-        const bool back_in = wh[2].is_in_contact || wh[3].is_in_contact;
-        if (front_in) ds.front_right_col = wheel_steered_right_col(wh[0], ds.next_steer_angle);
-        if (back_in) {
-            const bool positive_zero = ds.next_steer_angle == 0.0f && !signbit(ds.next_steer_angle);
-            if (front_in && positive_zero) {
-                ds.back_right_col = ds.front_right_col;
-            } else {
-                ds.back_right_col = wheel_steered_right_col(wh[2], 0.0f);
-            }
-        }
-        for (int i = 0; i < 4; ++i) wheel_drive_setup(c, ds, wh[i], i, wr, dt);
-        // sticky force
-        V3 sticky_sum = sticky_prev_world_normal_sum;
-        bool gate = sticky_prev_world_contacts > 0;
+    }
+}
+
+// The car's own forces: sticky force, flips and air control, jump state, auto-roll.
+RG_HDI void vehicle_controls(CarState& c, const CarConfig& cfg, const TickConfig& tc, WheelRuntime& wr,
+                             VehicleTick& v) {
+    const float dt = tc.tick_dt;
+    const CarControls& k = v.k;
+    CarFrame& f = v.f;
+    {
+        V3 sticky_sum = v.sticky_prev_world_normal_sum;
+        bool gate = v.sticky_prev_world_contacts > 0;
         if (c.tick_count_since_update == 0) {
-            sticky_sum = world_normal_sum;
-            gate = world_contacts > 0;
+            sticky_sum = v.world_normal_sum;
+            gate = v.world_contacts > 0;
         }
         if (gate) {
             const float l2 = len2(sticky_sum);
             const V3 up = l2 >= 1e-8f ? sticky_sum * (1.0f / sqrtf(l2)) : V3{0.0f, 0.0f, 0.0f};
-            const bool full_stick = (k.throttle != 0.0f) || (abs_snapshot_forward_speed > 25.0f);
+            const bool full_stick = (k.throttle != 0.0f) || (v.abs_snapshot_forward_speed > 25.0f);
             const float base = 0.5f;
             const float full = base + 1.0f;
             const float target = full_stick ? full : base;
@@ -1286,76 +1322,133 @@ RG_NOINL void vehicle_update(CarState& c, CarControls k_raw, const CarConfig& cf
             queue_force(f, ((accel * up) * kUuToBt) * tc.car_mass);
         }
     }
-
-    if (wheel_world_contact) car_record_world_surface(c, false);
+    const int prev_wheel_contacts = v.prev_wheel_contacts, num_contact = v.num_contact;
+    if (v.world_contacts > 0) car_record_world_surface(c, false);
     if (car_has_flip_or_jump(c) && !c.flip_or_jump_last_tick) c.last_flip_or_jump_start = c.tick_count_since_update;
-    const int air_gate_contacts = (c.tick_count_since_update != 0 || set_v3_tick)
+    const int air_gate_contacts = (c.tick_count_since_update != 0 || v.set_v3_tick)
                                       ? prev_wheel_contacts
                                       : (prev_wheel_contacts > num_contact ? prev_wheel_contacts : num_contact);
-    const int landing_prev_contacts = (c.tick_count_since_update == 0 && !set_v3_tick)
+    const int landing_prev_contacts = (c.tick_count_since_update == 0 && !v.set_v3_tick)
                                           ? (num_contact > prev_wheel_contacts ? num_contact : prev_wheel_contacts)
                                           : prev_wheel_contacts;
     const uint8_t flipping_before_air = c.is_flipping;
     const V3 air_damp_ang_vel = c.cal_tick_start_ang_vel;
     if (air_gate_contacts < 3) {
-        const V3 dodge_torque_bt = flip_torque(c, k, cfg, tc, raw_pitch, f);
+        const V3 dodge_torque_bt = flip_torque(c, k, cfg, tc, v.raw_pitch, f);
         if (!c.driving_disabled)
-            air_control(c, k, cfg, tc, landing_prev_contacts == 0, landing_prev_contacts == 0, pitchlock_restart_time,
+            air_control(c, k, cfg, tc, landing_prev_contacts == 0, landing_prev_contacts == 0, v.pitchlock_restart_time,
                         air_damp_ang_vel, f);
         if (dodge_torque_bt.x != 0.0f || dodge_torque_bt.y != 0.0f || dodge_torque_bt.z != 0.0f)
             queue_torque(f, dodge_torque_bt);
     } else {
         c.is_flipping = 0;
         if (landing_prev_contacts == 0 && !c.driving_disabled)
-            air_control(c, k, cfg, tc, true, true, pitchlock_restart_time, air_damp_ang_vel, f);
+            air_control(c, k, cfg, tc, true, true, v.pitchlock_restart_time, air_damp_ang_vel, f);
     }
     const bool flip_ended = air_gate_contacts < 3 && flipping_before_air && !c.is_flipping;
     update_jump_state(c, k, tc, f);
-    if ((c.is_jumping && !was_jumping) || (!air_jump_used_before && (c.has_double_jumped || c.has_flipped)))
+    if ((c.is_jumping && !v.was_jumping) || (!v.air_jump_used_before && (c.has_double_jumped || c.has_flipped)))
         wr.cal_game_jumped = 1;
-    if (!air_jump_used_before && (c.has_double_jumped || c.has_flipped)) wr.cal_game_double_jumped = 1;
+    if (!v.air_jump_used_before && (c.has_double_jumped || c.has_flipped)) wr.cal_game_double_jumped = 1;
     wr.cal_jump_inactive_time = c.is_jumping ? 0.0f : wr.cal_jump_inactive_time + dt;
-    const bool jump_changed = air_jump_started || (was_jumping && !c.is_jumping);
-    const bool flip_changed = flip_started || c.is_flipping != flipping_at_start;
+    const bool jump_changed = v.air_jump_started || (v.was_jumping && !c.is_jumping);
+    const bool flip_changed = v.flip_started || c.is_flipping != v.flipping_at_start;
     if (jump_changed || !c.just_respawned) {
         const float jump_ticks = rintf(c.jump_time / dt) + 1.0f;
         c.jump_time = jump_changed ? dt : (jump_ticks <= 1024.0f ? c.jump_time + dt : jump_ticks * dt);
     }
     if (flip_changed || !c.just_respawned) c.flip_time = flip_changed ? dt : c.flip_time + dt;
-    if (air_jump_started) {
+    if (v.air_jump_started) {
         c.jump_hold_broken = 0;
-    } else if (was_jumping && !k.jump) {
+    } else if (v.was_jumping && !k.jump) {
         c.jump_hold_broken = 1;
     }
     // auto-roll
-    if (!autoroll_prev_contact) {
-        autoroll_normal_sum = wr.cal_prev_wheel_normal_sum;
-        autoroll_world_contacts = wr.cal_prev_world_wheel_contacts;
+    if (!v.autoroll_prev_contact) {
+        v.autoroll_normal_sum = wr.cal_prev_wheel_normal_sum;
+        v.autoroll_world_contacts = wr.cal_prev_world_wheel_contacts;
     }
-    int autoroll_contacts = autoroll_world_contacts;
+    int autoroll_contacts = v.autoroll_world_contacts;
     bool autoroll_gate = autoroll_contacts < 4 && (autoroll_contacts > 0 || c.world_contact.has_contact);
-    if (!autoroll_prev_contact && prev_wheel_contacts > 0 && prev_wheel_contacts < 4) {
-        const bool sticky = autoroll_world_contacts > 0;
+    if (!v.autoroll_prev_contact && prev_wheel_contacts > 0 && prev_wheel_contacts < 4) {
+        const bool sticky = v.autoroll_world_contacts > 0;
         autoroll_gate = sticky || c.world_contact.has_contact;
         autoroll_contacts = sticky ? prev_wheel_contacts : 0;
     }
-    if (k.throttle && !c.is_flipping && !flipping_at_start && !flip_ended && autoroll_gate)
-        apply_auto_roll(c, cfg, tc, autoroll_contacts, autoroll_normal_sum, f);
+    if (k.throttle && !c.is_flipping && !v.flipping_at_start && !flip_ended && autoroll_gate)
+        apply_auto_roll(c, cfg, tc, autoroll_contacts, v.autoroll_normal_sum, f);
     c.set_wheel_normals_mask = 0;
     c.world_contact.has_contact = 0;
-    if (!c.just_respawned) wheel_suspension_and_friction(c, tc, wh, f);
-    apply_boost(c, k, tc, f);
+}
+
+// After the wheels' impulses: boost and what the wheel record keeps.
+RG_HDI void vehicle_end(CarState& c, const TickConfig& tc, WheelRuntime& wr, VehicleTick& v, WheelBallPushes& pushes) {
+    CarFrame& f = v.f;
+    apply_boost(c, v.k, tc, f);
     if (f.has_queued_jump_force) f.queued_force += f.queued_jump_force;
     wr.accumulated_force = f.queued_force;
     wr.accumulated_ang_accel = f.queued_ang_accel;
     wr.accumulated_torque_bt = f.queued_torque_bt;
-    wr.solver_time_step = dt;
-    if (tc.events.windows) wheel_world_event(c, wr, wh, pushes);
-    for (int i = 0; i < 4; ++i) {
-        const bool world = wh[i].is_in_contact && wh[i].is_in_contact_with_world;
-        wr.event_world_ids[i] = world ? wh[i].ground_static_id : -1;
-        wr.event_world_normals[i] = world ? wh[i].contact_normal_ws : V3{0.0f, 0.0f, 0.0f};
+    wr.solver_time_step = tc.tick_dt;
+    if (tc.events.windows) wheel_world_event(c, wr, v.wheel, pushes);
+}
+
+// The vehicle update of one car. The lanes of `lanes` hold the same car, `wr` and `v` in memory they share; with four
+// lanes each takes a wheel (its ray, drive, suspension and tyre terms, which depend on no other wheel), and lane 0 alone
+// everything else, the wheels' sums in the reference's wheel order (1, 0, 3, 2) among it. `mesh_hits`: the four wheels'
+// arena-mesh rays cast ahead (wheel_mesh_ray_ahead), or null to cast them here. `oth` may name cars only with one lane
+// (a wheel on another car pushes it at once, in wheel order).
+template <class L>
+RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw, const CarConfig& cfg,
+                           const TickConfig& tc, WheelRuntime& wr, const BallState& ball, const MeshDevice& mesh,
+                           const WheelOthers& oth, WheelBallPushes& pushes, const RayHit* mesh_hits, VehicleTick& v) {
+    constexpr int kOwn = 4 / L::kLanes;
+    WheelStep wh[kOwn];
+    auto each_wheel = [&](auto&& part) {
+#pragma unroll 1
+        for (int q = 0; q < kOwn; ++q) {
+            const int i = kOwn == 1 ? lanes.lane() : (q ^ 1);
+            part(i, wh[kOwn == 1 ? 0 : i]);
+        }
+    };
+    const bool first = lanes.lane() == 0;
+    if (first) {
+        pushes.count = 0;
+        pushes.world_event = 0u;
+        c.demo_no_contact_response = c.is_demoed ? 1 : 0;
     }
+    if (c.is_demoed) return;
+    if (first) vehicle_begin(c, k_raw, cfg, tc, wr, v);
+    lanes.sync();
+    each_wheel([&](int i, WheelStep& w) {
+        vehicle_wheel_cast(c, cfg, tc, wr, ball, mesh, oth, mesh_hits, v, i, w);
+        if (L::kLanes == 1) vehicle_wheel_on_car(c, cfg, tc, oth, w);
+        vehicle_wheel_share(wr, v, i, w);
+    });
+    lanes.sync();
+    if (first) vehicle_contacts(c, cfg, tc, wr, v, pushes);
+    lanes.sync();
+    each_wheel([&](int i, WheelStep& w) { wheel_drive_setup(c, v.ds, w, i, wr, tc.tick_dt); });
+    lanes.sync();
+    if (first) vehicle_controls(c, cfg, tc, wr, v);
+    lanes.sync();
+    if (!c.just_respawned && v.num_contact > 0) {
+        each_wheel([&](int i, WheelStep& w) { v.impulse[i] = wheel_suspension_impulse(c, tc, w, v.f); });
+        lanes.sync();
+        if (first) combine_wheel_impulses(c, v.impulse);
+        lanes.sync();
+        each_wheel([&](int i, WheelStep& w) { v.impulse[i] = wheel_friction_impulse(c, tc, w, v.f); });
+        lanes.sync();
+        if (first) combine_wheel_impulses(c, v.impulse);
+    }
+    if (first) vehicle_end(c, tc, wr, v, pushes);
+    lanes.sync();
+    each_wheel([&](int i, WheelStep& w) {
+        const bool world = w.is_in_contact && w.is_in_contact_with_world;
+        wr.event_world_ids[i] = world ? w.ground_static_id : -1;
+        wr.event_world_normals[i] = world ? w.contact_normal_ws : V3{0.0f, 0.0f, 0.0f};
+    });
+    lanes.sync();
 }
 
 // ---- world step: the car's external forces and integration (reference env_step.hpp:3737-3806,

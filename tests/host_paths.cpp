@@ -3,6 +3,25 @@
 
 #include "rg_tick.cuh"
 
+namespace {
+// A mesh's device view over its host tables.
+rg::MeshDevice host_view(const rg::MeshHost& h) {
+    rg::MeshDevice m;
+    m.tris = h.dev_tris.data();
+    m.tri_count = static_cast<int32_t>(h.dev_tris.size());
+    m.quant = h.quant;
+    m.aabb_min = h.aabb_min;
+    m.aabb_max = h.aabb_max;
+    m.grid_lo = h.grid_lo;
+    for (int a = 0; a < 3; ++a) m.grid_dims[a] = h.grid_dims[a];
+    m.inv_query_cell = 1.0f / h.query_cell;
+    m.cell_start = h.cell_start.data();
+    m.cell_entries = h.cell_entries.data();
+    m.rank_entries = h.rank_entries.data();
+    return m;
+}
+}  // namespace
+
 extern "C" {
 
 // n boxes against n triangles; out: hit, distance, point (5 floats per case)
@@ -46,16 +65,7 @@ int hp_query_boxes(const float* vertices_uu, long long nv, const int* indices, l
                    float* cell) {
     using rg::V3;
     const rg::MeshHost h = rg::build_mesh_host(vertices_uu, nv, indices, ni);
-    rg::MeshDevice m;
-    m.tris = h.dev_tris.data();
-    m.tri_count = static_cast<int32_t>(h.dev_tris.size());
-    m.quant = h.quant;
-    m.grid_lo = h.grid_lo;
-    for (int a = 0; a < 3; ++a) m.grid_dims[a] = h.grid_dims[a];
-    m.inv_query_cell = 1.0f / h.query_cell;
-    m.cell_start = h.cell_start.data();
-    m.cell_entries = h.cell_entries.data();
-    m.rank_entries = h.rank_entries.data();
+    const rg::MeshDevice m = host_view(h);
     *cell = h.query_cell;
     int wrong = 0;
     for (int i = 0; i < n; ++i) {
@@ -75,6 +85,114 @@ int hp_query_boxes(const float* vertices_uu, long long nv, const int* indices, l
         wrong += got != want;
     }
     return wrong;
+}
+
+// ---- whole ticks on the host: the parts of a tick in order, one arena after another, one lane per car ------------------
+struct HostBatch {
+    int32_t envs, max_cars, pad_count;
+    const int32_t* counts;
+    const uint8_t* teams;
+    const rg::CarConfig* cfgs;
+    rg::CarState* cars;
+    rg::BallState* balls;
+    rg::EnvState* env_states;
+    rg::PadState* pads;
+    rg::WheelRuntime* wheels;
+    rg::BallWorldScratch* ball_world;
+    rg::Broadphase* broadphase;
+    rg::CarWorldScratch* car_world;
+    rg::BallCarScratch* ball_car;
+    rg::CarCarManifold* pairs;
+    const float* pad_pos;
+    const uint8_t* pad_big;
+    uint64_t kickoff_seed;
+};
+
+// `ticks` ticks of every arena under controls [ticks, envs * max_cars] and the default config (report fields after the
+// last tick).
+void hp_step(const HostBatch* b, const rg_sim_config* cfg, const float* vertices_uu, long long nv, const int* indices,
+             long long ni, const rg::CarControls* controls, int ticks) {
+    const rg::MeshHost h = rg::build_mesh_host(vertices_uu, nv, indices, ni);
+    const rg::MeshDevice m = host_view(h);
+    rg::TickConfig tc{};
+    tc.tick_dt = cfg->tick_dt;
+    tc.gravity_z = cfg->gravity_z;
+    tc.ball_radius = cfg->ball_radius;
+    tc.ball_mass = cfg->ball_mass;
+    tc.ball_drag = cfg->ball_drag;
+    tc.ball_drag_scale = rg::ucrt_powf(1.0f - cfg->ball_drag, cfg->tick_dt);
+    tc.ball_friction = cfg->ball_friction;
+    tc.ball_restitution = cfg->ball_restitution;
+    tc.ball_max_speed = cfg->ball_max_speed;
+    tc.ball_max_ang_speed = cfg->ball_max_ang_speed;
+    tc.goal_base_threshold_y = cfg->goal_base_threshold_y;
+    tc.frame_frac = 0.5f;
+    tc.enable_scoring = cfg->enable_scoring;
+    tc.enable_boost_pads = cfg->enable_boost_pads;
+    tc.enable_car_car = cfg->enable_car_car_collisions;
+    tc.enable_demos = cfg->enable_demos;
+    tc.bump_force_scale = 1.0f;
+    tc.bump_cooldown_time = 0.25f;
+    tc.kickoff_seed = b->kickoff_seed;
+    tc.max_cars = b->max_cars;
+    tc.pad_count = b->pad_count;
+    tc.car_mass = cfg->car_mass;
+    tc.car_max_speed = cfg->car_max_speed;
+    tc.car_max_ang_speed = cfg->car_max_ang_speed;
+    rg::fill_car_constants(tc);
+    tc.arena_friction = cfg->arena_friction;
+    tc.arena_restitution = cfg->arena_restitution;
+    rg::PadLayout layout{};
+    layout.count = b->pad_count;
+    for (int p = 0; p < b->pad_count; ++p) {
+        layout.pos[p] = rg::V3{b->pad_pos[3 * p], b->pad_pos[3 * p + 1], b->pad_pos[3 * p + 2]};
+        layout.is_big[p] = b->pad_big[p];
+    }
+    const int mc = b->max_cars, slots = mc * (mc - 1) / 2;
+    std::vector<rg::CarTickRecord> recs(mc);
+    std::vector<rg::CarStage> stages(mc);
+    for (int e = 0; e < b->envs; ++e) {
+        const int base = e * mc, count = b->counts[e];
+        rg::BallState& ball = b->balls[e];
+        rg::EnvState& env = b->env_states[e];
+        for (int t = 0; t < ticks; ++t) {
+            rg::ArenaCars A{};
+            A.cars = b->cars + base;
+            A.wheels = b->wheels + base;
+            A.cfgs = b->cfgs + base;
+            A.pads = b->pads + static_cast<size_t>(e) * b->pad_count;
+            A.controls = controls + static_cast<size_t>(t) * b->envs * mc + base;
+            A.teams = b->teams + base;
+            A.pairs = b->pairs + static_cast<size_t>(e) * slots;
+            A.count = count;
+            A.max_cars = mc;
+            A.car_base = base;
+            rg::ArenaTickSnap snap;
+            rg::arena_tick_begin(env, ball, A, tc, layout, snap, tc.kickoff_seed, e);
+            for (int i = 0; i < count; ++i) {
+                rg::RespawnCtx rc{tc.kickoff_seed, e, env.tick, static_cast<uint32_t>(base + i + 1), A.teams[i]};
+                rg::car_tick_pre(A.cars[i], A.controls[i], A.cfgs[i], tc, A.wheels[i], rc, recs[i]);
+            }
+            for (int i = 0; i < count; ++i) {
+                rg::CarStage& st = stages[i];
+                rg::car_mesh_stage(rg::OneLane{}, A.cars[i], A.cfgs[i], b->car_world[base + i], m, st);
+                rg::car_proxy_ball_stage(ball, snap.ball_vel_bt, A.cars[i], A.cfgs[i], tc, recs[i].vel_bt,
+                                         recs[i].ang_vel, b->ball_car[base + i], st);
+                st.in_car_thread = 0;  // every vehicle update in the arena's car order
+                for (int w = 0; w < 4 && !A.cars[i].is_demoed; ++w) {
+                    uint8_t meets;
+                    rg::wheel_mesh_ray_ahead(A.cars[i], A.cfgs[i], m, w, rg::WheelOthers{nullptr, nullptr, 0, i, 0u},
+                                             st.wheel_mesh[w], meets);
+                }
+            }
+            rg::arena_tick_finish(env, ball, b->ball_world[e], b->broadphase[e], b->car_world + base,
+                                  b->ball_car + base, tc, m, A, recs.data(), snap, stages.data());
+            for (int i = 0; i < count; ++i)
+                rg::car_tick_post(A.cars[i], stages[i].pre, A.controls[i], A.wheels[i], tc, t + 1 == ticks, A.cfgs[i],
+                                  A.pads, layout, stages[i].pads);
+            rg::arena_tick_tail(env, ball, A, layout, tc, stages.data());
+        }
+    }
 }
 
 }  // extern "C"

@@ -12,6 +12,7 @@ from rocketgpu_b200 import build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "rocketgpu_b200", "csrc")
+MC = 6
 
 
 def _build(tmp, name, edits=()):
@@ -111,3 +112,98 @@ def test_query_grid_visits_what_a_scan_of_all_triangles_does(libs, mesh, arena_m
                                    len(boxes), ctypes.byref(cell))
     assert wrong == 0
     assert cell.value == (4.0 if mesh in ("largest coordinates", "many large triangles") else 2.0)
+
+
+PADS = [(0, -4240, 70), (-1792, -4184, 70), (1792, -4184, 70), (-940, -3308, 70), (940, -3308, 70), (0, -2816, 70),
+        (-3584, -2484, 70), (3584, -2484, 70), (-1788, -2302, 70), (1788, -2302, 70), (-2048, -1036, 70),
+        (0, -1024, 70), (2048, -1036, 70), (-1024, 0, 70), (1024, 0, 70), (-2048, 1036, 70), (0, 1024, 70),
+        (2048, 1036, 70), (-1788, 2302, 70), (1788, 2302, 70), (-3584, 2484, 70), (3584, 2484, 70), (0, 2816, 70),
+        (-940, 3308, 70), (940, 3308, 70), (-1792, 4184, 70), (1792, 4184, 70), (0, 4240, 70), (-3584, 0, 73),
+        (3584, 0, 73), (-3072, 4096, 73), (3072, 4096, 73), (-3072, -4096, 73), (3072, -4096, 73)]
+
+
+class HostBatch(ctypes.Structure):
+    ARRAYS = ("counts", "teams", "cfgs", "cars", "balls", "env_states", "pads", "wheels", "ball_world", "broadphase",
+              "car_world", "ball_car", "pairs", "pad_pos", "pad_big")
+    _fields_ = [("envs", ctypes.c_int32), ("max_cars", ctypes.c_int32), ("pad_count", ctypes.c_int32)] + \
+        [(a, ctypes.c_void_p) for a in ARRAYS] + [("kickoff_seed", ctypes.c_uint64)]
+
+
+def host_step(lib, sim, mesh, counts, teams, cfgs, seed, controls):
+    """The batch's state as it stands, stepped on the host: (cars, balls, envs, pads) after the ticks of `controls`
+    [ticks, envs * MC, 24]."""
+    arrays = {"counts": np.ascontiguousarray(counts, np.int32), "teams": teams, "cfgs": cfgs,
+              "cars": sim.download_car_states(), "balls": sim.download_ball_states(),
+              "env_states": sim.download_env_states(), "pads": sim.download_boost_pad_states(),
+              "pad_pos": np.array(PADS, np.float32), "pad_big": np.array([k >= 28 for k in range(34)], np.uint8)}
+    blob, at = sim.download_internal_state(), 0
+    names = {"wheel_runtime": "wheels", "car_pairs": "pairs"}
+    for name, size in sim.internal_state_layout():
+        if name != "car_stages":
+            arrays[names.get(name, name)] = np.concatenate([blob[at:at + size], np.zeros(16, np.uint8)])
+        at += size
+    arrays = {k: _aligned(x) for k, x in arrays.items()}
+    b = HostBatch(len(counts), MC, 34, *[arrays[a].ctypes.data for a in HostBatch.ARRAYS], seed)
+    v, i = (np.ascontiguousarray(mesh[0], np.float32), np.ascontiguousarray(mesh[1], np.int32))
+    lib.hp_step(ctypes.byref(b), ctypes.byref(sim.config.c), v.ctypes.data_as(ctypes.c_void_p),
+                ctypes.c_longlong(len(v)), i.ctypes.data_as(ctypes.c_void_p), ctypes.c_longlong(len(i)),
+                controls.ctypes.data_as(ctypes.c_void_p), len(controls))
+    return arrays["cars"], arrays["balls"], arrays["env_states"], arrays["pads"]
+
+
+def _aligned(a):
+    """A copy at a 16-byte boundary, as the structs' host build expects."""
+    raw = np.zeros(a.nbytes + 16, np.uint8)
+    off = -raw.ctypes.data % 16
+    out = raw[off:off + a.nbytes].view(a.dtype).reshape(a.shape)
+    out[...] = a
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mix", ["one car", "odd mix", "six cars in contact"])
+def test_ticks_match_the_headers_on_the_host(libs, arena_mesh, mix):
+    """The tick's kernels against the same headers stepped on the host, arena after arena, one lane per car and every
+    vehicle update in the arena's order: bitwise over play with landings, wheels on cars, bumps and ball touches. Car
+    totals leave partly filled warps and blocks."""
+    import torch
+
+    from rocketgpu_b200.batch_sim import BatchSim, SimConfig, car_preset
+    from tests import scenarios
+    n, ticks, rounds, seed = {"one car": (1, 4, 40, 3), "odd mix": (67, 8, 30, 5),
+                              "six cars in contact": (41, 8, 30, 7)}[mix]
+    rng = np.random.default_rng(seed)
+    counts = {"one car": np.array([1]), "odd mix": rng.integers(0, MC + 1, n),
+              "six cars in contact": np.full(n, MC)}[mix].astype(np.int32)
+    slot = np.arange(MC)[None, :]
+    teams = ((slot >= (counts // 2)[:, None]) & (slot < counts[:, None])).astype(np.uint8).reshape(-1)
+    cfgs = np.stack([car_preset(k) for k in range(6)])[rng.integers(0, 6, n * MC)]
+    sim = BatchSim(SimConfig(kickoff_settled=0, env_count=n, max_cars_per_env=MC), *arena_mesh)
+    sim.set_env_car_count(counts)
+    sim.set_teams(teams)
+    sim.set_car_configs(cfgs)
+    sim.reset_to_kickoff(seed)
+    if mix == "six cars in contact":
+        cars, balls = scenarios.contact_heavy(sim.download_car_states(), sim.download_ball_states(), counts, MC, seed)
+        sim.upload_car_states(cars)
+        sim.upload_ball_states(balls)
+    stream = scenarios.ControlStream(n * MC, seed, p_jump=0.1, hold_max=30)
+    active = (slot < counts[:, None]).reshape(-1)
+    for k in range(rounds):
+        controls = np.ascontiguousarray(np.stack([stream.next() for _ in range(ticks)]))
+        if mix == "six cars in contact":
+            chase = scenarios.chase_ball_controls(sim.download_car_states(), sim.download_ball_states(), MC, rng)
+            controls[:] = chase
+        want = host_step(libs[0], sim, arena_mesh, counts, teams, cfgs, seed, controls)
+        dev = torch.from_numpy(controls.reshape(-1)).cuda()
+        sim.step_with_device_controls(dev.data_ptr(), ticks, n * MC)
+        sim.synchronize()
+        got = (sim.download_car_states(), sim.download_ball_states(), sim.download_env_states(),
+               sim.download_boost_pad_states())
+        for name, g, w in zip(("cars", "balls", "envs", "pads"), got, want):
+            if name == "cars":
+                g, w = g[active], w[active]
+            assert _same(np.ascontiguousarray(g).view(np.float32), np.ascontiguousarray(w).view(np.float32)), (name, k)
+    moved = sim.download_car_states()[active][:, 28:40].copy().view(np.float32)
+    assert np.abs(moved[np.isfinite(moved)]).max() > 100.0
+    sim.close()
