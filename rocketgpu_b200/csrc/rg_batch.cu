@@ -242,7 +242,7 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
     return a.meshes ? a.meshes[a.mesh_of[e]] : a.mesh;
 }
 
-__global__ void __launch_bounds__(256) tick_kernel(TickArgs a, int ticks) {
+__global__ void __launch_bounds__(256) tick_kernel(const __grid_constant__ TickArgs a, int ticks) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= a.env_count) return;
     rg::BallState b = a.balls[e];
@@ -288,6 +288,9 @@ struct SlotTable {
     const uint64_t* seed;
 };
 
+// The kernels take their arguments as __grid_constant__: functions that are not inlined get references to the config,
+// the mesh and the pad layout, and of an ordinary parameter the compiler first made each thread a copy in local memory
+// (1.2 KB; at 16,384 mixed arenas a tick's kernels wrote 1.3 GB of local memory to HBM, now 0.2 GB: 1,692 -> 1,450 us).
 struct CarTickArgs {
     TickArgs base;
     rg::CarState* cars;
@@ -362,8 +365,8 @@ __device__ __forceinline__ rg::ArenaContactState arena_contact_state(const CarTi
 
 // Env commands between steps, one thread per arena (reference LaunchApplyEnvCommands / apply_env_commands_host,
 // src/rocketgpu.cpp:2136-2218).
-__global__ void apply_commands_kernel(CarTickArgs a, const rg::EnvCommand* cmds, int n, rg::CarControls* controls,
-                                      uint32_t* status) {
+__global__ void apply_commands_kernel(const __grid_constant__ CarTickArgs a, const rg::EnvCommand* cmds, int n,
+                                      rg::CarControls* controls, uint32_t* status) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const rg::EnvCommand c = cmds[e];
@@ -375,7 +378,7 @@ __global__ void apply_commands_kernel(CarTickArgs a, const rg::EnvCommand* cmds,
 
 // Tick part 1, one thread per arena in step order: this tick's env command (step_with_device_commands), vehicle
 // order, the ball's tick start, pad timers.
-__global__ void __launch_bounds__(256) arena_begin_kernel(CarTickArgs a, int t) {
+__global__ void __launch_bounds__(256) arena_begin_kernel(const __grid_constant__ CarTickArgs a, int t) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
@@ -397,7 +400,7 @@ __global__ void __launch_bounds__(256) arena_begin_kernel(CarTickArgs a, int t) 
 
 // Tick part 2, one thread per active car: the car's tick start (demolition timer and respawn, quantisation, controls,
 // jumps, dodges, boost) and the speed clamp.
-__global__ void __launch_bounds__(256) car_pre_kernel(CarTickArgs a, int t) {
+__global__ void __launch_bounds__(256) car_pre_kernel(const __grid_constant__ CarTickArgs a, int t) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
@@ -452,7 +455,8 @@ struct FourLanes {
 // the lanes); [mesh_blocks, mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact
 // geometry; the rest one thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets
 // another car's box.
-__global__ void __launch_bounds__(256) car_geometry_kernel(CarTickArgs a, int t, int mesh_blocks, int ball_blocks) {
+__global__ void __launch_bounds__(256)
+    car_geometry_kernel(const __grid_constant__ CarTickArgs a, int t, int mesh_blocks, int ball_blocks) {
     const int block = static_cast<int>(blockIdx.x);
     if (block < mesh_blocks) {
         const int k = static_cast<int>(block * blockDim.x + threadIdx.x) >> 2;
@@ -529,7 +533,8 @@ __device__ __forceinline__ void lanes_copy(T* dst, const T* src, int lane) {
         if (4 * i + lane < kWords) d[4 * i + lane] = w[i];
 }
 
-__global__ void __launch_bounds__(kVehicleThreads) car_vehicle_kernel(CarTickArgs a, int t) {
+__global__ void __launch_bounds__(kVehicleThreads)
+    car_vehicle_kernel(const __grid_constant__ CarTickArgs a, int t) {
     __shared__ __align__(16) unsigned char shared[kVehicleThreads / 4 * kVehicleSlotBytes];
     const FourLanes lanes;
     const int k = static_cast<int>(blockIdx.x * (kVehicleThreads / 4) + (threadIdx.x >> 2));
@@ -570,7 +575,7 @@ __global__ void __launch_bounds__(kVehicleThreads) car_vehicle_kernel(CarTickArg
 // One thread per arena fills a single wave at any batch this path runs, so these two kernels take the registers that
 // remove most of their spills (measured at 16,384 mixed arenas: the finish 4.09 -> 3.91 ms per 8-tick step; the car
 // kernels lost time under the same change, their spill-free register counts cost waves).
-__global__ void __maxnreg__(255) arena_finish_kernel(CarTickArgs a, int t) {
+__global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
@@ -586,7 +591,8 @@ __global__ void __maxnreg__(255) arena_finish_kernel(CarTickArgs a, int t) {
 }
 
 // Tick part 5, one thread per active car: its integration and post-tick.
-__global__ void __launch_bounds__(256) car_post_kernel(CarTickArgs a, int t, int report_fields) {
+__global__ void __launch_bounds__(256)
+    car_post_kernel(const __grid_constant__ CarTickArgs a, int t, int report_fields) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
@@ -602,7 +608,7 @@ __global__ void __launch_bounds__(256) car_post_kernel(CarTickArgs a, int t, int
 }
 
 // Tick part 6, one thread per arena in step order: pads, the driving countdown, extra ball hits, goal and timers.
-__global__ void __maxnreg__(255) arena_tail_kernel(CarTickArgs a, int t) {
+__global__ void __maxnreg__(255) arena_tail_kernel(const __grid_constant__ CarTickArgs a, int t) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
@@ -747,8 +753,8 @@ void step_car_path(rg_batch* b, const rg::CarControls* controls, int stride, int
 
 // reset_to_kickoff for every arena (reference BatchSim::reset_to_kickoff, src/rocketgpu.cpp:2085-2132).
 // Arenas [first, first + n) reset; their RNG draws use their index within the range (the whole batch: first = 0).
-__global__ void reset_kickoff_kernel(CarTickArgs a, const uint8_t* teams, rg::CarControls* controls, uint64_t seed,
-                                     int first, int n) {
+__global__ void reset_kickoff_kernel(const __grid_constant__ CarTickArgs a, const uint8_t* teams,
+                                     rg::CarControls* controls, uint64_t seed, int first, int n) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const int e = first + j;
