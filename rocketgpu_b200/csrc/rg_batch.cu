@@ -126,6 +126,7 @@ struct rg_batch {
     DeviceArray<uint8_t> mesh_of;
     std::vector<int32_t> host_car_count;
     std::vector<int32_t> host_arena_order, host_active_cars;
+    int sms = 1;                  // the device's multiprocessors
     int launch_threads = 32;      // threads per block of the per-arena kernels
     int car_threads = 64;         // threads per block of the per-car kernels
     int pair_slots = 0;
@@ -224,6 +225,35 @@ __global__ void canonicalize_balls_kernel(rg::BallState* balls, int n) {
     b.deactivation_time = 0.0f;
 }
 
+// A kernel with one thread per arena or car leaves idle lanes between them when the chip has room for more warps than
+// they fill: item k runs in thread k << shift, so that a warp holds fewer items, diverges less and touches fewer lines
+// per access. The shift is the largest, up to one item per warp, whose warps are all resident at once (`warps_per_sm`:
+// by the kernel's registers). Measured, us a tick at shift 0 and by this rule: the arena finish 171 -> 148 at 1,024 mixed
+// arenas, 541 -> 475 at 4,095 3v3 arenas, 397 -> 382 at 16,384 mixed ones (one item in two threads there); the tail 41 ->
+// 31, 55 -> 46, 62 -> 56; the post-tick 47 -> 41, 56 -> 51, 73 -> 71; 16,384 ball-only arenas 2,907 -> 2,279 us a 60-tick
+// pass. The car tick start lost (27 -> 48 at 1,024): its local copies of the structs then use 4 of each 32-byte sector;
+// the arena begin gained nothing. Those two run one item per thread.
+__device__ __forceinline__ int spread_item(int shift) {
+    const int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    return (g & ((1 << shift) - 1)) != 0 ? 0x7fffffff : g >> shift;
+}
+int spread_shift(int64_t items, int sms, int warps_per_sm) {
+    int shift = 0;
+    while (shift < 5 && ((items << (shift + 1)) + 31) / 32 <= static_cast<int64_t>(sms) * warps_per_sm) ++shift;
+    return shift;
+}
+int spread_blocks(int64_t items, int shift, int threads) {
+    return static_cast<int>(((items << shift) + threads - 1) / threads);
+}
+// Resident warps per SM of the spread kernels, from their registers per thread (65,536 per SM).
+constexpr int kWarpsBalls = 16, kWarpsFinish = 8, kWarpsPost = 32, kWarpsTail = 8;
+
+int device_sms(int device) {
+    int n = 1;
+    check(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+    return n;
+}
+
 struct TickArgs {
     rg::BallState* balls;
     rg::EnvState* envs;
@@ -242,8 +272,8 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
     return a.meshes ? a.meshes[a.mesh_of[e]] : a.mesh;
 }
 
-__global__ void __launch_bounds__(256) tick_kernel(const __grid_constant__ TickArgs a, int ticks) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
+    const int e = spread_item(shift);
     if (e >= a.env_count) return;
     rg::BallState b = a.balls[e];
     rg::EnvState env = a.envs[e];
@@ -575,8 +605,8 @@ __global__ void __launch_bounds__(kVehicleThreads)
 // One thread per arena fills a single wave at any batch this path runs, so these two kernels take the registers that
 // remove most of their spills (measured at 16,384 mixed arenas: the finish 4.09 -> 3.91 ms per 8-tick step; the car
 // kernels lost time under the same change, their spill-free register counts cost waves).
-__global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
+    const int k = spread_item(shift);
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
     if (arena_idle(a, e)) return;
@@ -592,8 +622,8 @@ __global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ Car
 
 // Tick part 5, one thread per active car: its integration and post-tick.
 __global__ void __launch_bounds__(256)
-    car_post_kernel(const __grid_constant__ CarTickArgs a, int t, int report_fields) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    car_post_kernel(const __grid_constant__ CarTickArgs a, int t, int report_fields, int shift) {
+    const int k = spread_item(shift);
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
     const int e = idx / a.max_cars;
@@ -608,8 +638,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // Tick part 6, one thread per arena in step order: pads, the driving countdown, extra ball hits, goal and timers.
-__global__ void __maxnreg__(255) arena_tail_kernel(const __grid_constant__ CarTickArgs a, int t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __maxnreg__(255) arena_tail_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
+    const int k = spread_item(shift);
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
     if (arena_idle(a, e)) return;
@@ -663,7 +693,39 @@ CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stri
     return a;
 }
 
-// Arenas with cars: four launches per tick (arena begin, per-car tick start, per-car vehicle update, arena finish).
+// One tick's launches. `mark` is called before each of the six phases and after the last.
+template <class Mark>
+void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, int report_fields, cudaStream_t s, Mark&& mark) {
+    const int64_t arenas = b->env_count, cars = b->active_car_count;
+    const int at = b->launch_threads, ct = b->car_threads;
+    const int car_blocks = spread_blocks(cars, 0, ct), wheel_blocks = spread_blocks(cars, 2, ct);
+    auto shift = [&](int64_t items, int warps) { return spread_shift(items, b->sms, warps); };
+    mark();
+    arena_begin_kernel<<<spread_blocks(arenas, 0, at), at, 0, s>>>(a, t);
+    mark();
+    if (cars) car_pre_kernel<<<car_blocks, ct, 0, s>>>(a, t);
+    mark();
+    // phase 2 (timing) is the geometry and the vehicle updates
+    if (cars) {
+        car_geometry_kernel<<<2 * wheel_blocks + car_blocks, ct, 0, s>>>(a, t, wheel_blocks, car_blocks);
+        car_vehicle_kernel<<<spread_blocks(cars, 2, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t);
+    }
+    mark();
+    const int finish = shift(arenas, kWarpsFinish);
+    arena_finish_kernel<<<spread_blocks(arenas, finish, at), at, 0, s>>>(a, t, finish);
+    mark();
+    if (cars) {
+        const int post = shift(cars, kWarpsPost);
+        car_post_kernel<<<spread_blocks(cars, post, ct), ct, 0, s>>>(a, t, report_fields, post);
+    }
+    mark();
+    const int tail = shift(arenas, kWarpsTail);
+    arena_tail_kernel<<<spread_blocks(arenas, tail, at), at, 0, s>>>(a, t, tail);
+    mark();
+}
+
+// Arenas with cars: seven launches per tick (arena begin, car tick start, contact geometry, vehicle updates, arena
+// finish, car post-tick, arena tail).
 void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, int ticks, cudaStream_t s,
                      const rg::EnvCommand* commands = nullptr, int command_stride = 0) {
     if (b->env_count == 0) return;
@@ -675,12 +737,6 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         a.pads = b->pads.ptr;
         b->pads_live = true;
     }
-    const int threads = b->launch_threads;
-    const int blocks = (b->env_count + threads - 1) / threads;
-    const int ct = b->car_threads;
-    const int car_blocks = (b->active_car_count + ct - 1) / ct;
-    const int wheel_blocks = (4 * b->active_car_count + ct - 1) / ct;
-    const int vehicle_blocks = (4 * b->active_car_count + kVehicleThreads - 1) / kVehicleThreads;
     auto mark = [&] {
         if (!b->timing) return;
         if (b->events_used == b->events.size()) {
@@ -690,26 +746,9 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         }
         check(cudaEventRecord(b->events[b->events_used++], s), "cudaEventRecord");
     };
-    for (int t = 0; t < ticks; ++t) {
-        mark();
-        arena_begin_kernel<<<blocks, threads, 0, s>>>(a, t);
-        mark();
-        if (car_blocks) car_pre_kernel<<<car_blocks, ct, 0, s>>>(a, t);
-        mark();
-        // phase 2 (timing) is the geometry and the vehicle updates
-        if (car_blocks)
-            car_geometry_kernel<<<2 * wheel_blocks + car_blocks, ct, 0, s>>>(a, t, wheel_blocks, car_blocks);
-        if (car_blocks) car_vehicle_kernel<<<vehicle_blocks, kVehicleThreads, 0, s>>>(a, t);
-        mark();
-        arena_finish_kernel<<<blocks, threads, 0, s>>>(a, t);
-        mark();
-        // report fields after the last tick, and after every tick of a command stream (reference StepEnvGeneric,
-        // env_step.hpp:7174: report_fields = last tick || has_commands)
-        if (car_blocks) car_post_kernel<<<car_blocks, ct, 0, s>>>(a, t, (t + 1 == ticks || commands) ? 1 : 0);
-        mark();
-        arena_tail_kernel<<<blocks, threads, 0, s>>>(a, t);
-        mark();
-    }
+    // report fields after the last tick, and after every tick of a command stream (reference StepEnvGeneric,
+    // env_step.hpp:7174: report_fields = last tick || has_commands)
+    for (int t = 0; t < ticks; ++t) launch_tick_kernels(b, a, t, (t + 1 == ticks || commands) ? 1 : 0, s, mark);
     check(cudaGetLastError(), "car tick launch");
 }
 
@@ -969,11 +1008,8 @@ void launch_tick(rg_batch* b, int ticks, cudaStream_t s) {
     a.mesh = b->mesh;
     a.meshes = b->mesh_table.ptr;
     a.mesh_of = b->mesh_table.ptr ? b->mesh_of.ptr : nullptr;
-    // One warp per block: an arena is one thread, so 16K arenas are only 512 warps; single-warp blocks spread them
-    // over all 148 SMs (128-thread blocks left 20 SMs idle at 16K arenas).
-    const int threads = b->launch_threads;
-    const int blocks = (b->env_count + threads - 1) / threads;
-    tick_kernel<<<blocks, threads, 0, s>>>(a, ticks);
+    const int threads = b->launch_threads, shift = spread_shift(b->env_count, b->sms, kWarpsBalls);
+    tick_kernel<<<spread_blocks(b->env_count, shift, threads), threads, 0, s>>>(a, ticks, shift);
     check(cudaGetLastError(), "tick_kernel launch");
 }
 
@@ -1341,6 +1377,7 @@ RG_API int rg_batch_create(const rg_sim_config* cfg, const rg_arena_layout* layo
         b->mesh_host = rg::build_mesh_host(layout->vertices_uu, layout->vertex_count, layout->indices,
                                            layout->index_count);
         DeviceGuard dg(device);
+        b->sms = device_sms(device);
         b->mesh = rg::upload_mesh(b->mesh_host);
         b->balls.alloc(b->env_count);
         b->envs.alloc(b->env_count);
@@ -2103,8 +2140,8 @@ RG_API int rg_batch_step_static_scratch(rg_batch* b, rg_ball_state* dev_balls, r
         a.mesh = b->mesh;
         a.meshes = b->mesh_table.ptr;
         a.mesh_of = b->mesh_table.ptr ? b->mesh_of.ptr : nullptr;
-        const int threads = b->launch_threads;
-        tick_kernel<<<(env_count + threads - 1) / threads, threads, 0, s>>>(a, ticks);
+        const int threads = b->launch_threads, shift = spread_shift(env_count, b->sms, kWarpsBalls);
+        tick_kernel<<<spread_blocks(env_count, shift, threads), threads, 0, s>>>(a, ticks, shift);
         check(cudaGetLastError(), "tick_kernel launch (static scratch)");
     });
 }

@@ -123,20 +123,7 @@ void server_launch_round(rg_server* s) {
     a.slots.tick = s->tick.ptr;
     a.slots.logical = s->logical.ptr;
     a.slots.seed = s->seed.ptr;
-    const int threads = b->launch_threads;
-    const int blocks = (b->env_count + threads - 1) / threads;
-    const int ct = b->car_threads;
-    const int car_blocks = (b->active_car_count + ct - 1) / ct;
-    arena_begin_kernel<<<blocks, threads, 0, s->stream>>>(a, 0);
-    if (car_blocks) car_pre_kernel<<<car_blocks, ct, 0, s->stream>>>(a, 0);
-    const int wheel_blocks = (4 * b->active_car_count + ct - 1) / ct;
-    const int vehicle_blocks = (4 * b->active_car_count + kVehicleThreads - 1) / kVehicleThreads;
-    if (car_blocks)
-        car_geometry_kernel<<<2 * wheel_blocks + car_blocks, ct, 0, s->stream>>>(a, 0, wheel_blocks, car_blocks);
-    if (car_blocks) car_vehicle_kernel<<<vehicle_blocks, kVehicleThreads, 0, s->stream>>>(a, 0);
-    arena_finish_kernel<<<blocks, threads, 0, s->stream>>>(a, 0);
-    if (car_blocks) car_post_kernel<<<car_blocks, ct, 0, s->stream>>>(a, 0, 0);
-    arena_tail_kernel<<<blocks, threads, 0, s->stream>>>(a, 0);
+    launch_tick_kernels(b, a, 0, 0, s->stream, [] {});
     check(cudaGetLastError(), "serving round launch");
 }
 
