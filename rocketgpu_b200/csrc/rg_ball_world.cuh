@@ -619,38 +619,18 @@ RG_HDI void mesh_query_box(const MeshDevice& m, V3 lo, V3 hi, F&& visit) {
     }
 }
 
-// One thread doing a query alone (see mesh_query_box_lanes).
+// One thread alone where several lanes may share the work.
 struct OneLane {
     static constexpr int kLanes = 1;
     RG_HD int lane() const { return 0; }
     RG_HD void sync() const {}
     RG_HD unsigned ballot(bool p) const { return p ? 1u : 0u; }
+    RG_HD uint32_t any(uint32_t bits) const { return bits; }
     template <class T>
     RG_HD T from(const T& v, int) const {
         return v;
     }
 };
-// mesh_query_box with the list shared by the lanes of `lanes` (threads of one warp that hold the same query): each lane
-// tests its entries of a round, `test(triangle, result)`, and lane 0 visits the results that hold in the list's order.
-template <class R, class L, class Test, class Visit>
-RG_HDI void mesh_query_box_lanes(const L& lanes, const MeshDevice& m, V3 lo, V3 hi, Test&& test, Visit&& visit) {
-    const MeshQuery q = mesh_query(m, lo, hi);
-    for (int e = q.begin; e < q.end; e += L::kLanes) {
-        const int k = e + lanes.lane();
-        R r;
-        bool holds = false;
-        if (k < q.end) {
-            const CellEntry en = q.list[k];
-            holds = q.overlaps(en) && test(m.tris[en.rank], r);
-        }
-        unsigned hits = lanes.ballot(holds);
-        while (hits != 0u) {
-            const R v = lanes.from(r, ctz32(hits));
-            hits &= hits - 1u;
-            if (lanes.lane() == 0) visit(v);
-        }
-    }
-}
 
 // Bullet's ray-vs-leaf-box test of the quantized BVH walk: the ray must cross the leaf's dequantized bounds within its
 // length (reference ArenaMeshBvhRayLeaf, include/rocketgpu/detail/arena/mesh_bvh.hpp:522-558, and the same slab test

@@ -465,6 +465,11 @@ struct FourLanes {
     __device__ int lane() const { return static_cast<int>(threadIdx.x & 3u); }
     __device__ void sync() const { __syncwarp(mask); }
     __device__ unsigned ballot(bool p) const { return (__ballot_sync(mask, p) >> base) & 15u; }
+    // the bits that any lane holds
+    __device__ uint32_t any(uint32_t bits) const {
+        bits |= __shfl_xor_sync(mask, bits, 1);
+        return bits | __shfl_xor_sync(mask, bits, 2);
+    }
     // lane `src`'s value (a struct of 32-bit words)
     template <class T>
     __device__ T from(const T& v, int src) const {
@@ -480,22 +485,121 @@ struct FourLanes {
     }
 };
 
+// The car/mesh geometry of a warp's eight cars, four lanes each. The lanes of a car share the scan of its query list
+// (bounds and separating axes) and note the triangles that need the narrowphase; then all 32 lanes take those of the
+// eight cars, one each, whichever car they belong to, and each car's first lane merges its results in leaf order. A car
+// in a corner or on a seam of small triangles has up to a dozen: GJK (30,000 cycles a triangle, EPA 90,000) one after
+// another in the car's own lanes made the launch wait for a few of them.
+constexpr int kMeshList = 24;  // triangles noted per car before they are worked off
+struct MeshWarp {
+    rg::CarMeshPose pose[8];
+    const rg::DevTri* tris[8];
+    int32_t rank[8][kMeshList];
+    rg::CarTriHit hit[32];
+};
+__device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshWarp& w) {
+    const FourLanes lanes;
+    const int lane32 = static_cast<int>(threadIdx.x & 31u), group = lane32 >> 2;
+    const bool first = lanes.lane() == 0;
+    int idx = 0, e = 0;
+    bool runs = k < a.active_car_count;
+    if (runs) {
+        idx = a.active_cars[k];
+        e = idx / a.max_cars;
+        runs = !arena_idle(a, e);
+    }
+    if (runs) {
+        const rg::CarState& car = a.cars[idx];
+        runs = !(car.is_demoed || car.just_respawned);
+        if (first) a.stages[idx].mesh_ran = runs ? 1u : 0u;
+    }
+    rg::CarMeshPose pose;
+    rg::CarQueryFrame qf;
+    rg::MeshQuery q;
+    const rg::DevTri* tris = nullptr;
+    q.begin = q.end = 0;
+    rg::CarWorldScratch ws;
+    rg::CarMeshManifold m;
+    if (runs) {
+        const rg::MeshDevice& mesh = arena_mesh(a.base, e);
+        pose = rg::car_mesh_pose(a.cars[idx], a.car_cfgs[idx]);
+        qf = rg::car_query_frame(a.cars[idx], a.car_cfgs[idx]);
+        q = rg::mesh_query(mesh, qf.lo, qf.hi);
+        tris = mesh.tris;
+        if (first) {
+            w.pose[group] = pose;
+            w.tris[group] = tris;
+            ws = a.car_world[idx];
+            m.begin(pose, ws);
+        }
+    }
+    int at = q.begin;
+    bool more;
+    do {
+        int noted = 0;
+        while (at < q.end && noted + 4 <= kMeshList) {
+            const int i = at + lanes.lane();
+            bool take = false;
+            int32_t rank = 0;
+            if (i < q.end) {
+                const rg::CellEntry en = q.list[i];
+                rank = en.rank;
+                take = q.overlaps(en) && rg::car_triangle_query(tris[rank], qf, pose.thr) == 2;
+            }
+            const unsigned taken = lanes.ballot(take);
+            if (take) w.rank[group][noted + __popc(taken & ((1u << lanes.lane()) - 1u))] = rank;
+            noted += __popc(taken);
+            at += 4;
+        }
+        more = at < q.end;
+        __syncwarp();
+        int start = 0, total = 0, end_of[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            const int n = __shfl_sync(0xffffffffu, noted, 4 * g);
+            start += g < group ? n : 0;
+            total += n;
+            end_of[g] = total;
+        }
+        for (int from = 0; from < total; from += 32) {
+            const int p = from + lane32;
+            if (p < total) {
+                int g = 0, before = 0;
+#pragma unroll
+                for (int j = 0; j < 7; ++j)
+                    if (p >= end_of[j]) {
+                        g = j + 1;
+                        before = end_of[j];
+                    }
+                w.hit[lane32] = rg::car_triangle_hit(w.pose[g], w.tris[g][w.rank[g][p - before]]);
+            }
+            __syncwarp();
+            if (first) {
+                const int hi = start + noted < from + 32 ? start + noted : from + 32;
+                for (int j = start > from ? start : from; j < hi; ++j) m.add(pose, w.hit[j - from]);
+            }
+            __syncwarp();
+        }
+    } while (__any_sync(0xffffffffu, more));
+    if (runs && first) {
+        m.finish(pose, ws);
+        rg::CarStage& st = a.stages[idx];
+        st.ws = ws;
+        st.res.latest_normal = m.last_normal;
+    }
+}
+
 // Tick part 3a, what reads only poses and so runs ahead of the vehicle updates, in blocks of three kinds that the chip
-// runs side by side: [0, mesh_blocks) four lanes per active car, the geometry of its arena contacts (triangles shared by
-// the lanes); [mesh_blocks, mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact
-// geometry; the rest one thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets
-// another car's box.
-__global__ void __launch_bounds__(256)
+// runs side by side: [0, mesh_blocks) four lanes per active car, the geometry of its arena contacts; [mesh_blocks,
+// mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact geometry; the rest one
+// thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets another car's box.
+constexpr int kGeometryThreads = 64;
+__global__ void __launch_bounds__(kGeometryThreads)
     car_geometry_kernel(const __grid_constant__ CarTickArgs a, int t, int mesh_blocks, int ball_blocks) {
     const int block = static_cast<int>(blockIdx.x);
     if (block < mesh_blocks) {
-        const int k = static_cast<int>(block * blockDim.x + threadIdx.x) >> 2;
-        if (k >= a.active_car_count) return;
-        const int idx = a.active_cars[k];
-        const int e = idx / a.max_cars;
-        if (arena_idle(a, e)) return;
-        rg::car_mesh_stage(FourLanes(), a.cars[idx], a.car_cfgs[idx], a.car_world[idx], arena_mesh(a.base, e),
-                           a.stages[idx]);
+        __shared__ MeshWarp warps[kGeometryThreads / 32];
+        car_mesh_warp(a, static_cast<int>(block * blockDim.x + threadIdx.x) >> 2, warps[threadIdx.x >> 5]);
         return;
     }
     if (block < mesh_blocks + ball_blocks) {
@@ -521,87 +625,75 @@ __global__ void __launch_bounds__(256)
         return;
     }
     const int base = e * a.max_cars, count = a.base.env_car_count[e], slot = idx - base;
-    const uint32_t excluded = rg::wheel_ray_excluded_bodies(car, a.car_cfgs[idx], a.broadphase + e, slot, count);
-    uint8_t meets = 0;
+    const uint32_t excluded = rg::wheel_ray_excluded_bodies(FourLanes(), car, a.car_cfgs[idx], a.broadphase + e, slot, count);
+    int met = -1;
     rg::wheel_mesh_ray_ahead(car, a.car_cfgs[idx], arena_mesh(a.base, e), wheel,
                              rg::WheelOthers{a.cars + base, a.car_cfgs + base, count, slot, excluded},
-                             st.wheel_mesh[wheel], meets);
-    st.wheel_meets_car[wheel] = static_cast<uint8_t>((meets ? rg::kWheelMeetsCar : 0) |
-                                                     ((excluded & 1u) ? rg::kWheelBallExcluded : 0));
+                             st.wheel_mesh[wheel], met);
+    st.wheel_meets_car[wheel] = static_cast<uint8_t>(
+        (met >= 0 ? rg::kWheelMeetsCar | (met << rg::kWheelMetShift) : 0) | ((excluded & 1u) ? rg::kWheelBallExcluded : 0));
 }
 
 // Tick part 3b, four lanes per active car: the vehicle update (tyres, drive, air control) and the car's staged
-// world-step parts, for cars whose wheels can land on no other car and under whose car no other wheel can land
-// (rg::arena_free_cars); the others are left to part 4. The car, its wheel record and its config are worked on in shared
-// memory: one thread per car on the structs in HBM took 893 us at 16,384 mixed arenas (11 warps per SM, 37 cycles per
-// instruction waiting for lines of 880-byte-strided structs that the L1 could not hold).
-struct alignas(16) VehicleSlot {
-    rg::CarState car;
-    rg::WheelRuntime wheels;
-    alignas(8) rg::CarConfig cfg;
-    rg::VehicleTick tick;
-};
-// lanes_copy's words: 16 bytes for the car, 4 for the wheel record (292 bytes), 8 for the config
-static_assert(offsetof(VehicleSlot, car) % 16 == 0 && offsetof(VehicleSlot, cfg) % 8 == 0, "aligned copies");
-// An odd number of 16-byte units, so that the same field of a warp's eight cars falls into eight different banks.
-constexpr size_t kVehicleSlotBytes = sizeof(VehicleSlot) / 16 % 2 == 1 ? sizeof(VehicleSlot) : sizeof(VehicleSlot) + 16;
+// world-step parts. Cars whose wheels meet no other car and that no other wheel meets update side by side; an arena's
+// others (rg::arena_cars_met) one after another in the game's order, by the first `order_blocks` blocks, four lanes per
+// arena, so that these chains start with the launch (in the arena's own thread of part 4 they took 80 us of a tick at
+// 16,384 mixed arenas). The
+// car, its wheel record and its config are worked on in shared memory: one thread per car on the structs in HBM took
+// 893 us at 16,384 mixed arenas (11 warps per SM, 37 cycles per instruction waiting for lines of 880-byte-strided structs
+// that the L1 could not hold).
+// The slot is an odd number of 16-byte units, so that the same field of a warp's eight cars falls into eight different
+// banks.
+constexpr size_t kVehicleSlotBytes =
+    sizeof(rg::VehicleSlot) / 16 % 2 == 1 ? sizeof(rg::VehicleSlot) : sizeof(rg::VehicleSlot) + 16;
 constexpr int kVehicleThreads = 64;
 
-// A struct copied by the four lanes of a group, word l, l + 4, ... by lane l.
-template <class Word, class T>
-__device__ __forceinline__ void lanes_copy(T* dst, const T* src, int lane) {
-    static_assert(sizeof(T) % sizeof(Word) == 0, "whole words: every struct of an array is aligned to one");
-    constexpr int kWords = sizeof(T) / sizeof(Word), kRounds = (kWords + 3) / 4;
-    const Word* s = reinterpret_cast<const Word*>(src);
-    Word* d = reinterpret_cast<Word*>(dst);
-    Word w[kRounds];
-#pragma unroll
-    for (int i = 0; i < kRounds; ++i)
-        if (4 * i + lane < kWords) w[i] = s[4 * i + lane];
-#pragma unroll
-    for (int i = 0; i < kRounds; ++i)
-        if (4 * i + lane < kWords) d[4 * i + lane] = w[i];
+// Out of line, so that the kernel keeps the registers of the common path (inlined, it took 168 instead of 108).
+__device__ __noinline__ void cars_in_order(const CarTickArgs& a, int e, int t, uint32_t which, rg::VehicleSlot& s) {
+    const int base = e * a.max_cars;
+    rg::arena_cars_in_order(FourLanes(), a.base.envs[e], a.base.balls[e], a.broadphase[e], a.base.tc,
+                            arena_mesh(a.base, e), arena_cars(a, e, t), a.records + base, a.stages + base, which, s);
 }
 
-__global__ void __launch_bounds__(kVehicleThreads)
-    car_vehicle_kernel(const __grid_constant__ CarTickArgs a, int t) {
+__global__ void __launch_bounds__(kVehicleThreads, 8)
+    car_vehicle_kernel(const __grid_constant__ CarTickArgs a, int t, int order_blocks) {
     __shared__ __align__(16) unsigned char shared[kVehicleThreads / 4 * kVehicleSlotBytes];
     const FourLanes lanes;
-    const int k = static_cast<int>(blockIdx.x * (kVehicleThreads / 4) + (threadIdx.x >> 2));
+    rg::VehicleSlot& s = *reinterpret_cast<rg::VehicleSlot*>(shared + (threadIdx.x >> 2) * kVehicleSlotBytes);
+    const int block = static_cast<int>(blockIdx.x);
+    if (block < order_blocks) {
+        const int k = block * (kVehicleThreads / 4) + static_cast<int>(threadIdx.x >> 2);
+        if (k >= a.base.env_count) return;
+        const int e = a.arena_order[k];
+        if (arena_idle(a, e)) return;
+        const uint32_t which = rg::arena_cars_met(a.stages + e * a.max_cars, a.base.env_car_count[e]);
+        if (which != 0u) cars_in_order(a, e, t, which, s);
+        return;
+    }
+    const int k = (block - order_blocks) * (kVehicleThreads / 4) + static_cast<int>(threadIdx.x >> 2);
     if (k >= a.active_car_count) return;
     const int idx = a.active_cars[k];
     const int e = idx / a.max_cars;
     if (arena_idle(a, e)) return;
-    const int base = e * a.max_cars;
-    const int count = a.base.env_car_count[e];
-    VehicleSlot& s = *reinterpret_cast<VehicleSlot*>(shared + (threadIdx.x >> 2) * kVehicleSlotBytes);
-    lanes_copy<uint4>(&s.car, a.cars + idx, lanes.lane());
-    lanes_copy<uint32_t>(&s.wheels, a.wheels + idx, lanes.lane());
-    lanes_copy<uint2>(&s.cfg, a.car_cfgs + idx, lanes.lane());
-    // the car's update runs here when no wheel of the arena meets another car, or when the sweep-box rule shows that
-    // no other car can be under its wheels nor it under theirs
-    const bool free =
-        !rg::arena_wheels_meet_cars(a.stages + base, count) ||
-        ((rg::arena_free_cars(a.cars + base, a.car_cfgs + base, a.broadphase[e], count) >> (idx - base)) & 1u);
-    rg::CarStage& st = a.stages[idx];
-    if (lanes.lane() == 0) st.in_car_thread = free ? 1u : 0u;
-    if (!free) return;  // the arena thread updates this car in the game's car order
+    const int base = e * a.max_cars, slot = idx - base;
+    if ((rg::arena_cars_met(a.stages + base, a.base.env_car_count[e]) >> slot) & 1u) return;
+    rg::CarStage* stages = a.stages + base;
+    const rg::MeshDevice& mesh = arena_mesh(a.base, e);
+    rg::vehicle_slot_load(lanes, s, a.cars + idx, a.wheels + idx, a.car_cfgs + idx);
     lanes.sync();
+    rg::CarStage& st = stages[slot];
     const rg::CarControls& ctrl =
         a.controls[control_row(a, e, t) * static_cast<size_t>(a.control_stride) + static_cast<size_t>(idx)];
     const uint32_t excluded = (st.wheel_meets_car[0] & rg::kWheelBallExcluded) ? 1u : 0u;
-    const rg::MeshDevice& mesh = arena_mesh(a.base, e);
     rg::vehicle_update(lanes, s.car, ctrl, s.cfg, a.base.tc, s.wheels, a.base.balls[e], mesh,
                        rg::WheelOthers{nullptr, nullptr, 0, -1, excluded}, a.records[idx].pushes, st.wheel_mesh, s.tick);
-    // the car's own part of the world step, while this thread has the car (rg::CarStage)
-    if (lanes.lane() == 0) rg::car_stage_compute(s.car, s.cfg, s.wheels, a.base.tc, mesh, idx - base, st);
+    // the car's own part of the world step, while these lanes have the car (rg::CarStage)
+    if (lanes.lane() == 0) rg::car_stage_compute(s.car, s.cfg, s.wheels, a.base.tc, mesh, slot, st);
     lanes.sync();
-    lanes_copy<uint4>(a.cars + idx, &s.car, lanes.lane());
-    lanes_copy<uint32_t>(a.wheels + idx, &s.wheels, lanes.lane());
+    rg::vehicle_slot_store(lanes, s, a.cars + idx, a.wheels + idx);
 }
 
-// Tick part 4, one thread per arena in step order: the vehicle updates (and staged parts) of cars whose wheels may
-// land on other cars, in the game's car order; wheel pushes on the ball; the world step's shared stages.
+// Tick part 4, one thread per arena in step order: wheel pushes on the ball, then the world step's shared stages.
 // One thread per arena fills a single wave at any batch this path runs, so these two kernels take the registers that
 // remove most of their spills (measured at 16,384 mixed arenas: the finish 4.09 -> 3.91 ms per 8-tick step; the car
 // kernels lost time under the same change, their spill-free register counts cost waves).
@@ -698,7 +790,7 @@ template <class Mark>
 void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, int report_fields, cudaStream_t s, Mark&& mark) {
     const int64_t arenas = b->env_count, cars = b->active_car_count;
     const int at = b->launch_threads, ct = b->car_threads;
-    const int car_blocks = spread_blocks(cars, 0, ct), wheel_blocks = spread_blocks(cars, 2, ct);
+    const int car_blocks = spread_blocks(cars, 0, ct);
     auto shift = [&](int64_t items, int warps) { return spread_shift(items, b->sms, warps); };
     mark();
     arena_begin_kernel<<<spread_blocks(arenas, 0, at), at, 0, s>>>(a, t);
@@ -707,8 +799,10 @@ void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, int rep
     mark();
     // phase 2 (timing) is the geometry and the vehicle updates
     if (cars) {
-        car_geometry_kernel<<<2 * wheel_blocks + car_blocks, ct, 0, s>>>(a, t, wheel_blocks, car_blocks);
-        car_vehicle_kernel<<<spread_blocks(cars, 2, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t);
+        const int lanes = spread_blocks(cars, 2, kGeometryThreads), each = spread_blocks(cars, 0, kGeometryThreads);
+        car_geometry_kernel<<<2 * lanes + each, kGeometryThreads, 0, s>>>(a, t, lanes, each);
+        const int order = spread_blocks(arenas, 2, kVehicleThreads);
+        car_vehicle_kernel<<<order + spread_blocks(cars, 2, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
     }
     mark();
     const int finish = shift(arenas, kWarpsFinish);

@@ -133,17 +133,29 @@ RG_HDI int car_triangle_query(const DevTri& t, const CarQueryFrame& f, float thr
 struct CarTriHit {
     V3 normal, raw_normal, point_b, raw_point_b;
     float distance;
-    bool hit;
+    uint32_t hit;
 };
-RG_HDI CarTriHit car_triangle_hit(V3 f, V3 r, V3 u, V3 pos_bt, const CarConfig& cfg, const DevTri& t, float thr) {
+// What the narrowphase reads of a car: its pose, and its box's offset, half extents and contact threshold.
+struct CarMeshPose {
+    V3 f, r, u, pos, offset, half;
+    float thr;
+};
+RG_HDI CarMeshPose car_mesh_pose(const CarState& c, const CarConfig& cfg) {
+    CarMeshPose p;
+    car_basis(c, p.f, p.r, p.u);
+    p.pos = c.pos_bt;
+    p.offset = cfg.hitbox_offset * (1.0f / 50.0f);
+    p.half = (bullet_hitbox_size(cfg) * 0.5f) * (1.0f / 50.0f);
+    p.thr = car_contact_threshold_bt(cfg);
+    return p;
+}
+RG_HDI CarTriHit car_triangle_hit(const CarMeshPose& c, const DevTri& t) {
     CarTriHit out;
-    out.hit = false;
+    out.hit = 0;
     float distance = 0.0f;
     V3 point_b{0.0f, 0.0f, 0.0f};
-    const V3 raw_half = (bullet_hitbox_size(cfg) * 0.5f) * (1.0f / 50.0f);
-    if (!gjk::box_triangle_contact(f, r, u, pos_bt, cfg.hitbox_offset * (1.0f / 50.0f), raw_half, t.a, t.b, t.c,
-                                   distance, point_b) ||
-        distance > thr)
+    if (!gjk::box_triangle_contact(c.f, c.r, c.u, c.pos, c.offset, c.half, t.a, t.b, t.c, distance, point_b) ||
+        distance > c.thr)
         return out;
     const V3 e1 = t.b - t.a, e2 = t.c - t.a;
     const V3 n{e1.y * e2.z - e1.z * e2.y, e1.z * e2.x - e1.x * e2.z, e1.x * e2.y - e1.y * e2.x};
@@ -156,7 +168,7 @@ RG_HDI CarTriHit car_triangle_hit(V3 f, V3 r, V3 u, V3 pos_bt, const CarConfig& 
     out.normal = normal;
     out.point_b = point_b;
     out.distance = distance;
-    out.hit = true;
+    out.hit = 1;
     return out;
 }
 
@@ -376,32 +388,28 @@ struct MeshContactEvents {
     V3 normal[4];
 };
 
-// The geometry of the car's contacts with the arena mesh for this tick: refresh the retained manifold, collect
-// candidates from the triangles the box overlaps and merge them into the manifold. It reads the car's pose and config
-// only, so it runs ahead of the car's vehicle update. The lanes of `lanes` share the triangles; lane 0 holds the
-// manifold and returns the last contact's triangle normal.
-template <class L>
-RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& cfg, CarWorldScratch& ws,
-                            const MeshDevice& mesh) {
-    const float thr = car_contact_threshold_bt(cfg);
-    V3 f, r, u;
-    car_basis(c, f, r, u);
-    const V3 pos = c.pos_bt;
+// The geometry of a car's contacts with the arena mesh for this tick: refresh the retained manifold, collect candidates
+// from the triangles the box overlaps, in leaf order, and merge them into the manifold. It reads the car's pose and
+// config only, so it runs ahead of the car's vehicle update.
+struct CarMeshManifold {
     MeshCandidate cand[4];
-    int n = 0;
     CarMeshPoint seeds[4];
+    int n;
+    bool seeded;
+    V3 last_normal;  // the last contact's triangle normal
+
     // retained points: distances refreshed at the current pose; points that drifted away leave
-    auto refresh = [&]() {
+    RG_HDI static void refresh(const CarMeshPose& c, CarWorldScratch& ws) {
         V3 wa[4], wb[4];
         for (int i = 0; i < ws.count; ++i) {
-            wa[i] = car_world_point(f, r, u, pos, ws.pts[i].local_a);
+            wa[i] = car_world_point(c.f, c.r, c.u, c.pos, ws.pts[i].local_a);
             wb[i] = ws.pts[i].local_b;
             ws.pts[i].distance = dot(wa[i] - wb[i], ws.pts[i].normal);
         }
         for (int i = ws.count - 1; i >= 0; --i) {
             const CarMeshPoint& p = ws.pts[i];
             const V3 pd = wb[i] - (wa[i] - p.normal * p.distance);
-            if (p.distance > thr || dot(pd, pd) > thr * thr) {
+            if (p.distance > c.thr || dot(pd, pd) > c.thr * c.thr) {
                 const int last = ws.count - 1;
                 if (i != last) {
                     ws.pts[i] = ws.pts[last];
@@ -411,19 +419,22 @@ RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& 
                 ws.count = last;
             }
         }
-    };
-    bool seeded = false;
-    if (lanes.lane() == 0 && ws.count > 0) {
-        refresh();
+    }
+    RG_HDI void begin(const CarMeshPose& c, CarWorldScratch& ws) {
+        n = 0;
+        seeded = false;
+        last_normal = V3{0.0f, 0.0f, 1.0f};
+        if (ws.count <= 0) return;
+        refresh(c, ws);
         for (int k = 0; k < ws.count; ++k) {
             const CarMeshPoint& p = ws.pts[k];
-            const V3 pwa = car_world_point(f, r, u, pos, p.local_a);
+            const V3 pwa = car_world_point(c.f, c.r, c.u, c.pos, p.local_a);
             MeshCandidate& m = cand[k];
             m.normal = p.normal;
             m.raw_normal = V3{0.0f, 0.0f, 1.0f};
             m.local_a = p.local_a;
             m.point_b = p.local_b;
-            m.rel_bt = pwa - pos;
+            m.rel_bt = pwa - c.pos;
             m.distance = p.distance;
             m.add_distance = p.distance;
             m.seed = k;
@@ -432,27 +443,22 @@ RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& 
         n = ws.count;
         seeded = true;
     }
-    V3 last_normal{0.0f, 0.0f, 1.0f};
-    const CarQueryFrame qf = car_query_frame(c, cfg);
-    auto test = [&](const DevTri& t, CarTriHit& h) {
-        if (car_triangle_query(t, qf, thr) != 2) return false;
-        h = car_triangle_hit(f, r, u, pos, cfg, t, thr);
-        return h.hit && !(h.distance > thr);
-    };
-    mesh_query_box_lanes<CarTriHit>(lanes, mesh, qf.lo, qf.hi, test, [&](const CarTriHit& h) {
+    // One triangle's narrowphase result, in leaf order.
+    RG_HDI void add(const CarMeshPose& c, const CarTriHit& h) {
+        if (!h.hit || h.distance > c.thr) return;
         MeshCandidate m;
         m.normal = h.normal;
         m.raw_normal = h.raw_normal;
         m.add_distance = h.distance;
         const V3 manifold_a = h.raw_point_b + h.raw_normal * h.distance;
-        m.local_a = car_local_point(f, r, u, pos, manifold_a);
+        m.local_a = car_local_point(c.f, c.r, c.u, c.pos, manifold_a);
         m.point_b = h.point_b;
-        const V3 ra = car_world_point(f, r, u, pos, m.local_a);
+        const V3 ra = car_world_point(c.f, c.r, c.u, c.pos, m.local_a);
         m.distance = dot(ra - m.point_b, m.normal);
-        m.rel_bt = ra - pos;
+        m.rel_bt = ra - c.pos;
         m.seed = -1;
         int merge = -1;
-        float shortest = thr * thr;
+        float shortest = c.thr * c.thr;
         for (int i = 0; i < n; ++i) {
             const V3 d = cand[i].local_a - m.local_a;
             const float dd = dot(d, d);
@@ -462,7 +468,7 @@ RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& 
             }
         }
         last_normal = h.raw_normal;
-        if (m.distance > thr) {
+        if (m.distance > c.thr) {
             if (merge >= 0) {
                 for (int i = merge; i + 1 < n; ++i) cand[i] = cand[i + 1];
                 --n;
@@ -478,26 +484,38 @@ RG_HDI V3 car_mesh_geometry(const L& lanes, const CarState& c, const CarConfig& 
             return;
         }
         cand[mesh_replace_index(cand, m)] = m;
-    });
-    if (lanes.lane() != 0) return last_normal;
-    // the manifold keeps this tick's candidates (seeded points carry over unchanged)
-    if (seeded) {
-        refresh();
-        ws.count = 0;
     }
-    for (int k = 0; k < n; ++k) {
-        if (seeded && cand[k].seed >= 0) {
-            ws.pts[ws.count++] = seeds[cand[k].seed];
-            continue;
+    // The manifold keeps this tick's candidates (seeded points carry over unchanged).
+    RG_HDI void finish(const CarMeshPose& c, CarWorldScratch& ws) {
+        if (seeded) {
+            refresh(c, ws);
+            ws.count = 0;
         }
-        CarMeshPoint p;
-        p.local_a = cand[k].local_a;
-        p.local_b = cand[k].point_b;
-        p.normal = cand[k].normal;
-        p.distance = dot(car_world_point(f, r, u, pos, p.local_a) - p.local_b, p.normal);
-        ws.pts[ws.count++] = p;
+        for (int k = 0; k < n; ++k) {
+            if (seeded && cand[k].seed >= 0) {
+                ws.pts[ws.count++] = seeds[cand[k].seed];
+                continue;
+            }
+            CarMeshPoint p;
+            p.local_a = cand[k].local_a;
+            p.local_b = cand[k].point_b;
+            p.normal = cand[k].normal;
+            p.distance = dot(car_world_point(c.f, c.r, c.u, c.pos, p.local_a) - p.local_b, p.normal);
+            ws.pts[ws.count++] = p;
+        }
     }
-    return last_normal;
+};
+// One car alone (car_geometry_kernel does eight at a time). Returns the last contact's triangle normal.
+RG_HDI V3 car_mesh_geometry(const CarState& c, const CarConfig& cfg, CarWorldScratch& ws, const MeshDevice& mesh) {
+    const CarMeshPose pose = car_mesh_pose(c, cfg);
+    const CarQueryFrame qf = car_query_frame(c, cfg);
+    CarMeshManifold m;
+    m.begin(pose, ws);
+    mesh_query_box(mesh, qf.lo, qf.hi, [&](const DevTri& t) {
+        if (car_triangle_query(t, qf, pose.thr) == 2) m.add(pose, car_triangle_hit(pose, t));
+    });
+    m.finish(pose, ws);
+    return m.last_normal;
 }
 
 // The contact rows of the manifold that car_mesh_geometry left, from the car's velocities as they stand now (body index

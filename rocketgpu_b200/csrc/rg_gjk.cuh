@@ -92,7 +92,7 @@ RG_HD V3 support_no_margin(const Shape& s, V3 d) {
     if (s.kind == kSphere) return V3{0.0f, 0.0f, 0.0f};
     const V3 dots{bdot(d, s.v[0]), bdot(d, s.v[1]), bdot(d, s.v[2])};
     const int ax = dots.x < dots.y ? (dots.y < dots.z ? 2 : 1) : (dots.x < dots.z ? 2 : 0);
-    return s.v[ax];
+    return ax == 0 ? s.v[0] : (ax == 1 ? s.v[1] : s.v[2]);
 }
 RG_HD V3 support_margin(const Shape& s, V3 d) {
     V3 n = d;
@@ -835,6 +835,9 @@ struct SubResult {
     RG_HD bool valid() const { return bc[0] >= 0.0f && bc[1] >= 0.0f && bc[2] >= 0.0f && bc[3] >= 0.0f; }
 };
 
+// The simplex lives in registers: every index is a constant once the loops are unrolled, and a vertex count picks by
+// comparison instead of by address (as arrays in local memory, a turn of the GJK loop spent most of its time on loads
+// and stores of them).
 struct VoronoiSimplex {
     int n;
     V3 w[4], p[4], q[4];
@@ -850,32 +853,44 @@ struct VoronoiSimplex {
         last_w = V3{1.0e18f, 1.0e18f, 1.0e18f};
         bc.reset();
         cp1 = cp2 = cv = V3{0.0f, 0.0f, 0.0f};
+        for (int i = 0; i < 4; ++i) w[i] = p[i] = q[i] = V3{0.0f, 0.0f, 0.0f};
     }
     RG_HD void add(V3 ww, V3 pp, V3 qq) {
         last_w = ww;
         needs_update = true;
-        w[n] = ww;
-        p[n] = pp;
-        q[n] = qq;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i != n) continue;
+            w[i] = ww;
+            p[i] = pp;
+            q[i] = qq;
+        }
         ++n;
     }
     RG_HD bool full() const { return n == 4; }
     RG_HD bool in_simplex(V3 ww) const {
-        for (int i = 0; i < n; ++i)
-            if (len2(w[i] - ww) <= 0.0001f) return true;
-        return ww.x == last_w.x && ww.y == last_w.y && ww.z == last_w.z;
+        bool in = ww.x == last_w.x && ww.y == last_w.y && ww.z == last_w.z;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) in = in || (i < n && len2(w[i] - ww) <= 0.0001f);
+        return in;
     }
-    RG_HD void remove_vertex(int i) {
+    // the last vertex takes vertex kAt's place
+    template <int kAt>
+    RG_HD void remove_vertex() {
         --n;
-        w[i] = w[n];
-        p[i] = p[n];
-        q[i] = q[n];
+#pragma unroll
+        for (int i = kAt + 1; i < 4; ++i) {
+            if (i != n) continue;
+            w[kAt] = w[i];
+            p[kAt] = p[i];
+            q[kAt] = q[i];
+        }
     }
     RG_HD void reduce(const SubResult& u) {
-        if (n >= 4 && !u.ud) remove_vertex(3);
-        if (n >= 3 && !u.uc) remove_vertex(2);
-        if (n >= 2 && !u.ub) remove_vertex(1);
-        if (n >= 1 && !u.ua) remove_vertex(0);
+        if (n >= 4 && !u.ud) remove_vertex<3>();
+        if (n >= 3 && !u.uc) remove_vertex<2>();
+        if (n >= 2 && !u.ub) remove_vertex<1>();
+        if (n >= 1 && !u.ua) remove_vertex<0>();
     }
     RG_HDI static void closest_triangle(V3 pt, V3 a, V3 b, V3 c, SubResult& r) {
         r.ua = r.ub = r.uc = r.ud = false;
@@ -941,72 +956,54 @@ struct VoronoiSimplex {
         if (signd * signd < (1.0e-4f * 1.0e-4f)) return -1;
         return signp * signd < 0.0f;
     }
-    RG_HDI static bool closest_tetra(V3 pt, V3 a, V3 b, V3 c, V3 d, SubResult& fin) {
-        SubResult t;
-        t.reset();
-        fin.closest = pt;
-        fin.ua = fin.ub = fin.uc = fin.ud = true;
-        const int oabc = outside_plane(pt, a, b, c, d);
-        const int oacd = outside_plane(pt, a, c, d, b);
-        const int oadb = outside_plane(pt, a, d, b, c);
-        const int obdc = outside_plane(pt, b, d, c, a);
-        if (oabc < 0 || oacd < 0 || oadb < 0 || obdc < 0) {
-            fin.degenerate = true;
-            return false;
+    // The closest point of the triangle (kTetra false: the first three vertices) or tetrahedron to the origin. One copy
+    // of closest_triangle serves the triangle and the tetrahedron's four faces (abc, acd, adb, bdc): lanes on different
+    // faces run the same instructions, and the loop's code stays small. Returns false when the origin is inside the
+    // tetrahedron or the tetrahedron is degenerate.
+    RG_HDI bool closest_faces(SubResult& fin) const {
+        const V3 pt{0.0f, 0.0f, 0.0f};
+        const V3 a = w[0], b = w[1], c = w[2], d = w[3];
+        unsigned faces = 1u;
+        if (n == 4) {
+            fin.closest = pt;
+            fin.ua = fin.ub = fin.uc = fin.ud = true;
+            faces = 0u;
+            bool degenerate = false;
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k) {
+                const V3 x = k == 3 ? b : a, y = k == 0 ? b : (k == 1 ? c : d);
+                const V3 z = k == 0 ? c : (k == 1 ? d : (k == 2 ? b : c));
+                const V3 o = k == 0 ? d : (k == 1 ? b : (k == 2 ? c : a));
+                const int out = outside_plane(pt, x, y, z, o);
+                degenerate = degenerate || out < 0;
+                faces |= out != 0 ? 1u << k : 0u;
+            }
+            if (degenerate) {
+                fin.degenerate = true;
+                return false;
+            }
+            if (faces == 0u) return false;
         }
-        if (!oabc && !oacd && !oadb && !obdc) return false;
         float best = 3.402823466e+38f;
-        if (oabc) {
-            closest_triangle(pt, a, b, c, t);
+#pragma unroll 1
+        for (; faces != 0u; faces &= faces - 1u) {
+            const int k = ctz32(faces);
+            const V3 x = k == 3 ? b : a, y = k == 0 ? b : (k == 1 ? c : d);
+            const V3 z = k == 0 ? c : (k == 1 ? d : (k == 2 ? b : c));
+            SubResult t;
+            closest_triangle(pt, x, y, z, t);
             const float sq = len2(t.closest - pt);
-            if (sq < best) {
-                best = sq;
-                fin.closest = t.closest;
-                fin.ua = t.ua;
-                fin.ub = t.ub;
-                fin.uc = t.uc;
-                fin.ud = false;
-                fin.set_bc(t.bc[0], t.bc[1], t.bc[2], 0.0f);
-            }
-        }
-        if (oacd) {
-            closest_triangle(pt, a, c, d, t);
-            const float sq = len2(t.closest - pt);
-            if (sq < best) {
-                best = sq;
-                fin.closest = t.closest;
-                fin.ua = t.ua;
-                fin.ub = false;
-                fin.uc = t.ub;
-                fin.ud = t.uc;
-                fin.set_bc(t.bc[0], 0.0f, t.bc[1], t.bc[2]);
-            }
-        }
-        if (oadb) {
-            closest_triangle(pt, a, d, b, t);
-            const float sq = len2(t.closest - pt);
-            if (sq < best) {
-                best = sq;
-                fin.closest = t.closest;
-                fin.ua = t.ua;
-                fin.ub = t.uc;
-                fin.uc = false;
-                fin.ud = t.ub;
-                fin.set_bc(t.bc[0], t.bc[2], 0.0f, t.bc[1]);
-            }
-        }
-        if (obdc) {
-            closest_triangle(pt, b, d, c, t);
-            const float sq = len2(t.closest - pt);
-            if (sq < best) {
-                best = sq;
-                fin.closest = t.closest;
-                fin.ua = false;
-                fin.ub = t.ua;
-                fin.uc = t.uc;
-                fin.ud = t.ub;
-                fin.set_bc(0.0f, t.bc[0], t.bc[2], t.bc[1]);
-            }
+            if (n == 4 && !(sq < best)) continue;
+            best = sq;
+            fin.closest = t.closest;
+            fin.ua = k != 3 && t.ua;
+            fin.ub = k == 0 ? t.ub : (k == 2 ? t.uc : (k == 3 && t.ua));
+            fin.uc = k == 0 || k == 3 ? t.uc : (k == 1 && t.ub);
+            fin.ud = k == 1 ? t.uc : (k >= 2 && t.ub);
+            fin.bc[0] = k == 3 ? 0.0f : t.bc[0];
+            fin.bc[1] = k == 0 ? t.bc[1] : (k == 1 ? 0.0f : (k == 2 ? t.bc[2] : t.bc[0]));
+            fin.bc[2] = k == 0 || k == 3 ? t.bc[2] : (k == 1 ? t.bc[1] : 0.0f);
+            fin.bc[3] = k == 0 ? 0.0f : (k == 1 ? t.bc[2] : t.bc[1]);
         }
         return true;
     }
@@ -1051,17 +1048,14 @@ struct VoronoiSimplex {
                     break;
                 }
                 case 3:
-                    closest_triangle(V3{0.0f, 0.0f, 0.0f}, w[0], w[1], w[2], bc);
-                    cp1 = p[0] * bc.bc[0] + p[1] * bc.bc[1] + p[2] * bc.bc[2];
-                    cp2 = q[0] * bc.bc[0] + q[1] * bc.bc[1] + q[2] * bc.bc[2];
-                    cv = cp1 - cp2;
-                    reduce(bc);
-                    valid_closest = bc.valid();
-                    break;
-                case 4: {
-                    if (closest_tetra(V3{0.0f, 0.0f, 0.0f}, w[0], w[1], w[2], w[3], bc)) {
-                        cp1 = p[0] * bc.bc[0] + p[1] * bc.bc[1] + p[2] * bc.bc[2] + p[3] * bc.bc[3];
-                        cp2 = q[0] * bc.bc[0] + q[1] * bc.bc[1] + q[2] * bc.bc[2] + q[3] * bc.bc[3];
+                case 4:
+                    if (closest_faces(bc)) {
+                        cp1 = p[0] * bc.bc[0] + p[1] * bc.bc[1] + p[2] * bc.bc[2];
+                        cp2 = q[0] * bc.bc[0] + q[1] * bc.bc[1] + q[2] * bc.bc[2];
+                        if (n == 4) {
+                            cp1 = cp1 + p[3] * bc.bc[3];
+                            cp2 = cp2 + q[3] * bc.bc[3];
+                        }
                         cv = cp1 - cp2;
                         reduce(bc);
                         valid_closest = bc.valid();
@@ -1072,7 +1066,6 @@ struct VoronoiSimplex {
                         cv = V3{0.0f, 0.0f, 0.0f};
                     }
                     break;
-                }
                 default: valid_closest = false; break;
             }
         }
@@ -1103,7 +1096,7 @@ RG_HD bool any_nan(V3 v) { return v.x != v.x || v.y != v.y || v.z != v.z; }
 // A car that the reference's EPA left NaN took 1,001 turns per triangle and per ball test, and the launch waited for its
 // one thread: wheel rays and vehicle updates of a tick 1,009 -> 292 us at 1,024 mixed arenas, 1,490 -> 1,099 us at
 // 16,384.
-RG_NOINL bool pair_detector(const Shape& a, const Xform& xa, const Shape& b, const Xform& xb, float max_dist_sq,
+RG_HDI bool pair_detector(const Shape& a, const Xform& xa, const Shape& b, const Xform& xb, float max_dist_sq,
                           V3& cached_axis, int& degenerate, float& squared_distance, V3& pa, V3& pb) {
     constexpr float kRelError2 = 1.0e-6f;
     if (any_nan(xa.o) || any_nan(xb.o)) return false;
@@ -1223,12 +1216,15 @@ RG_NOINL bool box_triangle_contact(V3 basis_f, V3 basis_r, V3 basis_u, V3 car_po
         Results r;
         V3 sep{0.0f, 0.0f, 0.0f}, wa{0.0f, 0.0f, 0.0f}, wb{0.0f, 0.0f, 0.0f};
         bool pen = false;
-        if (penetration(box, ta_x, tri, tb_x, guess, r)) {
+        // copies: what the out-of-line calls take by address must not pin the detector's operands to memory
+        const Shape pen_box = box, pen_tri = tri;
+        const Xform pen_a = ta_x, pen_b = tb_x;
+        if (penetration(pen_box, pen_a, pen_tri, pen_b, guess, r)) {
             wa = r.witness0;
             wb = r.witness1;
             sep = r.normal;
             pen = true;
-        } else if (distance(box, ta_x, tri, tb_x, guess, r)) {
+        } else if (distance(pen_box, pen_a, pen_tri, pen_b, guess, r)) {
             wa = r.witness0;
             wb = r.witness1;
             sep = r.normal;
@@ -1333,12 +1329,14 @@ RG_NOINL bool ball_box_contact(V3 cf, V3 cr, V3 cu, V3 car_pos_bt, V3 child_offs
         Results r;
         V3 sep{0.0f, 0.0f, 0.0f}, wa{0.0f, 0.0f, 0.0f}, wb{0.0f, 0.0f, 0.0f};
         bool pen = false;
-        if (penetration(box, xa, sphere, xb, guess, r)) {
+        const Shape pen_box = box, pen_sphere = sphere;  // copies, as in box_triangle_contact
+        const Xform pen_a = xa, pen_b = xb;
+        if (penetration(pen_box, pen_a, pen_sphere, pen_b, guess, r)) {
             wa = r.witness0;
             wb = r.witness1;
             sep = r.normal;
             pen = true;
-        } else if (distance(box, xa, sphere, xb, guess, r)) {
+        } else if (distance(pen_box, pen_a, pen_sphere, pen_b, guess, r)) {
             wa = r.witness0;
             wb = r.witness1;
             sep = r.normal;

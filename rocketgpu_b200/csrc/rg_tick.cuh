@@ -1241,10 +1241,12 @@ RG_HDI bool ball_car_box_overlaps(const BallState& b, const CarState& car, const
 // the ball's velocity, the other cars or the broadphase), nothing the arena does between the vehicle update and their
 // place in the world step changes what they read (car/car and car/ball contacts touch only the cars' contact
 // bookkeeping), and their effects on the car (the world-surface record, the contact normal) are applied by the arena
-// where the reference makes them. A car whose vehicle update must run in the arena's car order (arena_free_cars) has
-// its second part computed by the arena thread after all those updates.
-// Per wheel: its ray meets another car's box; the car's rays skip the ball (wheel_ray_excluded_bodies).
+// where the reference makes them. A car whose vehicle update must run in the arena's car order (arena_cars_met) has
+// its second part computed after all those updates (arena_cars_in_order).
+// Per wheel: its ray meets another car's box (the car's slot from bit kWheelMetShift); the car's rays skip the ball
+// (wheel_ray_excluded_bodies).
 constexpr uint8_t kWheelMeetsCar = 1, kWheelBallExcluded = 2;
+constexpr int kWheelMetShift = 2;
 struct CarStage {
     PreContactCar pre;
     V3 pred_n;
@@ -1256,7 +1258,7 @@ struct CarStage {
     CarStageRows rows;   // the query's rows, in the order it made them
     BpProxy proxy;       // the car's broadphase proxy (valid = 0 for a car demolished at the step's start)
     PadContacts pads;    // the car's pad contacts after its post-tick (pad_contacts_stage)
-    uint32_t in_car_thread;  // this tick's vehicle update and stage ran in the car's own thread (arena_free_cars)
+    uint32_t unused;
     RayHit wheel_mesh[4];    // the wheels' arena-mesh rays, cast ahead of the vehicle update (wheel_mesh_ray_ahead)
     uint8_t wheel_meets_car[4];  // kWheelMeetsCar, kWheelBallExcluded (0 for a demolished car)
     BallCarScratch ball_manifold;  // the car/ball manifold after this tick's geometry (car_ball_stage)
@@ -1305,20 +1307,14 @@ RG_HDI void car_proxy_ball_stage(const BallState& b, V3 ball_start_vel_bt, const
     st.ball_staged = 1u;
 }
 
-// The geometry of the car's arena contacts ahead of its vehicle update (car_mesh_geometry), by the lanes that share it.
-template <class L>
-RG_HDI void car_mesh_stage(const L& lanes, const CarState& car, const CarConfig& cfg, const CarWorldScratch& ws_in,
+// The geometry of one car's arena contacts ahead of its vehicle update (car_geometry_kernel does eight at a time).
+RG_HDI void car_mesh_stage(const CarState& car, const CarConfig& cfg, const CarWorldScratch& ws_in,
                            const MeshDevice& mesh, CarStage& st) {
-    const bool runs = !(car.is_demoed || car.just_respawned);
-    if (lanes.lane() == 0) st.mesh_ran = runs ? 1u : 0u;
-    if (!runs) return;
-    CarWorldScratch ws;
-    if (lanes.lane() == 0) ws = ws_in;
-    const V3 last_normal = car_mesh_geometry(lanes, car, cfg, ws, mesh);
-    if (lanes.lane() == 0) {
-        st.ws = ws;
-        st.res.latest_normal = last_normal;
-    }
+    st.mesh_ran = !(car.is_demoed || car.just_respawned) ? 1u : 0u;
+    if (!st.mesh_ran) return;
+    CarWorldScratch ws = ws_in;
+    st.res.latest_normal = car_mesh_geometry(car, cfg, ws, mesh);
+    st.ws = ws;
 }
 
 // The rest of the car's staged part, after its vehicle update.
@@ -1626,16 +1622,17 @@ RG_HDI void apply_ball_extra_hits(BallState& b, CarState* cars, int count, const
     if (any) ball_set_vel_bt(b, v);
 }
 
-// A tick of an arena with cars runs in six parts, so that each car's own work runs one thread per car:
+// A tick of an arena with cars runs in seven parts, so that each car's own work runs one thread per car:
 //   arena_tick_begin   (per arena)  this tick's env command, the game's vehicle order, the ball's tick start, pad timers;
 //   car_tick_pre       (per car)    the car's tick start (demolition timer and respawn, quantisation, controls, jumps);
-//   vehicle_update + car_stage_compute (per car, cars no other car's wheels can reach and whose wheels reach no other
-//                                   car, arena_free_cars)
-//                                   the vehicle update, then the car's prestep, predictive contact, broadphase proxy
-//                                   and mesh contact query (CarStage);
-//   arena_tick_finish  (per arena)  the other cars' vehicle updates in car order and their staged parts, the wheel
-//                                   pushes on the ball in car order, the world step's shared stages (manifold list,
-//                                   car/car, car/ball, ball/mesh contacts, the unified solves, the ball's
+//   car_mesh_stage, car_proxy_ball_stage, wheel_mesh_ray_ahead (per car or wheel)
+//                                   what reads only poses: the car's arena and ball contact geometry, its broadphase
+//                                   proxy, the wheels' rays (CarStage);
+//   vehicle_update + car_stage_compute (per car; cars whose wheels meet one another in the arena's car order,
+//                                   arena_cars_met)
+//                                   the vehicle update, then the car's prestep, predictive contact and contact rows;
+//   arena_tick_finish  (per arena)  the wheel pushes on the ball in car order, the world step's shared stages (manifold
+//                                   list, car/car, car/ball, ball/mesh contacts, the unified solves, the ball's
 //                                   integration);
 //   car_tick_post      (per car)    the car's integration and post-tick;
 //   arena_tick_tail    (per arena)  pads in car order, the driving countdown, extra ball hits, goal and timers.
@@ -1679,43 +1676,46 @@ RG_HDI void car_tick_pre(CarState& car, const CarControls& k, const CarConfig& c
     r.pushes.world_event = 0u;
 }
 
-// The cars of an arena whose vehicle update is independent of the other cars': no other car can be under one of its
-// wheel rays (each other car is demolished or excluded for its rays by the sweep-box rule, wheel_ray_excluded_bodies:
-// the reference never tests those) and it is under no other car's rays. Their updates (and their staged world-step
-// parts) run one thread per car; the other cars' updates run in the game's car order in the arena thread, because a
-// wheel that lands on another car pushes that car at once. Every thread of the arena evaluates this alike from the
-// cars' poses after their tick start, which no vehicle update changes.
-RG_HDI uint32_t arena_free_cars(const CarState* cars, const CarConfig* cfgs, const Broadphase& bp, int count) {
-    uint32_t reach[8];
-    uint32_t under = 0u;
-    for (int i = 0; i < count && i < 8; ++i) {
-        reach[i] = 0u;
-        if (cars[i].is_demoed) continue;
-        const uint32_t ex = wheel_ray_excluded_bodies(cars[i], cfgs[i], &bp, i, count);
-        for (int j = 0; j < count && j < 8; ++j)
-            if (j != i && !cars[j].is_demoed && !((ex >> (j + 1)) & 1u)) reach[i] |= 1u << j;
-        under |= reach[i];
-    }
-    uint32_t free = 0u;
-    for (int i = 0; i < count && i < 8; ++i)
-        if (reach[i] == 0u && !((under >> i) & 1u)) free |= 1u << i;
-    return free;
+// The arena's cars whose vehicle updates depend on one another, from the rays cast ahead: those with a wheel ray that
+// meets another car's box (the wheel may stand on that car and push it at once) and those met. Their updates run one
+// after another in the game's car order (arena_cars_in_order); no other car's update sees or changes another car, so the
+// rest run side by side. No vehicle update changes the poses, configs and demolition flags that the rays read.
+RG_HDI uint32_t arena_cars_met(const CarStage* stages, int count) {
+    uint32_t met = 0u;
+    for (int i = 0; i < count; ++i)
+        for (int w = 0; w < 4; ++w) {
+            const uint32_t m = stages[i].wheel_meets_car[w];
+            if (m & kWheelMeetsCar) met |= (1u << i) | (1u << (m >> kWheelMetShift));
+        }
+    return met;
 }
 
-// Whether any wheel ray of the arena's cars meets another car's box this tick (from the rays cast ahead). When none
-// does, no vehicle update pushes another car or sees one, and every car's update depends on the car alone.
-RG_HDI bool arena_wheels_meet_cars(const CarStage* stages, int count) {
-    uint32_t any = 0u;
-    for (int i = 0; i < count; ++i)
-        any |= stages[i].wheel_meets_car[0] | stages[i].wheel_meets_car[1] | stages[i].wheel_meets_car[2] |
-               stages[i].wheel_meets_car[3];
-    return (any & kWheelMeetsCar) != 0u;
+// The vehicle updates of the arena's cars in `which`, in the game's car order with their wheels seeing the other cars,
+// then their staged world-step parts (after every update: a later car's wheel may push an earlier one).
+template <class L>
+RG_HDI void arena_cars_in_order(const L& lanes, const EnvState& env, const BallState& b, const Broadphase& bp,
+                                const TickConfig& c, const MeshDevice& mesh, const ArenaCars& A, CarTickRecord* recs,
+                                CarStage* stages, uint32_t which, VehicleSlot& s) {
+    const int count = A.count;
+    for (int k = 0; k < count; ++k) {
+        const int i = car_visit_slot(env, k, count);
+        if (!((which >> i) & 1u)) continue;
+        vehicle_slot_load(lanes, s, A.cars + i, A.wheels + i, A.cfgs + i);
+        lanes.sync();
+        const uint32_t excluded = s.car.is_demoed ? 0u : wheel_ray_excluded_bodies(lanes, s.car, s.cfg, &bp, i, count);
+        vehicle_update(lanes, s.car, A.controls[i], s.cfg, c, s.wheels, b, mesh,
+                       WheelOthers{A.cars, A.cfgs, count, i, excluded}, recs[i].pushes, stages[i].wheel_mesh, s.tick);
+        lanes.sync();
+        vehicle_slot_store(lanes, s, A.cars + i, A.wheels + i);
+        lanes.sync();
+    }
+    for (int i = lanes.lane(); i < count; i += L::kLanes)
+        if ((which >> i) & 1u) car_stage_compute(A.cars[i], A.cfgs[i], A.wheels[i], c, mesh, i, stages[i]);
 }
 
 RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, Broadphase& bp, CarWorldScratch* cws,
                               BallCarScratch* bcs, const TickConfig& c, const MeshDevice& mesh, const ArenaCars& A,
                               CarTickRecord* recs, const ArenaTickSnap& as, CarStage* stages) {
-    // stages[i].in_car_thread: car i's vehicle update and staged parts ran in its own thread this tick
     const int count = A.count;
     int order[8];
     TickSnap snap;
@@ -1727,20 +1727,6 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
     }
     snap.ball_start_vel = as.ball_start_vel;
     snap.ball_vel_bt = as.ball_vel_bt;
-    // cars whose wheels may land on other cars: vehicle updates in the game's car order, wheels seeing other cars,
-    // then their staged world-step parts (after every update: a later car's wheel may push an earlier one)
-    uint32_t left = 0u;
-    for (int k = 0; k < count; ++k) {
-        const int i = order[k];
-        if (stages[i].in_car_thread) continue;
-        left |= 1u << i;
-        const uint32_t excluded = A.cars[i].is_demoed ? 0u : wheel_ray_excluded_bodies(A.cars[i], A.cfgs[i], &bp, i, count);
-        VehicleTick v;
-        vehicle_update(OneLane{}, A.cars[i], A.controls[i], A.cfgs[i], c, A.wheels[i], b, mesh,
-                       WheelOthers{A.cars, A.cfgs, count, i, excluded}, recs[i].pushes, stages[i].wheel_mesh, v);
-    }
-    for (int i = 0; i < count; ++i)
-        if ((left >> i) & 1u) car_stage_compute(A.cars[i], A.cfgs[i], A.wheels[i], c, mesh, i, stages[i]);
     if (c.events.windows) {
         // the vehicle updates' car-world events, in the game's car order (each update emits its own in the reference)
         for (int k = 0; k < count; ++k) {

@@ -270,7 +270,7 @@ RG_HDI bool wheel_ray_vs_ball(V3 src_bt, V3 dir, float max_len, const BallState&
     return true;
 }
 
-// The other cars of the arena a wheel ray may land on (null `cars`: none can be reached, see arena_free_cars),
+// The other cars of the arena a wheel ray may land on (null `cars`: it meets none, see arena_cars_met),
 // and the bodies (bit 0 the ball, bit i + 1 car slot i) the car's rays skip this tick (wheel_ray_excluded_bodies).
 struct WheelOthers {
     CarState* cars;
@@ -283,8 +283,10 @@ struct WheelOthers {
 // box around all four of the car's rays (reference WheelRayExcludedBodies with WheelRaysWhole,
 // raycast_wheels_and_contact_prep.hpp:9-25, 508-606, as StepEnvVehicleUpdateCarInline calls it, env_step.hpp:6232).
 // The ball is body 0, car slot i body i + 1; bodies without a stored box (not yet swept, or left the sweep) are tested.
-RG_HDI uint32_t wheel_ray_excluded_bodies(const CarState& c, const CarConfig& cfg, const Broadphase* bp, int self,
-                                          int count) {
+// The lanes of `lanes` hold the same car: with four, each takes a wheel's ray and a share of the bodies.
+template <class L>
+RG_HDI uint32_t wheel_ray_excluded_bodies(const L& lanes, const CarState& c, const CarConfig& cfg,
+                                          const Broadphase* bp, int self, int count) {
     const int bodies = count + 1 < kBpBodies ? count + 1 : kBpBodies;
     const uint32_t mask = (bp != nullptr && bodies > 0)
                               ? (bp->body_aabb_valid & ((1u << bodies) - 1u) & ~(1u << (self + 1)))
@@ -300,25 +302,37 @@ RG_HDI uint32_t wheel_ray_excluded_bodies(const CarState& c, const CarConfig& cf
         ((oz - front_bone) * kUuToBt + cfg.front_wheel_radius * kUuToBt) + ((14.5f - kWheelSuspensionSubtraction) * kUuToBt);
     const float back_len_bt =
         ((oz - back_bone) * kUuToBt + cfg.back_wheel_radius * kUuToBt) + ((14.5f - kWheelSuspensionSubtraction) * kUuToBt);
-    V3 mn{0.0f, 0.0f, 0.0f}, mx{0.0f, 0.0f, 0.0f};
-    for (int i = 0; i < 4; ++i) {
+    auto ray_box = [&](int i, V3& lo, V3& hi) {
         V3 offset = i < 2 ? cfg.front_wheels_offset : cfg.back_wheels_offset;
         if (i % 2) offset.y = -offset.y;
         offset.z = oz;
         const V3 from = c.pos_bt + rotate_via_basis(fw, rt, up, offset * kUuToBt);
         const V3 to = from + dir * (i < 2 ? front_len_bt : back_len_bt);
-        const V3 lo = vmin(from, to), hi = vmax(from, to);
+        lo = vmin(from, to);
+        hi = vmax(from, to);
+    };
+    V3 mn{0.0f, 0.0f, 0.0f}, mx{0.0f, 0.0f, 0.0f};
+    V3 own_lo, own_hi;
+    if (L::kLanes == 4) ray_box(lanes.lane(), own_lo, own_hi);
+    for (int i = 0; i < 4; ++i) {
+        V3 lo, hi;
+        if (L::kLanes == 4) {
+            lo = lanes.from(own_lo, i);
+            hi = lanes.from(own_hi, i);
+        } else {
+            ray_box(i, lo, hi);
+        }
         mn = i == 0 ? lo : vmin(mn, lo);
         mx = i == 0 ? hi : vmax(mx, hi);
     }
     uint32_t excluded = 0u;
-    for (int body = 0; body < bodies; ++body) {
+    for (int body = lanes.lane(); body < bodies; body += L::kLanes) {
         if (!((mask >> body) & 1u)) continue;
         const float* a = bp->body_aabb[body];
         if (a[3] < mn.x || mx.x < a[0] || a[4] < mn.y || mx.y < a[1] || a[5] < mn.z || mx.z < a[2])
             excluded |= 1u << body;
     }
-    return excluded;
+    return lanes.any(excluded);
 }
 
 // Distance from a point to a car's hitbox (core box plus margin) by Bullet's GJK pair detector with the Voronoi
@@ -1396,8 +1410,8 @@ RG_HDI void vehicle_end(CarState& c, const TickConfig& tc, WheelRuntime& wr, Veh
 // The vehicle update of one car. The lanes of `lanes` hold the same car, `wr` and `v` in memory they share; with four
 // lanes each takes a wheel (its ray, drive, suspension and tyre terms, which depend on no other wheel), and lane 0 alone
 // everything else, the wheels' sums in the reference's wheel order (1, 0, 3, 2) among it. `mesh_hits`: the four wheels'
-// arena-mesh rays cast ahead (wheel_mesh_ray_ahead), or null to cast them here. `oth` may name cars only with one lane
-// (a wheel on another car pushes it at once, in wheel order).
+// arena-mesh rays cast ahead (wheel_mesh_ray_ahead), or null to cast them here. Wheels that land on other cars (`oth`)
+// push them after all four rays, in wheel order: a push changes the other car's velocity, which no ray reads.
 template <class L>
 RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw, const CarConfig& cfg,
                            const TickConfig& tc, WheelRuntime& wr, const BallState& ball, const MeshDevice& mesh,
@@ -1422,9 +1436,15 @@ RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw
     lanes.sync();
     each_wheel([&](int i, WheelStep& w) {
         vehicle_wheel_cast(c, cfg, tc, wr, ball, mesh, oth, mesh_hits, v, i, w);
-        if (L::kLanes == 1) vehicle_wheel_on_car(c, cfg, tc, oth, w);
-        vehicle_wheel_share(wr, v, i, w);
     });
+    if (oth.cars) {
+        for (int kk = 0; kk < 4; ++kk) {
+            const int i = kk ^ 1;
+            if (kOwn == 4 || lanes.lane() == i) vehicle_wheel_on_car(c, cfg, tc, oth, wh[kOwn == 1 ? 0 : i]);
+            lanes.sync();
+        }
+    }
+    each_wheel([&](int i, WheelStep& w) { vehicle_wheel_share(wr, v, i, w); });
     lanes.sync();
     if (first) vehicle_contacts(c, cfg, tc, wr, v, pushes);
     lanes.sync();
@@ -1451,6 +1471,50 @@ RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw
     lanes.sync();
 }
 
+// One car's structs and its update's scratch while lanes work on them (shared memory on the device).
+struct alignas(16) VehicleSlot {
+    CarState car;
+    WheelRuntime wheels;
+    alignas(8) CarConfig cfg;
+    VehicleTick tick;
+};
+// The words that copies move: 16 bytes for the car, 4 for the wheel record (292 bytes), 8 for the config (120 bytes).
+struct alignas(16) Word16 {
+    uint32_t w[4];
+};
+struct alignas(8) Word8 {
+    uint32_t w[2];
+};
+static_assert(offsetof(VehicleSlot, car) % 16 == 0 && offsetof(VehicleSlot, cfg) % 8 == 0, "aligned copies");
+
+// A struct copied by the lanes of a group, word l, l + kLanes, ... by lane l.
+template <class Word, class L, class T>
+RG_HDI void lanes_copy(const L& lanes, T* dst, const T* src) {
+    static_assert(sizeof(T) % sizeof(Word) == 0, "whole words: every struct of an array is aligned to one");
+    constexpr int kWords = sizeof(T) / sizeof(Word), kRounds = (kWords + L::kLanes - 1) / L::kLanes;
+    const Word* s = reinterpret_cast<const Word*>(src);
+    Word* d = reinterpret_cast<Word*>(dst);
+    Word w[kRounds];
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i)
+        if (L::kLanes * i + lanes.lane() < kWords) w[i] = s[L::kLanes * i + lanes.lane()];
+#pragma unroll
+    for (int i = 0; i < kRounds; ++i)
+        if (L::kLanes * i + lanes.lane() < kWords) d[L::kLanes * i + lanes.lane()] = w[i];
+}
+template <class L>
+RG_HDI void vehicle_slot_load(const L& lanes, VehicleSlot& s, const CarState* car, const WheelRuntime* wheels,
+                              const CarConfig* cfg) {
+    lanes_copy<Word16>(lanes, &s.car, car);
+    lanes_copy<uint32_t>(lanes, &s.wheels, wheels);
+    lanes_copy<Word8>(lanes, &s.cfg, cfg);
+}
+template <class L>
+RG_HDI void vehicle_slot_store(const L& lanes, const VehicleSlot& s, CarState* car, WheelRuntime* wheels) {
+    lanes_copy<Word16>(lanes, car, &s.car);
+    lanes_copy<uint32_t>(lanes, wheels, &s.wheels);
+}
+
 // ---- world step: the car's external forces and integration (reference env_step.hpp:3737-3806,
 // host_validation_and_contact_debug.hpp:971-1022) ------------------------------------------------------------------
 struct PreContactCar {
@@ -1460,10 +1524,10 @@ struct PreContactCar {
 };
 // Wheel `i`'s arena-mesh ray as the car's vehicle update casts it (the same wheel set-up from the car's pose and
 // config), for running the rays of every car ahead of the updates, one thread per wheel.
-// Also reports whether the ray meets another car's box (`oth`: the arena's cars with this car's broadphase
-// exclusions), which is when the update can push that car and must run in the arena's car order.
+// Also reports the slot of the car whose box the ray meets first, or -1 (`oth`: the arena's cars with this car's
+// broadphase exclusions): the update may push that car and must run in the arena's car order.
 RG_HDI void wheel_mesh_ray_ahead(const CarState& c, const CarConfig& cfg, const MeshDevice& mesh, int i,
-                                 const WheelOthers& oth, RayHit& hit, uint8_t& meets_car) {
+                                 const WheelOthers& oth, RayHit& hit, int& met_car) {
     CarFrame f;
     car_basis(c, f.fwd, f.right, f.up);
     float front_bone, back_bone;
@@ -1476,7 +1540,7 @@ RG_HDI void wheel_mesh_ray_ahead(const CarState& c, const CarConfig& cfg, const 
     int best_idx;
     bool best_nr;
     wheel_ray_vs_cars(w, min_hit_dist_sq, oth, best, best_idx, best_nr);
-    meets_car = best.hit ? 1 : 0;
+    met_car = best.hit ? best_idx : -1;
 }
 
 RG_HDI void car_world_prestep(CarState& c, const CarConfig& cfg, const WheelRuntime& wr, const TickConfig& tc,

@@ -175,16 +175,18 @@ void hp_step(const HostBatch* b, const rg_sim_config* cfg, const float* vertices
             }
             for (int i = 0; i < count; ++i) {
                 rg::CarStage& st = stages[i];
-                rg::car_mesh_stage(rg::OneLane{}, A.cars[i], A.cfgs[i], b->car_world[base + i], m, st);
+                rg::car_mesh_stage(A.cars[i], A.cfgs[i], b->car_world[base + i], m, st);
                 rg::car_proxy_ball_stage(ball, snap.ball_vel_bt, A.cars[i], A.cfgs[i], tc, recs[i].vel_bt,
                                          recs[i].ang_vel, b->ball_car[base + i], st);
-                st.in_car_thread = 0;  // every vehicle update in the arena's car order
                 for (int w = 0; w < 4 && !A.cars[i].is_demoed; ++w) {
-                    uint8_t meets;
+                    int met;
                     rg::wheel_mesh_ray_ahead(A.cars[i], A.cfgs[i], m, w, rg::WheelOthers{nullptr, nullptr, 0, i, 0u},
-                                             st.wheel_mesh[w], meets);
+                                             st.wheel_mesh[w], met);
                 }
             }
+            rg::VehicleSlot slot;  // every vehicle update in the arena's car order
+            rg::arena_cars_in_order(rg::OneLane{}, env, ball, b->broadphase[e], tc, m, A, recs.data(), stages.data(),
+                                    (1u << count) - 1u, slot);
             rg::arena_tick_finish(env, ball, b->ball_world[e], b->broadphase[e], b->car_world + base,
                                   b->ball_car + base, tc, m, A, recs.data(), snap, stages.data());
             for (int i = 0; i < count; ++i)
