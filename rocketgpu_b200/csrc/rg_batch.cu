@@ -225,25 +225,27 @@ __global__ void canonicalize_balls_kernel(rg::BallState* balls, int n) {
     b.deactivation_time = 0.0f;
 }
 
-// A kernel with one thread per arena or car leaves idle lanes between them when the chip has room for more warps than
-// they fill: item k runs in thread k << shift, so that a warp holds fewer items, diverges less and touches fewer lines
-// per access. The shift is the largest, up to one item per warp, whose warps are all resident at once (`warps_per_sm`:
-// by the kernel's registers). Measured, us a tick at shift 0 and by this rule: the arena finish 171 -> 148 at 1,024 mixed
-// arenas, 541 -> 475 at 4,095 3v3 arenas, 397 -> 382 at 16,384 mixed ones (one item in two threads there); the tail 41 ->
-// 31, 55 -> 46, 62 -> 56; the post-tick 47 -> 41, 56 -> 51, 73 -> 71; 16,384 ball-only arenas 2,907 -> 2,279 us a 60-tick
-// pass. The car tick start lost (27 -> 48 at 1,024): its local copies of the structs then use 4 of each 32-byte sector;
-// the arena begin gained nothing. Those two run one item per thread.
+// A kernel with one thread per arena or car gives a warp fewer items, 32 >> shift, when the chip has room for more warps
+// than full ones would be, so that a warp diverges less and touches fewer lines per access. The shift is the largest, up
+// to one item per warp, whose warps are all resident at once (`warps_per_sm`: by the kernel's registers). The items take
+// the warp's first lanes: local memory interleaves its lanes by words, and items spread over the warp would use a part of
+// each 32-byte sector. Measured, us a tick with full warps and by this rule: the arena finish 171 -> 130 at 1,024 mixed
+// arenas, 541 -> 450 at 4,095 3v3 arenas, 397 -> 330 at 16,384 mixed ones; the tail 41 -> 28, 55 -> 45, 62 -> 54; the
+// post-tick 47 -> 39, 56 -> 51, 73 -> 71; 16,384 ball-only arenas 2,907 -> 2,279 us a 60-tick pass. The car tick start
+// lost (27 -> 44 at 1,024), the arena begin gained nothing: one item per thread in these two.
 __device__ __forceinline__ int spread_item(int shift) {
-    const int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    return (g & ((1 << shift) - 1)) != 0 ? 0x7fffffff : g >> shift;
+    const int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), per = 32 >> shift;
+    return (g & 31) < per ? (g >> 5) * per + (g & 31) : 0x7fffffff;
 }
 int spread_shift(int64_t items, int sms, int warps_per_sm) {
     int shift = 0;
     while (shift < 5 && ((items << (shift + 1)) + 31) / 32 <= static_cast<int64_t>(sms) * warps_per_sm) ++shift;
     return shift;
 }
+int blocks_for(int64_t items, int threads) { return static_cast<int>((items + threads - 1) / threads); }
 int spread_blocks(int64_t items, int shift, int threads) {
-    return static_cast<int>(((items << shift) + threads - 1) / threads);
+    const int64_t warps = ((items << shift) + 31) / 32;
+    return static_cast<int>((32 * warps + threads - 1) / threads);
 }
 // Resident warps per SM of the spread kernels, from their registers per thread (65,536 per SM).
 constexpr int kWarpsBalls = 16, kWarpsFinish = 8, kWarpsPost = 32, kWarpsTail = 8;
@@ -529,7 +531,8 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
         if (first) {
             w.pose[group] = pose;
             w.tris[group] = tris;
-            ws = a.car_world[idx];
+            ws.count = a.car_world[idx].count;
+            if (ws.count != 0) ws = a.car_world[idx];
             m.begin(pose, ws);
         }
     }
@@ -584,7 +587,10 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
     if (runs && first) {
         m.finish(pose, ws);
         rg::CarStage& st = a.stages[idx];
-        st.ws = ws;
+        if (ws.count != 0)
+            st.ws = ws;
+        else
+            st.ws.count = 0;
         st.res.latest_normal = m.last_normal;
     }
 }
@@ -694,9 +700,8 @@ __global__ void __launch_bounds__(kVehicleThreads, 8)
 }
 
 // Tick part 4, one thread per arena in step order: wheel pushes on the ball, then the world step's shared stages.
-// One thread per arena fills a single wave at any batch this path runs, so these two kernels take the registers that
-// remove most of their spills (measured at 16,384 mixed arenas: the finish 4.09 -> 3.91 ms per 8-tick step; the car
-// kernels lost time under the same change, their spill-free register counts cost waves).
+// The registers (255) are the ones that remove the spills. Bringing the sweep history (1.4 KB per arena) into shared memory
+// first, by the whole warp, was slower: 333 against 299 us at 16,384 mixed arenas, for the L1 that local memory lost.
 __global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
     const int k = spread_item(shift);
     if (k >= a.base.env_count) return;
@@ -790,19 +795,19 @@ template <class Mark>
 void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, int report_fields, cudaStream_t s, Mark&& mark) {
     const int64_t arenas = b->env_count, cars = b->active_car_count;
     const int at = b->launch_threads, ct = b->car_threads;
-    const int car_blocks = spread_blocks(cars, 0, ct);
+    const int car_blocks = blocks_for(cars, ct);
     auto shift = [&](int64_t items, int warps) { return spread_shift(items, b->sms, warps); };
     mark();
-    arena_begin_kernel<<<spread_blocks(arenas, 0, at), at, 0, s>>>(a, t);
+    arena_begin_kernel<<<blocks_for(arenas, at), at, 0, s>>>(a, t);
     mark();
     if (cars) car_pre_kernel<<<car_blocks, ct, 0, s>>>(a, t);
     mark();
     // phase 2 (timing) is the geometry and the vehicle updates
     if (cars) {
-        const int lanes = spread_blocks(cars, 2, kGeometryThreads), each = spread_blocks(cars, 0, kGeometryThreads);
+        const int lanes = blocks_for(4 * cars, kGeometryThreads), each = blocks_for(cars, kGeometryThreads);
         car_geometry_kernel<<<2 * lanes + each, kGeometryThreads, 0, s>>>(a, t, lanes, each);
-        const int order = spread_blocks(arenas, 2, kVehicleThreads);
-        car_vehicle_kernel<<<order + spread_blocks(cars, 2, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
+        const int order = blocks_for(4 * arenas, kVehicleThreads);
+        car_vehicle_kernel<<<order + blocks_for(4 * cars, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
     }
     mark();
     const int finish = shift(arenas, kWarpsFinish);

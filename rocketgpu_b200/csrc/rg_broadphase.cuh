@@ -72,6 +72,16 @@ struct BpProxy {
     uint8_t valid, is_ball;
 };
 
+// The bodies' proxies where they lie: the ball's, and car slot i's at byte offset i * stride from the first car's.
+struct BpProxies {
+    const BpProxy* ball;
+    const unsigned char* cars;
+    size_t stride;
+    RG_HD const BpProxy& operator[](int body) const {
+        return body == 0 ? *ball : *reinterpret_cast<const BpProxy*>(cars + static_cast<size_t>(body - 1) * stride);
+    }
+};
+
 RG_HD uint16_t sweep_quantize(float v, int is_max) {
     const float q = 65535.0f / (kSweepHalfExtentBt + kSweepHalfExtentBt);
     float s = (v + kSweepHalfExtentBt) * q;
@@ -351,7 +361,7 @@ struct Sweep {
     }
     // Bodies of a fresh sweep enter together: their edges are merged into the static edges, then each pair with a
     // static or an earlier body is found by scanning the last axis (reference add_bodies_merged).
-    RG_HDI void add_bodies_merged(const BpProxy* proxies) {
+    RG_HDI void add_bodies_merged(const BpProxies& proxies) {
         uint8_t new_handle[kBpBodies], new_body[kBpBodies];
         uint16_t q[kBpBodies][2][3];
         const int old_count = 2 * h.handle_count + 2;
@@ -442,7 +452,7 @@ struct Sweep {
         }
     }
     // Each body's swept AABB moves its edges; crossings update the pairs (reference update_aabbs).
-    RG_HDI void update_aabbs(const BpProxy* proxies) {
+    RG_HDI void update_aabbs(const BpProxies& proxies) {
         for (int o = 0; o < h.obj_count; ++o) {
             const int body = h.obj[o];
             if (body >= body_count) continue;
@@ -495,7 +505,7 @@ struct BpEntry {
 // `mesh_max`: the arena mesh's bounds (Bullet units); `pred_mask`: bodies with a predictive contact this tick;
 // `ball_static_skipped`: the ball sleeps, so its static pairs make no new manifold. Fills `out` (sorted) and returns
 // its length.
-RG_NOINL int bp_build_manifold_list(Broadphase& h, const BpProxy* proxies, int body_count, V3 mesh_min, V3 mesh_max,
+RG_NOINL int bp_build_manifold_list(Broadphase& h, const BpProxies& proxies, int body_count, V3 mesh_min, V3 mesh_max,
                                   uint32_t pred_mask, bool ball_static_skipped, BpEntry* out) {
     Sweep s{h, body_count};
     const bool fresh = h.handle_count == 0;

@@ -630,16 +630,6 @@ RG_HDI V3 car_pre_tick(CarState& c, const CarControls& k, const CarConfig& cfg, 
 }
 
 // ---- the world step of an arena with cars ------------------------------------------------------------------------
-// Per-tick snapshots the world step needs from the tick start: the velocities the broadphase predicts motion with
-// (reference car_predict_vel_bt / ball_predict_vel_bt, env_step.hpp:6847-6851, 6884).
-struct TickSnap {
-    V3 ball_vel_bt;
-    V3 car_vel_bt[8], car_ang_vel[8];
-    // uu velocities right after the tick-start quantisation, for the ball-hit impulse (reference cal_start_vel /
-    // cal_ball_start_vel)
-    V3 car_start_vel[8], ball_start_vel;
-};
-
 // The car's predictive (CCD) contact: its box centre's motion this tick (reference PredictiveContactRayForBody
 // body > 0, env_step.hpp:3930-4060; the free-box shortcuts there only skip rays that cannot hit).
 RG_HDI bool car_predictive_hit(const CarState& c, const CarConfig& cfg, const MeshDevice& m, float dt, V3& n,
@@ -1336,6 +1326,17 @@ RG_HDI void car_stage_compute(CarState& car, const CarConfig& cfg, const WheelRu
     st.res = res;
 }
 
+// What the world step needs from one car's tick start and vehicle update.
+struct CarTickRecord {
+    V3 start_vel;  // uu velocity right after the tick-start quantisation (ball-hit impulse)
+    V3 vel_bt, ang_vel;  // velocities the broadphase predicts motion with
+    WheelBallPushes pushes;
+};
+// The ball's velocities at the tick start.
+struct ArenaTickSnap {
+    V3 ball_start_vel, ball_vel_bt;
+};
+
 // One arena's world step with cars (reference WorldStepSoccar, env_step.hpp:4727-5623, on the path a custom-mesh
 // soccar arena takes): predictive rays, the broadphase's manifold list, the ball's and the cars' arena contacts, the
 // unified velocity and position solves, then integration; car-ball contacts (reference env_step.hpp:5045-5133)
@@ -1343,7 +1344,7 @@ RG_HDI void car_stage_compute(CarState& car, const CarConfig& cfg, const WheelRu
 // manifold list here.
 RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp, CarWorldScratch* cws,
                             BallCarScratch* bcs, const TickConfig& c, const MeshDevice& mesh, const ArenaCars& A,
-                            PreContactCar* pre, const TickSnap& snap, uint64_t env_tick,
+                            const CarTickRecord* recs, const ArenaTickSnap& snap, uint64_t env_tick,
                             const CarStage* stages) {
     const int count = A.count;
     const float sub_dt = c.tick_dt;
@@ -1352,16 +1353,12 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
     const bool ball_sleeping = ball_resolve_activation(b);
     if (vehicle_woke) b.deactivation_time = 0.0f;
     const V3 ext_delta = ball_sleeping ? V3{0.0f, 0.0f, 0.0f} : V3{0.0f, 0.0f, c.gravity_z * sub_dt};
-    for (int i = 0; i < count; ++i) pre[i] = stages[i].pre;
     const V3 solver_vel_bt = b.vel_bt;
-    // where the bodies stand at the step's start, for the ball-hit records (reference record_ball_car_info)
+    // where the bodies stand at the step's start, for the ball-hit records (reference record_ball_car_info); the cars'
+    // are kept only when car pairs may rewrite them
     const V3 hit_ball_pos = b.pos;
     V3 hit_car_pos[8];
     Q4 hit_car_rot[8];
-    for (int i = 0; i < count && i < 8; ++i) {
-        hit_car_pos[i] = A.cars[i].pos;
-        hit_car_rot[i] = A.cars[i].rot;
-    }
     const bool awake = !ball_sleeping || vehicle_woke;
     // predictive contacts (reference ComputePredictiveContactHits, env_step.hpp:4129-4168)
     const int body_count = count + 1 < kBpBodies ? count + 1 : kBpBodies;
@@ -1370,21 +1367,16 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
     float pred_d[kBpBodies];
     if (!(ball_sleeping && !vehicle_woke) && ball_predictive_hit(b, mesh, sub_dt, pred_n[0], pred_d[0])) pred_mask |= 1u;
     for (int i = 0; i + 1 < body_count; ++i) {
-        if (pre[i].is_demoed || !stages[i].pred_hit) continue;
+        if (!stages[i].pred_hit) continue;  // among them cars demolished at the step's start
         pred_n[i + 1] = stages[i].pred_n;
         pred_d[i + 1] = stages[i].pred_d;
         pred_mask |= 1u << (i + 1);
     }
     // broadphase proxies and the manifold list (reference BuildBulletManifoldList + SortBulletManifoldListByIsland)
-    BpProxy proxies[kBpBodies];
-    ball_proxy(proxies[0], b.pos_bt, snap.ball_vel_bt, c.ball_radius, sub_dt);
-    for (int i = 0; i + 1 < body_count; ++i) {
-        BpProxy& p = proxies[i + 1];
-        if (pre[i].is_demoed)
-            p.valid = 0;
-        else
-            p = stages[i].proxy;
-    }
+    // (a car demolished at the step's start has no valid proxy)
+    BpProxy ball_body;
+    ball_proxy(ball_body, b.pos_bt, snap.ball_vel_bt, c.ball_radius, sub_dt);
+    const BpProxies proxies{&ball_body, reinterpret_cast<const unsigned char*>(&stages[0].proxy), sizeof(CarStage)};
     BpEntry list[kBpMaxEntries];
     const int n_list = bp_build_manifold_list(bp, proxies, body_count, mesh.aabb_min, mesh.aabb_max, pred_mask,
                                               ball_sleeping && !vehicle_woke, list);
@@ -1398,6 +1390,10 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
         const int pc = count < 8 ? count : 8;
         const uint32_t all = pc >= 2 ? (1u << (pc * (pc - 1) / 2)) - 1u : 0u;
         if ((reject & all) != all) {
+            for (int i = 0; i < count && i < 8; ++i) {
+                hit_car_pos[i] = A.cars[i].pos;
+                hit_car_rot[i] = A.cars[i].rot;
+            }
             int8_t oi[28], oj[28];
             int no = 0;
             uint32_t listed = 0u;
@@ -1434,8 +1430,9 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
                 const bool i_body0 = bp.body_handle[i + 1] <= bp.body_handle[j + 1];
                 const int a = i_body0 ? j : i, b2 = i_body0 ? i : j;
                 car_car_resolve(A.cars[a], static_cast<uint32_t>(A.car_base + a + 1), A.teams[a], A.cfgs[a], A.cars[b2],
-                                static_cast<uint32_t>(A.car_base + b2 + 1), A.teams[b2], A.cfgs[b2], c, pre[a], pre[b2],
-                                snap.car_start_vel[a], snap.car_start_vel[b2], a, b2, A.pairs[car_pair_slot(i, j)], pr);
+                                static_cast<uint32_t>(A.car_base + b2 + 1), A.teams[b2], A.cfgs[b2], c, stages[a].pre,
+                                stages[b2].pre,
+                                recs[a].start_vel, recs[b2].start_vel, a, b2, A.pairs[car_pair_slot(i, j)], pr);
             }
         }
     }
@@ -1452,7 +1449,7 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
         // (reference BallCarRetainedPairOverlaps, triangle_and_carcar.hpp:1658-1698)
         const bool overlaps =
             ((car_car_touched >> i) & 1u)
-                ? ball_car_box_overlaps(b, car, A.cfgs[i], c, pre[i].is_demoed == 0)
+                ? ball_car_box_overlaps(b, car, A.cfgs[i], c, stages[i].pre.is_demoed == 0)
                 : (i + 1 < body_count && pc.valid != 0 && !car.just_respawned &&
                    !(pc.child_min.x > pb.child_max.x || pc.child_max.x < pb.child_min.x ||
                      pc.child_min.y > pb.child_max.y || pc.child_max.y < pb.child_min.y ||
@@ -1467,10 +1464,11 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
         } else {
             ball_car_contacts(bcs[i], b, car, A.cfgs[i], c, i, ext_delta, solver_vel_bt, sub_dt, bc);
         }
-        if (!pre[i].is_demoed && !car.just_respawned)
+        if (!stages[i].pre.is_demoed && !car.just_respawned)
             commit_ball_hit_from_manifold(b, car, bcs[i], static_cast<uint32_t>(A.car_base + i + 1), env_tick,
-                                          hit_car_pos[i], hit_car_rot[i], hit_ball_pos, snap.car_start_vel[i],
-                                          snap.ball_start_vel, A.teams[i], c.events);
+                                          car_car_touched != 0u ? hit_car_pos[i] : car.pos,
+                                          car_car_touched != 0u ? hit_car_rot[i] : car.rot, hit_ball_pos,
+                                          recs[i].start_vel, snap.ball_start_vel, A.teams[i], c.events);
     }
     // the ball's arena contacts (reference env_step.hpp:5219-5290): a sleeping ball a car touched is awake now,
     // and looks at the arena when it still holds arena contact points
@@ -1484,7 +1482,7 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
     cr.nv = cr.nf = cr.ns = 0;
     for (int i = 0; i < count; ++i) {
         CarState& car = A.cars[i];
-        if (pre[i].is_demoed || car.just_respawned) {
+        if (stages[i].pre.is_demoed || car.just_respawned) {
             cws[i].count = 0;
             continue;
         }
@@ -1496,6 +1494,10 @@ RG_NOINL void world_step_cars(BallState& b, BallWorldScratch& s, Broadphase& bp,
         if (!listed && cws[i].count == 0) continue;
         if (!listed) {
             cws[i].count = 0;  // what the query does for an unlisted manifold
+            continue;
+        }
+        if (stages[i].ws.count == 0) {  // the manifold stays or becomes empty: no contact, no rows
+            cws[i].count = 0;
             continue;
         }
         cws[i] = stages[i].ws;
@@ -1640,17 +1642,6 @@ RG_HDI void apply_ball_extra_hits(BallState& b, CarState* cars, int count, const
 // none of them moves), and the arena parts keep the reference's order for everything shared
 // (reference StepEnvGeneric, env_step.hpp:7088-7180).
 
-// What the world step needs from one car's tick start and vehicle update.
-struct CarTickRecord {
-    V3 start_vel;  // uu velocity right after the tick-start quantisation (ball-hit impulse)
-    V3 vel_bt, ang_vel;  // velocities the broadphase predicts motion with
-    WheelBallPushes pushes;
-};
-// The ball's velocities at the tick start.
-struct ArenaTickSnap {
-    V3 ball_start_vel, ball_vel_bt;
-};
-
 // respawn_seed and env_idx are the respawn draw's: the batch's last kickoff seed and the arena's logical index.
 RG_HDI void arena_tick_begin(EnvState& env, BallState& b, const ArenaCars& A, const TickConfig& c,
                              const PadLayout& pads_layout, ArenaTickSnap& as, uint64_t respawn_seed, int env_idx) {
@@ -1718,15 +1709,7 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
                               CarTickRecord* recs, const ArenaTickSnap& as, CarStage* stages) {
     const int count = A.count;
     int order[8];
-    TickSnap snap;
     for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
-    for (int i = 0; i < count && i < 8; ++i) {
-        snap.car_start_vel[i] = recs[i].start_vel;
-        snap.car_vel_bt[i] = recs[i].vel_bt;
-        snap.car_ang_vel[i] = recs[i].ang_vel;
-    }
-    snap.ball_start_vel = as.ball_start_vel;
-    snap.ball_vel_bt = as.ball_vel_bt;
     if (c.events.windows) {
         // the vehicle updates' car-world events, in the game's car order (each update emits its own in the reference)
         for (int k = 0; k < count; ++k) {
@@ -1743,9 +1726,7 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
         }
     }
     for (int k = 0; k < count; ++k) apply_wheel_ball_pushes(b, recs[order[k]].pushes, c);
-    PreContactCar pre[8];
-    world_step_cars(b, s, bp, cws, bcs, c, mesh, A, pre, snap, env.tick, stages);
-    for (int i = 0; i < count; ++i) stages[i].pre = pre[i];  // for the car's own finish (car_tick_post)
+    world_step_cars(b, s, bp, cws, bcs, c, mesh, A, recs, as, env.tick, stages);
 }
 
 // Tick part 5, per car: the car's integration, then its post-tick (reference WorldStepFinishCar + StepEnvPostCar,
