@@ -8,8 +8,8 @@ arena. Controls come from the seeded generator (throttle, steer, pitch, yaw, rol
 Bernoulli 0.1 / 0.3 / 0.1; each sample held for U{1..30} ticks). An arena resets to kickoff when its ball is scored or
 when no car has touched the ball for 300 ticks; the no-touch clocks start at seeded ages, so resets are spread over the
 ticks. A step is 8 ticks: one BatchSim::step_with_device_commands over a [8, car_capacity] control block resident in
-HBM, whose first tick applies the resets rg_batch_episode_commands chose after the previous step (6 kernels per tick
-plus the episode kernel, 49 launches per step).
+HBM, whose first tick applies the resets rg_batch_episode_commands chose after the previous step (4 kernels per tick,
+the turn that starts the first tick and the episode kernel, 34 launches per step).
 
 Steady state: every arena starts from kickoff, so SETTLE_STEPS untimed steps (320 ticks) run first, then W warm-up
 steps; the K timed steps follow. Every pass (the device-timed pass, the end-to-end pass and the CPU baseline / the
@@ -56,7 +56,8 @@ sys.path.insert(0, ROOT)
 ENVS = 16384
 EVENTS = 0  # --events: physics event records per arena (0: the stream is off)
 TICKS_PER_STEP = 8
-KERNELS_PER_TICK = 7  # arena begin, car tick start, wheel rays, vehicle updates, arena finish, car post-tick, arena tail
+KERNELS_PER_TICK = 4  # contact geometry, vehicle updates, arena finish, the turn to the next tick
+KERNELS_PER_STEP = 2  # the turn that starts the first tick, the episode commands
 SETTLE_STEPS = 40
 NO_TOUCH_TICKS = 300
 MAX_CARS = 6
@@ -71,18 +72,18 @@ WORKLOADS = {
 }
 # Algorithmic bytes of one launch (one tick) of each kernel of the car path: read + write of the state it owns, as
 # (bytes per arena, per active car, per car pair). Struct sizes: car 880, wheel record 292, car config 120, controls
-# 24, tick record 136, car stage 1,176 (prestep 56, predictive contact 20, proxy 148, car/mesh manifold 176, query
-# rows and result 776), car/mesh manifold 176, car/ball manifold 272, car-pair manifold 260, ball 288, ball contact
-# state 288, env 44, broadphase history 1,376, 34 pads x 16, tick snapshot 24.
+# 24, tick record 136, prestep and predictive contact 76, proxy 148, four wheel rays 160, car/mesh manifold 176, query
+# rows and result 776, car/ball manifold 272, car-pair manifold 260, ball 288, ball contact state 288, env 44,
+# broadphase history 1,376, 34 pads x 16, tick snapshot 24.
+_TURN = (2 * (288 + 44 + 34 * 16) + 24 + 16, 2 * (880 + 292) + 120 + 2 * 24 + 136 + 56, 0)
 KERNEL_BYTES = {
-    "arena_begin": (2 * (288 + 44 + 34 * 16) + 24 + 16, 0, 0),
-    "car_pre": (0, 2 * (880 + 292) + 120 + 24 + 136, 0),
-    "car_vehicle": (0, 2 * (880 + 292) + 120 + 24 + 288 + 136 + 176 + 1176, 0),
+    "turn_start": _TURN,
+    "car_geometry": (288 + 24 + 216, 880 + 120 + 2 * (176 + 272) + 148 + 160, 0),
+    "car_vehicle": (288, 2 * (880 + 292) + 120 + 24 + 136 + 160 + 176 + 776 + 76, 0),
     "arena_finish": (2 * (288 + 288 + 1344) + 44 + 24, 2 * (880 + 176 + 272) + 120 + 136 + 1176, 2 * 260),
-    "car_post": (0, 2 * 880 + 292 + 56 + 24, 0),
-    "arena_tail": (2 * (288 + 44 + 34 * 16), 2 * 880 + 120, 0),
+    "arena_turn": _TURN,
 }
-KERNEL_NAMES = ("arena_begin", "car_pre", "car_vehicle", "arena_finish", "car_post", "arena_tail")
+KERNEL_NAMES = ("turn_start", "car_geometry", "car_vehicle", "arena_finish", "arena_turn")
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per car of one car_vehicle_kernel launch, from an ncu
 # --set full capture of the mixed workload at 4,096 arenas (13,350 cars: 31.01 MB read + 13.92 MB written); a launch
 # at the bench's size is scaled by its cars (the kernel's traffic is per car: its state, stage and mesh reads).
@@ -476,7 +477,7 @@ def run_ours(args, world, rank, local):
                                 "max": float(np.max(step_ms)), "e2e_p50": float(np.percentile(e2e_ms, 50)),
                                 "e2e_p99": float(np.percentile(e2e_ms, 99))},
         "e2e": {"value": e2e, "unit": "arena-ticks/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        "gpu_launches": args.steps * (TICKS_PER_STEP * KERNELS_PER_TICK + 1) if mixed else args.steps,
+        "gpu_launches": args.steps * (TICKS_PER_STEP * KERNELS_PER_TICK + KERNELS_PER_STEP) if mixed else args.steps,
         "clocks": clocks.summary(),
     }
     if mixed:

@@ -85,6 +85,11 @@ struct DeviceArray {
 
 }  // namespace
 
+// A group of arenas that one warp of arena_turn_kernel works on: positions in the step order and in the active cars.
+struct TurnGroup {
+    int32_t arena_first, arena_count, car_first, car_count;
+};
+
 struct rg_batch {
     int device = 0;
     rg_sim_config cfg{};
@@ -113,6 +118,10 @@ struct rg_batch {
     DeviceArray<int32_t> arena_order;
     DeviceArray<int32_t> active_cars;
     int32_t active_car_count = 0;
+    DeviceArray<TurnGroup> turn_groups;
+    std::vector<TurnGroup> host_turn_groups;
+    int turn_car_room = 0;   // cars a turn's block has room for, and its bytes of shared memory
+    size_t turn_shared = 0;
     rg::PadLayout pad_layout{};
     DeviceArray<rg::ArenaRules> rules;  // a custom layout's spawns and goals (b->tc.rules points here), or empty
     // Pads stay at their initial state until a car exists or pads are uploaded; until then ball-only arenas skip them.
@@ -248,7 +257,7 @@ int spread_blocks(int64_t items, int shift, int threads) {
     return static_cast<int>((32 * warps + threads - 1) / threads);
 }
 // Resident warps per SM of the spread kernels, from their registers per thread (65,536 per SM).
-constexpr int kWarpsBalls = 16, kWarpsFinish = 8, kWarpsPost = 32, kWarpsTail = 8;
+constexpr int kWarpsBalls = 16, kWarpsFinish = 8;
 
 int device_sms(int device) {
     int n = 1;
@@ -345,6 +354,7 @@ struct CarTickArgs {
     const int32_t* active_cars;
     int32_t active_car_count;
     rg::CarStage* stages;
+    const TurnGroup* turn_groups;
     const rg::EnvCommand* commands;  // step_with_device_commands: tick t's command for arena e at t * stride + e
     int32_t command_stride;
     rg::CarControls* reset_controls;  // the batch's held controls, cleared by a kickoff reset
@@ -369,7 +379,7 @@ __device__ __forceinline__ bool arena_idle(const CarTickArgs& a, int e) {
 __device__ __forceinline__ rg::ArenaCars arena_cars(const CarTickArgs& a, int e, int t) {
     const int car_base = e * a.max_cars;
     rg::ArenaCars A;
-    A.cars = a.cars + car_base;
+    A.cars = A.slots = a.cars + car_base;
     A.wheels = a.wheels + car_base;
     A.cfgs = a.car_cfgs + car_base;
     A.pads = a.pads ? a.pads + static_cast<size_t>(e) * a.pad_layout.count : nullptr;
@@ -408,54 +418,173 @@ __global__ void apply_commands_kernel(const __grid_constant__ CarTickArgs a, con
                           controls + static_cast<size_t>(e) * a.max_cars, a.pad_layout, a.base.tc);
 }
 
-// Tick part 1, one thread per arena in step order: this tick's env command (step_with_device_commands), vehicle
-// order, the ball's tick start, pad timers.
-__global__ void __launch_bounds__(256) arena_begin_kernel(const __grid_constant__ CarTickArgs a, int t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.base.env_count) return;
-    const int e = a.arena_order[k];
-    if (arena_idle(a, e)) return;
-    if (a.commands) {
-        const rg::EnvCommand c = a.commands[static_cast<size_t>(t) * static_cast<size_t>(a.command_stride) + e];
-        if (rg::env_command_active(c))
-            rg::apply_env_command(c, e, a.base.envs[e], a.base.balls[e], arena_contact_state(a, e),
-                                  arena_cars(a, e, t), a.reset_controls + static_cast<size_t>(e) * a.max_cars,
-                                  a.pad_layout, a.base.tc);
-    }
-    rg::BallState b = a.base.balls[e];
-    rg::EnvState env = a.base.envs[e];
-    rg::arena_tick_begin(env, b, arena_cars(a, e, t), a.base.tc, a.pad_layout, a.snaps[e],
-                         a.slots.remaining ? a.slots.seed[e] : a.base.tc.kickoff_seed, logical_env(a, e));
-    a.base.balls[e] = b;
-    a.base.envs[e] = env;
+// ---- asynchronous copies into shared memory ----------------------------------------------------------------------
+template <int kBytes>
+__device__ __forceinline__ void copy_async(void* shared, const void* global) {
+#if defined(__CUDA_ARCH__)
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(shared));
+    if (kBytes == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(global) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(global), "n"(kBytes) : "memory");
+#else
+    memcpy(shared, global, kBytes);
+#endif
+}
+__device__ __forceinline__ void copy_async_wait() {
+#if defined(__CUDA_ARCH__)
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+}
+// `bytes` (a multiple of kWord, both ends aligned to it) by the lanes of a warp.
+template <int kWord>
+__device__ __forceinline__ void warp_load(void* shared, const void* global, int bytes, int lane) {
+    for (int at = kWord * lane; at < bytes; at += 32 * kWord)
+        copy_async<kWord>(static_cast<unsigned char*>(shared) + at, static_cast<const unsigned char*>(global) + at);
+}
+template <class Word>
+__device__ __forceinline__ void warp_store(void* global, const void* shared, int bytes, int lane) {
+    for (int at = static_cast<int>(sizeof(Word)) * lane; at < bytes; at += 32 * static_cast<int>(sizeof(Word)))
+        *reinterpret_cast<Word*>(static_cast<unsigned char*>(global) + at) =
+            *reinterpret_cast<const Word*>(static_cast<const unsigned char*>(shared) + at);
 }
 
-// Tick part 2, one thread per active car: the car's tick start (demolition timer and respawn, quantisation, controls,
-// jumps, dodges, boost) and the speed clamp.
-__global__ void __launch_bounds__(256) car_pre_kernel(const __grid_constant__ CarTickArgs a, int t) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.active_car_count) return;
-    const int idx = a.active_cars[k];
-    const int e = idx / a.max_cars;
-    if (arena_idle(a, e)) return;
-    const rg::CarControls& ctrl =
-        a.controls[control_row(a, e, t) * static_cast<size_t>(a.control_stride) + static_cast<size_t>(idx)];
-    const int le = logical_env(a, e);
-    rg::RespawnCtx rc;
-    rc.seed = a.slots.remaining ? a.slots.seed[e] : a.base.tc.kickoff_seed;
-    rc.env_idx = le;
-    rc.env_tick = a.base.envs[e].tick;
-    rc.car_id = static_cast<uint32_t>(le * a.max_cars + (idx - e * a.max_cars) + 1);
-    rc.team = a.teams[idx];
-    // the car's structs are worked on in local copies: one burst of independent loads, after which the warp's
-    // accesses to a field go to one interleaved local line instead of 32 lines of 880-byte-strided structs (measured:
-    // faster here, where the tick start touches most of the car; slower in the post-tick, which touches little)
-    rg::CarState car = a.cars[idx];
-    rg::WheelRuntime wr = a.wheels[idx];
-    const rg::CarConfig cfg = a.car_cfgs[idx];
-    rg::car_tick_pre(car, ctrl, cfg, a.base.tc, wr, rc, a.records[idx]);
-    a.cars[idx] = car;
-    a.wheels[idx] = wr;
+// Tick parts 5, 6, 1 and 2 in one launch, the turn from tick t to the next: each car's integration and post-tick (a lane
+// per car); each arena's pads, driving countdown, extra ball hits, goal and timers (a lane per arena); then, for the next
+// tick, the arena's env command, vehicle order, ball tick start and pad timers, and each car's tick start (demolition
+// timer and respawn, quantisation, controls, jumps, dodges, boost, speed clamp). A warp holds a group of whole arenas, so
+// its lanes need no other warp's; their cars, wheel records and pads are in shared memory from one end to the other
+// (asynchronous copies, all in flight at once). As four launches (post-tick, tail, begin, tick start) these parts loaded
+// the structs from HBM four times, field by field: 298 us a tick at 16,384 mixed arenas, 60 us for one 1v1 arena.
+// kTurnFinish: tick t ends; kTurnStart: tick t_next begins.
+constexpr int kTurnFinish = 1, kTurnStart = 2;
+__global__ void __launch_bounds__(32, 16)
+    arena_turn_kernel(const __grid_constant__ CarTickArgs a, int parts, int t, int report_fields, int t_next,
+                      int car_room) {
+    extern __shared__ __align__(16) unsigned char turn_shared[];
+    const int lane = static_cast<int>(threadIdx.x);
+    const TurnGroup g = a.turn_groups[blockIdx.x];
+    const int pad_bytes = a.pad_layout.count * static_cast<int>(sizeof(rg::PadState));
+    rg::CarState* cars = reinterpret_cast<rg::CarState*>(turn_shared);
+    rg::WheelRuntime* wheels = reinterpret_cast<rg::WheelRuntime*>(cars + car_room);
+    unsigned char* pads = reinterpret_cast<unsigned char*>(wheels + car_room);  // car_room is a multiple of 4: aligned
+    // this lane's car and this lane's arena; an idle arena (serving) and its cars stay out
+    int idx = -1, car_env = -1, e = -1, count = 0;
+    if (lane < g.car_count) {
+        idx = a.active_cars[g.car_first + lane];
+        car_env = idx / a.max_cars;
+        if (arena_idle(a, car_env)) idx = -1;
+    }
+    if (lane < g.arena_count) {
+        e = a.arena_order[g.arena_first + lane];
+        count = a.base.env_car_count[e];
+    }
+    int car_at = count;  // the arena's first car in the group
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int below = __shfl_up_sync(0xffffffffu, car_at, d);
+        if (lane >= d) car_at += below;
+    }
+    car_at -= count;
+    if (e >= 0 && arena_idle(a, e)) e = -1;
+    for (int j = 0; j < g.car_count; ++j) {
+        const int from = __shfl_sync(0xffffffffu, idx, j);
+        if (from < 0) continue;
+        warp_load<16>(cars + j, a.cars + from, sizeof(rg::CarState), lane);
+        warp_load<4>(wheels + j, a.wheels + from, sizeof(rg::WheelRuntime), lane);
+    }
+    if (a.pads)
+        for (int j = 0; j < g.arena_count; ++j) {
+            const int from = __shfl_sync(0xffffffffu, e, j);
+            if (from >= 0)
+                warp_load<16>(pads + j * pad_bytes, a.pads + static_cast<size_t>(from) * a.pad_layout.count, pad_bytes,
+                              lane);
+        }
+    // the lanes' own single loads meanwhile
+    rg::BallState b;
+    rg::EnvState env;
+    if (e >= 0) {
+        b = a.base.balls[e];
+        env = a.base.envs[e];
+    }
+    copy_async_wait();
+    __syncwarp();
+    auto arena = [&](int tick) {
+        rg::ArenaCars A = arena_cars(a, e, tick);
+        A.cars = cars + car_at;
+        A.wheels = wheels + car_at;
+        A.pads = a.pads ? reinterpret_cast<rg::PadState*>(pads + lane * pad_bytes) : nullptr;
+        return A;
+    };
+    if (parts & kTurnFinish) {
+        // a car's arena is the group's arena whose cars it is among: its pads lie at that arena's place
+        int mine = 0;
+        for (int j = 1; j < g.arena_count; ++j) {
+            const int first = __shfl_sync(0xffffffffu, car_at, j);
+            mine = lane >= first ? j : mine;
+        }
+        if (idx >= 0) {
+            // serving: report fields after the request's last tick, as a batch reports them after a step's last tick
+            const bool report = a.slots.remaining ? a.slots.remaining[car_env] == 1 : report_fields != 0;
+            const rg::CarControls& ctrl = a.controls[control_row(a, car_env, t) * static_cast<size_t>(a.control_stride) +
+                                                     static_cast<size_t>(idx)];
+            rg::car_tick_post(cars[lane], a.stages[idx].pre, ctrl, wheels[lane], a.base.tc, report, a.car_cfgs[idx],
+                              a.pads ? reinterpret_cast<const rg::PadState*>(pads + mine * pad_bytes) : nullptr,
+                              a.pad_layout, a.stages[idx].pads);
+        }
+        __syncwarp();
+        if (e >= 0) {
+            rg::arena_tick_tail(env, b, arena(t), a.pad_layout, a.base.tc,
+                                a.stages + static_cast<size_t>(e) * a.max_cars);
+            if (a.slots.remaining) {
+                --a.slots.remaining[e];
+                ++a.slots.tick[e];
+            }
+        }
+    }
+    if ((parts & kTurnStart) && e >= 0) {
+        const rg::ArenaCars A = arena(t_next);
+        if (a.commands) {
+            const rg::EnvCommand c =
+                a.commands[static_cast<size_t>(t_next) * static_cast<size_t>(a.command_stride) + e];
+            if (rg::env_command_active(c))
+                rg::apply_env_command(c, e, env, b, arena_contact_state(a, e), A,
+                                      a.reset_controls + static_cast<size_t>(e) * a.max_cars, a.pad_layout, a.base.tc);
+        }
+        rg::arena_tick_begin(env, b, A, a.base.tc, a.pad_layout, a.snaps[e],
+                             a.slots.remaining ? a.slots.seed[e] : a.base.tc.kickoff_seed, logical_env(a, e));
+    }
+    if (e >= 0) {
+        a.base.balls[e] = b;
+        a.base.envs[e] = env;
+    }
+    __syncwarp();
+    if ((parts & kTurnStart) && idx >= 0) {
+        const rg::CarControls& ctrl = a.controls[control_row(a, car_env, t_next) * static_cast<size_t>(a.control_stride) +
+                                                 static_cast<size_t>(idx)];
+        const int le = logical_env(a, car_env);
+        rg::RespawnCtx rc;
+        rc.seed = a.slots.remaining ? a.slots.seed[car_env] : a.base.tc.kickoff_seed;
+        rc.env_idx = le;
+        rc.env_tick = a.base.envs[car_env].tick;
+        rc.car_id = static_cast<uint32_t>(le * a.max_cars + (idx - car_env * a.max_cars) + 1);
+        rc.team = a.teams[idx];
+        rg::car_tick_pre(cars[lane], ctrl, a.car_cfgs[idx], a.base.tc, wheels[lane], rc, a.records[idx]);
+    }
+    __syncwarp();
+    for (int j = 0; j < g.car_count; ++j) {
+        const int to = __shfl_sync(0xffffffffu, idx, j);
+        if (to < 0) continue;
+        warp_store<rg::Word16>(a.cars + to, cars + j, sizeof(rg::CarState), lane);
+        warp_store<uint32_t>(a.wheels + to, wheels + j, sizeof(rg::WheelRuntime), lane);
+    }
+    if (a.pads)
+        for (int j = 0; j < g.arena_count; ++j) {
+            const int to = __shfl_sync(0xffffffffu, e, j);
+            if (to >= 0)
+                warp_store<rg::Word16>(a.pads + static_cast<size_t>(to) * a.pad_layout.count, pads + j * pad_bytes,
+                                       pad_bytes, lane);
+        }
 }
 
 // Four lanes of a warp that share one car: lane threadIdx.x & 3 of the group.
@@ -717,40 +846,6 @@ __global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ Car
     a.base.ball_world[e] = s;
 }
 
-// Tick part 5, one thread per active car: its integration and post-tick.
-__global__ void __launch_bounds__(256)
-    car_post_kernel(const __grid_constant__ CarTickArgs a, int t, int report_fields, int shift) {
-    const int k = spread_item(shift);
-    if (k >= a.active_car_count) return;
-    const int idx = a.active_cars[k];
-    const int e = idx / a.max_cars;
-    if (arena_idle(a, e)) return;
-    // serving: report fields after the request's last tick, as a batch reports them after a step's last tick
-    const bool report = a.slots.remaining ? a.slots.remaining[e] == 1 : report_fields != 0;
-    const rg::CarControls& ctrl =
-        a.controls[control_row(a, e, t) * static_cast<size_t>(a.control_stride) + static_cast<size_t>(idx)];
-    rg::car_tick_post(a.cars[idx], a.stages[idx].pre, ctrl, a.wheels[idx], a.base.tc, report, a.car_cfgs[idx],
-                      a.pads ? a.pads + static_cast<size_t>(e) * a.pad_layout.count : nullptr, a.pad_layout,
-                      a.stages[idx].pads);
-}
-
-// Tick part 6, one thread per arena in step order: pads, the driving countdown, extra ball hits, goal and timers.
-__global__ void __maxnreg__(255) arena_tail_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
-    const int k = spread_item(shift);
-    if (k >= a.base.env_count) return;
-    const int e = a.arena_order[k];
-    if (arena_idle(a, e)) return;
-    rg::BallState b = a.base.balls[e];
-    rg::EnvState env = a.base.envs[e];
-    rg::arena_tick_tail(env, b, arena_cars(a, e, t), a.pad_layout, a.base.tc, a.stages + static_cast<size_t>(e) * a.max_cars);
-    a.base.balls[e] = b;
-    a.base.envs[e] = env;
-    if (a.slots.remaining) {
-        --a.slots.remaining[e];
-        ++a.slots.tick[e];
-    }
-}
-
 CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stride) {
     CarTickArgs a;
     a.base.balls = b->balls.ptr;
@@ -782,6 +877,7 @@ CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stri
     a.active_cars = b->active_cars.ptr;
     a.active_car_count = b->active_car_count;
     a.stages = b->car_stages.ptr;
+    a.turn_groups = b->turn_groups.ptr;
     a.commands = nullptr;
     a.command_stride = 0;
     a.reset_controls = b->controls.ptr;
@@ -790,41 +886,35 @@ CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stri
     return a;
 }
 
-// One tick's launches. `mark` is called before each of the six phases and after the last.
+// A turn (arena_turn_kernel) of every arena.
+void launch_turn(const rg_batch* b, const CarTickArgs& a, int parts, int t, int report_fields, int t_next,
+                 cudaStream_t s) {
+    arena_turn_kernel<<<static_cast<int>(b->host_turn_groups.size()), 32, b->turn_shared, s>>>(
+        a, parts, t, report_fields, t_next, b->turn_car_room);
+}
+
+// One tick's launches between two turns. `mark` is called before each and after the last.
 template <class Mark>
-void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, int report_fields, cudaStream_t s, Mark&& mark) {
+void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, cudaStream_t s, Mark&& mark) {
     const int64_t arenas = b->env_count, cars = b->active_car_count;
-    const int at = b->launch_threads, ct = b->car_threads;
-    const int car_blocks = blocks_for(cars, ct);
-    auto shift = [&](int64_t items, int warps) { return spread_shift(items, b->sms, warps); };
     mark();
-    arena_begin_kernel<<<blocks_for(arenas, at), at, 0, s>>>(a, t);
-    mark();
-    if (cars) car_pre_kernel<<<car_blocks, ct, 0, s>>>(a, t);
-    mark();
-    // phase 2 (timing) is the geometry and the vehicle updates
     if (cars) {
         const int lanes = blocks_for(4 * cars, kGeometryThreads), each = blocks_for(cars, kGeometryThreads);
         car_geometry_kernel<<<2 * lanes + each, kGeometryThreads, 0, s>>>(a, t, lanes, each);
+    }
+    mark();
+    if (cars) {
         const int order = blocks_for(4 * arenas, kVehicleThreads);
         car_vehicle_kernel<<<order + blocks_for(4 * cars, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
     }
     mark();
-    const int finish = shift(arenas, kWarpsFinish);
+    const int at = b->launch_threads, finish = spread_shift(arenas, b->sms, kWarpsFinish);
     arena_finish_kernel<<<spread_blocks(arenas, finish, at), at, 0, s>>>(a, t, finish);
-    mark();
-    if (cars) {
-        const int post = shift(cars, kWarpsPost);
-        car_post_kernel<<<spread_blocks(cars, post, ct), ct, 0, s>>>(a, t, report_fields, post);
-    }
-    mark();
-    const int tail = shift(arenas, kWarpsTail);
-    arena_tail_kernel<<<spread_blocks(arenas, tail, at), at, 0, s>>>(a, t, tail);
     mark();
 }
 
-// Arenas with cars: seven launches per tick (arena begin, car tick start, contact geometry, vehicle updates, arena
-// finish, car post-tick, arena tail).
+// Arenas with cars: a turn that starts the first tick, then four launches per tick: contact geometry, vehicle updates,
+// arena finish, and the turn that ends this tick and starts the next.
 void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, int ticks, cudaStream_t s,
                      const rg::EnvCommand* commands = nullptr, int command_stride = 0) {
     if (b->env_count == 0) return;
@@ -845,9 +935,16 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         }
         check(cudaEventRecord(b->events[b->events_used++], s), "cudaEventRecord");
     };
-    // report fields after the last tick, and after every tick of a command stream (reference StepEnvGeneric,
-    // env_step.hpp:7174: report_fields = last tick || has_commands)
-    for (int t = 0; t < ticks; ++t) launch_tick_kernels(b, a, t, (t + 1 == ticks || commands) ? 1 : 0, s, mark);
+    for (int t = 0; t < ticks; ++t) {
+        mark();
+        if (t == 0) launch_turn(b, a, kTurnStart, 0, 0, 0, s);
+        launch_tick_kernels(b, a, t, s, mark);
+        // report fields after the last tick, and after every tick of a command stream (reference StepEnvGeneric,
+        // env_step.hpp:7174: report_fields = last tick || has_commands)
+        const bool last = t + 1 == ticks;
+        launch_turn(b, a, last ? kTurnFinish : kTurnFinish | kTurnStart, t, (last || commands) ? 1 : 0, t + 1, s);
+        mark();
+    }
     check(cudaGetLastError(), "car tick launch");
 }
 
@@ -1112,6 +1209,50 @@ void launch_tick(rg_batch* b, int ticks, cudaStream_t s) {
     check(cudaGetLastError(), "tick_kernel launch");
 }
 
+// The groups of a turn, along the step order: whole arenas, up to kTurnCars cars (or one arena). Fewer cars per group,
+// down to one arena, while the chip has warps to spare (kTurnWarps resident per SM, by the kernel's registers). Twelve
+// cars take 17 KB of shared memory, so that 13 groups are resident per SM: 187 us a turn at 16,384 mixed arenas, against
+// 221 with up to 32 cars, 216 with 8 (one arena of six, three of two). 168 registers instead of 128 gained 14 us there and
+// lost 18 of 130 us at 4,095 3v3 arenas, where the warps count.
+constexpr int kTurnWarps = 16, kTurnCars = 12, kTurnArenas = 16;
+constexpr size_t kTurnSharedMax = 48 * 1024;
+size_t turn_shared_bytes(int cars, int arenas, int pads) {
+    const size_t room = static_cast<size_t>((cars + 3) / 4 * 4);
+    return room * (sizeof(rg::CarState) + sizeof(rg::WheelRuntime)) +
+           static_cast<size_t>(arenas) * static_cast<size_t>(pads) * sizeof(rg::PadState);
+}
+void rebuild_turn_groups(rg_batch* b, cudaStream_t s) {
+    std::vector<TurnGroup>& groups = b->host_turn_groups;
+    groups.clear();
+    const int64_t warps = static_cast<int64_t>(b->sms) * kTurnWarps;
+    const int share = static_cast<int>(std::min<int64_t>(kTurnCars, (b->active_car_count + warps - 1) / warps));
+    TurnGroup g{0, 0, 0, 0};
+    int cars_most = 0, arenas_most = 0;
+    auto close = [&] {
+        if (g.arena_count == 0) return;
+        groups.push_back(g);
+        cars_most = std::max(cars_most, g.car_count);
+        arenas_most = std::max(arenas_most, g.arena_count);
+        g = TurnGroup{g.arena_first + g.arena_count, 0, g.car_first + g.car_count, 0};
+    };
+    for (int32_t e : b->host_arena_order) {
+        const int n = b->host_car_count[e];
+        if (g.arena_count == kTurnArenas || (g.car_count + n > share && g.car_count > 0) ||
+            turn_shared_bytes(std::max(cars_most, g.car_count + n), std::max(arenas_most, g.arena_count + 1),
+                              b->pad_layout.count) > kTurnSharedMax)
+            close();
+        ++g.arena_count;
+        g.car_count += n;
+    }
+    close();
+    b->turn_car_room = (cars_most + 3) / 4 * 4;
+    b->turn_shared = turn_shared_bytes(cars_most, arenas_most, b->pad_layout.count);
+    if (!groups.empty())
+        check(cudaMemcpyAsync(b->turn_groups.ptr, groups.data(), groups.size() * sizeof(TurnGroup),
+                              cudaMemcpyHostToDevice, s),
+              "turn groups");
+}
+
 // The step order (reference set_env_car_count rebuilds its step order, src/rocketgpu.cpp:2920-2932): arenas stably
 // sorted by car count, largest first (their warps run longest, so they start first and the short ones fill in behind
 // them), and the active car slots of those arenas in that order. The host copies stay in the batch
@@ -1136,6 +1277,7 @@ void rebuild_step_order(rg_batch* b, cudaStream_t s) {
                               s),
               "active cars");
     b->active_car_count = static_cast<int32_t>(cars.size());
+    rebuild_turn_groups(b, s);
 }
 
 rg::TickConfig resolve_tick_config(const rg_sim_config& c) {
@@ -1555,6 +1697,7 @@ RG_API int rg_batch_create(const rg_sim_config* cfg, const rg_arena_layout* layo
         b->episode_seen.alloc(cap);
         if (cap) check(cudaMemset(b->episode_seen.ptr, 0xff, cap * sizeof(uint64_t)), "episode state");
         b->arena_order.alloc(b->env_count);
+        b->turn_groups.alloc(b->env_count);
         b->active_cars.alloc(cap);
         rebuild_step_order(b.get(), nullptr);
         if (cap) {
@@ -1943,8 +2086,8 @@ RG_API int rg_batch_phase_times(rg_batch* b, float* out_ms, int64_t* out_ticks) 
     return guard([&] {
         if (!b || !out_ms) throw std::invalid_argument("null argument");
         DeviceGuard dg(b->device);
-        constexpr int kPhases = 6;
-        for (int k = 0; k < kPhases; ++k) out_ms[k] = 0.0f;
+        constexpr int kPhases = 5;
+        for (int k = 0; k < 6; ++k) out_ms[k] = 0.0f;
         const size_t ticks = b->events_used / (kPhases + 1);
         if (ticks) check(cudaEventSynchronize(b->events[b->events_used - 1]), "phase timing sync");
         for (size_t t = 0; t < ticks; ++t)

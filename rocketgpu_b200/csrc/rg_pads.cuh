@@ -192,17 +192,25 @@ RG_HDI void pad_touch_step(PadState& pad, int p, CarState& c, uint32_t car_id, b
     }
 }
 // Pickup: the car gets the pad's boost, the pad starts its cooldown (reference BoostPadGive, :2562-2585).
-// `cars` is the arena's car array; car ids are global slot + 1.
-RG_HDI void pad_give(CarState* cars, int car_base, int max_cars, PadState& pad, int p, uint32_t car_id,
-                     const TickConfig& tc) {
+// `cars` holds the arena's active cars, `slots` all its slots in the batch's array (the first `count` of them may be out
+// of date); car ids are global slot + 1.
+struct PadCars {
+    CarState *cars, *slots;
+    int count, car_base, max_cars;
+};
+RG_HDI void pad_give(const PadCars& A, PadState& pad, int p, uint32_t car_id, const TickConfig& tc) {
+    CarState* cars = A.cars;
+    const int car_base = A.car_base, max_cars = A.max_cars;
     CarState& c = cars[static_cast<int>(car_id - 1u) - car_base];
     const float boost_before = c.boost;
     car_set_boost_amount(c, fmin_(tc.boost_max / 100.0f, car_boost_amount(c) + (pad.is_big ? 1.0f : 0.12f)));
     pad.is_active = 0;
     pad.cooldown = (pad.is_big ? tc.boost_pad_cooldown_big : tc.boost_pad_cooldown_small) - tc.tick_dt;
     pad.pickup_frac_q = pad_frac_q(tc.frame_frac);
-    for (int i = 0; i < max_cars; ++i)
+    for (int i = 0; i < A.count; ++i)
         if (cars[i].boost_pad_touching == p + 1) cars[i].boost_pad_touching = 0;
+    for (int i = A.count; i < max_cars; ++i)
+        if (A.slots[i].boost_pad_touching == p + 1) A.slots[i].boost_pad_touching = 0;
     if (tc.events.windows) {
         PhysicsEvent e = new_event(kEventBoostPickup);
         e.car_id = car_id;
@@ -214,10 +222,10 @@ RG_HDI void pad_give(CarState* cars, int car_base, int max_cars, PadState& pad, 
     }
 }
 // More than one pad hit in one tick: visit them in order of entry (reference BoostPadSweepTouchSteps, :2587-2637).
-RG_HDI void pad_sweep_touch_steps(CarState* cars, int car_base, int max_cars, int slot, PadState* pads,
-                                  const PadLayout& L, const TickConfig& tc, uint64_t hits, uint64_t overlap) {
-    CarState& c = cars[slot];
-    const uint32_t car_id = static_cast<uint32_t>(car_base + slot + 1);
+RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, const PadLayout& L,
+                                  const TickConfig& tc, uint64_t hits, uint64_t overlap) {
+    CarState& c = A.cars[slot];
+    const uint32_t car_id = static_cast<uint32_t>(A.car_base + slot + 1);
     const V3 to_bt = pad_frame_pos(c, tc.frame_frac) * (1.0f / 50.0f);
     const V3 from_bt = pad_sweep_from_bt(c, to_bt);
     if (c.boost_pad_touching != 0 && ((hits >> (c.boost_pad_touching - 1)) & 1u) == 0u) {
@@ -247,7 +255,7 @@ RG_HDI void pad_sweep_touch_steps(CarState* cars, int car_base, int max_cars, in
         if (pad_eligible(c, tc)) {
             c.boost_pad_touching = static_cast<uint8_t>(p + 1);
             pad.cur_locked_car_id = car_id;
-            pad_give(cars, car_base, max_cars, pad, p, car_id, tc);
+            pad_give(A, pad, p, car_id, tc);
         } else if (((overlap >> p) & 1u) != 0u) {
             c.boost_pad_touching = static_cast<uint8_t>(p + 1);
         }
@@ -256,28 +264,21 @@ RG_HDI void pad_sweep_touch_steps(CarState* cars, int car_base, int max_cars, in
 
 // The pads' part of the tick tail (reference BoostPadTouchPassForEnv, :2706-2835, and PostTickBoostPadsForEnv,
 // :2851-2892). `order` lists the car slots in visit order.
-// `staged` (null: computed here) holds car slot i's pad contacts (pad_contacts_stage) at byte offset
-// i * staged_stride.
-RG_NOINL void pads_tail(CarState* cars, int car_base, int max_cars, const CarConfig* cfgs, int count, const int* order,
-                      PadState* pads, const PadLayout& L, const TickConfig& tc, const PadContacts* staged = nullptr,
-                      size_t staged_stride = sizeof(PadContacts)) {
+// `staged` holds car slot i's pad contacts (pad_contacts_stage) at byte offset i * staged_stride.
+RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* order, PadState* pads, const PadLayout& L,
+                        const TickConfig& tc, const PadContacts* staged, size_t staged_stride) {
+    CarState* cars = A.cars;
+    const int count = A.count, car_base = A.car_base;
     if (!tc.enable_boost_pads || tc.frame_frac < 0.0f) return;
     for (int k = 0; k < count; ++k) {
         const int i = order[k];
         CarState& c = cars[i];
-        uint64_t overlap = 0u, hits = 0u;
-        V3 frame_pos_bt{0.0f, 0.0f, 0.0f};
-        if (staged) {
-            const PadContacts& pc = *reinterpret_cast<const PadContacts*>(
-                reinterpret_cast<const unsigned char*>(staged) + static_cast<size_t>(i) * staged_stride);
-            hits = pc.hits;
-            overlap = pc.overlap;
-            frame_pos_bt = pc.frame_pos_bt;
-        } else if (!c.is_demoed) {
-            hits = pad_contacts_for_car(c, cfgs[i], pads, L, tc, overlap, frame_pos_bt);
-        }
+        const PadContacts& pc = *reinterpret_cast<const PadContacts*>(
+            reinterpret_cast<const unsigned char*>(staged) + static_cast<size_t>(i) * staged_stride);
+        const uint64_t hits = pc.hits, overlap = pc.overlap;
+        const V3 frame_pos_bt = pc.frame_pos_bt;
         if ((hits & (hits - 1u)) != 0u) {
-            pad_sweep_touch_steps(cars, car_base, max_cars, i, pads, L, tc, hits, overlap);
+            pad_sweep_touch_steps(A, i, pads, L, tc, hits, overlap);
         } else {
             const bool eligible = pad_eligible(c, tc);
             uint64_t near = hits;
@@ -335,7 +336,7 @@ RG_NOINL void pads_tail(CarState* cars, int car_base, int max_cars, const CarCon
             PadState& pad = pads[p];
             const uint32_t locked = pad.cur_locked_car_id;
             if ((locked | pad.prev_locked_car_id) == 0u) continue;
-            if (locked != 0 && pad.is_active) pad_give(cars, car_base, max_cars, pad, p, locked, tc);
+            if (locked != 0 && pad.is_active) pad_give(A, pad, p, locked, tc);
             pad.prev_locked_car_id = locked;
         }
     }

@@ -107,7 +107,7 @@ int64_t server_slot_bytes(int max_cars) {
     const int64_t per_arena = sizeof(rg::BallState) + sizeof(rg::EnvState) + sizeof(int32_t) +
                               sizeof(rg::BallWorldScratch) + 34 * sizeof(rg::PadState) + sizeof(rg::Broadphase) +
                               pairs * sizeof(rg::CarCarManifold) + sizeof(rg::ArenaTickSnap) + 2 * sizeof(int32_t) +
-                              sizeof(rg::EnvCommand) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
+                              sizeof(rg::EnvCommand) + sizeof(TurnGroup) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
     const int64_t per_car = sizeof(rg::CarState) + sizeof(rg::WheelRuntime) + sizeof(rg::CarConfig) +
                             (1 + kServerMaxTicks) * sizeof(rg::CarControls) + 1 + sizeof(rg::CarWorldScratch) +
                             sizeof(rg::BallCarScratch) + sizeof(rg::CarTickRecord) + sizeof(rg::CarStage) +
@@ -123,7 +123,9 @@ void server_launch_round(rg_server* s) {
     a.slots.tick = s->tick.ptr;
     a.slots.logical = s->logical.ptr;
     a.slots.seed = s->seed.ptr;
-    launch_tick_kernels(b, a, 0, 0, s->stream, [] {});
+    launch_turn(b, a, kTurnStart, 0, 0, 0, s->stream);
+    launch_tick_kernels(b, a, 0, s->stream, [] {});
+    launch_turn(b, a, kTurnFinish, 0, 0, 0, s->stream);
     check(cudaGetLastError(), "serving round launch");
 }
 

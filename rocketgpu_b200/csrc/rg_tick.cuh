@@ -290,7 +290,8 @@ RG_HDI void arena_tick(EnvState& env, BallState& b, BallWorldScratch& s, const T
 // One arena's cars during a tick: its max_cars slots of car state, wheel records and configs, its pads (null when the
 // batch never had a car, so every pad is still at its initial state) and this tick's control row.
 struct ArenaCars {
-    CarState* cars;
+    CarState* cars;        // the active cars, `count` of them
+    CarState* slots;       // all the arena's slots in the batch's array (`cars` may be a copy of the active ones)
     WheelRuntime* wheels;
     const CarConfig* cfgs;
     PadState* pads;
@@ -1757,8 +1758,8 @@ RG_HDI void arena_tick_tail(EnvState& env, BallState& b, const ArenaCars& A, con
     int order[8];
     for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
     if (A.pads)
-        pads_tail(A.cars, A.car_base, A.max_cars, A.cfgs, count, order, A.pads, pads_layout, c, &stages[0].pads,
-                  sizeof(CarStage));
+        pads_tail(PadCars{A.cars, A.slots, count, A.car_base, A.max_cars}, A.cfgs, order, A.pads, pads_layout, c,
+                  &stages[0].pads, sizeof(CarStage));
     for (int k = 0; k < count; ++k) {
         CarState& car = A.cars[order[k]];
         if (!car.is_demoed && car.driving_disabled) --car.driving_disabled;

@@ -157,7 +157,7 @@ void hp_step(const HostBatch* b, const rg_sim_config* cfg, const float* vertices
         rg::EnvState& env = b->env_states[e];
         for (int t = 0; t < ticks; ++t) {
             rg::ArenaCars A{};
-            A.cars = b->cars + base;
+            A.cars = A.slots = b->cars + base;
             A.wheels = b->wheels + base;
             A.cfgs = b->cfgs + base;
             A.pads = b->pads + static_cast<size_t>(e) * b->pad_count;
