@@ -713,7 +713,8 @@ RG_HDI bool mesh_ray_closest(const MeshDevice& m, V3 from, V3 to, float& out_fra
 // The ray of a body's motion this tick, from `cur` (backed off 0.04 bt) to `to`, against the mesh; a hit gives the hit
 // plane's normal (facing the ray's start) and the motion's signed distance past it (reference
 // PredictiveContactRayForBody tail, env_step.hpp:4075-4127).
-RG_HDI bool predictive_ray(const MeshDevice& m, V3 cur, V3 to, V3& out_n, float& out_dist) {
+// `clear`: bounds (lo, hi) that no triangle's bounds meet, or null: a ray inside them needs no query.
+RG_HDI bool predictive_ray(const MeshDevice& m, V3 cur, V3 to, V3& out_n, float& out_dist, const V3* clear = nullptr) {
     constexpr float kCcdMotionThresholdBt = 0.02f;
     constexpr float kRayBackoffBt = 0.04f;
     const V3 mv{to.x - cur.x, to.y - cur.y, to.z - cur.z};
@@ -724,6 +725,13 @@ RG_HDI bool predictive_ray(const MeshDevice& m, V3 cur, V3 to, V3& out_n, float&
                   cur.z - inv_len * mv.z * kRayBackoffBt};
     const V3 delta{to.x - from.x, to.y - from.y, to.z - from.z};
     if (!(len(delta) * 50.0f > 0.0f) || m.tri_count == 0) return false;
+    if (clear) {
+        const V3 end = from + delta;
+        const V3 lo = vmin(from, end), hi = vmax(from, end);
+        if (lo.x >= clear[0].x && lo.y >= clear[0].y && lo.z >= clear[0].z && hi.x <= clear[1].x &&
+            hi.y <= clear[1].y && hi.z <= clear[1].z)
+            return false;
+    }
     float f = 0.0f;
     const DevTri* t = nullptr;
     if (!mesh_ray_closest(m, from, from + delta, f, t) || !(f < 1.0f)) return false;

@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(32, 16)
                 rg::apply_env_command(c, e, env, b, arena_contact_state(a, e), A,
                                       a.reset_controls + static_cast<size_t>(e) * a.max_cars, a.pad_layout, a.base.tc);
         }
-        rg::arena_tick_begin(env, b, A, a.base.tc, a.pad_layout, a.snaps[e],
+        rg::arena_tick_begin(env, b, A, a.base.tc, a.snaps[e],
                              a.slots.remaining ? a.slots.seed[e] : a.base.tc.kickoff_seed, logical_env(a, e));
     }
     if (e >= 0) {
@@ -559,6 +559,13 @@ __global__ void __launch_bounds__(32, 16)
         a.base.envs[e] = env;
     }
     __syncwarp();
+    if (parts & kTurnStart)
+        for (int j = 0; j < g.arena_count; ++j) {  // pad timers: the lanes share the pads
+            const int ej = __shfl_sync(0xffffffffu, e, j), n = __shfl_sync(0xffffffffu, count, j);
+            if (ej < 0 || !a.pads) continue;
+            for (int p = lane; p < a.pad_layout.count; p += 32)
+                rg::pad_tick_begin(a.base.tc, n, reinterpret_cast<rg::PadState*>(pads + j * pad_bytes), p);
+        }
     if ((parts & kTurnStart) && idx >= 0) {
         const rg::CarControls& ctrl = a.controls[control_row(a, car_env, t_next) * static_cast<size_t>(a.control_stride) +
                                                  static_cast<size_t>(idx)];
@@ -666,7 +673,7 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
         }
     }
     int at = q.begin;
-    bool more;
+    bool more, met = false;  // whether any triangle's bounds meet the car's box
     do {
         int noted = 0;
         while (at < q.end && noted + 4 <= kMeshList) {
@@ -676,12 +683,15 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
             if (i < q.end) {
                 const rg::CellEntry en = q.list[i];
                 rank = en.rank;
-                take = q.overlaps(en) && rg::car_triangle_query(tris[rank], qf, pose.thr) == 2;
+                take = q.overlaps(en);
             }
+            at += 4;
+            if (lanes.ballot(take) == 0u) continue;
+            met = true;
+            take = take && rg::car_triangle_query(tris[rank], qf, pose.thr) == 2;
             const unsigned taken = lanes.ballot(take);
             if (take) w.rank[group][noted + __popc(taken & ((1u << lanes.lane()) - 1u))] = rank;
             noted += __popc(taken);
-            at += 4;
         }
         more = at < q.end;
         __syncwarp();
@@ -716,11 +726,19 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
     if (runs && first) {
         m.finish(pose, ws);
         rg::CarStage& st = a.stages[idx];
-        if (ws.count != 0)
+        st.box_clear = ws.count == 0 && !met ? 1u : 0u;
+        if (ws.count != 0) {
             st.ws = ws;
-        else
+        } else {
             st.ws.count = 0;
+            if (st.box_clear) {
+                st.ws.pts[0].local_a = qf.lo;
+                st.ws.pts[0].local_b = qf.hi;
+            }
+        }
         st.res.latest_normal = m.last_normal;
+    } else if (first && k < a.active_car_count) {
+        a.stages[a.active_cars[k]].box_clear = 0u;
     }
 }
 

@@ -125,15 +125,20 @@ RG_HDI uint32_t car_car_reject_mask(const CarState* cars, const CarConfig* cfgs,
     if (count < 2) return 0u;
     const int n = count < 8 ? count : 8;
     uint32_t live = 0u, reject = 0u;
-    for (int k = 0; k < n; ++k)
+    float radius[8];  // once per car: per pair, these were most of the pass
+    V3 pos[8];
+    for (int k = 0; k < n; ++k) {
         live |= static_cast<uint32_t>((cars[k].is_demoed == 0) & (cars[k].just_respawned == 0)) << k;
+        radius[k] = car_bounding_sphere_radius(cfgs[k]);
+        pos[k] = cars[k].pos;
+    }
     for (int hi = 1; hi < n; ++hi) {
         for (int lo = 0; lo < hi; ++lo) {
             const int slot = car_pair_slot(lo, hi);
             const uint32_t pair_live = (live >> lo) & (live >> hi) & 1u;
             const uint32_t empty = mans[slot].count == 0 ? 1u : 0u;
-            const float md = car_bounding_sphere_radius(cfgs[hi]) + car_bounding_sphere_radius(cfgs[lo]);
-            const uint32_t beyond = !(len2(cars[lo].pos - cars[hi].pos) < md * md) ? 1u : 0u;
+            const float md = radius[hi] + radius[lo];
+            const uint32_t beyond = !(len2(pos[lo] - pos[hi]) < md * md) ? 1u : 0u;
             reject |= (empty & (beyond | (pair_live ^ 1u))) << slot;
         }
     }

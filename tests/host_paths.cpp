@@ -168,7 +168,8 @@ void hp_step(const HostBatch* b, const rg_sim_config* cfg, const float* vertices
             A.max_cars = mc;
             A.car_base = base;
             rg::ArenaTickSnap snap;
-            rg::arena_tick_begin(env, ball, A, tc, layout, snap, tc.kickoff_seed, e);
+            rg::arena_tick_begin(env, ball, A, tc, snap, tc.kickoff_seed, e);
+            for (int p = 0; p < layout.count; ++p) rg::pad_tick_begin(tc, count, A.pads, p);
             for (int i = 0; i < count; ++i) {
                 rg::RespawnCtx rc{tc.kickoff_seed, e, env.tick, static_cast<uint32_t>(base + i + 1), A.teams[i]};
                 rg::car_tick_pre(A.cars[i], A.controls[i], A.cfgs[i], tc, A.wheels[i], rc, recs[i]);
