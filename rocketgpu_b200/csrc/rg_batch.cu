@@ -257,7 +257,7 @@ int spread_blocks(int64_t items, int shift, int threads) {
     return static_cast<int>((32 * warps + threads - 1) / threads);
 }
 // Resident warps per SM of the spread kernels, from their registers per thread (65,536 per SM).
-constexpr int kWarpsBalls = 16, kWarpsFinish = 8;
+constexpr int kWarpsBalls = 12, kWarpsFinish = 8;
 
 int device_sms(int device) {
     int n = 1;
@@ -283,7 +283,11 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
     return a.meshes ? a.meshes[a.mesh_of[e]] : a.mesh;
 }
 
-__global__ void __launch_bounds__(256) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
+// One thread owns one ball-only arena for all its ticks, bounded by the latency of its chain: two lanes of three idle at
+// 16,384 arenas. 168 registers hold the tick (12 bytes spilled; 266 at 144), and the twelve warps of an SM that they leave
+// room for are more than two lanes per item can fill there: 60 ticks of 16,384 arenas 2,194 us with 128 registers and 16
+// warps, 1,889 with 168 and 12, 1,888 with 255 and 8, 2,365 with 144 and 14.
+__global__ void __maxnreg__(168) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
     const int e = spread_item(shift);
     if (e >= a.env_count) return;
     rg::BallState b = a.balls[e];
