@@ -283,8 +283,8 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
     return a.meshes ? a.meshes[a.mesh_of[e]] : a.mesh;
 }
 
-// One thread owns one ball-only arena for all its ticks, bounded by the latency of its chain: two lanes of three idle at
-// 16,384 arenas. 168 registers hold the tick (12 bytes spilled; 266 at 144), and the twelve warps of an SM that they leave
+// One thread owns one ball-only arena for all its ticks, bounded by the latency of its chain: 16 lanes
+// of a warp idle at 16,384 arenas. 168 registers hold the tick (12 bytes spilled; 266 at 144), and the twelve warps of an SM that they leave
 // room for are more than two lanes per item can fill there: 60 ticks of 16,384 arenas 2,194 us with 128 registers and 16
 // warps, 1,889 with 168 and 12, 1,888 with 255 and 8, 2,365 with 144 and 14.
 __global__ void __maxnreg__(168) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
@@ -750,8 +750,11 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
 // runs side by side: [0, mesh_blocks) four lanes per active car, the geometry of its arena contacts; [mesh_blocks,
 // mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact geometry; the rest one
 // thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets another car's box.
+// Registers: the deepest part, the penetration search, would take 255, which leaves an SM eight warps; held to 168 for
+// twelve it spills 664 bytes in code that few cars reach. A tick's geometry with 255 and with 168 registers: 330 and 272 us
+// at 16,384 mixed arenas, 360 and 288 at 4,095 3v3 arenas that meet, 138 and 137 at 8,191 duels; 128 lose again.
 constexpr int kGeometryThreads = 64;
-__global__ void __launch_bounds__(kGeometryThreads)
+__global__ void __launch_bounds__(kGeometryThreads, 6)
     car_geometry_kernel(const __grid_constant__ CarTickArgs a, int t, int mesh_blocks, int ball_blocks) {
     const int block = static_cast<int>(blockIdx.x);
     if (block < mesh_blocks) {

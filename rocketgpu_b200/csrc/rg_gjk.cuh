@@ -167,35 +167,40 @@ RG_HDI Minkowski make_minkowski(const Shape& s0, const Xform& w0, const Shape& s
 struct SV {
     V3 d, w;
 };
-struct Simplex {
-    int c[4];  // indices into the vertex store
-    float p[4];
-    int rank;
-};
 
 enum GjkStatus { kGjkValid, kGjkInside, kGjkFailed };
 
+// The current simplex is kept in order in registers (constant indices once the loops are unrolled); btGjkEpa2's vertex
+// store, free list and second simplex only decide where a vertex lies, not which it is. Bounded by the latency of its
+// serial chain, as EPA is: a box deep in a triangle takes one lane 62,900 cycles with the simplex in a store behind
+// indices and EPA's faces read back as they are written, 42,000 with the simplex in registers and each face computed from
+// three vertices loaded once; a box above a triangle 17,700 and 16,000.
 struct Gjk {
     Minkowski shape;
     V3 ray;
     float distance;
-    Simplex simplices[2];
-    SV store[4];
-    int free_[4];
-    int nfree;
-    int current;
-    int simplex;  // index of the result simplex
+    V3 d[4], w[4];  // the simplex's vertices: direction and support point
+    float p[4];
+    int rank;
     GjkStatus status;
 
-    RG_HD void getsupport(V3 d, SV& sv) const {
-        sv.d = bdiv(d, blen(d));
+    RG_HD void getsupport(V3 dir, SV& sv) const {
+        sv.d = bdiv(dir, blen(dir));
         sv.w = shape.support(sv.d);
     }
-    RG_HD void removevertice(Simplex& s) { free_[nfree++] = s.c[--s.rank]; }
-    RG_HD void appendvertice(Simplex& s, V3 v) {
-        s.p[s.rank] = 0.0f;
-        s.c[s.rank] = free_[--nfree];
-        getsupport(v, store[s.c[s.rank++]]);
+    RG_HD void removevertice() { --rank; }
+    RG_HD V3 appendvertice(V3 v) {
+        SV sv;
+        getsupport(v, sv);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i != rank) continue;
+            d[i] = sv.d;
+            w[i] = sv.w;
+            p[i] = 0.0f;
+        }
+        ++rank;
+        return sv.w;
     }
     RG_HD static float det(V3 a, V3 b, V3 c) {
         return (a.y * b.z * c.x + a.z * b.x * c.y - a.x * b.z * c.y - a.y * b.x * c.z + a.x * b.y * c.z -
@@ -306,80 +311,74 @@ struct Gjk {
         float alpha = 0.0f;
         V3 lastw[4];
         int clastw = 0;
-        for (int i = 0; i < 4; ++i) free_[i] = i;
-        nfree = 4;
-        current = 0;
         status = kGjkValid;
         distance = 0.0f;
-        simplices[0].rank = 0;
+        rank = 0;
+        for (int i = 0; i < 4; ++i) {
+            d[i] = w[i] = V3{0.0f, 0.0f, 0.0f};
+            p[i] = 0.0f;
+        }
         ray = guess;
         const float sqrl = blen2(ray);
-        appendvertice(simplices[0], sqrl > 0.0f ? -ray : V3{1.0f, 0.0f, 0.0f});
-        simplices[0].p[0] = 1.0f;
-        ray = store[simplices[0].c[0]].w;
+        ray = appendvertice(sqrl > 0.0f ? -ray : V3{1.0f, 0.0f, 0.0f});
+        p[0] = 1.0f;
         sqdist = sqrl;
         lastw[0] = lastw[1] = lastw[2] = lastw[3] = ray;
         do {
-            const int next = 1 - current;
-            Simplex& cs = simplices[current];
-            Simplex& ns = simplices[next];
             const float rl = blen(ray);
             if (rl < kGjkMinDistance) {
                 status = kGjkInside;
                 break;
             }
-            appendvertice(cs, -ray);
-            const V3 w = store[cs.c[cs.rank - 1]].w;
+            const V3 nw = appendvertice(-ray);
             bool found = false;
-            for (int i = 0; i < 4; ++i) {
-                if (blen2(w - lastw[i]) < kGjkDuplicatedEps) {
-                    found = true;
-                    break;
-                }
-            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) found = found || blen2(nw - lastw[i]) < kGjkDuplicatedEps;
             if (found) {
-                removevertice(simplices[current]);
+                removevertice();
                 break;
             }
             clastw = (clastw + 1) & 3;
-            lastw[clastw] = w;
-            const float omega = bdot(ray, w) / rl;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i == clastw) lastw[i] = nw;
+            const float omega = bdot(ray, nw) / rl;
             alpha = omega > alpha ? omega : alpha;
             if (((rl - alpha) - (kGjkAccuracy * rl)) <= 0.0f) {
-                removevertice(simplices[current]);
+                removevertice();
                 break;
             }
-            float weights[4];
+            float weights[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             unsigned mask = 0;
-            switch (cs.rank) {
-                case 2: sqdist = project2(store[cs.c[0]].w, store[cs.c[1]].w, weights, mask); break;
-                case 3: sqdist = project3(store[cs.c[0]].w, store[cs.c[1]].w, store[cs.c[2]].w, weights, mask); break;
-                case 4:
-                    sqdist = project4(store[cs.c[0]].w, store[cs.c[1]].w, store[cs.c[2]].w, store[cs.c[3]].w, weights,
-                                      mask);
-                    break;
+            switch (rank) {
+                case 2: sqdist = project2(w[0], w[1], weights, mask); break;
+                case 3: sqdist = project3(w[0], w[1], w[2], weights, mask); break;
+                case 4: sqdist = project4(w[0], w[1], w[2], w[3], weights, mask); break;
             }
             if (sqdist >= 0.0f) {
-                ns.rank = 0;
                 ray = V3{0.0f, 0.0f, 0.0f};
-                current = next;
-                for (int i = 0, ni = cs.rank; i < ni; ++i) {
-                    if (mask & (1u << i)) {
-                        ns.c[ns.rank] = cs.c[i];
-                        ns.p[ns.rank++] = weights[i];
-                        ray += store[cs.c[i]].w * weights[i];
-                    } else {
-                        free_[nfree++] = cs.c[i];
+                int kept = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i >= rank || !(mask & (1u << i))) continue;
+                    ray += w[i] * weights[i];
+#pragma unroll
+                    for (int j = 0; j <= i; ++j) {
+                        if (j != kept) continue;
+                        d[j] = d[i];
+                        w[j] = w[i];
+                        p[j] = weights[i];
                     }
+                    ++kept;
                 }
+                rank = kept;
                 if (mask == 15) status = kGjkInside;
             } else {
-                removevertice(simplices[current]);
+                removevertice();
                 break;
             }
             if ((++iterations) >= kGjkMaxIterations) status = kGjkFailed;
         } while (status == kGjkValid);
-        simplex = current;
         switch (status) {
             case kGjkValid: distance = blen(ray); break;
             case kGjkInside: distance = 0.0f; break;
@@ -389,79 +388,88 @@ struct Gjk {
     }
 
     // Grow a degenerate simplex to a tetrahedron that encloses the origin (btGjkEpa2 EncloseOrigin).
-    RG_HDI bool enclose4() {
-        const Simplex& s = simplices[simplex];
-        return fabs_(det(store[s.c[0]].w - store[s.c[3]].w, store[s.c[1]].w - store[s.c[3]].w,
-                         store[s.c[2]].w - store[s.c[3]].w)) > 0.0f;
-    }
+    RG_HDI bool enclose4() { return fabs_(det(w[0] - w[3], w[1] - w[3], w[2] - w[3])) > 0.0f; }
     RG_HDI bool enclose3() {
-        Simplex& s = simplices[simplex];
-        const V3 n = bcross(store[s.c[1]].w - store[s.c[0]].w, store[s.c[2]].w - store[s.c[0]].w);
+        const V3 n = bcross(w[1] - w[0], w[2] - w[0]);
         if (blen2(n) > 0.0f) {
-            appendvertice(s, n);
+            appendvertice(n);
             if (enclose4()) return true;
-            removevertice(s);
-            appendvertice(s, -n);
+            removevertice();
+            appendvertice(-n);
             if (enclose4()) return true;
-            removevertice(s);
+            removevertice();
         }
         return false;
     }
     RG_HDI bool enclose2() {
-        Simplex& s = simplices[simplex];
-        const V3 d = store[s.c[1]].w - store[s.c[0]].w;
+        const V3 e = w[1] - w[0];
+#pragma unroll 1
         for (int i = 0; i < 3; ++i) {
             V3 axis{0.0f, 0.0f, 0.0f};
             set_comp(axis, i, 1.0f);
-            const V3 p = bcross(d, axis);
-            if (blen2(p) > 0.0f) {
-                appendvertice(s, p);
+            const V3 pp = bcross(e, axis);
+            if (blen2(pp) > 0.0f) {
+                appendvertice(pp);
                 if (enclose3()) return true;
-                removevertice(s);
-                appendvertice(s, -p);
+                removevertice();
+                appendvertice(-pp);
                 if (enclose3()) return true;
-                removevertice(s);
+                removevertice();
             }
         }
         return false;
     }
     RG_HDI bool enclose1() {
-        Simplex& s = simplices[simplex];
+#pragma unroll 1
         for (int i = 0; i < 3; ++i) {
             V3 axis{0.0f, 0.0f, 0.0f};
             set_comp(axis, i, 1.0f);
-            appendvertice(s, axis);
+            appendvertice(axis);
             if (enclose2()) return true;
-            removevertice(s);
-            appendvertice(s, -axis);
+            removevertice();
+            appendvertice(-axis);
             if (enclose2()) return true;
-            removevertice(s);
+            removevertice();
         }
         return false;
     }
-    RG_HDI bool enclose_origin() {
-        switch (simplices[simplex].rank) {
-            case 1: return enclose1();
-            case 2: return enclose2();
-            case 3: return enclose3();
-            case 4: return enclose4();
-        }
-        return false;
-    }
+    RG_HDI bool enclose_origin();
 };
+
+// GJK ends with fewer than four vertices only on degenerate overlaps: out of line and on a copy, so that the simplex of
+// the other calls stays in registers.
+RG_NOINL bool enclose_degenerate(Gjk& g) {
+    switch (g.rank) {
+        case 1: return g.enclose1();
+        case 2: return g.enclose2();
+        case 3: return g.enclose3();
+    }
+    return false;
+}
+RG_HDI bool Gjk::enclose_origin() {
+    if (rank == 4) return enclose4();
+    Gjk copy = *this;
+    const bool enclosed = enclose_degenerate(copy);
+    *this = copy;
+    return enclosed;
+}
 
 enum EpaStatus { kEpaValid, kEpaTouching, kEpaDegenerated, kEpaNonConvex, kEpaInvalidHull, kEpaOutOfFaces,
                  kEpaOutOfVertices, kEpaAccuracyReached, kEpaFallBack, kEpaFailed };
 
 struct Epa {
-    struct Face {
+    // 16-byte parts, so that a part is one load
+    struct alignas(16) Face {
         V3 n;
         float d;
-        int16_t c[3];  // vertex: 0..63 EPA store, 64+k GJK store k
+        int16_t c[3];  // vertices: 0..63 EPA's own, 64 + k the GJK simplex's
         int16_t f[3];
         int16_t l[2];
         uint8_t e[3];
         uint8_t pass;
+    };
+    struct alignas(16) Vertex {
+        V3 w;
     };
     struct List {
         int16_t root;
@@ -473,7 +481,8 @@ struct Epa {
     int result_rank;
     V3 normal;
     float depth;
-    SV sv_store[kEpaMaxVertices];
+    Vertex vw[kEpaMaxVertices + 4];
+    V3 vd[kEpaMaxVertices + 4];
     Face fc[kEpaMaxFaces];
     int nextsv;
     // The free faces: `stock` holds the faces given back (most recent first), `fresh` the first never-used slot.
@@ -481,9 +490,7 @@ struct Epa {
     // then fresh slots in index order, hands out the same faces in the same order without touching all 128.
     List hull, stock;
     int16_t fresh;
-    const Gjk* gjk;
 
-    RG_HD const SV& vtx(int16_t i) const { return i >= kEpaMaxVertices ? gjk->store[i - kEpaMaxVertices] : sv_store[i]; }
     RG_HD void bind(int16_t fa, int ea, int16_t fb, int eb) {
         fc[fa].e[ea] = static_cast<uint8_t>(eb);
         fc[fa].f[ea] = fb;
@@ -512,10 +519,10 @@ struct Epa {
         hull.count = stock.count = 0;
         fresh = 0;
     }
-    RG_HDI bool getedgedist(int16_t face, int16_t a, int16_t b, float& dist) {
-        const V3 aw = vtx(a).w, bw = vtx(b).w;
+    // `n`: the face's normal, not yet normalized.
+    RG_HDI static bool getedgedist(V3 n, V3 aw, V3 bw, float& dist) {
         const V3 ba = bw - aw;
-        const V3 n_ab = bcross(ba, fc[face].n);
+        const V3 n_ab = bcross(ba, n);
         const float a_dot_nab = bdot(aw, n_ab);
         if (a_dot_nab < 0.0f) {
             const float ba_l2 = blen2(ba);
@@ -534,39 +541,43 @@ struct Epa {
         }
         return false;
     }
+    // The face is computed before it is taken: one that fails stays where the next call finds it (btGjkEpa2 takes it,
+    // links it into the hull and gives it back).
     RG_HDI int16_t newface(int16_t a, int16_t b, int16_t c, bool forced) {
-        if (stock.root >= 0 || fresh < kEpaMaxFaces) {
-            int16_t face;
-            if (stock.root >= 0) {
-                face = stock.root;
-                remove(stock, face);
-            } else {
-                face = fresh++;
-            }
-            append(hull, face);
-            Face& F = fc[face];
-            F.pass = 0;
-            F.c[0] = a;
-            F.c[1] = b;
-            F.c[2] = c;
-            F.n = bcross(vtx(b).w - vtx(a).w, vtx(c).w - vtx(a).w);
-            const float l = blen(F.n);
-            if (l > kEpaAccuracy) {
-                if (!getedgedist(face, a, b, F.d) && !getedgedist(face, b, c, F.d) && !getedgedist(face, c, a, F.d)) {
-                    F.d = bdot(vtx(a).w, F.n) / l;
-                }
-                F.n = bdiv(F.n, l);
-                if (forced || (F.d >= -kEpaPlaneEps)) return face;
-                status = kEpaNonConvex;
-            } else {
-                status = kEpaDegenerated;
-            }
-            remove(hull, face);
-            append(stock, face);
+        if (!(stock.root >= 0 || fresh < kEpaMaxFaces)) {
+            status = kEpaOutOfFaces;
             return -1;
         }
-        status = kEpaOutOfFaces;
-        return -1;
+        const V3 wa = vw[a].w, wb = vw[b].w, wc = vw[c].w;
+        const V3 n = bcross(wb - wa, wc - wa);
+        const float l = blen(n);
+        if (!(l > kEpaAccuracy)) {
+            status = kEpaDegenerated;
+            return -1;
+        }
+        float dist = 0.0f;
+        if (!getedgedist(n, wa, wb, dist) && !getedgedist(n, wb, wc, dist) && !getedgedist(n, wc, wa, dist))
+            dist = bdot(wa, n) / l;
+        if (!(forced || (dist >= -kEpaPlaneEps))) {
+            status = kEpaNonConvex;
+            return -1;
+        }
+        int16_t face;
+        if (stock.root >= 0) {
+            face = stock.root;
+            remove(stock, face);
+        } else {
+            face = fresh++;
+        }
+        append(hull, face);
+        Face& F = fc[face];
+        F.n = bdiv(n, l);
+        F.d = dist;
+        F.c[0] = a;
+        F.c[1] = b;
+        F.c[2] = c;
+        F.pass = 0;
+        return face;
     }
     RG_HDI int16_t findbest() {
         int16_t minf = hull.root;
@@ -585,7 +596,7 @@ struct Epa {
         int nf;
     };
     // Recursive horizon walk of btGjkEpa2 (expand) with an explicit stack of (face, edge, stage) frames.
-    RG_HDI bool expand(int pass, int16_t w, int16_t f0, int e0, Horizon& horizon) {
+    RG_HDI bool expand(int pass, int16_t w, V3 ww, int16_t f0, int e0, Horizon& horizon) {
         const int i1m3[3] = {1, 2, 0};
         const int i2m3[3] = {2, 0, 1};
         struct Frame {
@@ -603,7 +614,7 @@ struct Epa {
             if (top.stage == 0) {
                 if (cf.pass != pass) {
                     const int e1 = i1m3[ce];
-                    if ((bdot(cf.n, vtx(w).w) - cf.d) < -kEpaPlaneEps) {
+                    if ((bdot(cf.n, ww) - cf.d) < -kEpaPlaneEps) {
                         const int16_t nf = newface(cf.c[e1], cf.c[ce], w, false);
                         if (nf >= 0) {
                             bind(nf, 0, top.f, ce);
@@ -658,32 +669,27 @@ struct Epa {
         return ret;
     }
     RG_HDI EpaStatus evaluate(Gjk& g, V3 guess) {
-        gjk = &g;
-        Simplex& simplex = g.simplices[g.simplex];
-        if ((simplex.rank > 1) && g.enclose_origin()) {
-            while (hull.root >= 0) {
-                const int16_t f = hull.root;
-                remove(hull, f);
-                append(stock, f);
-            }
+        if ((g.rank > 1) && g.enclose_origin()) {
             status = kEpaValid;
             nextsv = 0;
-            const V3 w0 = g.store[simplex.c[0]].w, w1 = g.store[simplex.c[1]].w, w2 = g.store[simplex.c[2]].w,
-                     w3 = g.store[simplex.c[3]].w;
-            if (Gjk::det(w0 - w3, w1 - w3, w2 - w3) < 0.0f) {
-                const int tc = simplex.c[0];
-                simplex.c[0] = simplex.c[1];
-                simplex.c[1] = tc;
-                const float tp = simplex.p[0];
-                simplex.p[0] = simplex.p[1];
-                simplex.p[1] = tp;
+            if (Gjk::det(g.w[0] - g.w[3], g.w[1] - g.w[3], g.w[2] - g.w[3]) < 0.0f) {
+                const V3 td = g.d[0], tw = g.w[0];
+                g.d[0] = g.d[1];
+                g.w[0] = g.w[1];
+                g.d[1] = td;
+                g.w[1] = tw;
             }
-            const int16_t s0 = static_cast<int16_t>(kEpaMaxVertices + simplex.c[0]);
-            const int16_t s1 = static_cast<int16_t>(kEpaMaxVertices + simplex.c[1]);
-            const int16_t s2 = static_cast<int16_t>(kEpaMaxVertices + simplex.c[2]);
-            const int16_t s3 = static_cast<int16_t>(kEpaMaxVertices + simplex.c[3]);
-            const int16_t tetra[4] = {newface(s0, s1, s2, true), newface(s1, s0, s3, true), newface(s2, s1, s3, true),
-                                      newface(s0, s2, s3, true)};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                vd[kEpaMaxVertices + i] = g.d[i];
+                vw[kEpaMaxVertices + i].w = g.w[i];
+            }
+            constexpr int16_t s0 = kEpaMaxVertices, s1 = s0 + 1, s2 = s0 + 2, s3 = s0 + 3;
+            int16_t tetra[4];
+#pragma unroll 1
+            for (int k = 0; k < 4; ++k)  // (s0, s1, s2), (s1, s0, s3), (s2, s1, s3), (s0, s2, s3)
+                tetra[k] = newface(k == 1 ? s1 : (k == 2 ? s2 : s0), k == 1 ? s0 : (k == 3 ? s2 : s1), k == 0 ? s2 : s3,
+                                   true);
             if (hull.count == 4) {
                 int16_t best = findbest();
                 Face outer = fc[best];
@@ -701,11 +707,15 @@ struct Epa {
                         const int16_t w = static_cast<int16_t>(nextsv++);
                         bool valid = true;
                         fc[best].pass = static_cast<uint8_t>(++pass);
-                        g.getsupport(fc[best].n, sv_store[w]);
-                        const float wdist = bdot(fc[best].n, sv_store[w].w) - fc[best].d;
+                        SV sv;
+                        g.getsupport(outer.n, sv);
+                        vd[w] = sv.d;
+                        vw[w].w = sv.w;
+                        const float wdist = bdot(outer.n, sv.w) - outer.d;
                         if (wdist > kEpaAccuracy) {
+#pragma unroll 1
                             for (int j = 0; (j < 3) && valid; ++j) {
-                                valid &= expand(pass, w, fc[best].f[j], fc[best].e[j], horizon);
+                                valid &= expand(pass, w, sv.w, fc[best].f[j], fc[best].e[j], horizon);
                             }
                             if (valid && (horizon.nf >= 3)) {
                                 bind(horizon.cf, 1, horizon.ff, 2);
@@ -733,9 +743,10 @@ struct Epa {
                 result_c[0] = outer.c[0];
                 result_c[1] = outer.c[1];
                 result_c[2] = outer.c[2];
-                result_p[0] = blen(bcross(vtx(outer.c[1]).w - projection, vtx(outer.c[2]).w - projection));
-                result_p[1] = blen(bcross(vtx(outer.c[2]).w - projection, vtx(outer.c[0]).w - projection));
-                result_p[2] = blen(bcross(vtx(outer.c[0]).w - projection, vtx(outer.c[1]).w - projection));
+                const V3 o0 = vw[outer.c[0]].w, o1 = vw[outer.c[1]].w, o2 = vw[outer.c[2]].w;
+                result_p[0] = blen(bcross(o1 - projection, o2 - projection));
+                result_p[1] = blen(bcross(o2 - projection, o0 - projection));
+                result_p[2] = blen(bcross(o0 - projection, o1 - projection));
                 const float sum = result_p[0] + result_p[1] + result_p[2];
                 result_p[0] /= sum;
                 result_p[1] /= sum;
@@ -749,7 +760,8 @@ struct Epa {
         normal = nl > 0.0f ? bdiv(normal, nl) : V3{1.0f, 0.0f, 0.0f};
         depth = 0.0f;
         result_rank = 1;
-        result_c[0] = static_cast<int16_t>(kEpaMaxVertices + simplex.c[0]);
+        vd[kEpaMaxVertices] = g.d[0];
+        result_c[0] = static_cast<int16_t>(kEpaMaxVertices);
         result_p[0] = 1.0f;
         return status;
     }
@@ -765,18 +777,13 @@ RG_NOINL bool penetration(const Shape& s0, const Xform& w0, const Shape& s1, con
     r.witness0 = r.witness1 = V3{0.0f, 0.0f, 0.0f};
     Gjk g;
     g.shape = make_minkowski(s0, w0, s1, w1, true);
-    g.ray = V3{0.0f, 0.0f, 0.0f};
-    g.nfree = 0;
-    g.status = kGjkFailed;
-    g.current = 0;
-    g.distance = 0.0f;
     if (g.evaluate(-guess) != kGjkInside) return false;
     Epa epa;
     epa.initialize();
     if (epa.evaluate(g, -guess) == kEpaFailed) return false;
     V3 wsum{0.0f, 0.0f, 0.0f};
     for (int i = 0; i < epa.result_rank; ++i) {
-        V3 dn = epa.vtx(epa.result_c[i]).d;
+        V3 dn = epa.vd[epa.result_c[i]];
         if (blen2(dn) < (1.1920929e-7f * 1.1920929e-7f)) dn = V3{-1.0f, -1.0f, -1.0f};
         dn = bnormalized(dn);
         const V3 sup = support_no_margin(s0, dn) + dn * s0.margin;
@@ -793,18 +800,13 @@ RG_NOINL bool distance(const Shape& s0, const Xform& w0, const Shape& s1, const 
     r.witness0 = r.witness1 = V3{0.0f, 0.0f, 0.0f};
     Gjk g;
     g.shape = make_minkowski(s0, w0, s1, w1, false);
-    g.ray = V3{0.0f, 0.0f, 0.0f};
-    g.nfree = 0;
-    g.status = kGjkFailed;
-    g.current = 0;
-    g.distance = 0.0f;
     if (g.evaluate(guess) != kGjkValid) return false;
     V3 a{0.0f, 0.0f, 0.0f}, b{0.0f, 0.0f, 0.0f};
-    const Simplex& s = g.simplices[g.simplex];
-    for (int i = 0; i < s.rank; ++i) {
-        const float p = s.p[i];
-        a += g.shape.support0(g.store[s.c[i]].d) * p;
-        b += g.shape.support1(-g.store[s.c[i]].d) * p;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (i >= g.rank) continue;
+        a += g.shape.support0(g.d[i]) * g.p[i];
+        b += g.shape.support1(-g.d[i]) * g.p[i];
     }
     r.witness0 = xform(w0, a);
     r.witness1 = xform(w0, b);
