@@ -341,10 +341,11 @@ RG_API int rg_batch_episode_commands(rg_batch* b, int32_t no_touch_ticks, uint64
                                      rg_env_command* device_commands, void* stream);
 
 /* How steps launch (no counterpart in the reference, whose tick-loop graph cache is internal, src/rocketgpu_cuda.cu:
- * 3764-3876): threads per block of the per-arena kernels and of the per-car kernels (32, 64, 128 or 256; defaults
- * 32 and 64), and use_graphs != 0 to capture each distinct step (same controls and commands pointers, strides and
- * tick count) into a CUDA graph on first use and replay it after (up to 16 kept; a change of car counts, pads,
- * kickoff seed, meshes or launch config drops them). Results do not depend on any of these. rocketgpu_b200.autotune
+ * 3764-3876): threads per block of the per-arena kernels (32, 64, 128 or 256; default 32), the same for the per-car
+ * kernels (default 64; checked and kept, but their blocks are fixed by their shared memory), and use_graphs != 0 to
+ * capture each distinct step (same controls and commands pointers, strides and tick count) into a CUDA graph on first
+ * use and replay it after (up to 16 kept; a change of car counts, pads, kickoff seed, meshes or launch config drops
+ * them). Results do not depend on any of these. rocketgpu_b200.autotune
  * picks them by timing. While phase timing is on, steps launch without graphs. */
 typedef struct rg_launch_config {
     int32_t arena_threads, car_threads, use_graphs, reserved;

@@ -1,10 +1,11 @@
 // rg_batch: the C ABI (include/rocketgpu_b200.h) and the sm_100a kernels behind it.
 //
-// Execution model. One CUDA thread owns one arena for the whole launch: it loads the arena's ball and env state from
-// HBM once, runs `ticks` ticks with the state in registers, and stores it back once. Arenas are independent (the
-// reference steps each env in isolation, include/rocketgpu/detail/step/env_step.hpp:7048), so a step is one launch
-// of single-warp blocks with no inter-thread communication; at 16K arenas that is 512 blocks, about 3.5 per SM on the
-// 148 SMs. Ticks per launch amortise the state load/store and launch latency.
+// Execution model. Arenas are independent (the reference steps each env in isolation,
+// include/rocketgpu/detail/step/env_step.hpp:7048). A ball-only batch runs all ticks of a step in one launch, a thread
+// per arena with the state in registers. A batch with cars runs four launches per tick, each split as its work allows:
+// arena_turn_kernel a warp per group of whole arenas, car_geometry_kernel and car_vehicle_kernel by car, lane group and
+// wheel, arena_finish_kernel a thread per arena; their order on the stream is the only synchronisation between arenas'
+// parts.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -120,7 +121,7 @@ struct rg_batch {
     int32_t active_car_count = 0;
     DeviceArray<TurnGroup> turn_groups;
     std::vector<TurnGroup> host_turn_groups;
-    int turn_car_room = 0;   // cars a turn's block has room for, and its bytes of shared memory
+    int turn_car_room = 0, turn_arena_room = 0;  // what a turn's block has room for, and its bytes of shared memory
     size_t turn_shared = 0;
     rg::PadLayout pad_layout{};
     DeviceArray<rg::ArenaRules> rules;  // a custom layout's spawns and goals (b->tc.rules points here), or empty
@@ -178,7 +179,7 @@ struct rg_batch {
     DeviceArray<rg::KickoffSettledRow> settle_rows;
     DeviceArray<int32_t> settle_entry;
     DeviceArray<rg::BallState> settle_ball;
-    // Phase timing (rg_batch_phase_timing): events around the six kernels of every tick, seven per tick.
+    // Phase timing (rg_batch_phase_timing): events around the kernels of every tick.
     bool timing = false;
     std::vector<cudaEvent_t> events;
     size_t events_used = 0;
@@ -239,9 +240,8 @@ __global__ void canonicalize_balls_kernel(rg::BallState* balls, int n) {
 // to one item per warp, whose warps are all resident at once (`warps_per_sm`: by the kernel's registers). The items take
 // the warp's first lanes: local memory interleaves its lanes by words, and items spread over the warp would use a part of
 // each 32-byte sector. Measured, us a tick with full warps and by this rule: the arena finish 171 -> 130 at 1,024 mixed
-// arenas, 541 -> 450 at 4,095 3v3 arenas, 397 -> 330 at 16,384 mixed ones; the tail 41 -> 28, 55 -> 45, 62 -> 54; the
-// post-tick 47 -> 39, 56 -> 51, 73 -> 71; 16,384 ball-only arenas 2,907 -> 2,279 us a 60-tick pass. The car tick start
-// lost (27 -> 44 at 1,024), the arena begin gained nothing: one item per thread in these two.
+// arenas, 541 -> 450 at 4,095 3v3 arenas, 397 -> 330 at 16,384 mixed ones; 16,384 ball-only arenas 2,907 -> 2,279 us a
+// 60-tick pass.
 __device__ __forceinline__ int spread_item(int shift) {
     const int g = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), per = 32 >> shift;
     return (g & 31) < per ? (g >> 5) * per + (g & 31) : 0x7fffffff;
@@ -283,10 +283,9 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
     return a.meshes ? a.meshes[a.mesh_of[e]] : a.mesh;
 }
 
-// One thread owns one ball-only arena for all its ticks, bounded by the latency of its chain: 16 lanes
-// of a warp idle at 16,384 arenas. 168 registers hold the tick (12 bytes spilled; 266 at 144), and the twelve warps of an SM that they leave
-// room for are more than two lanes per item can fill there: 60 ticks of 16,384 arenas 2,194 us with 128 registers and 16
-// warps, 1,889 with 168 and 12, 1,888 with 255 and 8, 2,365 with 144 and 14.
+// One thread owns one ball-only arena for all its ticks: a serial chain, bounded by its latency. 168 registers hold the
+// tick (24 bytes spilled; 266 at 144) and leave room for twelve warps of an SM: 60 ticks of 16,384 arenas 2,194 us with
+// 128 registers and 16 warps, 1,920 with 168 and 12, 1,933 with 255 and 8, 2,365 with 144 and 14.
 __global__ void __maxnreg__(168) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
     const int e = spread_item(shift);
     if (e >= a.env_count) return;
@@ -464,7 +463,7 @@ __device__ __forceinline__ void warp_store(void* global, const void* shared, int
 constexpr int kTurnFinish = 1, kTurnStart = 2;
 __global__ void __launch_bounds__(32, 16)
     arena_turn_kernel(const __grid_constant__ CarTickArgs a, int parts, int t, int report_fields, int t_next,
-                      int car_room) {
+                      int car_room, int arena_room) {
     extern __shared__ __align__(16) unsigned char turn_shared[];
     const int lane = static_cast<int>(threadIdx.x);
     const TurnGroup g = a.turn_groups[blockIdx.x];
@@ -489,6 +488,10 @@ __global__ void __launch_bounds__(32, 16)
         const int below = __shfl_up_sync(0xffffffffu, car_at, d);
         if (lane >= d) car_at += below;
     }
+    // A launch captured before a change of car counts reads the new groups: one that the launch has no room for, or
+    // whose arenas' cars are not the group's, is left as it is, as no index of it could be relied on.
+    const int cars_now = __shfl_sync(0xffffffffu, car_at, 31);
+    if (g.car_count > car_room || g.arena_count > arena_room || cars_now != g.car_count) return;
     car_at -= count;
     if (e >= 0 && arena_idle(a, e)) e = -1;
     for (int j = 0; j < g.car_count; ++j) {
@@ -915,7 +918,7 @@ CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stri
 void launch_turn(const rg_batch* b, const CarTickArgs& a, int parts, int t, int report_fields, int t_next,
                  cudaStream_t s) {
     arena_turn_kernel<<<static_cast<int>(b->host_turn_groups.size()), 32, b->turn_shared, s>>>(
-        a, parts, t, report_fields, t_next, b->turn_car_room);
+        a, parts, t, report_fields, t_next, b->turn_car_room, b->turn_arena_room);
 }
 
 // One tick's launches between two turns. `mark` is called before each and after the last.
@@ -1271,6 +1274,7 @@ void rebuild_turn_groups(rg_batch* b, cudaStream_t s) {
     }
     close();
     b->turn_car_room = (cars_most + 3) / 4 * 4;
+    b->turn_arena_room = arenas_most;
     b->turn_shared = turn_shared_bytes(cars_most, arenas_most, b->pad_layout.count);
     if (!groups.empty())
         check(cudaMemcpyAsync(b->turn_groups.ptr, groups.data(), groups.size() * sizeof(TurnGroup),

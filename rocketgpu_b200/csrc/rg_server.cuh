@@ -101,13 +101,13 @@ struct rg_server {
 namespace {
 
 // Device bytes one arena slot of a pool with `max_cars` car slots takes (the per-arena arrays rg_batch_create
-// allocates plus the server's slot tables and control rows).
+// allocates plus the server's slot tables and control rows; not the launch plan, TurnGroup, at most 16 bytes a slot).
 int64_t server_slot_bytes(int max_cars) {
     const int64_t pairs = static_cast<int64_t>(max_cars) * (max_cars - 1) / 2;
     const int64_t per_arena = sizeof(rg::BallState) + sizeof(rg::EnvState) + sizeof(int32_t) +
                               sizeof(rg::BallWorldScratch) + 34 * sizeof(rg::PadState) + sizeof(rg::Broadphase) +
                               pairs * sizeof(rg::CarCarManifold) + sizeof(rg::ArenaTickSnap) + 2 * sizeof(int32_t) +
-                              sizeof(rg::EnvCommand) + sizeof(TurnGroup) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
+                              sizeof(rg::EnvCommand) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
     const int64_t per_car = sizeof(rg::CarState) + sizeof(rg::WheelRuntime) + sizeof(rg::CarConfig) +
                             (1 + kServerMaxTicks) * sizeof(rg::CarControls) + 1 + sizeof(rg::CarWorldScratch) +
                             sizeof(rg::BallCarScratch) + sizeof(rg::CarTickRecord) + sizeof(rg::CarStage) +
