@@ -1238,7 +1238,9 @@ void launch_tick(rg_batch* b, int ticks, cudaStream_t s) {
 }
 
 // The groups of a turn, along the step order: whole arenas, up to kTurnCars cars (or one arena). Fewer cars per group,
-// down to one arena, while the chip has warps to spare (kTurnWarps resident per SM, by the kernel's registers). Twelve
+// down to one arena, while the chip has warps to spare (kTurnWarps resident per SM, by the kernel's registers), and no
+// more groups than those while whole arenas allow it: a few groups more are a second wave (8,191 duels in 2,731 groups of
+// three 119 us a turn, in 2,048 of four 72; 4,095 3v3 arenas one by one 131, by two 84). Twelve
 // cars take 17 KB of shared memory, so that 13 groups are resident per SM: 187 us a turn at 16,384 mixed arenas, against
 // 221 with up to 32 cars, 216 with 8 (one arena of six, three of two). 168 registers instead of 128 gained 14 us there and
 // lost 18 of 130 us at 4,095 3v3 arenas, where the warps count.
@@ -1251,28 +1253,32 @@ size_t turn_shared_bytes(int cars, int arenas, int pads) {
 }
 void rebuild_turn_groups(rg_batch* b, cudaStream_t s) {
     std::vector<TurnGroup>& groups = b->host_turn_groups;
-    groups.clear();
     const int64_t warps = static_cast<int64_t>(b->sms) * kTurnWarps;
-    const int share = static_cast<int>(std::min<int64_t>(kTurnCars, (b->active_car_count + warps - 1) / warps));
-    TurnGroup g{0, 0, 0, 0};
+    int share = static_cast<int>(std::min<int64_t>(kTurnCars, (b->active_car_count + warps - 1) / warps));
     int cars_most = 0, arenas_most = 0;
-    auto close = [&] {
-        if (g.arena_count == 0) return;
-        groups.push_back(g);
-        cars_most = std::max(cars_most, g.car_count);
-        arenas_most = std::max(arenas_most, g.arena_count);
-        g = TurnGroup{g.arena_first + g.arena_count, 0, g.car_first + g.car_count, 0};
-    };
-    for (int32_t e : b->host_arena_order) {
-        const int n = b->host_car_count[e];
-        if (g.arena_count == kTurnArenas || (g.car_count + n > share && g.car_count > 0) ||
-            turn_shared_bytes(std::max(cars_most, g.car_count + n), std::max(arenas_most, g.arena_count + 1),
-                              b->pad_layout.count) > kTurnSharedMax)
-            close();
-        ++g.arena_count;
-        g.car_count += n;
+    for (;; ++share) {
+        groups.clear();
+        cars_most = arenas_most = 0;
+        TurnGroup g{0, 0, 0, 0};
+        auto close = [&] {
+            if (g.arena_count == 0) return;
+            groups.push_back(g);
+            cars_most = std::max(cars_most, g.car_count);
+            arenas_most = std::max(arenas_most, g.arena_count);
+            g = TurnGroup{g.arena_first + g.arena_count, 0, g.car_first + g.car_count, 0};
+        };
+        for (int32_t e : b->host_arena_order) {
+            const int n = b->host_car_count[e];
+            if (g.arena_count == kTurnArenas || (g.car_count + n > share && g.car_count > 0) ||
+                turn_shared_bytes(std::max(cars_most, g.car_count + n), std::max(arenas_most, g.arena_count + 1),
+                                  b->pad_layout.count) > kTurnSharedMax)
+                close();
+            ++g.arena_count;
+            g.car_count += n;
+        }
+        close();
+        if (share >= kTurnCars || static_cast<int64_t>(groups.size()) <= warps) break;
     }
-    close();
     b->turn_car_room = (cars_most + 3) / 4 * 4;
     b->turn_arena_room = arenas_most;
     b->turn_shared = turn_shared_bytes(cars_most, arenas_most, b->pad_layout.count);
