@@ -84,10 +84,10 @@ KERNEL_BYTES = {
     "arena_turn": _TURN,
 }
 KERNEL_NAMES = ("turn_start", "car_geometry", "car_vehicle", "arena_finish", "arena_turn")
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per car of one car_vehicle_kernel launch, from an ncu
-# --set full capture of the mixed workload at 4,096 arenas (13,350 cars: 31.01 MB read + 13.92 MB written); a launch
-# at the bench's size is scaled by its cars (the kernel's traffic is per car: its state, stage and mesh reads).
-KERNEL_TRAFFIC_PER_CAR = {"car_vehicle": (31.014656e6 + 13.916416e6) / 13350}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per car of one launch of each kernel, from an ncu capture of
+# the mixed workload at 4,096 arenas (13,350 cars); a launch at the bench's size is scaled by its cars.
+KERNEL_TRAFFIC_PER_CAR = {"car_geometry": (16.827e6 + 2.588e6) / 13350, "car_vehicle": (27.513e6 + 0.764e6) / 13350,
+                          "arena_finish": (39.797e6 + 6.846e6) / 13350, "arena_turn": (36.203e6 + 1.715e6) / 13350}
 
 
 def peaks():
@@ -494,8 +494,7 @@ def run_ours(args, world, rank, local):
             "bound": "hbm", "kernel": top, "achieved": achieved, "peak": hbm, "unit": "GB/s",
             "frac": achieved / hbm, "peak_source": peak_kind,
             "traffic": KERNEL_TRAFFIC_PER_CAR[top] * cars_total if top in KERNEL_TRAFFIC_PER_CAR else None,
-            "traffic_note": "car_vehicle_kernel alone (the phase also holds car_rays_kernel), 4,096-arena ncu capture "
-                            "scaled by cars",
+            "traffic_note": "4,096-arena ncu capture scaled by cars",
             "algorithmic_bytes_per_launch": top_bytes, "avg_launch_ms": per_launch_ms[top],
             "note": "dominant kernel by device time; the tick is bound by latency and FP32 issue of serial per-arena "
                     "work, not by HBM; frac is the HBM fraction of its algorithmic state bytes"}
