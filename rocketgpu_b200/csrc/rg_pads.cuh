@@ -197,20 +197,18 @@ RG_HDI void pad_touch_step(PadState& pad, int p, CarState& c, uint32_t car_id, b
 struct PadCars {
     CarState *cars, *slots;
     int count, car_base, max_cars;
+    RG_HD CarState& car(int i) const { return i < count ? cars[i] : slots[i]; }
 };
 RG_HDI void pad_give(const PadCars& A, PadState& pad, int p, uint32_t car_id, const TickConfig& tc) {
-    CarState* cars = A.cars;
     const int car_base = A.car_base, max_cars = A.max_cars;
-    CarState& c = cars[static_cast<int>(car_id - 1u) - car_base];
+    CarState& c = A.car(static_cast<int>(car_id - 1u) - car_base);
     const float boost_before = c.boost;
     car_set_boost_amount(c, fmin_(tc.boost_max / 100.0f, car_boost_amount(c) + (pad.is_big ? 1.0f : 0.12f)));
     pad.is_active = 0;
     pad.cooldown = (pad.is_big ? tc.boost_pad_cooldown_big : tc.boost_pad_cooldown_small) - tc.tick_dt;
     pad.pickup_frac_q = pad_frac_q(tc.frame_frac);
-    for (int i = 0; i < A.count; ++i)
-        if (cars[i].boost_pad_touching == p + 1) cars[i].boost_pad_touching = 0;
-    for (int i = A.count; i < max_cars; ++i)
-        if (A.slots[i].boost_pad_touching == p + 1) A.slots[i].boost_pad_touching = 0;
+    for (int i = 0; i < max_cars; ++i)
+        if (A.car(i).boost_pad_touching == p + 1) A.car(i).boost_pad_touching = 0;
     if (tc.events.windows) {
         PhysicsEvent e = new_event(kEventBoostPickup);
         e.car_id = car_id;
@@ -224,7 +222,7 @@ RG_HDI void pad_give(const PadCars& A, PadState& pad, int p, uint32_t car_id, co
 // More than one pad hit in one tick: visit them in order of entry (reference BoostPadSweepTouchSteps, :2587-2637).
 RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, const PadLayout& L,
                                   const TickConfig& tc, uint64_t hits, uint64_t overlap) {
-    CarState& c = A.cars[slot];
+    CarState& c = A.car(slot);
     const uint32_t car_id = static_cast<uint32_t>(A.car_base + slot + 1);
     const V3 to_bt = pad_frame_pos(c, tc.frame_frac) * (1.0f / 50.0f);
     const V3 from_bt = pad_sweep_from_bt(c, to_bt);
@@ -267,12 +265,11 @@ RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, co
 // `staged` holds car slot i's pad contacts (pad_contacts_stage) at byte offset i * staged_stride.
 RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* order, PadState* pads, const PadLayout& L,
                         const TickConfig& tc, const PadContacts* staged, size_t staged_stride) {
-    CarState* cars = A.cars;
     const int count = A.count, car_base = A.car_base;
     if (!tc.enable_boost_pads || tc.frame_frac < 0.0f) return;
     for (int k = 0; k < count; ++k) {
         const int i = order[k];
-        CarState& c = cars[i];
+        CarState& c = A.car(i);
         const PadContacts& pc = *reinterpret_cast<const PadContacts*>(
             reinterpret_cast<const unsigned char*>(staged) + static_cast<size_t>(i) * staged_stride);
         const uint64_t hits = pc.hits, overlap = pc.overlap;
@@ -303,7 +300,7 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
         pad.cooldown = 0.0f;
         pad.is_active = 1;
         for (int k = count - 1; k >= 0; --k) {
-            CarState& c = cars[order[k]];
+            CarState& c = A.car(order[k]);
             if (c.is_demoed) continue;
             const V3 car_uu = pad_frame_pos(c, tc.frame_frac);
             V3 axes[3];
@@ -315,7 +312,7 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
     // the touch list (reference BoostPadTouchListStep, :2555-2561)
     for (int k = count - 1; k >= 0; --k) {
         const int i = order[k];
-        CarState& c = cars[i];
+        CarState& c = A.car(i);
         if (c.boost_pad_touching != 0) {
             const int p = c.boost_pad_touching - 1;
             PadState& pad = pads[p];

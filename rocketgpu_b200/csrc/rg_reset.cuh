@@ -272,10 +272,14 @@ struct KickoffReset {
     bool game_spawn = false;      // the countdown's kickoff: cars appear at their spots a tick and a half later
 };
 
-// The car slot visited k-th under `env`'s visit order (reference CarVisitSlot, rocketgpu.h:575-581).
-RG_HD int reset_visit_slot(const EnvState& env, int k, int count) {
-    if (env.car_visit_order_mode == 1 || env.car_visit_order_mode == 3)
-        return static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
+// The car slot visited k-th under `env`'s visit order (reference CarVisitSlot, rocketgpu.h:575-581). Nothing ties a
+// packed order to the car count: one kept across a change of counts, or uploaded, may name slots past the active cars. A
+// slot that the arena does not have reads as its last one.
+RG_HD int car_visit_slot(const EnvState& env, int k, int count, int max_cars) {
+    if (env.car_visit_order_mode == 1 || env.car_visit_order_mode == 3) {
+        const int slot = static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
+        return slot < max_cars ? slot : max_cars - 1;
+    }
     return env.car_visit_order_mode == 2 ? count - 1 - k : k;
 }
 
@@ -321,7 +325,7 @@ RG_HDI void reset_env_to_kickoff(int env_idx, uint64_t seed, EnvState& env, Ball
     }
     int blue_count = 0, orange_count = 0;
     for (int k = 0; k < count; ++k) {
-        if (teams[reset_visit_slot(next, k, count)] == 0)
+        if (teams[car_visit_slot(next, k, count, max_cars)] == 0)
             ++blue_count;
         else
             ++orange_count;
@@ -381,7 +385,7 @@ RG_HDI void reset_env_to_kickoff(int env_idx, uint64_t seed, EnvState& env, Ball
         int nth = 0;
         bool found = false;
         for (int k = 0; k < count && !found; ++k) {
-            const int s = reset_visit_slot(env, k, count);
+            const int s = car_visit_slot(env, k, count, max_cars);
             if (s == i) {
                 found = true;
             } else if (teams[s] == team) {

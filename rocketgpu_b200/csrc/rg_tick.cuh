@@ -292,6 +292,8 @@ RG_HDI void arena_tick(EnvState& env, BallState& b, BallWorldScratch& s, const T
 struct ArenaCars {
     CarState* cars;        // the active cars, `count` of them
     CarState* slots;       // all the arena's slots in the batch's array (`cars` may be a copy of the active ones)
+    // Slot i's car wherever it lies: a visit order may name slots past the active ones (car_visit_slot).
+    RG_HD CarState& car(int i) const { return i < count ? cars[i] : slots[i]; }
     WheelRuntime* wheels;
     const CarConfig* cfgs;
     PadState* pads;
@@ -302,13 +304,6 @@ struct ArenaCars {
     int count, max_cars, car_base;
 };
 
-// The slot visited k-th (reference CarVisitSlot, rocketgpu.h:575-581).
-RG_HD int car_visit_slot(const EnvState& env, int k, int count) {
-    if (env.car_visit_order_mode == 1 || env.car_visit_order_mode == 3)
-        return static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
-    if (env.car_visit_order_mode == 2) return count - 1 - k;
-    return k;
-}
 // The game's vehicle order kept across demolitions (reference UpdateGameCarVisitOrder, rocketgpu.h:592-634).
 RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int count) {
     if (env.car_visit_order_mode != 3) return;
@@ -1700,7 +1695,7 @@ RG_HDI void arena_cars_in_order(const L& lanes, const EnvState& env, const BallS
                                 CarStage* stages, uint32_t which, VehicleSlot& s) {
     const int count = A.count;
     for (int k = 0; k < count; ++k) {
-        const int i = car_visit_slot(env, k, count);
+        const int i = car_visit_slot(env, k, count, A.max_cars);
         if (!((which >> i) & 1u)) continue;
         vehicle_slot_load(lanes, s, A.cars + i, A.wheels + i, A.cfgs + i);
         lanes.sync();
@@ -1720,7 +1715,7 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
                               CarTickRecord* recs, const ArenaTickSnap& as, CarStage* stages) {
     const int count = A.count;
     int order[8];
-    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
+    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count, A.max_cars);
     if (c.events.windows) {
         // the vehicle updates' car-world events, in the game's car order (each update emits its own in the reference)
         for (int k = 0; k < count; ++k) {
@@ -1766,12 +1761,12 @@ RG_HDI void arena_tick_tail(EnvState& env, BallState& b, const ArenaCars& A, con
                             const TickConfig& c, const CarStage* stages) {
     const int count = A.count;
     int order[8];
-    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
+    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count, A.max_cars);
     if (A.pads)
         pads_tail(PadCars{A.cars, A.slots, count, A.car_base, A.max_cars}, A.cfgs, order, A.pads, pads_layout, c,
                   &stages[0].pads, sizeof(CarStage));
     for (int k = 0; k < count; ++k) {
-        CarState& car = A.cars[order[k]];
+        CarState& car = A.car(order[k]);
         if (!car.is_demoed && car.driving_disabled) --car.driving_disabled;
     }
     apply_ball_extra_hits(b, A.cars, count, c);
@@ -1849,7 +1844,8 @@ RG_HDI void apply_env_command(const EnvCommand& cmd, int env_idx, EnvState& env,
     clear_retained_car_contacts(cs, A.max_cars);
     // the countdown: driving off for its ticks (or until the game timers end it), the ball held in its plane
     // (reference ApplyEnvCommand, env_step.hpp:5747-5752)
-    for (int k = 0; k < count; ++k) A.cars[car_visit_slot(env, k, count)].driving_disabled = cmd.kickoff_countdown_ticks;
+    for (int k = 0; k < count; ++k)
+        A.car(car_visit_slot(env, k, count, A.max_cars)).driving_disabled = cmd.kickoff_countdown_ticks;
     ball.constrained_2d = cmd.kickoff_countdown_ticks;
     if (cmd.reset_scoreboard) {
         env.blue_score = 0;

@@ -1,0 +1,94 @@
+"""What a turn does with states that are not the tick's own: visit orders that name inactive slots. The headers run on the
+CPU, with an arena's active cars in a copy of their own as the turn keeps them, against the batch's array; on a GPU, the
+kernels against the headers."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from rocketgpu_b200 import build
+from tests.test_host_paths import CSRC, MC, ROOT, _build, _same, host_step
+
+OFF_MODE, OFF_ORDER = 17, 20  # env state: the visit order's mode and its slots, four bits each
+OFF_DEMOED, OFF_RESPAWN = 135, 108  # car state
+
+
+@pytest.fixture(scope="module")
+def turn(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("turn_paths") / "turn.so")
+    cuda = os.path.dirname(os.path.dirname(build.nvcc()))
+    subprocess.run(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-ffp-contract=off", "-w", "-I", CSRC, "-I",
+                    os.path.join(ROOT, "include"), "-I", os.path.join(cuda, "include"),
+                    os.path.join(ROOT, "tests", "turn_paths.cpp"), "-o", out], check=True)
+    return ctypes.CDLL(out)
+
+
+@pytest.mark.parametrize("command", [0, 1], ids=["tail", "kickoff command"])
+@pytest.mark.parametrize("mode,order", [(1, 0x76543210), (1, 0x76103245), (3, 0x76043215), (1, 0xFFFFFFFF), (2, 0)])
+def test_visit_order_past_the_active_cars(turn, command, mode, order):
+    for count in range(1, MC + 1):
+        for seed in range(40):
+            assert turn.tp_visit_order(command, mode, ctypes.c_uint32(order), count, seed) == 0, (count, seed)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", ["kept", "uploaded"])
+def test_car_count_lowered_after_play_matches_the_headers(tmp_path_factory, arena_mesh, order):
+    """Six cars, of which the first is demolished and comes back, so that the game's vehicle order ends with it, and is
+    demolished again; then two or three cars without a kickoff: the order visits inactive slots, and the first car, which
+    does nothing, not at all. Or an uploaded order that does so and names a slot that the arena does not have. Bitwise
+    as the headers step it on the host."""
+    import torch
+
+    from rocketgpu_b200.batch_sim import BatchSim, SimConfig, car_preset
+    lib = _build(str(tmp_path_factory.mktemp("host")), "as_is")
+    n, seed = 37, 5
+    rng = np.random.default_rng(seed)
+    sim = BatchSim(SimConfig(kickoff_settled=0, env_count=n, max_cars_per_env=MC), *arena_mesh)
+    sim.set_env_car_count(np.full(n, MC, np.int32))
+    teams = np.tile((np.arange(MC) >= 3).astype(np.uint8), n)
+    cfgs = np.tile(car_preset(0), (n * MC, 1))
+    sim.set_teams(teams)
+    sim.set_car_configs(cfgs)
+    sim.reset_to_kickoff(seed)
+    sim.step(4)
+
+    def demolish_first(seconds):
+        cars = sim.download_car_states()
+        cars[::MC, OFF_DEMOED] = 1
+        cars[::MC, OFF_RESPAWN:OFF_RESPAWN + 4] = np.frombuffer(np.float32(seconds).tobytes(), np.uint8)
+        sim.upload_car_states(cars)
+
+    demolish_first(3 / 120)
+    sim.step(8)
+    assert not sim.download_car_states()[::MC, OFF_DEMOED].any()
+    demolish_first(3.0)
+    sim.step(1)
+    want = 0x76043215
+    if order == "uploaded":
+        envs, want = sim.download_env_states(), 0x70643215
+        envs[:, OFF_MODE] = 1
+        envs[:, OFF_ORDER:OFF_ORDER + 4] = np.frombuffer(np.uint32(want).tobytes(), np.uint8)
+        sim.upload_env_states(envs)
+    assert (sim.download_env_states()[:, OFF_ORDER:OFF_ORDER + 4].copy().view(np.uint32) == want).all()
+    counts = (2 + np.arange(n) % 2).astype(np.int32)
+    sim.set_env_car_count(counts)
+    active = (np.arange(MC)[None, :] < counts[:, None]).reshape(-1)
+    for k in range(10):
+        controls = np.zeros((4, n * MC, 24), np.uint8)
+        axes = rng.uniform(-1, 1, (4, n * MC, 5)).astype(np.float32)
+        axes[..., 0] = 1.0
+        controls[..., :20] = axes.view(np.uint8)
+        want = host_step(lib, sim, arena_mesh, counts, teams, cfgs, seed, controls)
+        dev = torch.from_numpy(controls.reshape(-1)).cuda()
+        sim.step_with_device_controls(dev.data_ptr(), 4, n * MC)
+        sim.synchronize()
+        got = (sim.download_car_states(), sim.download_ball_states(), sim.download_env_states(),
+               sim.download_boost_pad_states())
+        for name, g, w in zip(("cars", "balls", "envs", "pads"), got, want):
+            if name == "cars":
+                g, w = g[active], w[active]
+            assert _same(np.ascontiguousarray(g).view(np.float32), np.ascontiguousarray(w).view(np.float32)), (name, k)
+    sim.close()

@@ -1,0 +1,141 @@
+// Host build of the arena parts of a turn for test_turn_paths.py.
+#include <cstring>
+#include <random>
+#include <vector>
+
+#include "rg_tick.cuh"
+
+namespace {
+
+constexpr int kSlots = 6, kRoom = 16;  // room for every slot that four bits of a packed order can name
+
+// One arena's state, in the middle of play: cars around the boost pads, some of them demolished.
+struct Arena {
+    rg::CarState slots[kRoom];
+    rg::WheelRuntime wheels[kRoom];
+    rg::CarConfig cfgs[kRoom];
+    rg::PadState pads[64];
+    rg::CarControls controls[kRoom];
+    uint8_t teams[kRoom];
+    rg::CarStage stages[kRoom];
+    rg::BallState ball;
+    rg::EnvState env;
+    rg::BallWorldScratch ball_world;
+    rg::Broadphase bp;
+    rg::CarWorldScratch car_world[kRoom];
+    rg::BallCarScratch ball_car[kRoom];
+};
+
+rg::PadLayout pad_layout() {
+    rg::PadLayout l;
+    memset(&l, 0, sizeof(l));
+    l.count = 20;
+    for (int p = 0; p < l.count; ++p) {
+        l.pos[p] = rg::V3{600.0f * static_cast<float>(p % 5) - 1200.0f, 700.0f * static_cast<float>(p / 5) - 1000.0f, 70.0f};
+        l.is_big[p] = p % 4 == 0;
+    }
+    return l;
+}
+
+rg::TickConfig tick_config() {
+    rg::TickConfig tc{};
+    tc.tick_dt = 1.0f / 120.0f;
+    tc.frame_frac = 0.5f;
+    tc.enable_boost_pads = 1;
+    tc.boost_max = 100.0f;
+    tc.boost_spawn_amount = 33.3f;
+    tc.boost_pad_cooldown_big = 10.0f;
+    tc.boost_pad_cooldown_small = 4.0f;
+    tc.car_max_ang_speed = 5.5f;
+    tc.max_cars = kSlots;
+    return tc;
+}
+
+void fill(Arena& a, const rg::PadLayout& l, const rg::TickConfig& tc, unsigned seed) {
+    memset(static_cast<void*>(&a), 0, sizeof(a));
+    std::mt19937 g(seed);
+    std::uniform_real_distribution<float> u(-1.0f, 1.0f);
+    for (int i = 0; i < kRoom; ++i) {
+        rg::CarState& c = a.slots[i];
+        const rg::V3 p = l.pos[g() % l.count];
+        c.pos_bt = rg::V3{p.x + 200.0f * u(g), p.y + 200.0f * u(g), 17.0f} * rg::kUuToBt;
+        c.tick_start_pos_bt = c.pos_bt - rg::V3{0.3f * u(g), 0.3f * u(g), 0.0f};
+        c.rot = rg::Q4{1.0f, 0.0f, 0.0f, 0.0f};
+        c.boost = 50.0f + 50.0f * u(g);
+        c.is_demoed = g() % 5 == 0;
+        c.driving_disabled = static_cast<uint16_t>(g() % 3);
+        c.boost_pad_touching = static_cast<uint8_t>(g() % (l.count + 1));
+        a.cfgs[i].hitbox_size = rg::V3{118.0f, 84.0f, 36.0f};
+        a.cfgs[i].hitbox_offset = rg::V3{13.9f, 0.0f, 20.8f};
+        a.teams[i] = static_cast<uint8_t>(i & 1);
+    }
+    for (int p = 0; p < 64; ++p) {
+        a.pads[p].is_active = g() % 3 != 0;
+        a.pads[p].is_big = l.is_big[p];
+        a.pads[p].cooldown = a.pads[p].is_active ? 0.0f : (g() % 2 ? 0.004f : 2.0f);
+    }
+    for (int i = 0; i < kRoom; ++i)
+        rg::pad_contacts_stage(a.slots[i], a.cfgs[i], a.pads, l, tc, a.stages[i].pads);
+}
+
+rg::ArenaCars arena_cars(Arena& a, int count) {
+    rg::ArenaCars A{};
+    A.cars = A.slots = a.slots;
+    A.wheels = a.wheels;
+    A.cfgs = a.cfgs;
+    A.pads = a.pads;
+    A.controls = a.controls;
+    A.teams = a.teams;
+    A.count = count;
+    A.max_cars = kSlots;
+    return A;
+}
+
+}  // namespace
+
+extern "C" {
+
+// An arena with `count` active cars of six slots, visited in a packed order: the tail of its tick (command 0) or a kickoff
+// command (1), once on the batch's array and once with the active cars in a copy of their own. Returns 0, or what is
+// wrong: 1 the copy's neighbours were written, 2 the results differ, 4 slots that the arena does not have were written.
+int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned seed) {
+    const rg::PadLayout l = pad_layout();
+    const rg::TickConfig tc = tick_config();
+    std::vector<Arena> both(2);
+    Arena &a = both[0], &b = both[1];
+    fill(a, l, tc, seed);
+    a.env.car_visit_order_mode = static_cast<uint8_t>(mode);
+    a.env.car_visit_order_packed = packed;
+    a.env.car_visit_present_mask = 0xFF;
+    memcpy(static_cast<void*>(&b), &a, sizeof(a));
+    std::vector<rg::CarState> before(a.slots, a.slots + kRoom);
+    rg::EnvCommand cmd;
+    memset(&cmd, 0, sizeof(cmd));
+    cmd.reset_to_kickoff = 1;
+    cmd.kickoff_countdown_ticks = 7;
+    auto run = [&](Arena& x, const rg::ArenaCars& A) {
+        const rg::ArenaContactState cs{&x.ball_world, &x.bp, x.car_world, x.ball_car, nullptr, 0};
+        if (command)
+            rg::apply_env_command(cmd, 0, x.env, x.ball, cs, A, x.controls, l, tc);
+        else
+            rg::arena_tick_tail(x.env, x.ball, A, l, tc, x.stages);
+    };
+    run(a, arena_cars(a, count));
+    std::vector<rg::CarState> packed_cars(kRoom + count + kRoom);
+    memset(static_cast<void*>(packed_cars.data()), 0, packed_cars.size() * sizeof(rg::CarState));
+    rg::ArenaCars A = arena_cars(b, count);
+    A.cars = packed_cars.data() + kRoom;
+    memcpy(static_cast<void*>(A.cars), b.slots, count * sizeof(rg::CarState));
+    run(b, A);
+    memcpy(static_cast<void*>(b.slots), A.cars, count * sizeof(rg::CarState));
+    int wrong = 0;
+    const rg::CarState zero = [] { rg::CarState z; memset(static_cast<void*>(&z), 0, sizeof(z)); return z; }();
+    for (int i = 0; i < kRoom; ++i)
+        if (memcmp(&packed_cars[i], &zero, sizeof(zero)) || memcmp(&packed_cars[kRoom + count + i], &zero, sizeof(zero)))
+            wrong |= 1;
+    if (memcmp(&a, &b, sizeof(a))) wrong |= 2;
+    if (memcmp(a.slots + kSlots, before.data() + kSlots, (kRoom - kSlots) * sizeof(rg::CarState))) wrong |= 4;
+    return wrong;
+}
+
+}  // extern "C"
