@@ -311,6 +311,12 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
     for (int k = 0; k < 8; ++k) order[k] = static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
     uint32_t present = env.car_visit_present_mask;
     auto is_present = [&](int slot) { return slot < count && ((present >> slot) & 1u) != 0u; };
+    // a slot's place, or 8: an uploaded order may leave slots out, which then keep out of it
+    auto place_of = [&](int slot) {
+        int p = 0;
+        while (p < 8 && order[p] != slot) ++p;
+        return p;
+    };
     auto last_present = [&]() {
         int q = -1;
         for (int k = 0; k < 8; ++k)
@@ -319,8 +325,8 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
     };
     for (int s = 0; s < count && s < 8; ++s) {
         if (((present >> s) & 1u) || cars[s].is_demoed) continue;
-        int p = 0;
-        while (order[p] != s) ++p;
+        const int p = place_of(s);
+        if (p == 8) continue;
         const int dst = last_present() + 1;
         for (int k = p; k > dst; --k) order[k] = order[k - 1];
         order[dst < p ? dst : p] = s;
@@ -328,8 +334,8 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
     }
     for (int s = 0; s < count && s < 8; ++s) {
         if (!((present >> s) & 1u) || !cars[s].is_demoed) continue;
-        int p = 0;
-        while (order[p] != s) ++p;
+        const int p = place_of(s);
+        if (p == 8) continue;
         const int q = last_present();
         order[p] = order[q];
         order[q] = s;

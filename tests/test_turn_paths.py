@@ -1,6 +1,6 @@
-"""What a turn does with states that are not the tick's own: visit orders that name inactive slots. The headers run on the
-CPU, with an arena's active cars in a copy of their own as the turn keeps them, against the batch's array; on a GPU, the
-kernels against the headers."""
+"""What a turn does with states that are not the tick's own: visit orders that name inactive slots or leave slots out. The
+headers run on the CPU, with an arena's active cars in a copy of their own as the turn keeps them, against the batch's
+array; on a GPU, the kernels against the headers."""
 import ctypes
 import os
 import subprocess
@@ -31,6 +31,47 @@ def test_visit_order_past_the_active_cars(turn, command, mode, order):
     for count in range(1, MC + 1):
         for seed in range(40):
             assert turn.tp_visit_order(command, mode, ctypes.c_uint32(order), count, seed) == 0, (count, seed)
+
+
+def _game_order(order, present, demoed):
+    """The game's order by its rule: a car that is back takes the place after the last car present, a demolished one trades
+    places with the last one present. Slots that the order leaves out stay out."""
+    count = len(demoed)
+
+    def last(order):
+        return max((k for k, s in enumerate(order) if s < count and present[s]), default=-1)
+
+    for s in range(count):
+        if not present[s] and not demoed[s] and s in order:
+            p, to = order.index(s), last(order) + 1
+            order.insert(min(p, to), order.pop(p))
+            present[s] = 1
+    for s in range(count):
+        if present[s] and demoed[s] and s in order:
+            p, q = order.index(s), last(order)
+            order[p], order[q] = order[q], s
+            present[s] = 0
+    return order, present
+
+
+def test_game_order_of_slots_in_it_and_left_out(turn):
+    """Whole orders and uploaded ones that leave slots out (mode 3 is accepted with any order), every demolition."""
+    rng = np.random.default_rng(2)
+    orders = [list(rng.permutation(8)) for _ in range(60)] + [list(rng.integers(0, 16, 8)) for _ in range(60)] + \
+        [[0] * 8, [7] * 8, [15] * 8]
+    for order in orders:
+        order = [int(s) for s in order]
+        if len(set(order)) != 8:  # the rule for a slot that stands twice is the first place's; keep to left-out ones
+            order = [s if s not in order[:k] else 8 + k % 8 for k, s in enumerate(order)]
+        for count in range(1, MC + 1):
+            for mask in (0xFF, 0, 0x15):
+                demoed = rng.integers(0, 2, count).astype(np.uint8)
+                present = ctypes.c_uint8(mask)
+                got = turn.tp_update_order(ctypes.c_uint32(sum(s << 4 * k for k, s in enumerate(order))),
+                                           ctypes.byref(present), count, demoed.ctypes.data_as(ctypes.c_void_p))
+                want, bits = _game_order(list(order), [mask >> s & 1 for s in range(16)], demoed)
+                assert got & 0xFFFFFFFF == sum(s << 4 * k for k, s in enumerate(want)), (order, count, mask, demoed)
+                assert present.value == sum(b << s for s, b in enumerate(bits[:8]))
 
 
 @pytest.mark.gpu

@@ -138,4 +138,18 @@ int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned s
     return wrong;
 }
 
+// The game's order after cars with the demolition flags `demoed` start a tick; `present` is the mask before and after.
+uint32_t tp_update_order(uint32_t packed, uint8_t* present, int count, const uint8_t* demoed) {
+    rg::EnvState env;
+    memset(&env, 0, sizeof(env));
+    env.car_visit_order_mode = 3;
+    env.car_visit_order_packed = packed;
+    env.car_visit_present_mask = *present;
+    std::vector<rg::CarState> cars(count);
+    for (int i = 0; i < count; ++i) cars[i].is_demoed = demoed[i];
+    rg::update_game_visit_order(env, cars.data(), count);
+    *present = env.car_visit_present_mask;
+    return env.car_visit_order_packed;
+}
+
 }  // extern "C"
