@@ -125,6 +125,13 @@ RG_HDI bool pad_box_overlap(V3 pad_pos_uu, bool is_big, V3 car_uu, const V3 axes
     return true;
 }
 
+// The pad that the car touches, or -1. A car uploaded from a layout with more pads may name one that this layout does not
+// have: no pad.
+RG_HD int pad_touched(const CarState& c, const PadLayout& L) {
+    const int p = c.boost_pad_touching - 1;
+    return p < L.count ? p : -1;
+}
+
 // Pads whose cylinder the car's frame-interpolated point swept through this tick, and the overlaps of the car's box
 // with those pads and with the pad it is touching (reference BoostPadContactsForCar, :2412-2505, custom-layout branch).
 RG_HDI uint64_t pad_contacts_for_car(const CarState& c, const CarConfig& cfg, const PadState* pads,
@@ -146,7 +153,8 @@ RG_HDI uint64_t pad_contacts_for_car(const CarState& c, const CarConfig& cfg, co
         if (pad_sweep_enter(L.pos[p], pads[p].is_big != 0, prev, car_bt, enter)) hits |= 1ull << p;
     }
     uint64_t check = hits;
-    if (c.boost_pad_touching != 0) check |= 1ull << (c.boost_pad_touching - 1);
+    const int touched = pad_touched(c, L);
+    if (touched >= 0) check |= 1ull << touched;
     if (check != 0u) {
         V3 axes[3];
         pad_frame_axes(c, tc, axes);
@@ -226,10 +234,9 @@ RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, co
     const uint32_t car_id = static_cast<uint32_t>(A.car_base + slot + 1);
     const V3 to_bt = pad_frame_pos(c, tc.frame_frac) * (1.0f / 50.0f);
     const V3 from_bt = pad_sweep_from_bt(c, to_bt);
-    if (c.boost_pad_touching != 0 && ((hits >> (c.boost_pad_touching - 1)) & 1u) == 0u) {
-        const int p = c.boost_pad_touching - 1;
-        pad_touch_step(pads[p], p, c, car_id, false, ((overlap >> p) & 1u) != 0u, false);
-    }
+    const int touched = pad_touched(c, L);
+    if (touched >= 0 && ((hits >> touched) & 1u) == 0u)
+        pad_touch_step(pads[touched], touched, c, car_id, false, ((overlap >> touched) & 1u) != 0u, false);
     for (uint64_t left = hits; left != 0u;) {
         int p = -1;
         float best = 0.0f;
@@ -279,7 +286,8 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
         } else {
             const bool eligible = pad_eligible(c, tc);
             uint64_t near = hits;
-            if (c.boost_pad_touching != 0) near |= 1ull << (c.boost_pad_touching - 1);
+            const int touched = pad_touched(c, L);
+            if (touched >= 0) near |= 1ull << touched;
             for (; near != 0u; near &= near - 1u) {
                 const int p = ctz64(near);
                 pad_touch_step(pads[p], p, c, static_cast<uint32_t>(car_base + i + 1), ((hits >> p) & 1u) != 0u,
@@ -313,8 +321,8 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
     for (int k = count - 1; k >= 0; --k) {
         const int i = order[k];
         CarState& c = A.car(i);
-        if (c.boost_pad_touching != 0) {
-            const int p = c.boost_pad_touching - 1;
+        const int p = pad_touched(c, L);
+        if (p >= 0) {
             PadState& pad = pads[p];
             if (pad.is_active && pad.cur_locked_car_id == 0 && pad_eligible(c, tc)) {
                 pad.cur_locked_car_id = static_cast<uint32_t>(car_base + i + 1);

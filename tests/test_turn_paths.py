@@ -1,6 +1,6 @@
-"""What a turn does with states that are not the tick's own: visit orders that name inactive slots or leave slots out. The
-headers run on the CPU, with an arena's active cars in a copy of their own as the turn keeps them, against the batch's
-array; on a GPU, the kernels against the headers."""
+"""What a turn does with states that are not the tick's own: visit orders that name inactive slots or leave slots out, pads
+that the layout does not have. The headers run on the CPU, with an arena's active cars in a copy of their own as the turn
+keeps them, against the batch's array; on a GPU, the kernels against the headers."""
 import ctypes
 import os
 import subprocess
@@ -31,6 +31,13 @@ def test_visit_order_past_the_active_cars(turn, command, mode, order):
     for count in range(1, MC + 1):
         for seed in range(40):
             assert turn.tp_visit_order(command, mode, ctypes.c_uint32(order), count, seed) == 0, (count, seed)
+
+
+@pytest.mark.parametrize("touching", [0, 1, 20, 21, 64, 65, 128, 255])
+def test_touched_pad_past_the_layout(turn, touching):
+    """The layout has 20 pads."""
+    for seed in range(60):
+        assert turn.tp_touching(touching, seed) == 0, seed
 
 
 def _game_order(order, present, demoed):

@@ -152,4 +152,35 @@ uint32_t tp_update_order(uint32_t packed, uint8_t* present, int count, const uin
     return env.car_visit_order_packed;
 }
 
+// A tick's pad contacts and tail of an arena whose car 0 touches pad number `touching` (0: none): 0, or 1 when a pad past
+// the layout's was read (one there takes cars, gives none) or changed.
+int tp_touching(int touching, unsigned seed) {
+    const rg::PadLayout l = pad_layout();
+    const rg::TickConfig tc = tick_config();
+    std::vector<rg::PadState> pads(2 * 256);  // the layout's, then other memory: in the second run all taken
+    std::vector<rg::CarState> got[2];
+    for (int k = 0; k < 2; ++k) {
+        std::vector<Arena> one(1);
+        Arena& a = one[0];
+        fill(a, l, tc, seed);
+        a.slots[0].boost_pad_touching = static_cast<uint8_t>(touching);
+        a.slots[0].is_demoed = 0;
+        memcpy(pads.data(), a.pads, l.count * sizeof(rg::PadState));
+        for (size_t p = l.count; p < pads.size(); ++p) {
+            memset(&pads[p], 0, sizeof(pads[p]));
+            pads[p].is_active = k == 0;
+            pads[p].is_big = k == 0;
+        }
+        const std::vector<rg::PadState> beyond(pads.begin() + l.count, pads.end());
+        for (int i = 0; i < kSlots; ++i)
+            rg::pad_contacts_stage(a.slots[i], a.cfgs[i], pads.data(), l, tc, a.stages[i].pads);
+        rg::ArenaCars A = arena_cars(a, kSlots);
+        A.pads = pads.data();
+        rg::arena_tick_tail(a.env, a.ball, A, l, tc, a.stages);
+        if (memcmp(beyond.data(), pads.data() + l.count, beyond.size() * sizeof(rg::PadState))) return 1;
+        got[k].assign(a.slots, a.slots + kSlots);
+    }
+    return memcmp(got[0].data(), got[1].data(), kSlots * sizeof(rg::CarState)) != 0;
+}
+
 }  // extern "C"
