@@ -269,7 +269,10 @@ RG_API void rg_batch_destroy(rg_batch* b);
 RG_API int64_t rg_batch_env_count(const rg_batch* b);    /* BatchSim::env_count (rocketgpu.h:1012) */
 RG_API int64_t rg_batch_car_capacity(const rg_batch* b); /* BatchSim::car_capacity (rocketgpu.h:1011) */
 
-/* BatchSim::set_env_car_count (rocketgpu.h:1017; range checks src/rocketgpu.cpp:2920-2932). */
+/* BatchSim::set_env_car_count (rocketgpu.h:1017; range checks src/rocketgpu.cpp:2920-2932). A step that the caller has
+ * captured into a CUDA graph of its own is laid out for the counts of its capture: capture it again after this call (the
+ * batch's own graphs are). A replay of the old one stays within the batch's arrays and steps no car twice, but arenas
+ * that it has no room for are stepped in part or not at all. */
 RG_API int rg_batch_set_env_car_count(rg_batch* b, const int32_t* host_counts, size_t count, void* stream);
 /* BatchSim::upload_ball_states / download_ball_states (rocketgpu.h:1023-1046). */
 RG_API int rg_batch_upload_ball_states(rg_batch* b, const rg_ball_state* host, size_t count, void* stream);

@@ -21,6 +21,7 @@
 #include "rg_mesh.h"
 #include "rg_reset.cuh"
 #include "rg_tick.cuh"
+#include "rg_turn.h"
 #include "rg_ucrt.cuh"
 #include "rocketgpu_b200.h"
 
@@ -86,11 +87,6 @@ struct DeviceArray {
 
 }  // namespace
 
-// A group of arenas that one warp of arena_turn_kernel works on: positions in the step order and in the active cars.
-struct TurnGroup {
-    int32_t arena_first, arena_count, car_first, car_count;
-};
-
 struct rg_batch {
     int device = 0;
     rg_sim_config cfg{};
@@ -119,10 +115,8 @@ struct rg_batch {
     DeviceArray<int32_t> arena_order;
     DeviceArray<int32_t> active_cars;
     int32_t active_car_count = 0;
-    DeviceArray<TurnGroup> turn_groups;
-    std::vector<TurnGroup> host_turn_groups;
-    int turn_car_room = 0, turn_arena_room = 0;  // what a turn's block has room for, and its bytes of shared memory
-    size_t turn_shared = 0;
+    DeviceArray<rg::TurnGroup> turn_groups;
+    rg::TurnPlan turn;
     rg::PadLayout pad_layout{};
     DeviceArray<rg::ArenaRules> rules;  // a custom layout's spawns and goals (b->tc.rules points here), or empty
     // Pads stay at their initial state until a car exists or pads are uploaded; until then ball-only arenas skip them.
@@ -357,7 +351,7 @@ struct CarTickArgs {
     const int32_t* active_cars;
     int32_t active_car_count;
     rg::CarStage* stages;
-    const TurnGroup* turn_groups;
+    const rg::TurnGroup* turn_groups;
     const rg::EnvCommand* commands;  // step_with_device_commands: tick t's command for arena e at t * stride + e
     int32_t command_stride;
     rg::CarControls* reset_controls;  // the batch's held controls, cleared by a kickoff reset
@@ -421,6 +415,11 @@ __global__ void apply_commands_kernel(const __grid_constant__ CarTickArgs a, con
                           controls + static_cast<size_t>(e) * a.max_cars, a.pad_layout, a.base.tc);
 }
 
+// The k-th active car, or -1: past the last one, or where a launch captured for more cars than there are now reads on.
+__device__ __forceinline__ int active_car(const CarTickArgs& a, int k) {
+    return k < a.active_car_count ? a.active_cars[k] : -1;
+}
+
 // ---- asynchronous copies into shared memory ----------------------------------------------------------------------
 template <int kBytes>
 __device__ __forceinline__ void copy_async(void* shared, const void* global) {
@@ -466,7 +465,9 @@ __global__ void __launch_bounds__(32, 16)
                       int car_room, int arena_room) {
     extern __shared__ __align__(16) unsigned char turn_shared[];
     const int lane = static_cast<int>(threadIdx.x);
-    const TurnGroup g = a.turn_groups[blockIdx.x];
+    const rg::TurnGroup g = a.turn_groups[blockIdx.x];
+    // a launch captured before a change of car counts has no room for this group, as the header warns: left as it is
+    if (g.car_count > car_room || g.arena_count > arena_room) return;
     const int pad_bytes = a.pad_layout.count * static_cast<int>(sizeof(rg::PadState));
     rg::CarState* cars = reinterpret_cast<rg::CarState*>(turn_shared);
     rg::WheelRuntime* wheels = reinterpret_cast<rg::WheelRuntime*>(cars + car_room);
@@ -488,10 +489,6 @@ __global__ void __launch_bounds__(32, 16)
         const int below = __shfl_up_sync(0xffffffffu, car_at, d);
         if (lane >= d) car_at += below;
     }
-    // A launch captured before a change of car counts reads the new groups: one that the launch has no room for, or
-    // whose arenas' cars are not the group's, is left as it is, as no index of it could be relied on.
-    const int cars_now = __shfl_sync(0xffffffffu, car_at, 31);
-    if (g.car_count > car_room || g.arena_count > arena_room || cars_now != g.car_count) return;
     car_at -= count;
     if (e >= 0 && arena_idle(a, e)) e = -1;
     for (int j = 0; j < g.car_count; ++j) {
@@ -646,10 +643,10 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
     const FourLanes lanes;
     const int lane32 = static_cast<int>(threadIdx.x & 31u), group = lane32 >> 2;
     const bool first = lanes.lane() == 0;
-    int idx = 0, e = 0;
-    bool runs = k < a.active_car_count;
+    const int idx = active_car(a, k);
+    int e = 0;
+    bool runs = idx >= 0;
     if (runs) {
-        idx = a.active_cars[k];
         e = idx / a.max_cars;
         runs = !arena_idle(a, e);
     }
@@ -744,8 +741,8 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
             }
         }
         st.res.latest_normal = m.last_normal;
-    } else if (first && k < a.active_car_count) {
-        a.stages[a.active_cars[k]].box_clear = 0u;
+    } else if (first && idx >= 0) {
+        a.stages[idx].box_clear = 0u;
     }
 }
 
@@ -767,8 +764,8 @@ __global__ void __launch_bounds__(kGeometryThreads, 6)
     }
     if (block < mesh_blocks + ball_blocks) {
         const int k = static_cast<int>((block - mesh_blocks) * blockDim.x + threadIdx.x);
-        if (k >= a.active_car_count) return;
-        const int idx = a.active_cars[k];
+        const int idx = active_car(a, k);
+        if (idx < 0) return;
         const int e = idx / a.max_cars;
         if (arena_idle(a, e)) return;
         rg::car_proxy_ball_stage(a.base.balls[e], a.snaps[e].ball_vel_bt, a.cars[idx], a.car_cfgs[idx], a.base.tc,
@@ -777,8 +774,8 @@ __global__ void __launch_bounds__(kGeometryThreads, 6)
     }
     const int g = static_cast<int>((block - mesh_blocks - ball_blocks) * blockDim.x + threadIdx.x);
     const int k = g >> 2, wheel = g & 3;
-    if (k >= a.active_car_count) return;
-    const int idx = a.active_cars[k];
+    const int idx = active_car(a, k);
+    if (idx < 0) return;
     const int e = idx / a.max_cars;
     if (arena_idle(a, e)) return;
     const rg::CarState& car = a.cars[idx];
@@ -834,8 +831,8 @@ __global__ void __launch_bounds__(kVehicleThreads, 8)
         return;
     }
     const int k = (block - order_blocks) * (kVehicleThreads / 4) + static_cast<int>(threadIdx.x >> 2);
-    if (k >= a.active_car_count) return;
-    const int idx = a.active_cars[k];
+    const int idx = active_car(a, k);
+    if (idx < 0) return;
     const int e = idx / a.max_cars;
     if (arena_idle(a, e)) return;
     const int base = e * a.max_cars, slot = idx - base;
@@ -917,8 +914,8 @@ CarTickArgs car_tick_args(rg_batch* b, const rg::CarControls* controls, int stri
 // A turn (arena_turn_kernel) of every arena.
 void launch_turn(const rg_batch* b, const CarTickArgs& a, int parts, int t, int report_fields, int t_next,
                  cudaStream_t s) {
-    arena_turn_kernel<<<static_cast<int>(b->host_turn_groups.size()), 32, b->turn_shared, s>>>(
-        a, parts, t, report_fields, t_next, b->turn_car_room, b->turn_arena_room);
+    arena_turn_kernel<<<b->turn.count, 32, b->turn.shared, s>>>(a, parts, t, report_fields, t_next, b->turn.car_room,
+                                                                b->turn.arena_room);
 }
 
 // One tick's launches between two turns. `mark` is called before each and after the last.
@@ -1237,57 +1234,6 @@ void launch_tick(rg_batch* b, int ticks, cudaStream_t s) {
     check(cudaGetLastError(), "tick_kernel launch");
 }
 
-// The groups of a turn, along the step order: whole arenas, up to kTurnCars cars (or one arena). Fewer cars per group,
-// down to one arena, while the chip has warps to spare (kTurnWarps resident per SM, by the kernel's registers), and no
-// more groups than those while whole arenas allow it: a few groups more are a second wave (8,191 duels in 2,731 groups of
-// three 119 us a turn, in 2,048 of four 72; 4,095 3v3 arenas one by one 131, by two 84). Twelve
-// cars take 17 KB of shared memory, so that 13 groups are resident per SM: 187 us a turn at 16,384 mixed arenas, against
-// 221 with up to 32 cars, 216 with 8 (one arena of six, three of two). 168 registers instead of 128 gained 14 us there and
-// lost 18 of 130 us at 4,095 3v3 arenas, where the warps count.
-constexpr int kTurnWarps = 16, kTurnCars = 12, kTurnArenas = 16;
-constexpr size_t kTurnSharedMax = 48 * 1024;
-size_t turn_shared_bytes(int cars, int arenas, int pads) {
-    const size_t room = static_cast<size_t>((cars + 3) / 4 * 4);
-    return room * (sizeof(rg::CarState) + sizeof(rg::WheelRuntime)) +
-           static_cast<size_t>(arenas) * static_cast<size_t>(pads) * sizeof(rg::PadState);
-}
-void rebuild_turn_groups(rg_batch* b, cudaStream_t s) {
-    std::vector<TurnGroup>& groups = b->host_turn_groups;
-    const int64_t warps = static_cast<int64_t>(b->sms) * kTurnWarps;
-    int share = static_cast<int>(std::min<int64_t>(kTurnCars, (b->active_car_count + warps - 1) / warps));
-    int cars_most = 0, arenas_most = 0;
-    for (;; ++share) {
-        groups.clear();
-        cars_most = arenas_most = 0;
-        TurnGroup g{0, 0, 0, 0};
-        auto close = [&] {
-            if (g.arena_count == 0) return;
-            groups.push_back(g);
-            cars_most = std::max(cars_most, g.car_count);
-            arenas_most = std::max(arenas_most, g.arena_count);
-            g = TurnGroup{g.arena_first + g.arena_count, 0, g.car_first + g.car_count, 0};
-        };
-        for (int32_t e : b->host_arena_order) {
-            const int n = b->host_car_count[e];
-            if (g.arena_count == kTurnArenas || (g.car_count + n > share && g.car_count > 0) ||
-                turn_shared_bytes(std::max(cars_most, g.car_count + n), std::max(arenas_most, g.arena_count + 1),
-                                  b->pad_layout.count) > kTurnSharedMax)
-                close();
-            ++g.arena_count;
-            g.car_count += n;
-        }
-        close();
-        if (share >= kTurnCars || static_cast<int64_t>(groups.size()) <= warps) break;
-    }
-    b->turn_car_room = (cars_most + 3) / 4 * 4;
-    b->turn_arena_room = arenas_most;
-    b->turn_shared = turn_shared_bytes(cars_most, arenas_most, b->pad_layout.count);
-    if (!groups.empty())
-        check(cudaMemcpyAsync(b->turn_groups.ptr, groups.data(), groups.size() * sizeof(TurnGroup),
-                              cudaMemcpyHostToDevice, s),
-              "turn groups");
-}
-
 // The step order (reference set_env_car_count rebuilds its step order, src/rocketgpu.cpp:2920-2932): arenas stably
 // sorted by car count, largest first (their warps run longest, so they start first and the short ones fill in behind
 // them), and the active car slots of those arenas in that order. The host copies stay in the batch
@@ -1307,12 +1253,20 @@ void rebuild_step_order(rg_batch* b, cudaStream_t s) {
         check(cudaMemcpyAsync(b->arena_order.ptr, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                               s),
               "step order");
+    // Past the active cars and past the groups, where an earlier plan had more of them, there are none: a launch captured
+    // for that plan reads no car and no arena twice.
+    const size_t active = cars.size();
+    if (active < static_cast<size_t>(b->active_car_count)) cars.resize(b->active_car_count, -1);
     if (!cars.empty())
         check(cudaMemcpyAsync(b->active_cars.ptr, cars.data(), cars.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
                               s),
               "active cars");
-    b->active_car_count = static_cast<int32_t>(cars.size());
-    rebuild_turn_groups(b, s);
+    b->active_car_count = static_cast<int32_t>(active);
+    rg::plan_turn(b->turn, order, b->host_car_count, b->active_car_count, b->sms, b->pad_layout.count);
+    if (!b->turn.groups.empty())
+        check(cudaMemcpyAsync(b->turn_groups.ptr, b->turn.groups.data(), b->turn.groups.size() * sizeof(rg::TurnGroup),
+                              cudaMemcpyHostToDevice, s),
+              "turn groups");
 }
 
 rg::TickConfig resolve_tick_config(const rg_sim_config& c) {
@@ -1723,6 +1677,10 @@ RG_API int rg_batch_create(const rg_sim_config* cfg, const rg_arena_layout* layo
                   "car-car manifolds");
         b->car_records.alloc(cap);
         b->car_stages.alloc(cap);
+        if (cap) {
+            check(cudaMemset(b->car_records.ptr, 0, cap * sizeof(rg::CarTickRecord)), "car records");
+            check(cudaMemset(b->car_stages.ptr, 0, cap * sizeof(rg::CarStage)), "car stages");
+        }
         b->arena_snaps.alloc(b->env_count);
         b->command_scratch.alloc(b->env_count);
         b->device_status.alloc(1);

@@ -1,5 +1,5 @@
 """What a turn does with states that are not the tick's own: visit orders that name inactive slots or leave slots out, pads
-that the layout does not have. The headers run on the CPU, with an arena's active cars in a copy of their own as the turn
+that the layout does not have, launches captured for other car counts. The headers run on the CPU, with an arena's active cars in a copy of their own as the turn
 keeps them, against the batch's array; on a GPU, the kernels against the headers."""
 import ctypes
 import os
@@ -79,6 +79,68 @@ def test_game_order_of_slots_in_it_and_left_out(turn):
                 want, bits = _game_order(list(order), [mask >> s & 1 for s in range(16)], demoed)
                 assert got & 0xFFFFFFFF == sum(s << 4 * k for k, s in enumerate(want)), (order, count, mask, demoed)
                 assert present.value == sum(b << s for s, b in enumerate(bits[:8]))
+
+
+@pytest.mark.parametrize("n,sms,pads", [(1, 148, 34), (37, 4, 34), (700, 4, 64), (5000, 148, 34)])
+def test_turn_plans_one_after_another(turn, n, sms, pads):
+    """Car counts raised, lowered, set to none and mixed: a launch captured for any earlier plan finds no arena twice."""
+    rng = np.random.default_rng(n)
+    counts = [np.full(n, MC), rng.integers(0, MC + 1, n), np.full(n, 2), np.zeros(n), rng.integers(0, 2, n),
+              np.arange(n) % 3 * 2, np.full(n, 1), rng.integers(0, MC + 1, n)]
+    counts = np.ascontiguousarray(counts, np.int32)
+    assert turn.tp_plans(counts.ctypes.data_as(ctypes.c_void_p), len(counts), n, sms, pads) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("old,new", [((6, 6, 6, 6), (2, 4, 1, 6)), ((2, 4, 6, 2), (6, 2, 2, 4)), ((1, 1, 2, 2), (6, 0, 3, 4)),
+                                     ((6, 2, 4, 0), (0, 0, 1, 0))])
+def test_replay_of_a_capture_after_car_counts_change(arena_mesh, old, new):
+    """A caller's own capture of a step, replayed after the car counts change. The counts of the first two cases, lowered or
+    traded between arenas, fit what was captured, and it steps them as a new launch would; otherwise it only has to end,
+    and a new launch steps on."""
+    import torch
+
+    from rocketgpu_b200.batch_sim import BatchSim, SimConfig
+    n = 600
+    old, new = (np.array(c, np.int32).repeat(n // 4) for c in (old, new))
+    controls = torch.zeros((4 * n * MC, 24), dtype=torch.uint8, device="cuda")
+    controls.view(torch.float32)[:, 0] = 1.0
+
+    def batch():
+        sim = BatchSim(SimConfig(kickoff_settled=0, env_count=n, max_cars_per_env=MC), *arena_mesh)
+        sim.set_env_car_count(old)
+        sim.set_teams(np.tile((np.arange(MC) % 2).astype(np.uint8), n))
+        sim.reset_to_kickoff(3)
+        return sim
+
+    def state(sim):
+        torch.cuda.synchronize()
+        cars = sim.download_car_states().reshape(n, MC, -1)[np.arange(MC)[None] < new[:, None]]
+        return cars, sim.download_ball_states(), sim.download_env_states(), sim.download_boost_pad_states()
+
+    sim, ref = batch(), batch()
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=side):
+        sim.step_with_device_controls(controls.data_ptr(), 4, n * MC, side.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    ref.step_with_device_controls(controls.data_ptr(), 4, n * MC)
+    for s in (sim, ref):
+        s.set_env_car_count(new)
+    graph.replay()
+    torch.cuda.synchronize()
+    if (new >= 1).all() and new.sum() <= old.sum():
+        ref.step_with_device_controls(controls.data_ptr(), 4, n * MC)
+        for a, b in zip(state(sim), state(ref)):
+            assert np.array_equal(a, b)
+    for s in (sim, ref):
+        s.reset_to_kickoff(8)
+        s.step_with_device_controls(controls.data_ptr(), 4, n * MC)
+    state(sim)
+    sim.close()
+    ref.close()
 
 
 @pytest.mark.gpu

@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "rg_tick.cuh"
+#include "rg_turn.h"
 
 namespace {
 
@@ -181,6 +182,48 @@ int tp_touching(int touching, unsigned seed) {
         got[k].assign(a.slots, a.slots + kSlots);
     }
     return memcmp(got[0].data(), got[1].data(), kSlots * sizeof(rg::CarState)) != 0;
+}
+
+// Plans of a turn for `plans` rows of car counts of n arenas, one after another as a batch makes them. Returns 0, or what is
+// wrong: 1 a plan's own groups do not hold every arena and active car once, in order and within the launch's room; 2 the
+// grid of an earlier plan over a later plan's groups works on an arena twice.
+int tp_plans(const int32_t* counts, int plans, int n, int sms, int pads) {
+    rg::TurnPlan plan;
+    std::vector<int> grids;
+    int wrong = 0;
+    for (int k = 0; k < plans; ++k) {
+        const std::vector<int32_t> count(counts + static_cast<size_t>(k) * n, counts + static_cast<size_t>(k + 1) * n);
+        std::vector<int32_t> order(n);
+        for (int e = 0; e < n; ++e) order[e] = e;
+        std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return count[x] > count[y]; });
+        int active = 0;
+        for (int32_t c : count) active += c;
+        rg::plan_turn(plan, order, count, active, sms, pads);
+        grids.push_back(plan.count);
+        int arena = 0, car = 0;
+        for (int g = 0; g < plan.count; ++g) {
+            const rg::TurnGroup& t = plan.groups[g];
+            int cars = 0;
+            for (int j = 0; j < t.arena_count; ++j) cars += count[order[t.arena_first + j]];
+            if (t.arena_first != arena || t.car_first != car || cars != t.car_count || t.arena_count < 1 ||
+                t.arena_count > std::min(plan.arena_room, 32) || t.car_count > std::min(plan.car_room, 32))
+                wrong |= 1;
+            arena += t.arena_count;
+            car += t.car_count;
+        }
+        if (arena != n || car != active || plan.car_room % 4 ||
+            plan.shared != rg::turn_shared_bytes(plan.car_room, plan.arena_room, pads))
+            wrong |= 1;
+        for (int grid : grids) {
+            std::vector<int> seen(n, 0);
+            for (int g = 0; g < grid; ++g) {
+                const rg::TurnGroup& t = plan.groups[g];
+                for (int j = 0; j < t.arena_count; ++j)
+                    if (++seen[order[t.arena_first + j]] > 1) wrong |= 2;
+            }
+        }
+    }
+    return wrong;
 }
 
 }  // extern "C"
