@@ -60,7 +60,7 @@ void edge_info(std::vector<HostTri>& tris, int ia, int ib) {
     const HostTri& tb = tris[ib];
     const V3 va[3] = {ta.a, ta.b, ta.c};
     const V3 vb[3] = {tb.a, tb.b, tb.c};
-    int sa[2] = {-1, -1}, sb[2] = {-1, -1};
+    int sa[3] = {-1, -1, -1}, sb[3] = {-1, -1, -1};  // a triangle that lies on another shares all three
     int shared = 0;
     for (int i = 0; i < 3; ++i) {
         for (int j = 0; j < 3; ++j) {
