@@ -411,6 +411,7 @@ __global__ void apply_commands_kernel(const __grid_constant__ CarTickArgs a, con
     const rg::EnvCommand c = cmds[e];
     if (!rg::env_command_active(c)) return;
     rg::ArenaCars A = arena_cars(a, e, 0);
+    rg::bound_visit_order(a.base.envs[e], A.count, a.max_cars);
     rg::apply_env_command(c, e, a.base.envs[e], a.base.balls[e], arena_contact_state(a, e), A,
                           controls + static_cast<size_t>(e) * a.max_cars, a.pad_layout, a.base.tc);
 }
@@ -510,6 +511,7 @@ __global__ void __launch_bounds__(32, 16)
     if (e >= 0) {
         b = a.base.balls[e];
         env = a.base.envs[e];
+        rg::bound_visit_order(env, count, a.max_cars);
     }
     copy_async_wait();
     __syncwarp();
@@ -1027,6 +1029,7 @@ __global__ void reset_kickoff_kernel(const __grid_constant__ CarTickArgs a, cons
         a.ball_car[car_base + k].count = 0;
     }
     for (int k = 0; k < a.pair_slots; ++k) a.pairs[static_cast<size_t>(e) * a.pair_slots + k].count = 0;
+    rg::bound_visit_order(a.base.envs[e], a.base.env_car_count[e], a.max_cars);
     rg::reset_env_to_kickoff(j, seed, a.base.envs[e], a.base.balls[e], a.base.ball_world[e], a.cars + car_base,
                              a.wheels + car_base, a.car_cfgs + car_base, controls + car_base,
                              a.pads ? a.pads + static_cast<size_t>(e) * a.pad_layout.count : nullptr, a.pad_layout,

@@ -200,23 +200,25 @@ RG_HDI void pad_touch_step(PadState& pad, int p, CarState& c, uint32_t car_id, b
     }
 }
 // Pickup: the car gets the pad's boost, the pad starts its cooldown (reference BoostPadGive, :2562-2585).
-// `cars` holds the arena's active cars, `slots` all its slots in the batch's array (the first `count` of them may be out
-// of date); car ids are global slot + 1.
+// `cars` holds the arena's active cars (all its slots, when inactive ones are visited), `slots` all its slots in the batch's
+// array (the first `count` of them may be out of date); car ids are global slot + 1.
 struct PadCars {
     CarState *cars, *slots;
     int count, car_base, max_cars;
-    RG_HD CarState& car(int i) const { return i < count ? cars[i] : slots[i]; }
 };
 RG_HDI void pad_give(const PadCars& A, PadState& pad, int p, uint32_t car_id, const TickConfig& tc) {
+    CarState* cars = A.cars;
     const int car_base = A.car_base, max_cars = A.max_cars;
-    CarState& c = A.car(static_cast<int>(car_id - 1u) - car_base);
+    CarState& c = cars[static_cast<int>(car_id - 1u) - car_base];
     const float boost_before = c.boost;
     car_set_boost_amount(c, fmin_(tc.boost_max / 100.0f, car_boost_amount(c) + (pad.is_big ? 1.0f : 0.12f)));
     pad.is_active = 0;
     pad.cooldown = (pad.is_big ? tc.boost_pad_cooldown_big : tc.boost_pad_cooldown_small) - tc.tick_dt;
     pad.pickup_frac_q = pad_frac_q(tc.frame_frac);
-    for (int i = 0; i < max_cars; ++i)
-        if (A.car(i).boost_pad_touching == p + 1) A.car(i).boost_pad_touching = 0;
+    for (int i = 0; i < A.count; ++i)
+        if (cars[i].boost_pad_touching == p + 1) cars[i].boost_pad_touching = 0;
+    for (int i = A.count; i < max_cars; ++i)
+        if (A.slots[i].boost_pad_touching == p + 1) A.slots[i].boost_pad_touching = 0;
     if (tc.events.windows) {
         PhysicsEvent e = new_event(kEventBoostPickup);
         e.car_id = car_id;
@@ -230,7 +232,7 @@ RG_HDI void pad_give(const PadCars& A, PadState& pad, int p, uint32_t car_id, co
 // More than one pad hit in one tick: visit them in order of entry (reference BoostPadSweepTouchSteps, :2587-2637).
 RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, const PadLayout& L,
                                   const TickConfig& tc, uint64_t hits, uint64_t overlap) {
-    CarState& c = A.car(slot);
+    CarState& c = A.cars[slot];
     const uint32_t car_id = static_cast<uint32_t>(A.car_base + slot + 1);
     const V3 to_bt = pad_frame_pos(c, tc.frame_frac) * (1.0f / 50.0f);
     const V3 from_bt = pad_sweep_from_bt(c, to_bt);
@@ -272,11 +274,12 @@ RG_HDI void pad_sweep_touch_steps(const PadCars& A, int slot, PadState* pads, co
 // `staged` holds car slot i's pad contacts (pad_contacts_stage) at byte offset i * staged_stride.
 RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* order, PadState* pads, const PadLayout& L,
                         const TickConfig& tc, const PadContacts* staged, size_t staged_stride) {
+    CarState* cars = A.cars;
     const int count = A.count, car_base = A.car_base;
     if (!tc.enable_boost_pads || tc.frame_frac < 0.0f) return;
     for (int k = 0; k < count; ++k) {
         const int i = order[k];
-        CarState& c = A.car(i);
+        CarState& c = cars[i];
         const PadContacts& pc = *reinterpret_cast<const PadContacts*>(
             reinterpret_cast<const unsigned char*>(staged) + static_cast<size_t>(i) * staged_stride);
         const uint64_t hits = pc.hits, overlap = pc.overlap;
@@ -308,7 +311,7 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
         pad.cooldown = 0.0f;
         pad.is_active = 1;
         for (int k = count - 1; k >= 0; --k) {
-            CarState& c = A.car(order[k]);
+            CarState& c = cars[order[k]];
             if (c.is_demoed) continue;
             const V3 car_uu = pad_frame_pos(c, tc.frame_frac);
             V3 axes[3];
@@ -320,7 +323,7 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
     // the touch list (reference BoostPadTouchListStep, :2555-2561)
     for (int k = count - 1; k >= 0; --k) {
         const int i = order[k];
-        CarState& c = A.car(i);
+        CarState& c = cars[i];
         const int p = pad_touched(c, L);
         if (p >= 0) {
             PadState& pad = pads[p];
@@ -345,6 +348,14 @@ RG_NOINL void pads_tail(const PadCars& A, const CarConfig* cfgs, const int* orde
             pad.prev_locked_car_id = locked;
         }
     }
+}
+
+// The pads' part for an order that visits inactive slots: with all cars where those are, in the batch's array.
+RG_NOINL void pads_tail_slots(const PadCars& A, const CarConfig* cfgs, const int* order, PadState* pads,
+                              const PadLayout& L, const TickConfig& tc, const PadContacts* staged, size_t staged_stride) {
+    for (int i = 0; i < A.count; ++i) A.slots[i] = A.cars[i];
+    pads_tail(PadCars{A.slots, A.slots, A.count, A.car_base, A.max_cars}, cfgs, order, pads, L, tc, staged, staged_stride);
+    for (int i = 0; i < A.count; ++i) A.cars[i] = A.slots[i];
 }
 
 }  // namespace rg

@@ -272,15 +272,34 @@ struct KickoffReset {
     bool game_spawn = false;      // the countdown's kickoff: cars appear at their spots a tick and a half later
 };
 
-// The car slot visited k-th under `env`'s visit order (reference CarVisitSlot, rocketgpu.h:575-581). Nothing ties a
-// packed order to the car count: one kept across a change of counts, or uploaded, may name slots past the active cars. A
-// slot that the arena does not have reads as its last one.
-RG_HD int car_visit_slot(const EnvState& env, int k, int count, int max_cars) {
-    if (env.car_visit_order_mode == 1 || env.car_visit_order_mode == 3) {
-        const int slot = static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
-        return slot < max_cars ? slot : max_cars - 1;
-    }
+// The car slot visited k-th under `env`'s visit order (reference CarVisitSlot, rocketgpu.h:575-581).
+RG_HD int car_visit_slot(const EnvState& env, int k, int count) {
+    if (env.car_visit_order_mode == 1 || env.car_visit_order_mode == 3)
+        return static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
     return env.car_visit_order_mode == 2 ? count - 1 - k : k;
+}
+// Nothing ties a packed order to the car count: one kept across a change of counts, or uploaded, may name slots past the
+// active cars. A visited slot that the arena does not have becomes its last one where a kernel that visits cars first
+// loads the env, so that no other part has to look.
+RG_NOINL uint32_t bounded_visit_order(uint32_t packed, int count, int max_cars) {
+    for (int k = 0; k < count; ++k)
+        if (static_cast<int>((packed >> (4 * k)) & 0xFu) >= max_cars)
+            packed = (packed & ~(0xFu << (4 * k))) | (static_cast<uint32_t>(max_cars - 1) << (4 * k));
+    return packed;
+}
+// Whether the order visits slots below `slots` only.
+RG_HDI bool visit_order_within(const EnvState& env, int count, int slots) {
+    const uint32_t packed = env.car_visit_order_packed;
+    // a place's slot plus 16 - slots carries into bit 4 when it is not below; even places, then odd ones
+    const uint32_t add = static_cast<uint32_t>(16 - slots) * 0x01010101u;
+    const uint32_t even = ((packed & 0x0F0F0F0Fu) + add) & 0x10101010u;
+    const uint32_t odd = (((packed >> 4) & 0x0F0F0F0Fu) + add) & 0x10101010u;
+    return (((even >> 4) | odd) & ((1u << (4 * count)) - 1u)) == 0u ||
+           (env.car_visit_order_mode != 1 && env.car_visit_order_mode != 3);
+}
+RG_HDI void bound_visit_order(EnvState& env, int count, int max_cars) {
+    if (!visit_order_within(env, count, max_cars))
+        env.car_visit_order_packed = bounded_visit_order(env.car_visit_order_packed, count, max_cars);
 }
 
 // The whole arena (reference ResetEnvToKickoffState + ResetKickoffBall + ResetBoostPads + ResetKickoffCar,
@@ -325,7 +344,7 @@ RG_HDI void reset_env_to_kickoff(int env_idx, uint64_t seed, EnvState& env, Ball
     }
     int blue_count = 0, orange_count = 0;
     for (int k = 0; k < count; ++k) {
-        if (teams[car_visit_slot(next, k, count, max_cars)] == 0)
+        if (teams[car_visit_slot(next, k, count)] == 0)
             ++blue_count;
         else
             ++orange_count;
@@ -385,7 +404,7 @@ RG_HDI void reset_env_to_kickoff(int env_idx, uint64_t seed, EnvState& env, Ball
         int nth = 0;
         bool found = false;
         for (int k = 0; k < count && !found; ++k) {
-            const int s = car_visit_slot(env, k, count, max_cars);
+            const int s = car_visit_slot(env, k, count);
             if (s == i) {
                 found = true;
             } else if (teams[s] == team) {

@@ -292,8 +292,6 @@ RG_HDI void arena_tick(EnvState& env, BallState& b, BallWorldScratch& s, const T
 struct ArenaCars {
     CarState* cars;        // the active cars, `count` of them
     CarState* slots;       // all the arena's slots in the batch's array (`cars` may be a copy of the active ones)
-    // Slot i's car wherever it lies: a visit order may name slots past the active ones (car_visit_slot).
-    RG_HD CarState& car(int i) const { return i < count ? cars[i] : slots[i]; }
     WheelRuntime* wheels;
     const CarConfig* cfgs;
     PadState* pads;
@@ -304,12 +302,15 @@ struct ArenaCars {
     int count, max_cars, car_base;
 };
 
-// The game's vehicle order kept across demolitions (reference UpdateGameCarVisitOrder, rocketgpu.h:592-634).
-RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int count) {
-    if (env.car_visit_order_mode != 3) return;
+// The game's vehicle order kept across demolitions (reference UpdateGameCarVisitOrder, rocketgpu.h:592-634), for the
+// arena's cars with the demolition flags `demoed`. Out of line: it runs in the ticks in which a car goes or comes back.
+struct GameVisitOrder {
+    uint32_t packed, present;
+};
+RG_NOINL GameVisitOrder changed_visit_order(GameVisitOrder o, uint32_t demoed, int count) {
     int order[8];
-    for (int k = 0; k < 8; ++k) order[k] = static_cast<int>((env.car_visit_order_packed >> (4 * k)) & 0xFu);
-    uint32_t present = env.car_visit_present_mask;
+    for (int k = 0; k < 8; ++k) order[k] = static_cast<int>((o.packed >> (4 * k)) & 0xFu);
+    uint32_t present = o.present;
     auto is_present = [&](int slot) { return slot < count && ((present >> slot) & 1u) != 0u; };
     // a slot's place, or 8: an uploaded order may leave slots out, which then keep out of it
     auto place_of = [&](int slot) {
@@ -324,7 +325,7 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
         return q;
     };
     for (int s = 0; s < count && s < 8; ++s) {
-        if (((present >> s) & 1u) || cars[s].is_demoed) continue;
+        if (((present | demoed) >> s) & 1u) continue;
         const int p = place_of(s);
         if (p == 8) continue;
         const int dst = last_present() + 1;
@@ -333,7 +334,7 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
         present |= 1u << s;
     }
     for (int s = 0; s < count && s < 8; ++s) {
-        if (!((present >> s) & 1u) || !cars[s].is_demoed) continue;
+        if (!((present & demoed) >> s & 1u)) continue;
         const int p = place_of(s);
         if (p == 8) continue;
         const int q = last_present();
@@ -343,8 +344,17 @@ RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int cou
     }
     uint32_t packed = 0;
     for (int k = 0; k < 8; ++k) packed |= (static_cast<uint32_t>(order[k]) & 0xFu) << (4 * k);
-    env.car_visit_order_packed = packed;
-    env.car_visit_present_mask = static_cast<uint8_t>(present);
+    return GameVisitOrder{packed, present};
+}
+RG_HDI void update_game_visit_order(EnvState& env, const CarState* cars, int count) {
+    if (env.car_visit_order_mode != 3) return;
+    uint32_t demoed = 0u;
+    for (int s = 0; s < count && s < 8; ++s) demoed |= static_cast<uint32_t>(cars[s].is_demoed != 0) << s;
+    const uint32_t present = env.car_visit_present_mask;
+    if (((present ^ demoed) & ((1u << count) - 1u)) == ((1u << count) - 1u)) return;  // those present are those not demolished
+    const GameVisitOrder o = changed_visit_order(GameVisitOrder{env.car_visit_order_packed, present}, demoed, count);
+    env.car_visit_order_packed = o.packed;
+    env.car_visit_present_mask = static_cast<uint8_t>(o.present);
 }
 
 // A car's tick start (reference StepEnvPreTickCar, env_step.hpp:6751-6873): working fields back from the report
@@ -1701,7 +1711,7 @@ RG_HDI void arena_cars_in_order(const L& lanes, const EnvState& env, const BallS
                                 CarStage* stages, uint32_t which, VehicleSlot& s) {
     const int count = A.count;
     for (int k = 0; k < count; ++k) {
-        const int i = car_visit_slot(env, k, count, A.max_cars);
+        const int i = car_visit_slot(env, k, count);
         if (!((which >> i) & 1u)) continue;
         vehicle_slot_load(lanes, s, A.cars + i, A.wheels + i, A.cfgs + i);
         lanes.sync();
@@ -1721,7 +1731,7 @@ RG_HDI void arena_tick_finish(EnvState& env, BallState& b, BallWorldScratch& s, 
                               CarTickRecord* recs, const ArenaTickSnap& as, CarStage* stages) {
     const int count = A.count;
     int order[8];
-    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count, A.max_cars);
+    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
     if (c.events.windows) {
         // the vehicle updates' car-world events, in the game's car order (each update emits its own in the reference)
         for (int k = 0; k < count; ++k) {
@@ -1767,12 +1777,17 @@ RG_HDI void arena_tick_tail(EnvState& env, BallState& b, const ArenaCars& A, con
                             const TickConfig& c, const CarStage* stages) {
     const int count = A.count;
     int order[8];
-    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count, A.max_cars);
-    if (A.pads)
-        pads_tail(PadCars{A.cars, A.slots, count, A.car_base, A.max_cars}, A.cfgs, order, A.pads, pads_layout, c,
-                  &stages[0].pads, sizeof(CarStage));
+    for (int k = 0; k < count; ++k) order[k] = car_visit_slot(env, k, count);
+    const bool inactive = !visit_order_within(env, count, count);
+    if (A.pads) {
+        const PadCars P{A.cars, A.slots, count, A.car_base, A.max_cars};
+        if (inactive && A.cars != A.slots)
+            pads_tail_slots(P, A.cfgs, order, A.pads, pads_layout, c, &stages[0].pads, sizeof(CarStage));
+        else
+            pads_tail(P, A.cfgs, order, A.pads, pads_layout, c, &stages[0].pads, sizeof(CarStage));
+    }
     for (int k = 0; k < count; ++k) {
-        CarState& car = A.car(order[k]);
+        CarState& car = (order[k] < count ? A.cars : A.slots)[order[k]];
         if (!car.is_demoed && car.driving_disabled) --car.driving_disabled;
     }
     apply_ball_extra_hits(b, A.cars, count, c);
@@ -1850,8 +1865,10 @@ RG_HDI void apply_env_command(const EnvCommand& cmd, int env_idx, EnvState& env,
     clear_retained_car_contacts(cs, A.max_cars);
     // the countdown: driving off for its ticks (or until the game timers end it), the ball held in its plane
     // (reference ApplyEnvCommand, env_step.hpp:5747-5752)
-    for (int k = 0; k < count; ++k)
-        A.car(car_visit_slot(env, k, count, A.max_cars)).driving_disabled = cmd.kickoff_countdown_ticks;
+    for (int k = 0; k < count; ++k) {
+        const int i = car_visit_slot(env, k, count);
+        (i < count ? A.cars : A.slots)[i].driving_disabled = cmd.kickoff_countdown_ticks;
+    }
     ball.constrained_2d = cmd.kickoff_countdown_ticks;
     if (cmd.reset_scoreboard) {
         env.blue_score = 0;

@@ -33,6 +33,20 @@ def test_visit_order_past_the_active_cars(turn, command, mode, order):
             assert turn.tp_visit_order(command, mode, ctypes.c_uint32(order), count, seed) == 0, (count, seed)
 
 
+def test_visited_slots_that_the_arena_does_not_have(turn):
+    """The places visited read as the last slot where they name none of the arena's; all else stays."""
+    rng = np.random.default_rng(4)
+    for order in rng.integers(0, 16, (400, 8)).tolist() + [list(range(8)), [15] * 8]:
+        packed = sum(s << 4 * k for k, s in enumerate(order))
+        for mode in range(4):
+            for max_cars in range(1, MC + 1):
+                for count in range(max_cars + 1):
+                    want = packed if mode in (0, 2) else sum(
+                        (min(s, max_cars - 1) if k < count else s) << 4 * k for k, s in enumerate(order))
+                    got = turn.tp_bound(mode, ctypes.c_uint32(packed), count, max_cars)
+                    assert got & 0xFFFFFFFF == want, (order, mode, count, max_cars)
+
+
 @pytest.mark.parametrize("touching", [0, 1, 20, 21, 64, 65, 128, 255])
 def test_touched_pad_past_the_layout(turn, touching):
     """The layout has 20 pads."""

@@ -96,8 +96,8 @@ rg::ArenaCars arena_cars(Arena& a, int count) {
 
 extern "C" {
 
-// An arena with `count` active cars of six slots, visited in a packed order: the tail of its tick (command 0) or a kickoff
-// command (1), once on the batch's array and once with the active cars in a copy of their own. Returns 0, or what is
+// An arena with `count` active cars of six slots, visited in a packed order: a tick's start and tail (command 0) or a kickoff
+// command and a tick's start (1), once on the batch's array and once with the active cars in a copy of their own. Returns 0, or what is
 // wrong: 1 the copy's neighbours were written, 2 the results differ, 4 slots that the arena does not have were written.
 int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned seed) {
     const rg::PadLayout l = pad_layout();
@@ -116,10 +116,12 @@ int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned s
     cmd.kickoff_countdown_ticks = 7;
     auto run = [&](Arena& x, const rg::ArenaCars& A) {
         const rg::ArenaContactState cs{&x.ball_world, &x.bp, x.car_world, x.ball_car, nullptr, 0};
+        rg::ArenaTickSnap snap;
+        rg::bound_visit_order(x.env, count, kSlots);
         if (command)
             rg::apply_env_command(cmd, 0, x.env, x.ball, cs, A, x.controls, l, tc);
-        else
-            rg::arena_tick_tail(x.env, x.ball, A, l, tc, x.stages);
+        rg::arena_tick_begin(x.env, x.ball, A, tc, snap, 0, 0);
+        if (!command) rg::arena_tick_tail(x.env, x.ball, A, l, tc, x.stages);
     };
     run(a, arena_cars(a, count));
     std::vector<rg::CarState> packed_cars(kRoom + count + kRoom);
@@ -137,6 +139,16 @@ int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned s
     if (memcmp(&a, &b, sizeof(a))) wrong |= 2;
     if (memcmp(a.slots + kSlots, before.data() + kSlots, (kRoom - kSlots) * sizeof(rg::CarState))) wrong |= 4;
     return wrong;
+}
+
+// The packed order after bound_visit_order.
+uint32_t tp_bound(int mode, uint32_t packed, int count, int max_cars) {
+    rg::EnvState env;
+    memset(&env, 0, sizeof(env));
+    env.car_visit_order_mode = static_cast<uint8_t>(mode);
+    env.car_visit_order_packed = packed;
+    rg::bound_visit_order(env, count, max_cars);
+    return env.car_visit_order_packed;
 }
 
 // The game's order after cars with the demolition flags `demoed` start a tick; `present` is the mask before and after.
