@@ -356,11 +356,14 @@ typedef struct rg_launch_config {
 RG_API int rg_batch_set_launch_config(rg_batch* b, const rg_launch_config* config);
 RG_API int rg_batch_get_launch_config(const rg_batch* b, rg_launch_config* config);
 
-/* Per-kernel device time of the stepping path, for profiling (no counterpart in the reference). While enabled, every
- * tick of a car step records CUDA events on the step's stream around its kernels: the turn that starts the step's first
- * tick, the contact geometry, the vehicle updates, the arena finish, and the turn that ends the tick and starts the
- * next. rg_batch_phase_times waits for the last event, returns the device milliseconds of each summed over the ticks
- * since enabling or the previous call (out_ms[6], the last one 0) and the tick count, and starts a new sum. Enabling or
+/* Device time of the stepping path, for profiling (no counterpart in the reference). While enabled, every tick of a car
+ * step records CUDA events on the step's stream. enable = 1 (or any other value but 0 and 2): around the tick's six parts
+ * (arena begin, car tick start, contact geometry and vehicle updates, arena finish, car post-tick, arena tail), of which
+ * the first and the last two, otherwise one launch between two ticks, are launched apart; results do not depend on it.
+ * enable = 2: around the launches as they are without timing (the turn that starts the step's first tick, the contact
+ * geometry, the vehicle updates, the arena finish, the turn that ends the tick and starts the next). rg_batch_phase_times
+ * waits for the last event, returns the device milliseconds of each part or launch summed over the ticks since enabling or
+ * the previous call (out_ms[6]; the sixth is 0 with enable = 2) and the tick count, and starts a new sum. Enabling or
  * disabling also starts a new sum. */
 RG_API int rg_batch_phase_timing(rg_batch* b, int32_t enable);
 RG_API int rg_batch_phase_times(rg_batch* b, float* out_ms, int64_t* out_ticks);

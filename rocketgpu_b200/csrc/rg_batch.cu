@@ -87,6 +87,8 @@ struct DeviceArray {
 
 }  // namespace
 
+constexpr int kTimingOff = 0, kTimingParts = 1, kTimingLaunches = 2;
+
 struct rg_batch {
     int device = 0;
     rg_sim_config cfg{};
@@ -173,8 +175,8 @@ struct rg_batch {
     DeviceArray<rg::KickoffSettledRow> settle_rows;
     DeviceArray<int32_t> settle_entry;
     DeviceArray<rg::BallState> settle_ball;
-    // Phase timing (rg_batch_phase_timing): events around the kernels of every tick.
-    bool timing = false;
+    // Phase timing (rg_batch_phase_timing): events around the parts or the launches of every tick.
+    int timing = kTimingOff;
     std::vector<cudaEvent_t> events;
     size_t events_used = 0;
     void drop_graphs() {
@@ -459,8 +461,9 @@ __device__ __forceinline__ void warp_store(void* global, const void* shared, int
 // its lanes need no other warp's; their cars, wheel records and pads are in shared memory from one end to the other
 // (asynchronous copies, all in flight at once). As four launches (post-tick, tail, begin, tick start) these parts loaded
 // the structs from HBM four times, field by field: 298 us a tick at 16,384 mixed arenas, 60 us for one 1v1 arena.
-// kTurnFinish: tick t ends; kTurnStart: tick t_next begins.
-constexpr int kTurnFinish = 1, kTurnStart = 2;
+// kTurnFinish: tick t ends; kTurnStart: tick t_next begins. Each consists of two parts that phase timing launches apart.
+constexpr int kTurnPost = 1, kTurnTail = 2, kTurnBegin = 4, kTurnPre = 8;
+constexpr int kTurnFinish = kTurnPost | kTurnTail, kTurnStart = kTurnBegin | kTurnPre;
 __global__ void __launch_bounds__(32, 16)
     arena_turn_kernel(const __grid_constant__ CarTickArgs a, int parts, int t, int report_fields, int t_next,
                       int car_room, int arena_room) {
@@ -522,7 +525,7 @@ __global__ void __launch_bounds__(32, 16)
         A.pads = a.pads ? reinterpret_cast<rg::PadState*>(pads + lane * pad_bytes) : nullptr;
         return A;
     };
-    if (parts & kTurnFinish) {
+    if (parts & kTurnPost) {
         // a car's arena is the group's arena whose cars it is among: its pads lie at that arena's place
         int mine = 0;
         for (int j = 1; j < g.arena_count; ++j) {
@@ -539,16 +542,15 @@ __global__ void __launch_bounds__(32, 16)
                               a.pad_layout, a.stages[idx].pads);
         }
         __syncwarp();
-        if (e >= 0) {
-            rg::arena_tick_tail(env, b, arena(t), a.pad_layout, a.base.tc,
-                                a.stages + static_cast<size_t>(e) * a.max_cars);
-            if (a.slots.remaining) {
-                --a.slots.remaining[e];
-                ++a.slots.tick[e];
-            }
+    }
+    if ((parts & kTurnTail) && e >= 0) {
+        rg::arena_tick_tail(env, b, arena(t), a.pad_layout, a.base.tc, a.stages + static_cast<size_t>(e) * a.max_cars);
+        if (a.slots.remaining) {
+            --a.slots.remaining[e];
+            ++a.slots.tick[e];
         }
     }
-    if ((parts & kTurnStart) && e >= 0) {
+    if ((parts & kTurnBegin) && e >= 0) {
         const rg::ArenaCars A = arena(t_next);
         if (a.commands) {
             const rg::EnvCommand c =
@@ -565,14 +567,14 @@ __global__ void __launch_bounds__(32, 16)
         a.base.envs[e] = env;
     }
     __syncwarp();
-    if (parts & kTurnStart)
+    if (parts & kTurnBegin)
         for (int j = 0; j < g.arena_count; ++j) {  // pad timers: the lanes share the pads
             const int ej = __shfl_sync(0xffffffffu, e, j), n = __shfl_sync(0xffffffffu, count, j);
             if (ej < 0 || !a.pads) continue;
             for (int p = lane; p < a.pad_layout.count; p += 32)
                 rg::pad_tick_begin(a.base.tc, n, reinterpret_cast<rg::PadState*>(pads + j * pad_bytes), p);
         }
-    if ((parts & kTurnStart) && idx >= 0) {
+    if ((parts & kTurnPre) && idx >= 0) {
         const rg::CarControls& ctrl = a.controls[control_row(a, car_env, t_next) * static_cast<size_t>(a.control_stride) +
                                                  static_cast<size_t>(idx)];
         const int le = logical_env(a, car_env);
@@ -920,16 +922,18 @@ void launch_turn(const rg_batch* b, const CarTickArgs& a, int parts, int t, int 
                                                                 b->turn.arena_room);
 }
 
-// One tick's launches between two turns. `mark` is called before each and after the last.
+// One tick's launches between two turns. `mark` is called before each and after the last; by part (phase timing), the
+// geometry and the vehicle updates are one.
 template <class Mark>
-void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, cudaStream_t s, Mark&& mark) {
+void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, cudaStream_t s, Mark&& mark,
+                         bool by_part = false) {
     const int64_t arenas = b->env_count, cars = b->active_car_count;
     mark();
     if (cars) {
         const int lanes = blocks_for(4 * cars, kGeometryThreads), each = blocks_for(cars, kGeometryThreads);
         car_geometry_kernel<<<2 * lanes + each, kGeometryThreads, 0, s>>>(a, t, lanes, each);
     }
-    mark();
+    if (!by_part) mark();
     if (cars) {
         const int order = blocks_for(4 * arenas, kVehicleThreads);
         car_vehicle_kernel<<<order + blocks_for(4 * cars, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
@@ -954,7 +958,7 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         b->pads_live = true;
     }
     auto mark = [&] {
-        if (!b->timing) return;
+        if (b->timing == kTimingOff) return;
         if (b->events_used == b->events.size()) {
             cudaEvent_t e;
             check(cudaEventCreate(&e), "cudaEventCreate");
@@ -963,13 +967,24 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
         check(cudaEventRecord(b->events[b->events_used++], s), "cudaEventRecord");
     };
     for (int t = 0; t < ticks; ++t) {
-        mark();
-        if (t == 0) launch_turn(b, a, kTurnStart, 0, 0, 0, s);
-        launch_tick_kernels(b, a, t, s, mark);
         // report fields after the last tick, and after every tick of a command stream (reference StepEnvGeneric,
         // env_step.hpp:7174: report_fields = last tick || has_commands)
         const bool last = t + 1 == ticks;
-        launch_turn(b, a, last ? kTurnFinish : kTurnFinish | kTurnStart, t, (last || commands) ? 1 : 0, t + 1, s);
+        const int report = last || commands ? 1 : 0;
+        mark();
+        if (b->timing == kTimingParts) {
+            launch_turn(b, a, kTurnBegin, 0, 0, t, s);
+            mark();
+            launch_turn(b, a, kTurnPre, 0, 0, t, s);
+            launch_tick_kernels(b, a, t, s, mark, true);
+            launch_turn(b, a, kTurnPost, t, report, 0, s);
+            mark();
+            launch_turn(b, a, kTurnTail, t, 0, 0, s);
+        } else {
+            if (t == 0) launch_turn(b, a, kTurnStart, 0, 0, 0, s);
+            launch_tick_kernels(b, a, t, s, mark);
+            launch_turn(b, a, last ? kTurnFinish : kTurnFinish | kTurnStart, t, report, t + 1, s);
+        }
         mark();
     }
     check(cudaGetLastError(), "car tick launch");
@@ -979,7 +994,7 @@ void launch_car_tick(rg_batch* b, const rg::CarControls* controls, int stride, i
 // with these pointers are captured once and replayed after.
 void step_car_path(rg_batch* b, const rg::CarControls* controls, int stride, int ticks, cudaStream_t s,
                    const rg::EnvCommand* commands, int command_stride) {
-    if (!b->use_graphs || b->timing) {
+    if (!b->use_graphs || b->timing != kTimingOff) {
         launch_car_tick(b, controls, stride, ticks, s, commands, command_stride);
         return;
     }
@@ -2073,7 +2088,7 @@ RG_API int rg_batch_get_launch_config(const rg_batch* b, rg_launch_config* c) {
 RG_API int rg_batch_phase_timing(rg_batch* b, int32_t enable) {
     return guard([&] {
         if (!b) throw std::invalid_argument("null argument");
-        b->timing = enable != 0;
+        b->timing = enable == kTimingLaunches ? kTimingLaunches : (enable != 0 ? kTimingParts : kTimingOff);
         b->events_used = 0;
     });
 }
@@ -2082,14 +2097,14 @@ RG_API int rg_batch_phase_times(rg_batch* b, float* out_ms, int64_t* out_ticks) 
     return guard([&] {
         if (!b || !out_ms) throw std::invalid_argument("null argument");
         DeviceGuard dg(b->device);
-        constexpr int kPhases = 5;
+        const int phases = b->timing == kTimingLaunches ? 5 : 6;
         for (int k = 0; k < 6; ++k) out_ms[k] = 0.0f;
-        const size_t ticks = b->events_used / (kPhases + 1);
+        const size_t ticks = b->events_used / (phases + 1);
         if (ticks) check(cudaEventSynchronize(b->events[b->events_used - 1]), "phase timing sync");
         for (size_t t = 0; t < ticks; ++t)
-            for (int k = 0; k < kPhases; ++k) {
+            for (int k = 0; k < phases; ++k) {
                 float ms = 0.0f;
-                check(cudaEventElapsedTime(&ms, b->events[(kPhases + 1) * t + k], b->events[(kPhases + 1) * t + k + 1]),
+                check(cudaEventElapsedTime(&ms, b->events[(phases + 1) * t + k], b->events[(phases + 1) * t + k + 1]),
                       "phase timing");
                 out_ms[k] += ms;
             }
