@@ -101,13 +101,13 @@ struct rg_server {
 namespace {
 
 // Device bytes one arena slot of a pool with `max_cars` car slots takes (the per-arena arrays rg_batch_create
-// allocates plus the server's slot tables and control rows; not the launch plan, TurnGroup, at most 16 bytes a slot).
+// allocates, without the host commands' array that a pool gives back, plus the server's slot tables and control rows).
 int64_t server_slot_bytes(int max_cars) {
     const int64_t pairs = static_cast<int64_t>(max_cars) * (max_cars - 1) / 2;
     const int64_t per_arena = sizeof(rg::BallState) + sizeof(rg::EnvState) + sizeof(int32_t) +
                               sizeof(rg::BallWorldScratch) + 34 * sizeof(rg::PadState) + sizeof(rg::Broadphase) +
                               pairs * sizeof(rg::CarCarManifold) + sizeof(rg::ArenaTickSnap) + 2 * sizeof(int32_t) +
-                              sizeof(rg::EnvCommand) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
+                              sizeof(rg::TurnGroup) + sizeof(int64_t) + 3 * sizeof(int32_t) + sizeof(uint64_t);
     const int64_t per_car = sizeof(rg::CarState) + sizeof(rg::WheelRuntime) + sizeof(rg::CarConfig) +
                             (1 + kServerMaxTicks) * sizeof(rg::CarControls) + 1 + sizeof(rg::CarWorldScratch) +
                             sizeof(rg::BallCarScratch) + sizeof(rg::CarTickRecord) + sizeof(rg::CarStage) +
@@ -290,6 +290,7 @@ RG_API int rg_server_open(const rg_server_config* scfg, const rg_sim_config* sim
         const int rc = rg_batch_create(&pc, layout, device, &s->pool);
         if (rc != 0) throw std::runtime_error(std::string("pool: ") + g_last_error);
         DeviceGuard dg(device);
+        s->pool->command_scratch.reset();  // no host commands reach a pool
         check(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "cudaStreamCreate");
         s->remaining.alloc(s->capacity);
         s->tick.alloc(s->capacity);
