@@ -344,12 +344,12 @@ RG_API int rg_batch_episode_commands(rg_batch* b, int32_t no_touch_ticks, uint64
                                      rg_env_command* device_commands, void* stream);
 
 /* How steps launch (no counterpart in the reference, whose tick-loop graph cache is internal, src/rocketgpu_cuda.cu:
- * 3764-3876): threads per block of the per-arena kernels (32, 64, 128 or 256; default 32), the same for the per-car
- * kernels (default 64; checked and kept, but their blocks are fixed by their shared memory), and use_graphs != 0 to
+ * 3764-3876): threads per block of the kernels with a thread per arena (32, 64, 128 or 256; default 32), car_threads
+ * (default 64; checked and kept, but the per-car kernels' blocks are fixed by their shared memory), and use_graphs != 0 to
  * capture each distinct step (same controls and commands pointers, strides and tick count) into a CUDA graph on first
  * use and replay it after (up to 16 kept; a change of car counts, pads, kickoff seed, meshes or launch config drops
- * them). Results do not depend on any of these. rocketgpu_b200.autotune
- * picks them by timing. While phase timing is on, steps launch without graphs. */
+ * them). Results do not depend on any of these. rocketgpu_b200.autotune picks arena_threads and use_graphs by timing.
+ * While phase timing is on, steps launch without graphs. */
 typedef struct rg_launch_config {
     int32_t arena_threads, car_threads, use_graphs, reserved;
 } rg_launch_config;

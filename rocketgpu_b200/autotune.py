@@ -1,9 +1,10 @@
-"""Launch autotuner: picks threads per block for the per-arena and per-car kernels and whether steps replay CUDA
-graphs, by timing the caller's own step on the caller's batch.
+"""Launch autotuner: picks threads per block of the kernels with a thread per arena (the world step; a ball-only batch's
+tick) and whether steps replay CUDA graphs, by timing the caller's own step on the caller's batch.
 
-Results never depend on the launch config (each arena and each car is one thread whatever the block size, and a
-graph replays exactly the launches it captured), so the tuner may time candidates on consecutive steps of a live
-batch; run it once the workload is in steady state.
+Results never depend on the launch config (an arena is one thread whatever the block size, and a graph replays exactly
+the launches it captured), so the tuner may time candidates on consecutive steps of a live batch; run it once the workload
+is in steady state. car_threads is part of the config but reaches no launch: the blocks of the kernels that share a car
+among lanes are fixed by their shared memory. One value of it is tried unless the caller names more.
 """
 from __future__ import annotations
 
@@ -16,7 +17,7 @@ from . import abi
 from .batch_sim import _check
 
 ARENA_THREADS = (32, 64, 128)
-CAR_THREADS = (32, 64, 128, 256)
+CAR_THREADS = (64,)
 
 
 def get_config(sim) -> dict:

@@ -133,8 +133,8 @@ struct rg_batch {
     std::vector<int32_t> host_car_count;
     std::vector<int32_t> host_arena_order, host_active_cars;
     int sms = 1;                  // the device's multiprocessors
-    int launch_threads = 32;      // threads per block of the per-arena kernels
-    int car_threads = 64;         // threads per block of the per-car kernels
+    int launch_threads = 32;      // threads per block of the kernels with a thread per arena
+    int car_threads = 64;         // kept for the launch config; reaches no launch
     int pair_slots = 0;
     // CUDA graphs of whole steps (rg_launch_config.use_graphs): one per (controls, stride, commands, stride, ticks),
     // captured on first use and replayed after; any change to what a step's launches capture (car counts, pads,
