@@ -70,24 +70,38 @@ WORKLOADS = {
     "balls": "ball-only arenas, 16384 arenas/GPU, procedural 11k-tri arena, 8 ticks per step",
     "serve": "serving loop (see config.workload)",
 }
-# Algorithmic bytes of one launch (one tick) of each kernel of the car path: read + write of the state it owns, as
-# (bytes per arena, per active car, per car pair). Struct sizes: car 880, wheel record 292, car config 120, controls
-# 24, tick record 136, prestep and predictive contact 76, proxy 148, four wheel rays 160, car/mesh manifold 176, query
-# rows and result 776, car/ball manifold 272, car-pair manifold 260, ball 288, ball contact state 288, env 44,
-# broadphase history 1,376, 34 pads x 16, tick snapshot 24.
-_TURN = (2 * (288 + 44 + 34 * 16) + 24 + 16, 2 * (880 + 292) + 120 + 2 * 24 + 136 + 56, 0)
+# Algorithmic bytes of one launch of each kernel of the car path: read + write of the state it owns, as
+# (bytes per arena, per active car, per car pair). The turn that starts a step only starts a tick, the one that ends it
+# only ends one; arena_turn is the mean of the step's launches but the first. Struct sizes: car 880, wheel record 292, car
+# config 120, controls 24, tick record 136, prestep and predictive contact 76, proxy 148, four wheel rays 160, car/mesh
+# manifold 176, query rows and result 776, car/ball manifold 272, car-pair manifold 260, ball 288, ball contact state
+# 288, env 44, broadphase history 1,376, 34 pads x 16, tick snapshot 24.
+_TURN_STATE = (2 * (288 + 44 + 34 * 16), 2 * (880 + 292) + 120)
+_TURN_STARTS = (24 + 16, 24 + 136)  # tick snapshot and env command; controls and tick record
+_TURN_ENDS = (0, 24 + 56)  # controls, prestep
+_STARTS = (TICKS_PER_STEP - 1) / TICKS_PER_STEP
 KERNEL_BYTES = {
-    "turn_start": _TURN,
+    "turn_start": (_TURN_STATE[0] + _TURN_STARTS[0], _TURN_STATE[1] + _TURN_STARTS[1], 0),
     "car_geometry": (288 + 24 + 216, 880 + 120 + 2 * (176 + 272) + 148 + 160, 0),
     "car_vehicle": (288, 2 * (880 + 292) + 120 + 24 + 136 + 160 + 176 + 776 + 76, 0),
     "arena_finish": (2 * (288 + 288 + 1344) + 44 + 24, 2 * (880 + 176 + 272) + 120 + 136 + 1176, 2 * 260),
-    "arena_turn": _TURN,
+    "arena_turn": tuple(s + e + _STARTS * b for s, e, b in zip(_TURN_STATE, _TURN_ENDS, _TURN_STARTS)) + (0,),
 }
 KERNEL_NAMES = ("turn_start", "car_geometry", "car_vehicle", "arena_finish", "arena_turn")
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per car of one launch of each kernel, from an ncu capture of
 # the mixed workload at 4,096 arenas (13,350 cars); a launch at the bench's size is scaled by its cars.
 KERNEL_TRAFFIC_PER_CAR = {"car_geometry": (16.827e6 + 2.588e6) / 13350, "car_vehicle": (27.513e6 + 0.764e6) / 13350,
                           "arena_finish": (39.797e6 + 6.846e6) / 13350, "arena_turn": (36.203e6 + 1.715e6) / 13350}
+
+
+def kernel_times(phase_ms, ticks):
+    """({kernel: ms a launch}, {kernel: ms a step}) of `ticks` ticks' summed times, KERNEL_NAMES' order: every kernel is
+    launched once a tick, but the turn that starts a step once a step (its time holds the other ticks' gaps between two
+    events, some 2 us each)."""
+    steps = max(1, ticks // TICKS_PER_STEP)
+    launches = {name: steps if name == "turn_start" else max(1, ticks) for name in KERNEL_NAMES}
+    ms = dict(zip(KERNEL_NAMES, phase_ms))
+    return {n: ms[n] / launches[n] for n in ms}, {n: ms[n] / steps for n in ms}
 
 
 def peaks():
@@ -483,9 +497,8 @@ def run_ours(args, world, rank, local):
     if mixed:
         cars_total = int(w.counts.sum())
         pairs_total = int((w.counts * (w.counts - 1) // 2).sum())
-        ticks = max(1, phase_ticks.value)
-        per_launch_ms = {name: phase_ms[k] / ticks for k, name in enumerate(KERNEL_NAMES)}
-        top = max(per_launch_ms, key=per_launch_ms.get)
+        per_launch_ms, per_step_ms = kernel_times(phase_ms, phase_ticks.value)
+        top = max(per_step_ms, key=per_step_ms.get)
         pa, pc, pp = KERNEL_BYTES[top]
         top_bytes = ENVS * pa + cars_total * pc + pairs_total * pp
         achieved = top_bytes / (per_launch_ms[top] / 1e3) / 1e9
@@ -498,7 +511,7 @@ def run_ours(args, world, rank, local):
             "algorithmic_bytes_per_launch": top_bytes, "avg_launch_ms": per_launch_ms[top],
             "note": "dominant kernel by device time; the tick is bound by latency and FP32 issue of serial per-arena "
                     "work, not by HBM; frac is the HBM fraction of its algorithmic state bytes"}
-        line["kernel_ms_per_step"] = {name: ms * TICKS_PER_STEP for name, ms in per_launch_ms.items()}
+        line["kernel_ms_per_step"] = per_step_ms
         # the same digest as the reference CUDA arm's (--impl reference --ref-backend cuda) after the same ticks
         line["final_state_sha"] = hashlib.sha256(final_a[0].tobytes() + final_a[1].tobytes()).hexdigest()[:16]
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
