@@ -252,8 +252,8 @@ int spread_blocks(int64_t items, int shift, int threads) {
     const int64_t warps = ((items << shift) + 31) / 32;
     return static_cast<int>((32 * warps + threads - 1) / threads);
 }
-// Resident warps per SM of the spread kernels, from their registers per thread (65,536 per SM).
-constexpr int kWarpsBalls = 12, kWarpsFinish = 8;
+// Registers per thread of the spread kernels.
+constexpr int kRegistersBalls = 168, kRegistersFinish = 255;
 
 int device_sms(int device) {
     int n = 1;
@@ -282,7 +282,7 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
 // One thread owns one ball-only arena for all its ticks: a serial chain, bounded by its latency. 168 registers hold the
 // tick (24 bytes spilled; 266 at 144) and leave room for twelve warps of an SM: 60 ticks of 16,384 arenas 2,194 us with
 // 128 registers and 16 warps, 1,920 with 168 and 12, 1,933 with 255 and 8, 2,365 with 144 and 14.
-__global__ void __maxnreg__(168) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
+__global__ void __maxnreg__(kRegistersBalls) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
     const int e = spread_item(shift);
     if (e >= a.env_count) return;
     rg::BallState b = a.balls[e];
@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(kVehicleThreads, 8)
 // Tick part 4, one thread per arena in step order: wheel pushes on the ball, then the world step's shared stages.
 // The registers (255) are the ones that remove the spills. Bringing the sweep history (1.4 KB per arena) into shared memory
 // first, by the whole warp, was slower: 333 against 299 us at 16,384 mixed arenas, for the L1 that local memory lost.
-__global__ void __maxnreg__(255) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
+__global__ void __maxnreg__(kRegistersFinish) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
     const int k = spread_item(shift);
     if (k >= a.base.env_count) return;
     const int e = a.arena_order[k];
@@ -939,7 +939,7 @@ void launch_tick_kernels(const rg_batch* b, const CarTickArgs& a, int t, cudaStr
         car_vehicle_kernel<<<order + blocks_for(4 * cars, kVehicleThreads), kVehicleThreads, 0, s>>>(a, t, order);
     }
     mark();
-    const int at = b->launch_threads, finish = spread_shift(arenas, b->sms, kWarpsFinish);
+    const int at = b->launch_threads, finish = spread_shift(arenas, b->sms, rg::resident_warps(kRegistersFinish, at));
     arena_finish_kernel<<<spread_blocks(arenas, finish, at), at, 0, s>>>(a, t, finish);
     mark();
 }
@@ -1247,7 +1247,8 @@ void launch_tick(rg_batch* b, int ticks, cudaStream_t s) {
     a.mesh = b->mesh;
     a.meshes = b->mesh_table.ptr;
     a.mesh_of = b->mesh_table.ptr ? b->mesh_of.ptr : nullptr;
-    const int threads = b->launch_threads, shift = spread_shift(b->env_count, b->sms, kWarpsBalls);
+    const int threads = b->launch_threads;
+    const int shift = spread_shift(b->env_count, b->sms, rg::resident_warps(kRegistersBalls, threads));
     tick_kernel<<<spread_blocks(b->env_count, shift, threads), threads, 0, s>>>(a, ticks, shift);
     check(cudaGetLastError(), "tick_kernel launch");
 }
@@ -2393,7 +2394,8 @@ RG_API int rg_batch_step_static_scratch(rg_batch* b, rg_ball_state* dev_balls, r
         a.mesh = b->mesh;
         a.meshes = b->mesh_table.ptr;
         a.mesh_of = b->mesh_table.ptr ? b->mesh_of.ptr : nullptr;
-        const int threads = b->launch_threads, shift = spread_shift(env_count, b->sms, kWarpsBalls);
+        const int threads = b->launch_threads;
+        const int shift = spread_shift(env_count, b->sms, rg::resident_warps(kRegistersBalls, threads));
         tick_kernel<<<spread_blocks(env_count, shift, threads), threads, 0, s>>>(a, ticks, shift);
         check(cudaGetLastError(), "tick_kernel launch (static scratch)");
     });

@@ -1,4 +1,4 @@
-// The launch plan of a turn (arena_turn_kernel): which arenas each of its warps works on. Host code.
+// Launch plans, host code: how many warps an SM holds, and which arenas each warp of a turn (arena_turn_kernel) works on.
 #pragma once
 
 #include <algorithm>
@@ -8,6 +8,12 @@
 #include "rg_tick.cuh"
 
 namespace rg {
+
+// Warps of a kernel that are resident on an SM at once, by its registers per thread (65,536 an SM, allocated to a thread
+// in eights), in blocks of `threads`.
+inline int resident_warps(int registers, int threads) {
+    return 65536 / ((registers + 7) / 8 * 8 * threads) * (threads / 32);
+}
 
 // A group of arenas that one warp of arena_turn_kernel works on: positions in the step order and in the active cars.
 struct TurnGroup {

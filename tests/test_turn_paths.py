@@ -95,6 +95,35 @@ def test_game_order_of_slots_in_it_and_left_out(turn):
                 assert present.value == sum(b << s for s, b in enumerate(bits[:8]))
 
 
+def test_resident_warps_by_block_size(turn):
+    """168 registers: twelve warps of an SM, but one block of 256 threads; 255: eight, in blocks of any size."""
+    assert [turn.tp_resident_warps(168, t) for t in (32, 64, 128, 256)] == [12, 12, 12, 8]
+    assert [turn.tp_resident_warps(255, t) for t in (32, 64, 128, 256)] == [8, 8, 8, 8]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 37, 5000, 40000])
+def test_ball_batches_by_block_size(arena_mesh, n):
+    """A ball-only batch's arenas are spread over more warps at some block sizes than at others, with the same results."""
+    from rocketgpu_b200 import abi, autotune
+    from rocketgpu_b200.batch_sim import BatchSim, SimConfig
+    from tests import scenarios
+    ball = np.zeros(288, np.uint8)
+    abi.lib().rg_default_ball_state(ball.ctypes.data)
+    start = scenarios.ball_states(ball, n, seed=n)
+    out = []
+    for threads in (32, 64, 128, 256):
+        sim = BatchSim(SimConfig(kickoff_settled=0, env_count=n, max_cars_per_env=0), *arena_mesh)
+        autotune.set_config(sim, threads, 64, False)
+        sim.upload_ball_states(start)
+        sim.step(24)
+        out.append((sim.download_ball_states(), sim.download_env_states()))
+        sim.close()
+    assert not np.array_equal(out[0][0], start)
+    for balls, envs in out[1:]:
+        assert np.array_equal(balls, out[0][0]) and np.array_equal(envs, out[0][1])
+
+
 @pytest.mark.parametrize("n,sms,pads", [(1, 148, 34), (37, 4, 34), (700, 4, 64), (5000, 148, 34)])
 def test_turn_plans_one_after_another(turn, n, sms, pads):
     """Car counts raised, lowered, set to none and mixed: a launch captured for any earlier plan finds no arena twice."""

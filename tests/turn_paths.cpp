@@ -141,6 +141,8 @@ int tp_visit_order(int command, int mode, uint32_t packed, int count, unsigned s
     return wrong;
 }
 
+int tp_resident_warps(int registers, int threads) { return rg::resident_warps(registers, threads); }
+
 // The packed order after bound_visit_order.
 uint32_t tp_bound(int mode, uint32_t packed, int count, int max_cars) {
     rg::EnvState env;
