@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(kVehicleThreads, 8)
     const rg::CarControls& ctrl =
         a.controls[control_row(a, e, t) * static_cast<size_t>(a.control_stride) + static_cast<size_t>(idx)];
     const uint32_t excluded = (st.wheel_meets_car[0] & rg::kWheelBallExcluded) ? 1u : 0u;
-    rg::vehicle_update(lanes, s.car, ctrl, s.cfg, a.base.tc, s.wheels, a.base.balls[e], mesh,
+    rg::vehicle_update(lanes, s.car, ctrl, s.cfg, a.base.tc, s.wheels, a.base.balls[e],
                        rg::WheelOthers{nullptr, nullptr, 0, -1, excluded}, a.records[idx].pushes, st.wheel_mesh, s.tick);
     // the car's own part of the world step, while these lanes have the car (rg::CarStage)
     if (lanes.lane() == 0) rg::car_stage_compute(s.car, s.cfg, s.wheels, a.base.tc, mesh, slot, st);

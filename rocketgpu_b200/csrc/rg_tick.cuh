@@ -1266,7 +1266,7 @@ struct CarStage {
     uint32_t box_clear;
     RayHit wheel_mesh[4];    // the wheels' arena-mesh rays, cast ahead of the vehicle update (wheel_mesh_ray_ahead)
     uint8_t wheel_meets_car[4];  // kWheelMeetsCar, kWheelBallExcluded (0 for a demolished car)
-    BallCarScratch ball_manifold;  // the car/ball manifold after this tick's geometry (car_ball_stage)
+    BallCarScratch ball_manifold;  // the car/ball manifold after this tick's geometry (car_proxy_ball_stage)
     uint32_t ball_staged;          // ball_manifold holds this tick's update
     MeshContactEvents mesh_events;  // the query's car-world events (when events are on)
 };
@@ -1716,7 +1716,7 @@ RG_HDI void arena_cars_in_order(const L& lanes, const EnvState& env, const BallS
         vehicle_slot_load(lanes, s, A.cars + i, A.wheels + i, A.cfgs + i);
         lanes.sync();
         const uint32_t excluded = s.car.is_demoed ? 0u : wheel_ray_excluded_bodies(lanes, s.car, s.cfg, &bp, i, count);
-        vehicle_update(lanes, s.car, A.controls[i], s.cfg, c, s.wheels, b, mesh,
+        vehicle_update(lanes, s.car, A.controls[i], s.cfg, c, s.wheels, b,
                        WheelOthers{A.cars, A.cfgs, count, i, excluded}, recs[i].pushes, stages[i].wheel_mesh, s.tick);
         lanes.sync();
         vehicle_slot_store(lanes, s, A.cars + i, A.wheels + i);

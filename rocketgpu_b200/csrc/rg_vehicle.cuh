@@ -572,21 +572,15 @@ RG_HDI void wheel_ray_vs_cars(const WheelStep& w, float min_hit_dist_sq_bt, cons
     }
 }
 
-// A wheel's suspension ray against the arena mesh (or its result `mesh_hit`, cast ahead by wheel_mesh_ray), the
-// other cars' boxes and the ball; the closest hit becomes the wheel's contact.
+// A wheel's suspension ray against the other cars' boxes and the ball, after `mesh_hit`, its result against the arena mesh
+// (cast ahead by wheel_mesh_ray); the closest hit becomes the wheel's contact.
 RG_HDI void wheel_ray_cast(const CarState& c, WheelStep& w, const BallState& ball, const TickConfig& tc,
-                           const MeshDevice& mesh, float min_hit_dist_sq_bt, const WheelOthers& oth,
-                           const RayHit* mesh_hit = nullptr) {
+                           float min_hit_dist_sq_bt, const WheelOthers& oth, const RayHit& mesh_hit) {
     const float real_ray_length =
         w.suspension_rest_length + w.max_suspension_travel + w.wheel_radius - kWheelSuspensionSubtraction;
     const float real_ray_length_bt = (w.suspension_rest_length * kUuToBt + w.wheel_radius * kUuToBt) +
                                      (w.max_suspension_travel - kWheelSuspensionSubtraction) * kUuToBt;
-    RayHit hit;
-    if (mesh_hit) {
-        hit = *mesh_hit;
-    } else {
-        wheel_mesh_ray(w, mesh, min_hit_dist_sq_bt, hit);
-    }
+    RayHit hit = mesh_hit;
     bool hit_world = hit.hit != 0;
     int32_t ground_car_idx = -1;
     bool selected_no_response = false;
@@ -1160,12 +1154,12 @@ RG_HDI void vehicle_begin(CarState& c, CarControls k_raw, const CarConfig& cfg, 
 
 // Wheel i's ray and what the wheel gets from it.
 RG_HDI void vehicle_wheel_cast(const CarState& c, const CarConfig& cfg, const TickConfig& tc, const WheelRuntime& wr,
-                               const BallState& ball, const MeshDevice& mesh, const WheelOthers& oth,
-                               const RayHit* mesh_hits, const VehicleTick& v, int i, WheelStep& w) {
+                               const BallState& ball, const WheelOthers& oth, const RayHit* mesh_hits,
+                               const VehicleTick& v, int i, WheelStep& w) {
     init_wheel(w, c, cfg, i, v.f, i < 2 ? v.front_bone : v.back_bone);
     w.suspension_force_scale = w.is_front_wheel ? v.front_scale : v.back_scale;
     w.extra_pushback = wr.extra_pushback[i];
-    wheel_ray_cast(c, w, ball, tc, mesh, v.min_hit_dist_sq, oth, mesh_hits ? mesh_hits + i : nullptr);
+    wheel_ray_cast(c, w, ball, tc, v.min_hit_dist_sq, oth, mesh_hits[i]);
     if (w.is_in_contact) w.extra_pushback = 0.0f;
     if (w.is_in_contact_with_world) world_wheel_pushback(c, tc, w, v.f);
 }
@@ -1410,12 +1404,12 @@ RG_HDI void vehicle_end(CarState& c, const TickConfig& tc, WheelRuntime& wr, Veh
 // The vehicle update of one car. The lanes of `lanes` hold the same car, `wr` and `v` in memory they share; with four
 // lanes each takes a wheel (its ray, drive, suspension and tyre terms, which depend on no other wheel), and lane 0 alone
 // everything else, the wheels' sums in the reference's wheel order (1, 0, 3, 2) among it. `mesh_hits`: the four wheels'
-// arena-mesh rays cast ahead (wheel_mesh_ray_ahead), or null to cast them here. Wheels that land on other cars (`oth`)
+// arena-mesh rays, cast ahead (wheel_mesh_ray_ahead). Wheels that land on other cars (`oth`)
 // push them after all four rays, in wheel order: a push changes the other car's velocity, which no ray reads.
 template <class L>
 RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw, const CarConfig& cfg,
-                           const TickConfig& tc, WheelRuntime& wr, const BallState& ball, const MeshDevice& mesh,
-                           const WheelOthers& oth, WheelBallPushes& pushes, const RayHit* mesh_hits, VehicleTick& v) {
+                           const TickConfig& tc, WheelRuntime& wr, const BallState& ball, const WheelOthers& oth,
+                           WheelBallPushes& pushes, const RayHit* mesh_hits, VehicleTick& v) {
     constexpr int kOwn = 4 / L::kLanes;
     WheelStep wh[kOwn];
     auto each_wheel = [&](auto&& part) {
@@ -1435,7 +1429,7 @@ RG_HDI void vehicle_update(const L& lanes, CarState& c, const CarControls& k_raw
     if (first) vehicle_begin(c, k_raw, cfg, tc, wr, v);
     lanes.sync();
     each_wheel([&](int i, WheelStep& w) {
-        vehicle_wheel_cast(c, cfg, tc, wr, ball, mesh, oth, mesh_hits, v, i, w);
+        vehicle_wheel_cast(c, cfg, tc, wr, ball, oth, mesh_hits, v, i, w);
     });
     if (oth.cars) {
         for (int kk = 0; kk < 4; ++kk) {
