@@ -280,7 +280,7 @@ __device__ __forceinline__ const rg::MeshDevice& arena_mesh(const TickArgs& a, i
 }
 
 // One thread owns one ball-only arena for all its ticks: a serial chain, bounded by its latency. 168 registers hold the
-// tick (24 bytes spilled; 266 at 144) and leave room for twelve warps of an SM: 60 ticks of 16,384 arenas 2,194 us with
+// tick (18 bytes spilled; 266 at 144) and leave room for twelve warps of an SM: 60 ticks of 16,384 arenas 2,194 us with
 // 128 registers and 16 warps, 1,920 with 168 and 12, 1,933 with 255 and 8, 2,365 with 144 and 14.
 __global__ void __maxnreg__(kRegistersBalls) tick_kernel(const __grid_constant__ TickArgs a, int ticks, int shift) {
     const int e = spread_item(shift);
@@ -460,7 +460,8 @@ __device__ __forceinline__ void warp_store(void* global, const void* shared, int
 // timer and respawn, quantisation, controls, jumps, dodges, boost, speed clamp). A warp holds a group of whole arenas, so
 // its lanes need no other warp's; their cars, wheel records and pads are in shared memory from one end to the other
 // (asynchronous copies, all in flight at once). As four launches (post-tick, tail, begin, tick start) these parts loaded
-// the structs from HBM four times, field by field: 298 us a tick at 16,384 mixed arenas, 60 us for one 1v1 arena.
+// the structs from HBM four times, field by field: 298 us a tick at 16,384 mixed arenas, 60 us for one 1v1 arena; in one
+// launch 177 and 34.
 // kTurnFinish: tick t ends; kTurnStart: tick t_next begins. Each consists of two parts that phase timing launches apart.
 constexpr int kTurnPost = 1, kTurnTail = 2, kTurnBegin = 4, kTurnPre = 8;
 constexpr int kTurnFinish = kTurnPost | kTurnTail, kTurnStart = kTurnBegin | kTurnPre;
@@ -755,7 +756,7 @@ __device__ __forceinline__ void car_mesh_warp(const CarTickArgs& a, int k, MeshW
 // mesh_blocks + ball_blocks) one thread per active car, its broadphase proxy and ball contact geometry; the rest one
 // thread per wheel, the wheel's suspension ray against the arena mesh and whether it meets another car's box.
 // Registers: the deepest part, the penetration search, would take 255, which leaves an SM eight warps; held to 168 for
-// twelve it spills 664 bytes in code that few cars reach. A tick's geometry with 255 and with 168 registers: 330 and 272 us
+// twelve it spills 988 bytes in code that few cars reach. A tick's geometry with 255 and with 168 registers: 330 and 272 us
 // at 16,384 mixed arenas, 360 and 288 at 4,095 3v3 arenas that meet, 138 and 137 at 8,191 duels; 128 lose again.
 constexpr int kGeometryThreads = 64;
 __global__ void __launch_bounds__(kGeometryThreads, 6)
@@ -812,7 +813,8 @@ constexpr size_t kVehicleSlotBytes =
     sizeof(rg::VehicleSlot) / 16 % 2 == 1 ? sizeof(rg::VehicleSlot) : sizeof(rg::VehicleSlot) + 16;
 constexpr int kVehicleThreads = 64;
 
-// Out of line, so that the kernel keeps the registers of the common path (inlined, it took 168 instead of 108).
+// Out of line, so that the common path keeps the kernel's 128 registers: 8 bytes of it are spilled, 376 with the chains
+// inlined.
 __device__ __noinline__ void cars_in_order(const CarTickArgs& a, int e, int t, uint32_t which, rg::VehicleSlot& s) {
     const int base = e * a.max_cars;
     rg::arena_cars_in_order(FourLanes(), a.base.envs[e], a.base.balls[e], a.broadphase[e], a.base.tc,
@@ -858,7 +860,7 @@ __global__ void __launch_bounds__(kVehicleThreads, 8)
 }
 
 // Tick part 4, one thread per arena in step order: wheel pushes on the ball, then the world step's shared stages.
-// The registers (255) are the ones that remove the spills. Bringing the sweep history (1.4 KB per arena) into shared memory
+// With 255 registers 36 bytes are spilled. Bringing the sweep history (1.4 KB per arena) into shared memory
 // first, by the whole warp, was slower: 333 against 299 us at 16,384 mixed arenas, for the L1 that local memory lost.
 __global__ void __maxnreg__(kRegistersFinish) arena_finish_kernel(const __grid_constant__ CarTickArgs a, int t, int shift) {
     const int k = spread_item(shift);

@@ -31,10 +31,11 @@ struct TurnPlan {
 // The groups of a turn, along the step order: whole arenas, up to kTurnCars cars (or one arena). Fewer cars per group,
 // down to one arena, while the chip has warps to spare (kTurnWarps resident per SM, by the kernel's registers), and no
 // more groups than those while whole arenas allow it: a few groups more are a second wave (8,191 duels in 2,731 groups of
-// three 119 us a turn, in 2,048 of four 72; 4,095 3v3 arenas one by one 131, by two 84). Twelve
-// cars take 17 KB of shared memory, so that 13 groups are resident per SM: 187 us a turn at 16,384 mixed arenas, against
-// 221 with up to 32 cars, 216 with 8 (one arena of six, three of two). 168 registers instead of 128 gained 14 us there and
-// lost 18 of 130 us at 4,095 3v3 arenas, where the warps count.
+// three 119 us a turn, in 2,048 of four 75; 4,095 3v3 arenas one by one 131, by two 83). Groups of nine cars and more take
+// so much shared memory that fewer are resident (twelve cars 17 KB, 13 per SM): between that number and kTurnWarps the
+// rule still counts a second wave as one. At kTurnCars the count no longer decides: 177 us a turn at 16,384 mixed arenas;
+// when it was 187, up to 32 cars took 221 and up to 8 (one arena of six, three of two) 216. 168 registers instead of 128
+// gained 14 us there and lost 18 of 130 us at 4,095 3v3 arenas, where the warps count.
 constexpr int kTurnWarps = 16, kTurnCars = 12, kTurnArenas = 16;
 constexpr size_t kTurnSharedMax = 48 * 1024;
 inline size_t turn_shared_bytes(int cars, int arenas, int pads) {
